@@ -1118,7 +1118,7 @@ size_t correlator_footprint(int kind, const int shape[3], double cell,
     if (precision != FC_FP64) {                              // FP32 density,
       bytes += g.ncells() * 4 + (size_t)g.shape[0] * g.shape[1] * 32;  // row table
       const int m = g.shape[2] / 2;
-      if (m >= 64 && m <= 2048 && (m & (m - 1)) == 0)        // paired z pass:
+      if (m >= 32 && m <= 2048 && (m & (m - 1)) == 0)        // paired z pass:
         bytes += (size_t)g.shape[0] * g.shape[1] * (h * eb + 32);  // W2, table
     }
     const int nlm = maxell == 0 ? 1 : maxell == 2 ? 6 : 15;

@@ -1,14 +1,7 @@
-// fc_fft.cuh -- shared-memory Stockham FFT engine for the fused correlator
-// passes.
-//
-// A CTA transforms B columns of length L held in shared memory as
-// buf[i * BP + b] (row i of column b, BP = B + 1 to spread banks).  The
-// transform is an iterative mixed-radix Stockham autosort (radices 8, 4, 2,
-// 3, 5, 7) between two shared buffers: each pass reads a butterfly's R
-// inputs, applies the twiddles and the radix-R DFT in registers and writes
-// the outputs to their Stockham positions in the other buffer.  Twiddles come from a table of e^{-2 pi i m / Lt} (Lt a
-// multiple of L) computed in FP64 on the host.  Forward is sign -1 and the
-// inverse is unnormalised, as in FFTW and cuFFT.
+// fc_fft.cuh -- complex arithmetic, small DFTs and the register-resident FFT
+// of power-of-two lengths for the fused correlator passes.  Twiddles come
+// from tables of e^{-2 pi i m / Lt} computed in FP64 on the host.  Forward is
+// sign -1 and the inverse is unnormalised, as in FFTW and cuFFT.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -172,6 +165,13 @@ __device__ __forceinline__ CPairS cmul(CPairS a, float2 w) {
   r.y = a.x * w.y + a.y * w.x;
   return r;
 }
+// a * conj(b), pair by pair.
+__device__ __forceinline__ CPair cmulc(CPair a, CPair b) {
+  CPair r;
+  r.x = __ffma2_rn(a.y, b.y, __fmul2_rn(a.x, b.x));
+  r.y = __ffma2_rn(a.y, b.x, -__fmul2_rn(a.x, b.y));
+  return r;
+}
 // (sign * i) * a
 template <typename C>
 __device__ __forceinline__ C cmuli(C a, int sign) {
@@ -256,143 +256,21 @@ struct Dft<8, C> {
 template <typename C>
 struct Dft<3, C> {
   __device__ static void run(C *v, int sign) {
-    using T = decltype(v[0].x);
+    using T = typename Real<C>::type;
     const T s3 = (T)0.86602540378443864676 * sign;
     const C t = cadd(v[1], v[2]);
     const C d = csub(v[1], v[2]);
     C m;
-    m.x = v[0].x - (T)0.5 * t.x;
-    m.y = v[0].y - (T)0.5 * t.y;
+    m.x = v[0].x + (T)-0.5 * t.x;
+    m.y = v[0].y + (T)-0.5 * t.y;
     C sd;
-    sd.x = -s3 * d.y;
+    sd.x = (-s3) * d.y;
     sd.y = s3 * d.x;
     v[0] = cadd(v[0], t);
     v[1] = cadd(m, sd);
     v[2] = csub(m, sd);
   }
 };
-
-// Generic odd prime radix (5, 7): O(R^2) complex products with the R-th
-// roots of unity evaluated once per butterfly by sincospi (correctly
-// rounded to within an ulp); these radices are rare in practice.
-template <int R, typename C>
-struct DftGeneric {
-  __device__ static void run(C *v, int sign) {
-    using T = decltype(v[0].x);
-    C w[R];
-#pragma unroll
-    for (int m = 0; m < R; ++m) {
-      double s, c;
-      sincospi(2.0 * m / R, &s, &c);
-      w[m].x = (T)c;
-      w[m].y = (T)(sign * s);
-    }
-    C in[R];
-#pragma unroll
-    for (int u = 0; u < R; ++u) in[u] = v[u];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      C acc = in[0];
-#pragma unroll
-      for (int u = 1; u < R; ++u) acc = cadd(acc, cmul(in[u], w[(u * q) % R]));
-      v[q] = acc;
-    }
-  }
-};
-template <typename C>
-struct Dft<5, C> : DftGeneric<5, C> {};
-template <typename C>
-struct Dft<7, C> : DftGeneric<7, C> {};
-
-// Plan of one transform length: up to 12 passes.
-struct FftPlan {
-  int L;          // transform length
-  int npass;
-  int radix[12];
-  int ns[12];     // product of the radices before each pass
-  int nsmask[12]; // ns - 1 when ns is a power of two, else -1
-  int tab_scale;  // root-table order / L
-};
-
-// One Stockham pass of radix R: reads the B columns from src, writes the
-// result to dst (both [L][BP] in shared memory).  Each thread handles one
-// butterfly at a time, so only R complex values live in registers.  B is a
-// compile-time constant so the butterfly decomposition is shifts and masks.
-template <int R, int B, typename C>
-__device__ __forceinline__ void stockham_pass(const C *src, C *dst, int L,
-                                              int Ns, int nsmask,
-                                              const C *__restrict__ tab,
-                                              int tab_scale, int sign) {
-  constexpr int BP = B + 1;
-  const int LR = L / R;
-  const int nbf = LR * B;
-  const int step = (L / (Ns * R)) * tab_scale;
-  for (int bf = threadIdx.x; bf < nbf; bf += blockDim.x) {
-    const int j = bf / B;
-    const int b = bf - j * B;
-    const int k = nsmask >= 0 ? (j & nsmask) : (j % Ns);
-    C v[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = src[(j + q * LR) * BP + b];
-    if (Ns > 1) {
-      // q * k * step < L * tab_scale: no reduction needed.
-      const int ks = k * step;
-#pragma unroll
-      for (int q = 1; q < R; ++q) {
-        C w = __ldg(&tab[q * ks]);
-        if (sign > 0) w.y = -w.y;
-        v[q] = cmul(v[q], w);
-      }
-    }
-    Dft<R, C>::run(v, sign);
-    const int o = ((j - k) * R + k) * BP + b;
-#pragma unroll
-    for (int q = 0; q < R; ++q) dst[o + q * Ns * BP] = v[q];
-  }
-  __syncthreads();
-}
-
-// Transforms the B columns in a (the caller has synchronised after filling
-// it), ping-ponging with b; returns the buffer that holds the result
-// (synchronised).
-template <int B, typename C>
-__device__ C *fft_columns(C *a, C *b, const FftPlan &p,
-                          const C *__restrict__ tab, int sign) {
-  C *src = a, *dst = b;
-  for (int s = 0; s < p.npass; ++s) {
-    const int R = p.radix[s];
-    const int Ns = p.ns[s];
-    const int m = p.nsmask[s];
-    switch (R) {
-      case 8:
-        stockham_pass<8, B>(src, dst, p.L, Ns, m, tab, p.tab_scale, sign);
-        break;
-      case 4:
-        stockham_pass<4, B>(src, dst, p.L, Ns, m, tab, p.tab_scale, sign);
-        break;
-      case 2:
-        stockham_pass<2, B>(src, dst, p.L, Ns, m, tab, p.tab_scale, sign);
-        break;
-      case 3:
-        stockham_pass<3, B>(src, dst, p.L, Ns, m, tab, p.tab_scale, sign);
-        break;
-      case 5:
-        stockham_pass<5, B>(src, dst, p.L, Ns, m, tab, p.tab_scale, sign);
-        break;
-      default:
-        stockham_pass<7, B>(src, dst, p.L, Ns, m, tab, p.tab_scale, sign);
-        break;
-    }
-    C *t = src;
-    src = dst;
-    dst = t;
-  }
-  return src;
-}
-
-}  // namespace fc
-
-namespace fc {
 
 // ---------------------------------------------------------------------------
 // Register-resident FFT for power-of-two lengths 64 <= L <= 4096.

@@ -75,31 +75,10 @@ __device__ __forceinline__ RowPoly row_poly(const YlmParams &p, double x,
   RowPoly r;
   r.ell = p.ell;
   r.value0 = (float)p.value0;
-  const double x2 = x * x, y2 = y * y, s = x2 + y2, n = p.norm;
-  double c[5] = {0, 0, 0, 0, 0};
-  if (p.ell == 2) {
-    switch (p.m) {
-      case 2: c[0] = x2 - y2; break;
-      case 1: c[1] = x; break;
-      case 0: c[0] = -s; c[2] = 2.0; break;
-      case -1: c[1] = y; break;
-      default: c[0] = x * y; break;
-    }
-  } else if (p.ell == 4) {
-    switch (p.m) {
-      case 4: c[0] = x2 * x2 - 6.0 * x2 * y2 + y2 * y2; break;
-      case 3: c[1] = x * (x2 - 3.0 * y2); break;
-      case 2: c[0] = y2 * y2 - x2 * x2; c[2] = 6.0 * (x2 - y2); break;
-      case 1: c[1] = -x * s; c[3] = 4.0 / 3.0 * x; break;
-      case 0: c[0] = 0.375 * s * s; c[2] = -3.0 * s; c[4] = 1.0; break;
-      case -1: c[1] = -y * s; c[3] = 4.0 / 3.0 * y; break;
-      case -2: c[0] = -2.0 * x * y * s; c[2] = 12.0 * x * y; break;
-      case -3: c[1] = 3.0 * x2 * y - y2 * y; break;
-      default: c[0] = 4.0 * x * (x2 * y - y2 * y); break;
-    }
-  }
-  for (int i = 0; i < 5; ++i) r.c[i] = (float)(n * c[i]);
-  r.rxy2 = (float)s;
+  double c[5];
+  row_poly_coefs(p, x, y, c);
+  for (int i = 0; i < 5; ++i) r.c[i] = (float)c[i];
+  r.rxy2 = (float)(x * x + y * y);
   return r;
 }
 
@@ -160,286 +139,15 @@ __device__ __forceinline__ RowPoly load_row_poly(const float4 *__restrict__ tab,
   return r;
 }
 
-// ------------------------------------------------------------------ zfwd
-// B rows of N2 reals per CTA: (optionally Y_lm-weighted) packed as
-// z_j = x_2j + i x_2j+1, length-M complex DFT, then the real-to-complex
-// split X_k = E_k + e^{-2 pi i k/N2} O_k for k <= M.
-template <typename T, bool WEIGHT>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2))
-    k_zfwd(const T *__restrict__ rho, C2<T> *__restrict__ W, FusedGeom g,
-           YlmParams p, double x0, double y0, double z0,
-           const C2<T> *__restrict__ tabz) {
-  using C = C2<T>;
-  constexpr int B = Tile<T>::B;
-  constexpr int BP = B + 1;
-  extern __shared__ unsigned char smem_raw[];
-  C *buf = reinterpret_cast<C *>(smem_raw);
-  const int M = g.m;
-  C *buf2 = buf + M * BP;
-  const int64_t nrows = (int64_t)g.n0 * g.n1;
-  const int64_t row0 = (int64_t)blockIdx.x * B;
-  for (int idx = threadIdx.x; idx < M * B; idx += blockDim.x) {
-    const int b = idx / M;
-    const int j = idx - b * M;
-    const int64_t row = row0 + b;
-    C z;
-    z.x = 0;
-    z.y = 0;
-    if (row < nrows) {
-      const typename Vec2<T>::type v =
-          reinterpret_cast<const typename Vec2<T>::type *>(rho + row * g.n2)[j];
-      z = v;
-      if (WEIGHT) {
-        const int x = (int)(row / g.n1);
-        const int y = (int)(row - (int64_t)x * g.n1);
-        const double cx = x0 + x * 1.0;
-        const double cy = y0 + y * 1.0;
-        z.x = weight_value<T>(p, v.x, cx, cy, z0 + (2 * j) * 1.0);
-        z.y = weight_value<T>(p, v.y, cx, cy, z0 + (2 * j + 1) * 1.0);
-      }
-    }
-    buf[j * BP + b] = z;
-  }
-  __syncthreads();
-  buf = fft_columns<B>(buf, buf2, g.pz, tabz, -1);
-  const int H = M + 1;
-  for (int idx = threadIdx.x; idx < H * B; idx += blockDim.x) {
-    const int b = idx / H;
-    const int k = idx - b * H;
-    const int64_t row = row0 + b;
-    if (row >= nrows) continue;
-    const C a = buf[(k == M ? 0 : k) * BP + b];
-    const C c = cconj(buf[(k == 0 ? 0 : M - k) * BP + b]);
-    C e, d, o;
-    e.x = (T)0.5 * (a.x + c.x);
-    e.y = (T)0.5 * (a.y + c.y);
-    d = csub(a, c);
-    o.x = (T)0.5 * d.y;  // -i (a - c) / 2
-    o.y = (T)-0.5 * d.x;
-    W[row * g.hp + k] = cadd(e, cmul(__ldg(&tabz[k]), o));
-  }
-}
-
-// Loads a B-column tile of a strided axis into shared memory.
-// Loads are issued in groups of 8 before any shared-memory store so each
-// thread keeps eight global reads in flight.
-template <int B, typename C>
-__device__ __forceinline__ void load_columns(C *buf, const C *__restrict__ src,
-                                             int64_t base, int64_t stride,
-                                             int L, int kz0, int h) {
-  constexpr int BP = B + 1;
-  const int n = L * B;
-  for (int idx0 = threadIdx.x; idx0 < n; idx0 += 8 * blockDim.x) {
-    C v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int idx = idx0 + u * blockDim.x;
-      const int i = idx / B;
-      const int b = idx - i * B;
-      v[u].x = 0;
-      v[u].y = 0;
-      if (idx < n && kz0 + b < h) v[u] = src[base + i * stride + kz0 + b];
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int idx = idx0 + u * blockDim.x;
-      if (idx < n) {
-        const int i = idx / B;
-        buf[i * BP + (idx - i * B)] = v[u];
-      }
-    }
-  }
-  __syncthreads();
-}
-
-// ------------------------------------------------------------------ yfwd
-template <typename T>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2))
-    k_yfwd(C2<T> *__restrict__ W, FusedGeom g, const C2<T> *__restrict__ taby) {
-  using C = C2<T>;
-  constexpr int B = Tile<T>::B;
-  constexpr int BP = B + 1;
-  extern __shared__ unsigned char smem_raw[];
-  C *buf = reinterpret_cast<C *>(smem_raw);
-  const int kz0 = blockIdx.x * B;
-  const int x = blockIdx.y;
-  const int64_t base = (int64_t)x * g.n1 * g.hp;
-  load_columns<B>(buf, W, base, g.hp, g.n1, kz0, g.h);
-  buf = fft_columns<B>(buf, buf + g.n1 * BP, g.py, taby, -1);
-  for (int idx = threadIdx.x; idx < g.n1 * B; idx += blockDim.x) {
-    const int i = idx / B;
-    const int b = idx - i * B;
-    if (kz0 + b < g.h) W[base + (int64_t)i * g.hp + kz0 + b] = buf[i * BP + b];
-  }
-}
-
-// ----------------------------------------------------------------- xcorr
-// MODE 0: G = DFT_x(W) (grid2's transform).  MODE 1: the fused product,
-// k-subgrid extraction, inverse and pruning described at the top.
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2))
-    k_xcorr(const C2<T> *__restrict__ W, const C2<T> *__restrict__ G,
-            C2<T> *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
-            const C2<T> *__restrict__ tabx, const T *__restrict__ ktab) {
-  using C = C2<T>;
-  constexpr int B = Tile<T>::B;
-  constexpr int BP = B + 1;
-  extern __shared__ unsigned char smem_raw[];
-  C *buf = reinterpret_cast<C *>(smem_raw);
-  const int kz0 = blockIdx.x * B;
-  const int yy = blockIdx.y;
-  const int64_t stride = (int64_t)g.n1 * g.hp;
-  const int64_t base = (int64_t)yy * g.hp;
-  C *other = buf + g.n0 * BP;
-  load_columns<B>(buf, W, base, stride, g.n0, kz0, g.h);
-  {
-    C *res = fft_columns<B>(buf, other, g.px, tabx, -1);
-    other = res == buf ? other : buf;
-    buf = res;
-  }
-  if constexpr (MODE == 0) {
-    for (int idx = threadIdx.x; idx < g.n0 * B; idx += blockDim.x) {
-      const int i = idx / B;
-      const int b = idx - i * B;
-      if (kz0 + b < g.h) out[base + i * stride + kz0 + b] = buf[i * BP + b];
-    }
-  } else {
-    // P = F * conj(G).
-    for (int idx = threadIdx.x; idx < g.n0 * B; idx += blockDim.x) {
-      const int i = idx / B;
-      const int b = idx - i * B;
-      if (kz0 + b < g.h)
-        buf[i * BP + b] = cmulc(buf[i * BP + b], G[base + i * stride + kz0 + b]);
-    }
-    __syncthreads();
-    // k-subgrid: this CTA owns the sources with ky index yy and kz in its
-    // block.  Direct targets k = kz + oz read P[(i - ox) mod N0][yy][kz];
-    // reflected targets k = oz - kz (kz >= 1) read P[(ox - i) mod N0][yy][kz]
-    // for j with (oy - j) mod N1 == yy.  Every ksub cell has exactly one
-    // source element, so these read-modify-writes never collide.
-    if (ksub != nullptr) {
-      const int ox = g.ks0 / 2, oy = g.ks1 / 2, oz = g.ks2 / 2;
-      if (kz0 <= oz) {
-        for (int refl = 0; refl < 2; ++refl) {
-          int j = refl == 0 ? (yy + oy) % g.n1 : ((oy - yy) % g.n1 + g.n1) % g.n1;
-          for (; j < g.ks1; j += g.n1) {
-            for (int idx = threadIdx.x; idx < g.ks0 * B; idx += blockDim.x) {
-              const int i = idx / B;
-              const int b = idx - i * B;
-              const int kzi = kz0 + b;
-              if (kzi >= g.h || kzi > oz || (refl == 1 && kzi == 0)) continue;
-              const int k = refl == 0 ? kzi + oz : oz - kzi;
-              const int x = refl == 0 ? ((i - ox) % g.n0 + g.n0) % g.n0
-                                      : ((ox - i) % g.n0 + g.n0) % g.n0;
-              const double re = (double)buf[x * BP + b].x;
-              const size_t cell = ((size_t)i * g.ks1 + j) * g.ks2 + k;
-              ksub[cell] += (double)ktab[cell] * re;
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
-    buf = fft_columns<B>(buf, other, g.px, tabx, +1);
-    const int64_t obase = (int64_t)yy * g.hp;
-    const int64_t ostride = (int64_t)g.n1 * g.hp;
-    for (int idx = threadIdx.x; idx < g.rs * B; idx += blockDim.x) {
-      const int ri = idx / B;
-      const int b = idx - ri * B;
-      if (kz0 + b >= g.h) continue;
-      const int x = ((ri - g.ro) % g.n0 + g.n0) % g.n0;
-      out[obase + ri * ostride + kz0 + b] = buf[x * BP + b];
-    }
-  }
-}
-
-// ------------------------------------------------------------------ yinv
-template <typename T>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2))
-    k_yinv(const C2<T> *__restrict__ Wr, C2<T> *__restrict__ Wry, FusedGeom g,
-           const C2<T> *__restrict__ taby) {
-  using C = C2<T>;
-  constexpr int B = Tile<T>::B;
-  constexpr int BP = B + 1;
-  extern __shared__ unsigned char smem_raw[];
-  C *buf = reinterpret_cast<C *>(smem_raw);
-  const int kz0 = blockIdx.x * B;
-  const int ri = blockIdx.y;
-  const int64_t base = (int64_t)ri * g.n1 * g.hp;
-  load_columns<B>(buf, Wr, base, g.hp, g.n1, kz0, g.h);
-  buf = fft_columns<B>(buf, buf + g.n1 * BP, g.py, taby, +1);
-  const int64_t obase = (int64_t)ri * g.rs * g.hp;
-  for (int idx = threadIdx.x; idx < g.rs * B; idx += blockDim.x) {
-    const int rj = idx / B;
-    const int b = idx - rj * B;
-    if (kz0 + b >= g.h) continue;
-    const int y = ((rj - g.ro) % g.n1 + g.n1) % g.n1;
-    Wry[obase + (int64_t)rj * g.hp + kz0 + b] = buf[y * BP + b];
-  }
-}
-
-// ----------------------------------------------------------------- zinv
-// B rows (ri, rj) per CTA: complex-to-real inverse along z (unnormalised,
-// the imaginary parts of the DC and Nyquist terms ignored), then
-// rsub[ri][rj][rk] += Y_lm(r) * value at z = (N2 - rs/2 + rk) mod N2.
-template <typename T>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 3 : 2))
-    k_zinv_rsub(const C2<T> *__restrict__ Wry, double *__restrict__ rsub,
-                FusedGeom g, const C2<T> *__restrict__ tabz,
-                const T *__restrict__ rtab) {
-  using C = C2<T>;
-  constexpr int B = Tile<T>::B;
-  constexpr int BP = B + 1;
-  extern __shared__ unsigned char smem_raw[];
-  C *buf = reinterpret_cast<C *>(smem_raw);
-  const int M = g.m;
-  const int nrows = g.rs * g.rs;
-  const int row0 = blockIdx.x * B;
-  C *buf2 = buf + M * BP;
-  for (int idx = threadIdx.x; idx < M * B; idx += blockDim.x) {
-    const int b = idx / M;
-    const int k = idx - b * M;
-    const int row = row0 + b;
-    C z;
-    z.x = 0;
-    z.y = 0;
-    if (row < nrows) {
-      const C *X = Wry + (int64_t)row * g.hp;
-      C a = X[k];
-      C c = cconj(X[M - k]);
-      if (k == 0) {
-        a.y = 0;
-        c.y = 0;  // X[M] is the Nyquist term
-      }
-      const C e = cadd(a, c);
-      const C o = cmul(csub(a, c), cconj(__ldg(&tabz[k])));  // e^{+2 pi i k/N2}
-      z.x = e.x - o.y;
-      z.y = e.y + o.x;
-    }
-    buf[k * BP + b] = z;
-  }
-  __syncthreads();
-  buf = fft_columns<B>(buf, buf2, g.pz, tabz, +1);
-  for (int idx = threadIdx.x; idx < g.rs * B; idx += blockDim.x) {
-    const int b = idx / g.rs;
-    const int rk = idx - b * g.rs;
-    const int row = row0 + b;
-    if (row >= nrows) continue;
-    const int z = ((rk - g.ro) % g.n2 + g.n2) % g.n2;
-    const C zz = buf[(z >> 1) * BP + b];
-    const double v = (double)((z & 1) ? zz.y : zz.x);
-    const size_t cell = (size_t)row * g.rs + rk;
-    rsub[cell] += (double)rtab[cell] * v;
-  }
-}
-
 // --------------------------------------------------------------------------
-// Power-of-two lengths: the same passes with the register-resident engine
-// (reg_fft in fc_fft.cuh).  B2 columns per CTA keep the CTA at <= 1024
+// Power-of-two lengths, with the register-resident engine (reg_fft in
+// fc_fft.cuh); other lengths are fc_fused_gen.cu's.  B2 columns per CTA keep the CTA at <= 1024
 // threads (TPC = L/8 threads per column).
 template <typename T, int L>
 struct P2 {
-  static constexpr int B = (Tile<T>::B < 8192 / L) ? Tile<T>::B : 8192 / L;
+  // (Rows of 32 elements, which only the z passes take, need more of them.)
+  static constexpr int B = L == 32 ? 4 * Tile<T>::B
+                           : (Tile<T>::B < 8192 / L) ? Tile<T>::B : 8192 / L;
   static constexpr int TPC = L / 8;
   static constexpr int THREADS = TPC * B;
   // Exchange rows of B elements: a 128-byte shared-memory line holds R of
@@ -1526,31 +1234,6 @@ __global__ void k_to_float(const double *__restrict__ in, float *__restrict__ ou
     out[i] = (float)(in[i] - shift);
 }
 
-// Radices of a length, largest first (8, 4, 2, 3, 5, 7); false if L has a
-// prime factor above 7.
-bool plan_length(int L, int tab_scale, FftPlan *p) {
-  p->L = L;
-  p->tab_scale = tab_scale;
-  p->npass = 0;
-  int n = L;
-  const int radices[] = {8, 4, 2, 3, 5, 7};
-  for (int r : radices) {
-    while (n % r == 0) {
-      if (p->npass == 12) return false;
-      p->radix[p->npass++] = r;
-      n /= r;
-    }
-  }
-  if (n != 1) return false;
-  int ns = 1;
-  for (int s = 0; s < p->npass; ++s) {
-    p->ns[s] = ns;
-    p->nsmask[s] = (ns & (ns - 1)) == 0 ? ns - 1 : -1;
-    ns *= p->radix[s];
-  }
-  return true;
-}
-
 template <typename C>
 std::vector<C> root_table(int order) {
   std::vector<C> t(order);
@@ -1561,14 +1244,6 @@ std::vector<C> root_table(int order) {
     t[m].y = (decltype(t[m].y))(-sin(a));
   }
   return t;
-}
-
-// Threads per CTA for a pass of length L over B columns: one thread per
-// radix-8 butterfly where possible, between 128 and 256.
-int threads_for(int L, int B) {
-  int t = (L / 8) * B;
-  t = ((t + 31) / 32) * 32;
-  return std::max(128, std::min(256, t));
 }
 
 // ----------------------------------------------------- power-of-two dispatch
@@ -1588,6 +1263,7 @@ size_t p2_row_smem() {
 template <typename F>
 void with_p2(int L, F &&f) {
   switch (L) {
+    case 32: f.template operator()<32>(); break;
     case 64: f.template operator()<64>(); break;
     case 128: f.template operator()<128>(); break;
     case 256: f.template operator()<256>(); break;
@@ -1639,18 +1315,8 @@ void p2_set_limits() {
 }  // namespace
 
 bool FusedSurvey::supported(const int shape[3], int rsize) {
-  if (shape[2] % 2 != 0) return false;
-  FftPlan p;
-  if (!plan_length(shape[0], 1, &p) || !plan_length(shape[1], 1, &p) ||
-      !plan_length(shape[2] / 2, 2, &p))
-    return false;
-  // Two shared tiles of L x (B+1) complex must fit in 200 KB.
-  for (int a = 0; a < 3; ++a) {
-    const int L = a == 2 ? shape[2] / 2 : shape[a];
-    if (2 * (size_t)L * 5 * 16 > 200 * 1024 || 2 * (size_t)L * 9 * 8 > 200 * 1024)
-      return false;
-  }
-  return rsize > 0;
+  return gen_supported(shape[0], false) && gen_supported(shape[1], false) &&
+         gen_supported(shape[2], true) && rsize > 0;
 }
 
 FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
@@ -1667,9 +1333,10 @@ FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
   g.ks0 = kshape[0];
   g.ks1 = kshape[1];
   g.ks2 = kshape[2];
-  FC_REQUIRE(plan_length(g.n0, 1, &g.px) && plan_length(g.n1, 1, &g.py) &&
-                 plan_length(g.m, 2, &g.pz),
-             FC_ERR_UNSUPPORTED, "grid size has a prime factor above 7");
+  // Axes that the power-of-two passes do not take.
+  if (!is_p2(g.n0)) gx.init(g.n0, false, fp64);
+  if (!is_p2(g.n1)) gy.init(g.n1, false, fp64);
+  if (!p2_rows()) gz.init(g.n2, true, fp64);
   const size_t eb = fp64 ? 16 : 8;
   if (fp64) {
     upload(tabx, root_table<double2>(g.n0));
@@ -1703,37 +1370,9 @@ void FusedSurvey::upload(DeviceBuffer &dst, const std::vector<V> &v) {
                      cudaMemcpyHostToDevice));
 }
 
-size_t FusedSurvey::smem(int L) const {
-  const int B = fp64_ ? Tile<double>::B : Tile<float>::B;
-  return 2 * (size_t)L * (B + 1) * (fp64_ ? 16 : 8);
-}
-
-template <typename T>
-static void set_limits_for() {
-  const int big = 200 * 1024;
-  FC_CUDA(cudaFuncSetAttribute(k_zfwd<T, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_zfwd<T, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_yfwd<T>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_xcorr<T, 0>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_xcorr<T, 1>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_yinv<T>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_zinv_rsub<T>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-}
-
 void FusedSurvey::set_smem_limits() {
-  if (fp64_)
-    set_limits_for<double>();
-  else
-    set_limits_for<float>();
-  for (int L : {g.n0, g.n1, g.m}) {
-    if (!is_p2(L)) continue;
+  for (int L : {is_p2(g.n0) ? g.n0 : 0, is_p2(g.n1) ? g.n1 : 0, p2_rows() ? g.m : 0}) {
+    if (L == 0) continue;
     if (fp64_)
       with_p2(L, [&]<int LL>() { p2_set_limits<double, LL>(); });
     else
@@ -1756,7 +1395,7 @@ const void *FusedSurvey::prepare_input(const void *rho, bool f32,
 template <typename T>
 void FusedSurvey::zfwd(const void *rho, bool weight, const YlmParams &p,
                        const double xyz0[3], cudaStream_t s) {
-  if (is_p2(g.m)) {
+  if (p2_rows()) {
     with_p2(g.m, [&]<int L>() {
       using Q = P2<T, L>;
       const int64_t nrows = (int64_t)g.n0 * g.n1;
@@ -1793,20 +1432,7 @@ void FusedSurvey::zfwd(const void *rho, bool weight, const YlmParams &p,
     FC_LAUNCH_CHECK();
     return;
   }
-  constexpr int B = Tile<T>::B;
-  const int64_t nrows = (int64_t)g.n0 * g.n1;
-  const unsigned blocks = (unsigned)((nrows + B - 1) / B);
-  const int threads = threads_for(g.m, B);
-  const size_t sm = smem(g.m);
-  if (weight)
-    k_zfwd<T, true><<<blocks, threads, sm, s>>>(
-        (const T *)rho, W.as<C2<T>>(), g, p, xyz0[0], xyz0[1], xyz0[2],
-        tabz.as<C2<T>>());
-  else
-    k_zfwd<T, false><<<blocks, threads, sm, s>>>(
-        (const T *)rho, W.as<C2<T>>(), g, p, xyz0[0], xyz0[1], xyz0[2],
-        tabz.as<C2<T>>());
-  FC_LAUNCH_CHECK();
+  gen_zfwd<T>(gz, g, (const T *)rho, W.as<C2<T>>(), weight, p, xyz0, s);
 }
 
 template <typename T>
@@ -1828,11 +1454,7 @@ void FusedSurvey::yfwd(cudaStream_t s) {
     FC_LAUNCH_CHECK();
     return;
   }
-  constexpr int B = Tile<T>::B;
-  dim3 grid((g.h + B - 1) / B, g.n0);
-  k_yfwd<T><<<grid, threads_for(g.n1, B), smem(g.n1), s>>>(W.as<C2<T>>(), g,
-                                                           taby.as<C2<T>>());
-  FC_LAUNCH_CHECK();
+  gen_yfwd<T>(gy, g, W.as<C2<T>>(), s);
 }
 
 template <typename T>
@@ -1866,26 +1488,20 @@ void FusedSurvey::xcorr(bool product, double *ksub, const void *ktab_v,
     FC_LAUNCH_CHECK();
     return;
   }
-  constexpr int B = Tile<T>::B;
-  dim3 grid((g.h + B - 1) / B, g.n1);
-  const int threads = threads_for(g.n0, B);
-  const size_t sm = smem(g.n0);
-  if (!product) {
-    k_xcorr<T, 0><<<grid, threads, sm, s>>>(
-        W.as<C2<T>>(), nullptr, G.as<C2<T>>(), nullptr, g, tabx.as<C2<T>>(),
-        nullptr);
-  } else {
-    k_xcorr<T, 1><<<grid, threads, sm, s>>>(
-        W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, g, tabx.as<C2<T>>(),
-        ktab);
-  }
-  FC_LAUNCH_CHECK();
+  if (product)
+    gen_x<T>(gx, g, 1, W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, ktab, T(0), s);
+  else
+    gen_x<T>(gx, g, 0, W.as<C2<T>>(), nullptr, G.as<C2<T>>(), nullptr, nullptr, T(0), s);
 }
 
 template <typename T>
 void FusedSurvey::xcorr00(double *ksub, const void *ktab_v, double w00,
                           cudaStream_t s) {
   const T *ktab = static_cast<const T *>(ktab_v);
+  if (!is_p2(g.n0)) {
+    gen_x<T>(gx, g, 2, nullptr, G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, ktab, (T)w00, s);
+    return;
+  }
   with_p2(g.n0, [&]<int L>() {
     using Q = P2<T, L>;
     if constexpr (std::is_same_v<T, float>) {
@@ -1924,17 +1540,13 @@ void FusedSurvey::yinv(cudaStream_t s) {
     FC_LAUNCH_CHECK();
     return;
   }
-  constexpr int B = Tile<T>::B;
-  dim3 grid((g.h + B - 1) / B, g.rs);
-  k_yinv<T><<<grid, threads_for(g.n1, B), smem(g.n1), s>>>(
-      Wr.as<C2<T>>(), Wry.as<C2<T>>(), g, taby.as<C2<T>>());
-  FC_LAUNCH_CHECK();
+  gen_yinv<T>(gy, g, Wr.as<C2<T>>(), Wry.as<C2<T>>(), s);
 }
 
 template <typename T>
 void FusedSurvey::zinv(double *rsub, const void *rtab_v, cudaStream_t s) {
   const T *rtab = static_cast<const T *>(rtab_v);
-  if (is_p2(g.m)) {
+  if (p2_rows()) {
     with_p2(g.m, [&]<int L>() {
       using Q = P2<T, L>;
       const int nrows = g.rs * g.rs;
@@ -1945,12 +1557,7 @@ void FusedSurvey::zinv(double *rsub, const void *rtab_v, cudaStream_t s) {
     FC_LAUNCH_CHECK();
     return;
   }
-  constexpr int B = Tile<T>::B;
-  const int nrows = g.rs * g.rs;
-  const unsigned blocks = (unsigned)((nrows + B - 1) / B);
-  k_zinv_rsub<T><<<blocks, threads_for(g.m, B), smem(g.m), s>>>(
-      Wry.as<C2<T>>(), rsub, g, tabz.as<C2<T>>(), rtab);
-  FC_LAUNCH_CHECK();
+  gen_zinv<T>(gz, g, Wry.as<C2<T>>(), rsub, rtab, s);
 }
 
 const void *FusedSurvey::r_table(int ell, int m, const double *raxis,
@@ -2022,7 +1629,10 @@ void FusedSurvey::grid2(const void *rho_in, cudaStream_t s, const KAxes &ka) {
   }
 }
 
-bool FusedSurvey::pairs() const { return !fp64_ && is_p2(g.m); }
+bool FusedSurvey::p2_rows() const {
+  return g.n2 % 2 == 0 && (g.m == 32 || is_p2(g.m));
+}
+bool FusedSurvey::pairs() const { return !fp64_ && p2_rows(); }
 
 void FusedSurvey::zfwd_pair(const void *rho_in, int ell_a, int m_a, int ell_b,
                             int m_b, const double xyz0[3], cudaStream_t s,
@@ -2059,7 +1669,7 @@ int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
   const YlmParams pr = make_ylm_params(ell, m, 4.0 * M_PI / ncells);
   const void *ktab = ksub ? k_table(ell, m, ka, s) : nullptr;
   const void *rtab = r_table(ell, m, raxis, pr, s);
-  const bool from_g = ell == 0 && g_of_input && is_p2(g.n0);
+  const bool from_g = ell == 0 && g_of_input;
   auto run = [&](auto tag) {
     using T = decltype(tag);
     if (from_g) {

@@ -7,21 +7,9 @@
 #include <vector>
 
 #include "fc_common.cuh"
-#include "fc_fft.cuh"
+#include "fc_fused_gen.h"
 
 namespace fc {
-
-// Geometry shared by the fused kernels (passed by value).
-struct FusedGeom {
-  int n0, n1, n2;  // grid shape
-  int m;           // N2 / 2: complex length of the z transform
-  int h;           // N2 / 2 + 1: half-complex z extent
-  int hp;          // row pitch of W, G, Wr, Wry: h rounded up to 16, so
-                   // every 16-column group starts on a 128-byte line
-  int rs, ro;      // r-subgrid edge and its centre offset (rs / 2)
-  int ks0, ks1, ks2;  // k-subgrid shape
-  FftPlan px, py, pz;
-};
 
 // Device pointers of the k axes and the per-axis |W|^2 window tables.
 struct KAxes {
@@ -37,8 +25,8 @@ struct PhaseHook {
 
 class FusedSurvey {
  public:
-  // True when every transform length factors into 2, 3, 5, 7, N2 is even
-  // and the shared-memory tiles fit.
+  // True when every side factors into 2, 3, 5, 7 and the shared-memory tiles
+  // fit.
   static bool supported(const int shape[3], int rsize);
 
   FusedSurvey(const int shape[3], int rsize, const int kshape[3], bool fp64);
@@ -91,8 +79,9 @@ class FusedSurvey {
  private:
   template <typename V>
   void upload(DeviceBuffer &dst, const std::vector<V> &v);
-  size_t smem(int L) const;
   void set_smem_limits();
+  // Whether the z passes are the power-of-two ones (even rows of m pairs).
+  bool p2_rows() const;
   template <typename T>
   void zfwd(const void *rho, bool weight, const YlmParams &p,
             const double xyz0[3], cudaStream_t s);
@@ -115,6 +104,7 @@ class FusedSurvey {
   void zinv(double *rsub, const void *rtab, cudaStream_t s);
 
   bool fp64_;
+  GenAxis gx, gy, gz;  // of the axes that are not powers of two
   DeviceBuffer tabx, taby, tabz;
   DeviceBuffer W, G, Wr, Wry, rho32;
   DeviceBuffer W2, rowtab2;  // the second term of a paired z pass

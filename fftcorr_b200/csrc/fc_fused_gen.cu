@@ -1,0 +1,741 @@
+// fc_fused_gen.cu -- the passes of the fused correlator (fc_fused.cu) along
+// an axis whose length is not a power of two, any product of 2, 3, 5 and 7,
+// even or odd, with the transform of fc_gfft.cuh.
+//
+// The column passes (x, y) take adjacent columns of one plane per CTA, 128
+// bytes of a row; the row passes (z) take pairs of rows, both of which ride
+// through one complex transform of the full row length as its real and
+// imaginary parts (so an odd row length needs nothing of its own) and are
+// separated by X_a(k) = (Z(k) + conj Z(N-k)) / 2 and X_b(k) = (Z(k) -
+// conj Z(N-k)) / 2i.  First passes read device memory into registers, last
+// passes write it from registers.
+//
+// Measured per launch on a 250 x 360 x 378 FP32 grid (34M cells, one B200),
+// against the engine before it (mixed radices chosen largest power of two
+// first, loads and stores as passes of their own through shared memory, one
+// column per thread, per-element modulos): z 339 -> 100 us, y 164 -> 67 us,
+// x with product and inverse 611 -> 134 us, inverse y 41 -> 19 us; a cross
+// correlation at ell <= 4 18.4 -> 5.6 ms.  The y pass moves 274 MB at 4.1
+// TB/s; all are bound by instruction issue and by barriers between the
+// passes (two or three CTAs of an SM at up to 80 registers).  One column per
+// thread instead of two took y 91 us and x 184 us; 64-byte rows (half the
+// tile, more CTAs) y 76 and x 162 us, from bank conflicts and scattered
+// twiddle loads.
+#include <algorithm>
+
+#include "fc_fused_gen.h"
+
+namespace fc {
+namespace {
+
+template <typename T>
+using C2 = typename Vec2<T>::type;
+
+constexpr int kRowThreads = 128;
+constexpr size_t kGenSmem = 200 * 1024;
+
+// What a thread carries through a transform: two complex columns (or row
+// pairs) in FP32, which share twiddles, indices and 16-byte accesses and use
+// the packed two-lane instructions, one in FP64.
+template <typename T>
+struct GElem;
+template <>
+struct GElem<float> {
+  using E = CPair;
+  static constexpr int W = 2;  // complex values per element
+  // The element at p, of which n values exist; the others are zero.
+  __device__ static CPair load(const float2 *p, int n) {
+    const float4 q = n > 0 ? *reinterpret_cast<const float4 *>(p) : make_float4(0, 0, 0, 0);
+    return cpack(make_float2(q.x, q.y), n > 1 ? make_float2(q.z, q.w) : make_float2(0, 0));
+  }
+  __device__ static void store(float2 *p, const CPair &v, int n) {
+    const float2 a = clane0(v), b = clane1(v);
+    if (n > 1) *reinterpret_cast<float4 *>(p) = make_float4(a.x, a.y, b.x, b.y);
+    else if (n > 0) *p = a;
+  }
+};
+template <>
+struct GElem<double> {
+  using E = double2;
+  static constexpr int W = 1;
+  __device__ static double2 load(const double2 *p, int n) {
+    return n > 0 ? *p : make_double2(0, 0);
+  }
+  __device__ static void store(double2 *p, const double2 &v, int n) {
+    if (n > 0) *p = v;
+  }
+};
+
+// A column pass takes B elements of a row per CTA.  With B = 8 a row is 128
+// bytes of device memory and of shared memory, which each 8-lane phase of a
+// 16-byte access covers without bank conflicts; longer transforms take 4,
+// padded, so that two CTAs still fit an SM.
+constexpr int pitch_of(int B) { return B == 8 ? 8 : B + 1; }
+template <typename T, int B>
+constexpr int kCols = B * GElem<T>::W;
+inline int col_width(int L) { return L <= 430 ? 8 : 4; }
+// Most threads of a y and of an x pass.
+constexpr int kYThreads = 512, kXThreads = 384;
+
+// A middle (or, with first, the first) pass over B columns of elements
+// between two shared buffers.
+template <int SIGN, int B, typename E, typename Tw>
+__device__ __forceinline__ void col_pass(const GPass &ps, const Tw *__restrict__ tw,
+                                         const E *src, E *dst, bool first) {
+  constexpr int BP = pitch_of(B);
+  with_radix(ps.R, [&]<int R>() {
+    for (int bf = threadIdx.x; bf < ps.LR * B; bf += blockDim.x) {
+      const int j = bf / B, b = bf % B;
+      E v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = src[(j + q * ps.LR) * BP + b];
+      int k = 0;
+      if (!first) {
+        k = j - gdiv(j, ps.Ns, ps.mNs) * ps.Ns;
+        g_twiddle<R, SIGN>(v, tw + ps.tw, ps.Ns, k);
+      }
+      GDft<R, SIGN, E>::run(v);
+      E *o = dst + ((j - k) * R + k) * BP + b;
+#pragma unroll
+      for (int q = 0; q < R; ++q) o[q * ps.Ns * BP] = v[q];
+    }
+  });
+  __syncthreads();
+}
+
+// The first pass, read from device memory (columns at and above nb are
+// zero), into dst.
+template <int SIGN, int B, typename T>
+__device__ __forceinline__ void col_first(const GPass &ps, const C2<T> *__restrict__ src,
+                                          int64_t stride, int nb,
+                                          typename GElem<T>::E *dst) {
+  using GE = GElem<T>;
+  using E = typename GE::E;
+  constexpr int BP = pitch_of(B);
+  with_radix(ps.R, [&]<int R>() {
+    for (int bf = threadIdx.x; bf < ps.LR * B; bf += blockDim.x) {
+      const int j = bf / B, b = bf % B;
+      const C2<T> *p = src + j * stride + GE::W * b;
+      E v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        v[q] = GE::load(p + (int64_t)(q * ps.LR) * stride, nb - GE::W * b);
+      GDft<R, SIGN, E>::run(v);
+      E *o = dst + j * R * BP + b;
+#pragma unroll
+      for (int q = 0; q < R; ++q) o[q * BP] = v[q];
+    }
+  });
+  __syncthreads();
+}
+
+// The last pass: store(i, b, value) for every output row i.
+template <int SIGN, int B, typename E, typename Tw, typename Store>
+__device__ __forceinline__ void col_last(const GPass &ps, const Tw *__restrict__ tw,
+                                         const E *src, Store store) {
+  constexpr int BP = pitch_of(B);
+  with_radix(ps.R, [&]<int R>() {
+    for (int bf = threadIdx.x; bf < ps.LR * B; bf += blockDim.x) {
+      const int j = bf / B, b = bf % B;
+      E v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = src[(j + q * ps.LR) * BP + b];
+      g_twiddle<R, SIGN>(v, tw + ps.tw, ps.Ns, j);
+      GDft<R, SIGN, E>::run(v);
+#pragma unroll
+      for (int q = 0; q < R; ++q) store(j + q * ps.LR, b, v[q]);
+    }
+  });
+}
+
+// The passes between the first and the last; returns the buffer they end in.
+template <int SIGN, int B, typename E, typename Tw>
+__device__ __forceinline__ E *col_middle(const GPlan &p, const Tw *__restrict__ tw,
+                                         E *src, E *dst) {
+  for (int s = 1; s + 1 < p.npass; ++s) {
+    col_pass<SIGN, B>(p.p[s], tw, src, dst, false);
+    E *t = src;
+    src = dst;
+    dst = t;
+  }
+  return src;
+}
+
+// ------------------------------------------------------------------ y
+template <typename T, int B>
+__global__ void __launch_bounds__(kYThreads, sizeof(T) == 4 ? 2 : 1)
+    k_gyfwd(C2<T> *W, FusedGeom g, const __grid_constant__ GPlan plan,
+            const C2<T> *__restrict__ tw) {
+  using GE = GElem<T>;
+  using E = typename GE::E;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  E *buf = reinterpret_cast<E *>(smem_raw);
+  const int kz0 = blockIdx.x * kCols<T, B>;
+  const int nb = g.h - kz0;
+  C2<T> *col = W + (int64_t)blockIdx.y * g.n1 * g.hp + kz0;
+  col_first<-1, B, T>(plan.p[0], col, g.hp, nb, buf);
+  const E *res = col_middle<-1, B>(plan, tw, buf, buf + g.n1 * pitch_of(B));
+  col_last<-1, B>(plan.p[plan.npass - 1], tw, res, [&](int i, int b, const E &v) {
+    GE::store(col + (int64_t)i * g.hp + GE::W * b, v, nb - GE::W * b);
+  });
+}
+
+template <typename T, int B>
+__global__ void __launch_bounds__(kYThreads, sizeof(T) == 4 ? 2 : 1)
+    k_gyinv(const C2<T> *__restrict__ Wr, C2<T> *__restrict__ Wry, FusedGeom g,
+            const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw) {
+  using GE = GElem<T>;
+  using E = typename GE::E;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  E *buf = reinterpret_cast<E *>(smem_raw);
+  const int kz0 = blockIdx.x * kCols<T, B>;
+  const int nb = g.h - kz0;
+  const C2<T> *col = Wr + (int64_t)blockIdx.y * g.n1 * g.hp + kz0;
+  C2<T> *out = Wry + (int64_t)blockIdx.y * g.rs * g.hp + kz0;
+  col_first<1, B, T>(plan.p[0], col, g.hp, nb, buf);
+  const E *res = col_middle<1, B>(plan, tw, buf, buf + g.n1 * pitch_of(B));
+  col_last<1, B>(plan.p[plan.npass - 1], tw, res, [&](int y, int b, const E &v) {
+    int rj = y + g.ro;
+    if (rj >= g.n1) rj -= g.n1;
+    for (; rj < g.rs; rj += g.n1)
+      GE::store(out + (int64_t)rj * g.hp + GE::W * b, v, nb - GE::W * b);
+  });
+}
+
+// ------------------------------------------------------------------ x
+// The real parts of an element's values.
+__device__ __forceinline__ double real_part(const CPair &v, int l) {
+  return (double)(l ? v.x.y : v.x.x);
+}
+__device__ __forceinline__ double real_part(const double2 &v, int) { return v.x; }
+
+// w |q|^2 as an element.
+__device__ __forceinline__ CPair abs2_elem(const CPair &q, float w) {
+  CPair r;
+  r.x = f2splat(w) * __ffma2_rn(q.x, q.x, q.y * q.y);
+  r.y = f2splat(0.f);
+  return r;
+}
+__device__ __forceinline__ double2 abs2_elem(const double2 &q, double w) {
+  return make_double2(w * (q.x * q.x + q.y * q.y), 0.0);
+}
+
+// MODE 0: G = DFT_x(W).  MODE 1: P = DFT_x(W) conj(G); MODE 2 (ell = 0 of an
+// autocorrelation): P = w00 |G|^2.  Then the k-subgrid extraction, straight
+// from the registers that hold P (every k-subgrid cell has one source
+// element, so the read-modify-writes never collide), and the inverse,
+// stored at the r-subgrid's rows.
+template <typename T, int B, int MODE>
+__global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
+    k_gx(const C2<T> *__restrict__ W, const C2<T> *__restrict__ G,
+         C2<T> *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
+         const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw,
+         const T *__restrict__ ktab, T w00) {
+  using GE = GElem<T>;
+  using E = typename GE::E;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  E *buf = reinterpret_cast<E *>(smem_raw);
+  constexpr int BP = pitch_of(B);
+  E *other = buf + g.n0 * BP;
+  const int kz0 = blockIdx.x * kCols<T, B>;
+  const int nb = g.h - kz0;
+  const int yy = blockIdx.y;
+  const int64_t stride = (int64_t)g.n1 * g.hp;
+  const int64_t base = (int64_t)yy * g.hp + kz0;
+  const GPass &last = plan.p[plan.npass - 1];
+  E *cur = buf;
+  if constexpr (MODE != 2) {
+    col_first<-1, B, T>(plan.p[0], W + base, stride, nb, buf);
+    cur = col_middle<-1, B>(plan, tw, buf, other);
+    other = cur == buf ? other : buf;
+  }
+  if constexpr (MODE == 0) {
+    col_last<-1, B>(last, tw, cur, [&](int i, int b, const E &v) {
+      GE::store(out + base + (int64_t)i * stride + GE::W * b, v, nb - GE::W * b);
+    });
+  } else {
+    const int ox = g.ks0 / 2, oy = g.ks1 / 2, oz = g.ks2 / 2;
+    int jr0 = yy + oy, jr1 = oy - yy;
+    if (jr0 >= g.n1) jr0 -= g.n1;
+    if (jr1 < 0) jr1 += g.n1;
+    const bool extract =
+        ksub != nullptr && kz0 <= oz && (jr0 < g.ks1 || jr1 < g.ks1);
+    auto to_ksub = [&](int x, int kz, double re) {
+#pragma unroll
+      for (int refl = 0; refl < 2; ++refl) {
+        if (refl && kz == 0) continue;
+        int i = refl ? ox - x : x + ox;
+        i = i < 0 ? i + g.n0 : (i >= g.n0 ? i - g.n0 : i);
+        for (; i < g.ks0; i += g.n0)
+          for (int j = refl ? jr1 : jr0; j < g.ks1; j += g.n1) {
+            const size_t cell =
+                ((size_t)i * g.ks1 + j) * g.ks2 + (refl ? oz - kz : oz + kz);
+            ksub[cell] += (double)ktab[cell] * re;
+          }
+      }
+    };
+    if constexpr (MODE == 1) {
+      with_radix(last.R, [&]<int R>() {
+        for (int bf = threadIdx.x; bf < last.LR * B; bf += blockDim.x) {
+          const int j = bf / B, b = bf % B;
+          const C2<T> *gp = G + base + j * stride + GE::W * b;
+          E gv[R], v[R];
+#pragma unroll
+          for (int q = 0; q < R; ++q)
+            gv[q] = GE::load(gp + (int64_t)(q * last.LR) * stride, nb - GE::W * b);
+#pragma unroll
+          for (int q = 0; q < R; ++q) v[q] = cur[(j + q * last.LR) * BP + b];
+          g_twiddle<R, -1>(v, tw + last.tw, last.Ns, j);
+          GDft<R, -1, E>::run(v);
+#pragma unroll
+          for (int q = 0; q < R; ++q) {
+            v[q] = cmulc(v[q], gv[q]);
+            other[(j + q * last.LR) * BP + b] = v[q];
+          }
+          if (extract) {
+#pragma unroll
+            for (int l = 0; l < GE::W; ++l) {
+              const int kz = kz0 + GE::W * b + l;
+              if (kz > oz) continue;
+#pragma unroll
+              for (int q = 0; q < R; ++q)
+                to_ksub(j + q * last.LR, kz, real_part(v[q], l));
+            }
+          }
+        }
+      });
+      E *t = cur;
+      cur = other;
+      other = t;
+    } else {
+      for (int idx = threadIdx.x; idx < g.n0 * B; idx += blockDim.x) {
+        const int x = idx / B, b = idx % B;
+        const E p = abs2_elem(
+            GE::load(G + base + x * stride + GE::W * b, nb - GE::W * b), w00);
+        if (extract) {
+#pragma unroll
+          for (int l = 0; l < GE::W; ++l)
+            if (kz0 + GE::W * b + l <= oz)
+              to_ksub(x, kz0 + GE::W * b + l, real_part(p, l));
+        }
+        cur[x * BP + b] = p;
+      }
+    }
+    __syncthreads();
+    col_pass<1, B>(plan.p[0], tw, cur, other, true);
+    const E *res = col_middle<1, B>(plan, tw, other, cur);
+    col_last<1, B>(last, tw, res, [&](int x, int b, const E &v) {
+      int ri = x + g.ro;
+      if (ri >= g.n0) ri -= g.n0;
+      for (; ri < g.rs; ri += g.n0)
+        GE::store(out + base + ri * stride + GE::W * b, v, nb - GE::W * b);
+    });
+  }
+}
+
+// ------------------------------------------------------------------ z
+// The z polynomial of Y_lm r^ell with the row's (x, y) fixed (row_poly in
+// fc_fused.cu), in the pass's precision, formed in FP64.
+template <typename T>
+struct RowCoef {
+  T c[5], rxy2;
+};
+
+// Y_lm D of a cell at z: D (c0 + c1 z + .. + c4 z^4) / r^ell.
+template <typename T, int ELL>
+__device__ __forceinline__ T row_value(const RowCoef<T> &r, T D, T z) {
+  const T z2 = z * z;
+  if constexpr (sizeof(T) == 4) {
+    const float ir2 = __fdividef(1.0f, r.rxy2 + z2 + 1e-20f);
+    if constexpr (ELL == 2) return D * ((r.c[2] * z + r.c[1]) * z + r.c[0]) * ir2;
+    return D * ((((r.c[4] * z + r.c[3]) * z + r.c[2]) * z + r.c[1]) * z + r.c[0]) *
+           (ir2 * ir2);
+  } else {
+    const double ir2 = 1.0 / (r.rxy2 + z2 + 1e-20);
+    if constexpr (ELL == 2) return D * ((r.c[2] * z + r.c[1]) * z + r.c[0]) * ir2;
+    return D * ((((r.c[4] * z + r.c[3]) * z + r.c[2]) * z + r.c[1]) * z + r.c[0]) *
+           ir2 * ir2;
+  }
+}
+
+// Shared index of element i of a row: one pad element in 8 spreads the
+// strided accesses over the banks.
+__device__ __forceinline__ int rpos(int i) { return i + (i >> 3); }
+
+// A pass over np rows of elements between shared buffers.
+template <int SIGN, typename E, typename Tw>
+__device__ __forceinline__ void row_pass(const GPass &ps, const Tw *__restrict__ tw,
+                                         const E *src, E *dst, int np, int pitch) {
+  with_radix(ps.R, [&]<int R>() {
+    for (int bf = threadIdx.x; bf < ps.LR * np; bf += blockDim.x) {
+      const int b = gdiv(bf, ps.LR, ps.mLR);
+      const int j = bf - b * ps.LR;
+      E v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = src[b * pitch + rpos(j + q * ps.LR)];
+      const int k = j - gdiv(j, ps.Ns, ps.mNs) * ps.Ns;
+      g_twiddle<R, SIGN>(v, tw + ps.tw, ps.Ns, k);
+      GDft<R, SIGN, E>::run(v);
+      const int o = (j - k) * R + k;
+#pragma unroll
+      for (int q = 0; q < R; ++q) dst[b * pitch + rpos(o + q * ps.Ns)] = v[q];
+    }
+  });
+  __syncthreads();
+}
+
+// Real component c (grid row c of the element's 2 W) of an element.
+__device__ __forceinline__ float &comp(CPair &v, int c) {
+  return c == 0 ? v.x.x : c == 1 ? v.y.x : c == 2 ? v.x.y : v.y.y;
+}
+__device__ __forceinline__ double &comp(double2 &v, int c) { return c ? v.y : v.x; }
+
+// ELL: -1 unweighted, else the weight's multipole.  np elements per CTA, each
+// of 2 W rows.
+template <typename T, int ELL>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
+    k_gzfwd(const T *__restrict__ rho, C2<T> *__restrict__ W, FusedGeom g,
+            const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw, int np,
+            YlmParams p, double x0, double y0, double z0) {
+  using E = typename GElem<T>::E;
+  constexpr int NR = 2 * GElem<T>::W;  // grid rows per element
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ RowCoef<T> rc[NR * kGenMaxPairs];
+  const int N = g.n2;
+  const int pitch = rpos(N - 1) + 1;
+  E *buf = reinterpret_cast<E *>(smem_raw);
+  E *other = buf + np * pitch;
+  const int64_t nrows = (int64_t)g.n0 * g.n1;
+  const int64_t row0 = (int64_t)blockIdx.x * NR * np;
+  if constexpr (ELL > 0) {
+    if ((int)threadIdx.x < NR * np) {
+      const int64_t row = min(row0 + threadIdx.x, nrows - 1);
+      const int x = (int)(row / g.n1);
+      const int y = (int)(row - (int64_t)x * g.n1);
+      double c[5];
+      row_poly_coefs(p, x0 + x * 1.0, y0 + y * 1.0, c);
+      RowCoef<T> r;
+      for (int i = 0; i < 5; ++i) r.c[i] = (T)c[i];
+      r.rxy2 = (T)((x0 + x) * (x0 + x) + (y0 + y) * (y0 + y));
+      rc[threadIdx.x] = r;
+    }
+    __syncthreads();
+  }
+  const GPass &f = plan.p[0];
+  with_radix(f.R, [&]<int R>() {
+    for (int bf = threadIdx.x; bf < f.LR * np; bf += blockDim.x) {
+      const int b = gdiv(bf, f.LR, f.mLR);
+      const int j = bf - b * f.LR;
+      const int64_t ra = row0 + NR * b;
+      const T *src = rho + (ra < nrows ? ra : 0) * N + j;
+      E v[R];
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        const bool on = ra + c < nrows;
+#pragma unroll
+        for (int q = 0; q < R; ++q) comp(v[q], c) = on ? src[c * N + q * f.LR] : (T)0;
+      }
+      if constexpr (ELL == 0) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+          v[q].x = v[q].x * (T)p.value0;
+          v[q].y = v[q].y * (T)p.value0;
+        }
+      } else if constexpr (ELL > 0) {
+        const T zj = (T)(z0 + j);
+#pragma unroll
+        for (int c = 0; c < NR; ++c) {
+          const RowCoef<T> a = rc[NR * b + c];
+#pragma unroll
+          for (int q = 0; q < R; ++q)
+            comp(v[q], c) = row_value<T, ELL>(a, comp(v[q], c), zj + (T)(q * f.LR));
+        }
+      }
+      GDft<R, -1, E>::run(v);
+#pragma unroll
+      for (int q = 0; q < R; ++q) buf[b * pitch + rpos(j * R + q)] = v[q];
+    }
+  });
+  __syncthreads();
+  for (int s = 1; s < plan.npass; ++s) {
+    row_pass<-1>(plan.p[s], tw, buf, other, np, pitch);
+    E *t = buf;
+    buf = other;
+    other = t;
+  }
+  for (int b = 0; b < np; ++b) {
+    const int64_t ra = row0 + NR * b;
+    if (ra >= nrows) break;
+    C2<T> *dst = W + ra * g.hp;
+    for (int k = threadIdx.x; k < g.h; k += blockDim.x) {
+      E z = buf[b * pitch + rpos(k)];
+      E c = buf[b * pitch + rpos(k == 0 ? 0 : N - k)];
+#pragma unroll
+      for (int l = 0; l < NR; l += 2) {
+        const T zx = comp(z, l), zy = comp(z, l + 1);
+        const T cx = comp(c, l), cy = -comp(c, l + 1);
+        C2<T> xa, xb;
+        xa.x = (T)0.5 * (zx + cx);
+        xa.y = (T)0.5 * (zy + cy);
+        xb.x = (T)0.5 * (zy - cy);
+        xb.y = (T)0.5 * (cx - zx);
+        if (ra + l < nrows) dst[l * g.hp + k] = xa;
+        if (ra + l + 1 < nrows) dst[(l + 1) * g.hp + k] = xb;
+      }
+    }
+  }
+}
+
+// Pairs of rows of Wry to real rows, accumulated into the r-subgrid.
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
+    k_gzinv(const C2<T> *__restrict__ Wry, double *__restrict__ rsub, FusedGeom g,
+            const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw, int np,
+            const T *__restrict__ rtab) {
+  using E = typename GElem<T>::E;
+  constexpr int NR = 2 * GElem<T>::W;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int N = g.n2;
+  const int pitch = rpos(N - 1) + 1;
+  E *buf = reinterpret_cast<E *>(smem_raw);
+  E *other = buf + np * pitch;
+  const int nrows = g.rs * g.rs;
+  const int row0 = blockIdx.x * NR * np;
+  const GPass &f = plan.p[0];
+  with_radix(f.R, [&]<int R>() {
+    for (int bf = threadIdx.x; bf < f.LR * np; bf += blockDim.x) {
+      const int b = gdiv(bf, f.LR, f.mLR);
+      const int j = bf - b * f.LR;
+      const int ra = row0 + NR * b;
+      const C2<T> *src = Wry + (int64_t)(ra < nrows ? ra : 0) * g.hp;
+      E v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int k = j + q * f.LR;
+        const int kk = k < g.h ? k : N - k;
+        const bool real = kk == 0 || 2 * kk == N;  // DC and Nyquist
+#pragma unroll
+        for (int l = 0; l < NR; l += 2) {
+          C2<T> xa, xb;
+          xa.x = xa.y = xb.x = xb.y = 0;
+          if (ra + l < nrows) xa = src[l * g.hp + kk];
+          if (ra + l + 1 < nrows) xb = src[(l + 1) * g.hp + kk];
+          const T sg = real ? (T)0 : k >= g.h ? (T)-1 : (T)1;
+          comp(v[q], l) = xa.x - sg * xb.y;
+          comp(v[q], l + 1) = sg * xa.y + xb.x;
+        }
+      }
+      GDft<R, 1, E>::run(v);
+#pragma unroll
+      for (int q = 0; q < R; ++q) buf[b * pitch + rpos(j * R + q)] = v[q];
+    }
+  });
+  __syncthreads();
+  for (int s = 1; s + 1 < plan.npass; ++s) {
+    row_pass<1>(plan.p[s], tw, buf, other, np, pitch);
+    E *t = buf;
+    buf = other;
+    other = t;
+  }
+  const GPass &l = plan.p[plan.npass - 1];
+  with_radix(l.R, [&]<int R>() {
+    for (int bf = threadIdx.x; bf < l.LR * np; bf += blockDim.x) {
+      const int b = gdiv(bf, l.LR, l.mLR);
+      const int j = bf - b * l.LR;
+      const int ra = row0 + NR * b;
+      if (ra >= nrows) break;
+      E v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = buf[b * pitch + rpos(j + q * l.LR)];
+      g_twiddle<R, 1>(v, tw + l.tw, l.Ns, j);
+      GDft<R, 1, E>::run(v);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        int rk = j + q * l.LR + g.ro;
+        if (rk >= N) rk -= N;
+        for (; rk < g.rs; rk += N) {
+#pragma unroll
+          for (int c = 0; c < NR; ++c) {
+            if (ra + c >= nrows) continue;
+            const size_t cell = (size_t)(ra + c) * g.rs + rk;
+            rsub[cell] += (double)rtab[cell] * (double)comp(v[q], c);
+          }
+        }
+      }
+    }
+  });
+}
+
+size_t col_smem(int L) { return 2 * (size_t)L * pitch_of(col_width(L)) * 16; }
+
+// Threads of a column pass: one butterfly each of the pass with the most, or
+// an equal share of several.
+int col_threads(const GPlan &p, int most) {
+  int n = 0;
+  for (int s = 0; s < p.npass; ++s)
+    if (p.p[s].R > 1) n = std::max(n, p.p[s].LR * col_width(p.L));
+  const int rounds = (n + most - 1) / most;
+  const int t = rounds > 0 ? (n + rounds - 1) / rounds : 32;
+  return std::max(64, (t + 31) / 32 * 32);
+}
+
+// Elements (of 2 W rows) per CTA of a z pass: about one butterfly of the
+// first pass per thread, within the shared memory and the coefficient table,
+// and few enough that `total` elements still make two CTAs per SM.
+size_t row_smem(int L, int np) { return 2 * (size_t)np * (L + L / 8 + 1) * 16; }
+int row_elems(const GPlan &p, int64_t total) {
+  int np = (kRowThreads + p.p[0].LR / 2) / p.p[0].LR;
+  np = std::min(np, (int)(44 * 1024 / row_smem(p.L, 1)));
+  np = (int)std::min<int64_t>(np, total / (2 * sm_count()));
+  return std::max(1, std::min(np, kGenMaxPairs));
+}
+int row_threads(const GPlan &p, int np) {
+  int n = 0;
+  for (int s = 0; s < p.npass; ++s)
+    if (p.p[s].R > 1) n = std::max(n, p.p[s].LR * np);
+  return std::max(32, std::min(kRowThreads, (n + 31) / 32 * 32));
+}
+
+template <typename K>
+void big_smem(K kernel) {
+  FC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kGenSmem));
+}
+
+template <typename T, int B>
+void col_limits() {
+  big_smem(k_gyfwd<T, B>);
+  big_smem(k_gyinv<T, B>);
+  big_smem(k_gx<T, B, 0>);
+  big_smem(k_gx<T, B, 1>);
+  big_smem(k_gx<T, B, 2>);
+}
+template <typename T>
+void set_limits(int L, bool row) {
+  if (row) {
+    big_smem(k_gzfwd<T, -1>);
+    big_smem(k_gzfwd<T, 0>);
+    big_smem(k_gzfwd<T, 2>);
+    big_smem(k_gzfwd<T, 4>);
+    big_smem(k_gzinv<T>);
+  } else if (col_width(L) == 8) {
+    col_limits<T, 8>();
+  } else {
+    col_limits<T, 4>();
+  }
+}
+
+}  // namespace
+
+bool gen_supported(int L, bool row) {
+  GPlan p;
+  if (!gplan_length(L, &p)) return false;
+  if (row) return row_smem(L, 1) <= kGenSmem;
+  return col_smem(L) <= kGenSmem;
+}
+
+void GenAxis::init(int L, bool row, bool fp64) {
+  FC_REQUIRE(gplan_length(L, &plan), FC_ERR_UNSUPPORTED,
+             "grid size has a prime factor above 7");
+  auto put = [&](const auto &t) {
+    tw.resize(t.size() * sizeof(t[0]));
+    FC_CUDA(cudaMemcpy(tw.get(), t.data(), t.size() * sizeof(t[0]),
+                       cudaMemcpyHostToDevice));
+  };
+  if (fp64) {
+    put(gplan_twiddles<double2>(plan));
+    set_limits<double>(L, row);
+  } else {
+    put(gplan_twiddles<float2>(plan));
+    set_limits<float>(L, row);
+  }
+}
+
+template <typename T>
+void gen_zfwd(const GenAxis &a, const FusedGeom &g, const T *rho, C2<T> *W, bool weight,
+              const YlmParams &p, const double xyz0[3], cudaStream_t s) {
+  constexpr int NR = 2 * GElem<T>::W;
+  const int64_t nrows = (int64_t)g.n0 * g.n1;
+  const int np = row_elems(a.plan, (nrows + NR - 1) / NR);
+  const unsigned blocks = (unsigned)((nrows + NR * np - 1) / (NR * np));
+  const size_t sm = row_smem(g.n2, np);
+  auto go = [&](auto kernel) {
+    kernel<<<blocks, row_threads(a.plan, np), sm, s>>>(rho, W, g, a.plan, a.tw.as<C2<T>>(), np, p,
+                                           xyz0[0], xyz0[1], xyz0[2]);
+  };
+  if (!weight) go(k_gzfwd<T, -1>);
+  else if (p.ell == 0) go(k_gzfwd<T, 0>);
+  else if (p.ell == 2) go(k_gzfwd<T, 2>);
+  else go(k_gzfwd<T, 4>);
+  FC_LAUNCH_CHECK();
+}
+
+// Calls f.template operator()<B>() for the axis's column width.
+template <typename F>
+void with_width(const GenAxis &a, F &&f) {
+  if (col_width(a.plan.L) == 8) f.template operator()<8>();
+  else f.template operator()<4>();
+}
+
+template <typename T>
+void gen_yfwd(const GenAxis &a, const FusedGeom &g, C2<T> *W, cudaStream_t s) {
+  with_width(a, [&]<int B>() {
+    constexpr int NC = kCols<T, B>;
+    k_gyfwd<T, B><<<dim3((g.h + NC - 1) / NC, g.n0), col_threads(a.plan, kYThreads),
+                    col_smem(g.n1), s>>>(W, g, a.plan, a.tw.as<C2<T>>());
+  });
+  FC_LAUNCH_CHECK();
+}
+
+template <typename T>
+void gen_x(const GenAxis &a, const FusedGeom &g, int mode, const C2<T> *W, const C2<T> *G,
+           C2<T> *out, double *ksub, const T *ktab, T w00, cudaStream_t s) {
+  with_width(a, [&]<int B>() {
+    constexpr int NC = kCols<T, B>;
+    auto go = [&](auto kernel) {
+      kernel<<<dim3((g.h + NC - 1) / NC, g.n1), col_threads(a.plan, kXThreads), col_smem(g.n0), s>>>(
+          W, G, out, ksub, g, a.plan, a.tw.as<C2<T>>(), ktab, w00);
+    };
+    if (mode == 0) go(k_gx<T, B, 0>);
+    else if (mode == 1) go(k_gx<T, B, 1>);
+    else go(k_gx<T, B, 2>);
+  });
+  FC_LAUNCH_CHECK();
+}
+
+template <typename T>
+void gen_yinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wr, C2<T> *Wry,
+              cudaStream_t s) {
+  with_width(a, [&]<int B>() {
+    constexpr int NC = kCols<T, B>;
+    k_gyinv<T, B><<<dim3((g.h + NC - 1) / NC, g.rs), col_threads(a.plan, kYThreads),
+                    col_smem(g.n1), s>>>(Wr, Wry, g, a.plan, a.tw.as<C2<T>>());
+  });
+  FC_LAUNCH_CHECK();
+}
+
+template <typename T>
+void gen_zinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wry, double *rsub,
+              const T *rtab, cudaStream_t s) {
+  constexpr int NR = 2 * GElem<T>::W;
+  const int nrows = g.rs * g.rs;
+  const int np = row_elems(a.plan, (nrows + NR - 1) / NR);
+  k_gzinv<T><<<(nrows + NR * np - 1) / (NR * np), row_threads(a.plan, np), row_smem(g.n2, np), s>>>(
+      Wry, rsub, g, a.plan, a.tw.as<C2<T>>(), np, rtab);
+  FC_LAUNCH_CHECK();
+}
+
+#define FC_GEN(T)                                                                      \
+  template void gen_zfwd<T>(const GenAxis &, const FusedGeom &, const T *, C2<T> *,    \
+                            bool, const YlmParams &, const double[3], cudaStream_t);   \
+  template void gen_yfwd<T>(const GenAxis &, const FusedGeom &, C2<T> *, cudaStream_t); \
+  template void gen_x<T>(const GenAxis &, const FusedGeom &, int, const C2<T> *,       \
+                         const C2<T> *, C2<T> *, double *, const T *, T, cudaStream_t); \
+  template void gen_yinv<T>(const GenAxis &, const FusedGeom &, const C2<T> *,         \
+                            C2<T> *, cudaStream_t);                                    \
+  template void gen_zinv<T>(const GenAxis &, const FusedGeom &, const C2<T> *,         \
+                            double *, const T *, cudaStream_t);
+FC_GEN(float)
+FC_GEN(double)
+
+}  // namespace fc

@@ -1,0 +1,34 @@
+"""The fused passes along axes of every kind of length against the oracle:
+single-radix and length-1 axes, odd rows, axes long enough for the narrow
+column tiles, and a k-subgrid that reaches the Nyquist planes of even and odd
+sides."""
+import numpy as np
+import pytest
+
+import fftcorr_b200 as fb
+from fftcorr_b200.correlate import TSC_ALIASED_CORRECTION
+from oracle import fc_oracle as O
+from test_gpu_parity import FP64_RTOL, _compare_results
+
+pytestmark = pytest.mark.gpu
+
+CELL = 10.0
+
+
+@pytest.mark.parametrize("shape", [(7, 450, 9), (486, 5, 14), (12, 432, 250), (1, 30, 21),
+                                   (10, 27, 35), (128, 6, 63), (45, 64, 128)])
+@pytest.mark.parametrize("kmax", [0.15, 0.35])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_survey_axis_lengths(shape, kmax, precision):
+    rng = np.random.default_rng(5)
+    a, b = rng.standard_normal(shape), rng.standard_normal(shape)
+    posmin = np.array([-40.0, 25.0, -35.0])
+    rmax = CELL * min(5, min(shape))
+    args = (CELL, posmin, TSC_ALIASED_CORRECTION, rmax, 6.0, kmax, 0.03, 4)
+    c = fb.Correlator(shape, *args, precision=precision)
+    c.autocorrelate(a)
+    _compare_results(c.results(), O.survey_correlate(a, *args), FP64_RTOL, "auto",
+                     fp32=precision == "fp32")
+    c.cross_correlate(a, b)
+    _compare_results(c.results(), O.survey_correlate(a, *args, grid2=b), FP64_RTOL,
+                     "cross", fp32=precision == "fp32")
