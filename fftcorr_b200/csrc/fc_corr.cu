@@ -192,6 +192,21 @@ __global__ void k_cell_bins(const double *__restrict__ ax,
   }
 }
 
+// Sets *differ when a subgrid cell and its mirror image (n - 1 - c) have
+// different bins.
+__global__ void k_bins_differ(const int *__restrict__ bins, size_t n, int *differ) {
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n / 2;
+       c += (size_t)gridDim.x * blockDim.x)
+    if (bins[c] != bins[n - 1 - c]) *differ = 1;
+}
+
+// Subgrid cells of a bin index to the cells the fused passes store.
+__global__ void k_half_cells(uint32_t *perm, size_t n, FusedGeom g, int k) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x)
+    perm[i] = (uint32_t)(k ? half_k_cell(g, perm[i]) : half_r_cell(g, perm[i]));
+}
+
 // Converts an FP64 complex grid to FP32 (set_grid2_fft in mixed precision).
 // rows of h complex values, written `pitch` elements apart.
 __global__ void k_z2c(const double2 *in, float2 *out, size_t n, int h,
@@ -451,12 +466,16 @@ struct Correlator {
       FC_CUDA(cudaEventCreate(&ev_stop));
       const char *mode = std::getenv("FFTCORR_B200_FFT");
       const bool want_fused = !(mode && std::string(mode) == "cufft");
+      upload_axes();
+      const bool even = build_bins();
       if (kind == FC_SURVEY && want_fused &&
-          FusedSurvey::supported(geo.shape, geo.rsize))
-        fused.reset(new FusedSurvey(geo.shape, geo.rsize, geo.kshape, fp64()));
+          FusedSurvey::supported(geo.shape, geo.rsize)) {
+        fused.reset(
+            new FusedSurvey(geo.shape, geo.rsize, geo.kshape, fp64(), even));
+        half_cells();
+      }
       allocate();
       if (!fused) make_plans();
-      build_bins();
       // Every (ell, m) weight table now: a correlation (a served job on a
       // resident correlator in particular) then allocates nothing.
       if (fused)
@@ -488,10 +507,23 @@ struct Correlator {
   bool fp64() const { return precision == FC_FP64; }
   size_t real_bytes() const { return fp64() ? 8 : 4; }
 
+  // Cells of the subgrids as they are stored.
+  size_t rsub_cells() const { return fused ? fused->r_cells() : geo.rcells(); }
+  size_t ksub_cells() const { return fused ? fused->k_cells() : geo.kcells(); }
+
   void allocate() {
     if (!fused) work.resize(geo.nreal_padded() * real_bytes());
-    rsub.resize(geo.rcells() * sizeof(double));
-    ksub.resize(geo.kcells() * sizeof(double));
+    rsub.resize(rsub_cells() * sizeof(double));
+    ksub.resize(ksub_cells() * sizeof(double));
+    d_rhist.resize(std::max(1, geo.nrows * geo.nr) * sizeof(double));
+    d_khist.resize(std::max(1, geo.nrows * geo.nk) * sizeof(double));
+    d_zerolag.resize(sizeof(double));
+    FC_CUDA(cudaMemset(d_rhist.get(), 0, d_rhist.bytes()));
+    FC_CUDA(cudaMemset(d_khist.get(), 0, d_khist.bytes()));
+    FC_CUDA(cudaMemset(d_zerolag.get(), 0, d_zerolag.bytes()));
+  }
+
+  void upload_axes() {
     d_raxis.resize(geo.rsize * sizeof(double));
     FC_CUDA(cudaMemcpy(d_raxis.get(), geo.raxis.data(),
                        geo.rsize * sizeof(double), cudaMemcpyHostToDevice));
@@ -509,12 +541,6 @@ struct Correlator {
                        cudaMemcpyHostToDevice));
     FC_CUDA(cudaMemcpy(d_kwin.get(), wn.data(), nk * sizeof(double),
                        cudaMemcpyHostToDevice));
-    d_rhist.resize(std::max(1, geo.nrows * geo.nr) * sizeof(double));
-    d_khist.resize(std::max(1, geo.nrows * geo.nk) * sizeof(double));
-    d_zerolag.resize(sizeof(double));
-    FC_CUDA(cudaMemset(d_rhist.get(), 0, d_rhist.bytes()));
-    FC_CUDA(cudaMemset(d_khist.get(), 0, d_khist.bytes()));
-    FC_CUDA(cudaMemset(d_zerolag.get(), 0, d_zerolag.bytes()));
   }
 
   // Creates both plans; on a failure neither is left behind (the
@@ -557,8 +583,10 @@ struct Correlator {
     FC_CUFFT(cufftSetStream(plan_c2r, stream));
   }
 
-  void build_bins() {
+  // Returns whether every r-subgrid cell has the bin of its mirror image.
+  bool build_bins() {
     const double *kaxes = d_kaxes.as<double>();
+    int differ = 0;
     {
       DeviceBuffer b(geo.rcells() * sizeof(int) + 16);
       const double *ra = d_raxis.as<double>();
@@ -566,6 +594,13 @@ struct Correlator {
           ra, ra, ra, geo.rsize, geo.rsize, geo.rsize, dr_(), geo.nr,
           b.as<int>());
       FC_LAUNCH_CHECK();
+      DeviceBuffer flag(sizeof(int));
+      FC_CUDA(cudaMemsetAsync(flag.get(), 0, sizeof(int), stream));
+      k_bins_differ<<<grid_for(geo.rcells(), 256), 256, 0, stream>>>(
+          b.as<int>(), geo.rcells(), flag.as<int>());
+      FC_LAUNCH_CHECK();
+      FC_CUDA(cudaMemcpyAsync(&differ, flag.get(), sizeof(int), cudaMemcpyDeviceToHost,
+                              stream));
       rbins.build(b.as<int>(), geo.rcells(), geo.nr, stream);
     }
     {
@@ -576,6 +611,19 @@ struct Correlator {
           b.as<int>());
       FC_LAUNCH_CHECK();
       kbins.build(b.as<int>(), geo.kcells(), geo.nk, stream);
+    }
+    return differ == 0;
+  }
+
+  // The bin indices' cells as the fused passes store them.
+  void half_cells() {
+    for (int k = 0; k < 2; ++k) {
+      BinIndex &b = k ? kbins : rbins;
+      const size_t n = (size_t)b.ninrange;
+      if (n == 0) continue;
+      k_half_cells<<<grid_for(n, 256), 256, 0, stream>>>(b.perm.as<uint32_t>(), n,
+                                                         fused->g, k);
+      FC_LAUNCH_CHECK();
     }
   }
 
@@ -708,13 +756,14 @@ struct Correlator {
   }
 
   void zero_sub(bool r, bool k) {
-    if (r) FC_CUDA(cudaMemsetAsync(rsub.get(), 0, geo.rcells() * sizeof(double), stream));
-    if (k) FC_CUDA(cudaMemsetAsync(ksub.get(), 0, geo.kcells() * sizeof(double), stream));
+    if (r) FC_CUDA(cudaMemsetAsync(rsub.get(), 0, rsub_cells() * sizeof(double), stream));
+    if (k) FC_CUDA(cudaMemsetAsync(ksub.get(), 0, ksub_cells() * sizeof(double), stream));
   }
 
   void save_zerolag() {
-    const size_t rz = ((size_t)geo.rmax_cells * geo.rsize + geo.rmax_cells) *
-                          geo.rsize + geo.rmax_cells;
+    const size_t rz = fused ? fused->zero_lag()
+                            : ((size_t)geo.rmax_cells * geo.rsize + geo.rmax_cells) *
+                                      geo.rsize + geo.rmax_cells;
     FC_CUDA(cudaMemcpyAsync(d_zerolag.get(), rsub.as<double>() + rz,
                             sizeof(double), cudaMemcpyDeviceToDevice, stream));
   }
@@ -912,7 +961,8 @@ struct Correlator {
       size_t next = 0;
       bool second_ready = false;
       for (int ell = 0; ell <= maxell; ell += 2) {
-        zero_sub(true, true);
+        // The multipole's first term overwrites the subgrids.
+        bool first = true;
         for (; next < owned.size() && owned[next][0] == ell; ++next) {
           const int m = owned[next][1];
           bool z_done = false;
@@ -930,9 +980,11 @@ struct Correlator {
           // alone for the ell = 0 term of an autocorrelation.
           n_fft += fused->term(in, ell, m, xyz0, (double)ncells,
                                ksub.as<double>(), rsub.as<double>(),
-                               d_raxis.as<double>(), ka, stream, ph, prepared,
-                               z_done);
+                               d_raxis.as<double>(), ka, stream, ph, first,
+                               prepared, z_done);
+          first = false;
         }
+        if (first) zero_sub(true, true);
         hist_rows(ell, true, true);
         if (ell == 0) save_zerolag();
       }
@@ -1113,8 +1165,9 @@ size_t correlator_footprint(int kind, const int shape[3], double cell,
   if (kind == FC_SURVEY && want_fused && FusedSurvey::supported(g.shape, g.rsize)) {
     const size_t h = (g.shape[2] / 2 + 1 + 15) / 16 * 16;   // row pitch
     bytes += 2 * (size_t)g.shape[0] * g.shape[1] * h * eb;   // W, G
-    bytes += (size_t)g.rsize * g.shape[1] * h * eb;          // Wr
-    bytes += (size_t)g.rsize * g.rsize * h * eb;             // Wry
+    // Wr and Wry, and below the r-subgrid, whole: the even form keeps half.
+    bytes += (size_t)g.rsize * g.shape[1] * h * eb;
+    bytes += (size_t)g.rsize * g.rsize * h * eb;
     if (precision != FC_FP64) {                              // FP32 density,
       bytes += g.ncells() * 4 + (size_t)g.shape[0] * g.shape[1] * 32;  // row table
       const int m = g.shape[2] / 2;

@@ -15,6 +15,18 @@
 //   yinv   Wry[ri][rj][kz] = IDFT_y(Wr) at the rs rows of the r-subgrid
 //   zinv   rsub[ri][rj][rk] += Y_lm(r) 4 pi/N * C2R_z(Wry)[rk] (fft_grid.cc:
 //          182-210)
+// Both histograms are over |k| and |r|, and Y_lm is even for even ell, so only
+// the part of P that is even in k contributes: Re P, whose inverse transform
+// is even in r.  The k-subgrid is stored for kz >= 0 alone.  Where every
+// r-subgrid cell and its mirror image fall into the same bin (the bins of r
+// and -r are computed from rounded coordinates, so this is checked when a
+// correlator is made), the inverse takes Re P -- two real columns ride
+// through one complex transform -- and stops at the rows x >= 0, half the
+// work of the inverse passes; otherwise it transforms P itself.  Per launch
+// at 512^3 FP32: x pass 324 -> 279 us, inverse y 37 -> 22 us, inverse z 23 ->
+// 14 us (a correlation 11.8 -> 10.8 ms); at 256^3 FP64: 105 -> 85 us, 15 -> 9
+// us, 9 -> 8 us; the x pass at 64^3, whose extraction walked the k-subgrid's
+// rows one after another, 27 -> 11 us.
 // grid2's transform G (correlator.h:53-77) is zfwd (no weighting) + yfwd +
 // DFT_x.  Bytes per (ell, m) at 512^3 FP32: ~4 GB instead of ~11 GB for
 // separate make_ylm / cuFFT r2c / multiply / extract / cuFFT c2r passes.
@@ -171,6 +183,25 @@ struct P2 {
   }
 };
 
+// The same layout with BB columns.
+template <typename T, int L, int BB>
+struct P2B {
+  static constexpr int TPC = L / 8;
+  static constexpr int THREADS = TPC * BB;
+  static constexpr int RB = BB * (int)sizeof(C2<T>);
+  static constexpr int R = RB >= 128 ? 1 : 128 / RB;
+  __device__ static __forceinline__ int row(int i) {
+    return i ^ ((i >> 3) & (R - 1));
+  }
+  static constexpr bool kFastRead = (TPC / 8) % R == 0;
+  __device__ static __forceinline__ int rd_base(int t, int b) {
+    return kFastRead ? row(t) * BB + b : 0;
+  }
+  __device__ static __forceinline__ int rd(int base, int t, int b, int u) {
+    return kFastRead ? base + u * TPC * BB : row(t + TPC * u) * BB + b;
+  }
+};
+
 template <typename T, int L>
 __global__ void __launch_bounds__(P2<T, L>::THREADS)
     k_yfwd_p2(C2<T> *__restrict__ W, FusedGeom g,
@@ -234,14 +265,79 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
   }
 }
 
-template <typename T, int L, int MODE>
-__global__ void __launch_bounds__(P2<T, L>::THREADS)
-    k_xcorr_p2(const C2<T> *__restrict__ W, const C2<T> *__restrict__ G,
-               C2<T> *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
-               const C2<T> *__restrict__ tabx, const T *__restrict__ ktab,
-               T w00) {
-  using C = C2<T>;
-  using Q = P2<T, L>;
+// Adds a thread's real parts re[u] of P at rows t + TPC u, columns kz ..
+// kz + W - 1, to the stored half of the k-subgrid (half_k_cell; the last cell
+// may be the row's padding), or overwrites it when `first`.  A cell has one
+// source element, so nothing collides.
+template <int L, int W, typename KT, typename Re>
+__device__ __forceinline__ void to_half_k(double *__restrict__ ksub,
+                                          const KT *__restrict__ ktab,
+                                          const FusedGeom &g, int t, int jr, int kz,
+                                          bool first, Re re) {
+  constexpr int TPC = L / 8;
+  constexpr int N = 4 / W;  // rows whose loads go out together
+  const int ox = g.ks0 / 2;
+  for (int j = jr; j < g.ks1; j += g.n1)
+#pragma unroll
+    for (int u0 = 0; u0 < 8; u0 += N) {
+      size_t cell[N];
+      double w[N][W], acc[N][W];
+      bool on[N];
+#pragma unroll
+      for (int s = 0; s < N; ++s) {
+        const int i = (t + TPC * (u0 + s) + ox) & (L - 1);
+        on[s] = i < g.ks0;
+        cell[s] = ((size_t)i * g.ks1 + j) * g.kp + kz;
+#pragma unroll
+        for (int l = 0; l < W; ++l) {
+          w[s][l] = acc[s][l] = 0.0;
+          if (on[s]) {
+            w[s][l] = (double)ktab[cell[s] + l];
+            if (!first) acc[s][l] = ksub[cell[s] + l];
+          }
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < N; ++s)
+#pragma unroll
+        for (int l = 0; l < W; ++l)
+          if (on[s]) ksub[cell[s] + l] = acc[s][l] + w[s][l] * re(u0 + s, l);
+    }
+  // A k-subgrid of L + 1 rows holds row L / 2 of P at both of its ends.
+  if (g.ks0 > L && t == (L / 2) % TPC)
+    for (int j = jr; j < g.ks1; j += g.n1) {
+      const size_t c = ((size_t)L * g.ks1 + j) * g.kp + kz;
+      for (int l = 0; l < W; ++l)
+        ksub[c + l] = (first ? 0.0 : ksub[c + l]) +
+                      (double)ktab[c + l] * re(L / 2 / TPC, l);
+    }
+}
+
+// The columns A and B of Z = DFT(a + i b), a and b real, from Z at x and at
+// -x: A = (Z(x) + conj Z(-x)) / 2, B = (Z(x) - conj Z(-x)) / 2i.
+template <typename C>
+__device__ __forceinline__ void split_pair(const C &z, const C &m, C *a, C *b) {
+  using T = decltype(z.x);
+  a->x = (T)0.5 * (z.x + m.x);
+  a->y = (T)0.5 * (z.y - m.y);
+  b->x = (T)0.5 * (z.y + m.y);
+  b->y = (T)0.5 * (m.x - z.x);
+}
+
+// FP64.  MODE 0: out = G = DFT_x(W).  MODE 1: the product, extraction and
+// inverse described at the top; MODE 2 (ell = 0 of an autocorrelation): the
+// weighted field is w00 * rho, whose transform is w00 * G, so P = w00 |G|^2
+// and neither W nor a forward transform is needed.  EVEN: the inverse of
+// Re P, two real columns to a complex one: half of the CTA's threads
+// transform half as many columns, the others leave.
+template <int L, int MODE, bool EVEN>
+__global__ void __launch_bounds__(P2<double, L>::THREADS)
+    k_xcorr_p2(const double2 *__restrict__ W, const double2 *__restrict__ G,
+               double2 *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
+               const double2 *__restrict__ tabx, const double *__restrict__ ktab,
+               double w00, int first) {
+  using C = double2;
+  using Q = P2<double, L>;
   extern __shared__ unsigned char smem_raw[];
   C *ex = reinterpret_cast<C *>(smem_raw);
   const int t = threadIdx.x / Q::B;
@@ -257,34 +353,19 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
   // In product mode the G column is loaded together with the W column, so
   // both streams are in flight during the forward transform.
   C gv[MODE == 1 ? 8 : 1];
-  if constexpr (MODE == 2) {
-    // ell = 0 of an autocorrelation: the weighted field is w00 * rho, whose
-    // transform is w00 * G, so the product is w00 |G|^2 and neither W nor a
-    // forward transform is needed.
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      C gg;
-      gg.x = 0;
-      gg.y = 0;
-      if (valid) gg = G[base + (t + Q::TPC * u) * stride];
-      v[u].x = w00 * (gg.x * gg.x + gg.y * gg.y);
-      v[u].y = 0;
+  for (int u = 0; u < 8; ++u) {
+    v[u] = make_double2(0, 0);
+    const int64_t at = base + (t + Q::TPC * u) * stride;
+    if constexpr (MODE == 2) {
+      if (valid) {
+        const C q = G[at];
+        v[u].x = w00 * (q.x * q.x + q.y * q.y);
+      }
+    } else {
+      if (valid) v[u] = W[at];
     }
-  } else {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      v[u].x = 0;
-      v[u].y = 0;
-      if (valid) v[u] = W[base + (t + Q::TPC * u) * stride];
-    }
-  }
-  if constexpr (MODE == 1) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      gv[u].x = 0;
-      gv[u].y = 0;
-      if (valid) gv[u] = G[base + (t + Q::TPC * u) * stride];
-    }
+    if constexpr (MODE == 1) gv[u] = valid ? G[at] : make_double2(0, 0);
   }
   const int rb = Q::rd_base(t, b);
   auto exr = [&](int u) { return &ex[Q::rd(rb, t, b, u)]; };
@@ -299,69 +380,49 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
 #pragma unroll
       for (int u = 0; u < 8; ++u) v[u] = cmulc(v[u], gv[u]);
     }
-    // k-subgrid extraction (see k_xcorr): needs P at arbitrary rows.  Only
-    // CTAs whose y feeds a k-subgrid row (for either sign of ky) and whose
-    // kz range reaches it stage P in shared memory.
-    const int ox = g.ks0 / 2, oy = g.ks1 / 2, oz = g.ks2 / 2;
-    const int jr0 = (yy + oy) % g.n1;
-    const int jr1 = ((oy - yy) % g.n1 + g.n1) % g.n1;
-    if (ksub != nullptr && kz0 <= oz && (jr0 < g.ks1 || jr1 < g.ks1)) {
+    const int jr = (yy + g.ks1 / 2) % g.n1;
+    if (ksub != nullptr && jr < g.ks1 && kzi <= g.ks2 / 2)
+      to_half_k<L, 1>(ksub, ktab, g, t, jr, kzi, first != 0,
+                      [&](int u, int) { return v[u].x; });
+    if constexpr (EVEN) {
+      constexpr int H = Q::B / 2;
+      using QH = P2B<double, L, H>;
+      double *st = reinterpret_cast<double *>(smem_raw);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) *exf(t + Q::TPC * u) = v[u];
+      for (int u = 0; u < 8; ++u) st[(t + Q::TPC * u) * Q::B + b] = v[u].x;
       __syncthreads();
-      if (valid && kzi <= oz) {
-        if (g.ks0 <= 3 * Q::TPC && g.ks1 <= g.n1) {
-          // At most three x rows per thread and one row j per reflection:
-          // each reflection's loads are issued together.
+      if (threadIdx.x >= QH::THREADS) return;
+      const int t2 = threadIdx.x / H, b2 = threadIdx.x % H;
+      C z[8];
 #pragma unroll
-          for (int refl = 0; refl < 2; ++refl) {
-            const int j = refl == 0 ? jr0 : jr1;
-            if (j >= g.ks1 || (refl == 1 && kzi == 0)) continue;
-            const int k = refl == 0 ? kzi + oz : oz - kzi;
-            size_t cell[3];
-            double acc[3], w[3], re[3];
-#pragma unroll
-            for (int s = 0; s < 3; ++s) {
-              const int i = t + s * Q::TPC;
-              cell[s] = ((size_t)i * g.ks1 + j) * g.ks2 + k;
-              if (i < g.ks0) {
-                const int x = refl == 0 ? (i - ox) & (L - 1)
-                                        : (ox - i) & (L - 1);
-                re[s] = (double)exf(x)->x;
-                w[s] = (double)ktab[cell[s]];
-                acc[s] = ksub[cell[s]];
-              }
-            }
-#pragma unroll
-            for (int s = 0; s < 3; ++s)
-              if (t + s * Q::TPC < g.ks0) ksub[cell[s]] = acc[s] + w[s] * re[s];
-          }
-        } else {
-          for (int refl = 0; refl < 2; ++refl) {
-            if (refl == 1 && kzi == 0) continue;
-            const int k = refl == 0 ? kzi + oz : oz - kzi;
-            for (int j = refl == 0 ? jr0 : jr1; j < g.ks1; j += g.n1) {
-              for (int i = t; i < g.ks0; i += Q::TPC) {
-                const int x = refl == 0 ? (i - ox) & (L - 1)
-                                        : (ox - i) & (L - 1);
-                const double re = (double)exf(x)->x;
-                const size_t cell = ((size_t)i * g.ks1 + j) * g.ks2 + k;
-                ksub[cell] += (double)ktab[cell] * re;
-              }
-            }
-          }
-        }
-      }
+      for (int u = 0; u < 8; ++u) z[u] = ex[(t2 + Q::TPC * u) * H + b2];
       __syncthreads();
-    }
-    reg_fft<L>(v, t, exf, exr, tabx, +1);
-    if (valid) {
-      const int64_t obase = (int64_t)yy * g.hp + kzi;
+      const int rb2 = QH::rd_base(t2, b2);
+      auto zf = [&](int i) { return &ex[QH::row(i) * H + b2]; };
+      reg_fft<L>(z, t2, zf, [&](int u) { return &ex[QH::rd(rb2, t2, b2, u)]; }, tabx, +1);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const int x = t + Q::TPC * u;
-        for (int ri = (x + g.ro) & (L - 1); ri < g.rs; ri += L)
-          out[obase + ri * stride] = v[u];
+        const int x = t2 + Q::TPC * u;
+        if (x <= g.ro || x >= L - g.ro) *zf(x) = z[u];
+      }
+      __syncthreads();
+      const int c = kz0 + 2 * b2;
+      for (int x = t2; x <= g.ro; x += Q::TPC) {
+        C A, B;
+        split_pair(*zf(x & (L - 1)), *zf((L - x) & (L - 1)), &A, &B);
+        C *o = out + x * stride + (int64_t)yy * g.hp + c;
+        if (c < g.h) o[0] = A;
+        if (c + 1 < g.h) o[1] = B;
+      }
+    } else {
+      reg_fft<L>(v, t, exf, exr, tabx, +1);
+      if (valid) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int x = t + Q::TPC * u;
+          for (int ri = (x + g.ro) & (L - 1); ri < g.rs; ri += L)
+            out[base + ri * stride] = v[u];
+        }
       }
     }
   }
@@ -445,7 +506,7 @@ template <typename T, int L>
 __global__ void __launch_bounds__(P2<T, L>::THREADS)
     k_zinv_p2(const C2<T> *__restrict__ Wry, double *__restrict__ rsub,
               FusedGeom g, const C2<T> *__restrict__ tabz,
-              const T *__restrict__ rtab) {
+              const T *__restrict__ rtab, int first) {
   using C = C2<T>;
   using Q = P2<T, L>;
   constexpr int RP = L + L / 8 + 1;
@@ -453,7 +514,7 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
   C *ex = reinterpret_cast<C *>(smem_raw);
   const int b = threadIdx.x / Q::TPC;
   const int t = threadIdx.x - b * Q::TPC;
-  const int nrows = g.rs * g.rs;
+  const int nrows = g.nri * g.rs;
   const int row = blockIdx.x * Q::B + b;
   const bool valid = row < nrows;
   C v[8];
@@ -488,7 +549,7 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
       const double val = (double)(h ? v[u].y : v[u].x);
       for (int rk = (z + g.ro) % g.n2; rk < g.rs; rk += g.n2) {
         const size_t cell = (size_t)row * g.rs + rk;
-        rsub[cell] += (double)rtab[cell] * val;
+        rsub[cell] = (first ? 0.0 : rsub[cell]) + (double)rtab[cell] * val;
       }
     }
   }
@@ -699,80 +760,17 @@ __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
 // k-subgrid extraction and the inverse transform, stored only at the
 // r-subgrid's rows.  G is read after the forward transform, so a thread
 // holds one pair of columns at a time and two CTAs fit an SM; the other
-// CTA's warps cover those loads.
+// CTA's warps cover those loads.  EVEN: the inverse of Re P: a pair of real
+// columns is one complex column, so half of the CTA's threads carry the
+// columns of two pairs through one transform each and the others leave.
 constexpr int kXB = 16;  // columns per CTA of the FP32 x passes
 
-// k-subgrid extraction of k_xcorr_pp (as in k_xcorr_p2) for the columns c0
-// and c0 + 1 of thread (t, p), from P staged in the exchange slots.  Not
-// inlined, so that its registers do not weigh on the kernel's transforms;
-// only the CTAs whose y and kz reach the k-subgrid call it.
-template <int L>
-__device__ __noinline__ void xcorr_pp_extract(const CPair *ex, int t, int p,
-                                              int c0, int jr0, int jr1, int ks0,
-                                              int ks1, int ks2, int n1,
-                                              double *__restrict__ ksub,
-                                              const float *__restrict__ ktab) {
-  using Q = PY<L, kXB>;
-  const int ox = ks0 / 2, oz = ks2 / 2;
-  auto exf = [&](int i) { return &ex[Q::row(i) * Q::PB + p]; };
-  if (ks0 <= 3 * Q::TPC && ks1 <= n1) {
-    // At most three x rows per thread and one row j per reflection: each
-    // reflection's loads are issued together.
-#pragma unroll
-    for (int refl = 0; refl < 2; ++refl) {
-      const int j = refl == 0 ? jr0 : jr1;
-      if (j >= ks1) continue;
-      size_t cell[3][2];
-      double acc[3][2], w[3][2], re[3][2];
-      bool on[3][2];
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const int i = t + s * Q::TPC;
-        const int x = refl == 0 ? (i - ox) & (L - 1) : (ox - i) & (L - 1);
-#pragma unroll
-        for (int ln = 0; ln < 2; ++ln) {
-          const int kzi = c0 + ln;
-          on[s][ln] = i < ks0 && kzi <= oz && !(refl == 1 && kzi == 0);
-          const int k = refl == 0 ? kzi + oz : oz - kzi;
-          cell[s][ln] = ((size_t)i * ks1 + j) * ks2 + k;
-          if (on[s][ln]) {
-            re[s][ln] = (double)(ln ? exf(x)->x.y : exf(x)->x.x);
-            w[s][ln] = (double)ktab[cell[s][ln]];
-            acc[s][ln] = ksub[cell[s][ln]];
-          }
-        }
-      }
-#pragma unroll
-      for (int s = 0; s < 3; ++s)
-#pragma unroll
-        for (int ln = 0; ln < 2; ++ln)
-          if (on[s][ln]) ksub[cell[s][ln]] = acc[s][ln] + w[s][ln] * re[s][ln];
-    }
-    return;
-  }
-  for (int ln = 0; ln < 2; ++ln) {
-    const int kzi = c0 + ln;
-    if (kzi > oz) continue;
-    for (int refl = 0; refl < 2; ++refl) {
-      if (refl == 1 && kzi == 0) continue;
-      const int k = refl == 0 ? kzi + oz : oz - kzi;
-      for (int j = refl == 0 ? jr0 : jr1; j < ks1; j += n1) {
-        for (int i = t; i < ks0; i += Q::TPC) {
-          const int x = refl == 0 ? (i - ox) & (L - 1) : (ox - i) & (L - 1);
-          const double re = (double)(ln ? exf(x)->x.y : exf(x)->x.x);
-          const size_t cell = ((size_t)i * ks1 + j) * ks2 + k;
-          ksub[cell] += (double)ktab[cell] * re;
-        }
-      }
-    }
-  }
-}
-
-template <int L, int MODE, bool SPLIT>
+template <int L, int MODE, bool SPLIT, bool EVEN>
 __device__ __forceinline__ void xcorr_pp_body(
     const float2 *__restrict__ W, const float2 *__restrict__ G,
     float2 *__restrict__ out, double *__restrict__ ksub, const FusedGeom &g,
-    const float2 *__restrict__ tabx, const float *__restrict__ ktab, float w00) {
+    const float2 *__restrict__ tabx, const float *__restrict__ ktab, float w00,
+    int first) {
   using Q = PY<L, kXB>;
   extern __shared__ unsigned char smem_raw[];
   CPair *ex = reinterpret_cast<CPair *>(smem_raw);
@@ -812,65 +810,108 @@ __device__ __forceinline__ void xcorr_pp_body(
     });
     cp_async_wait_all();
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      v[u] = cmulc(v[u], load_pair(reinterpret_cast<const float2 *>(exr(u))));
-  }
-  // k-subgrid extraction, as in k_xcorr_p2, for both columns of the pair.
-  const int oy = g.ks1 / 2, oz = g.ks2 / 2;
-  const int jr0 = (yy + oy) % g.n1;
-  const int jr1 = ((oy - yy) % g.n1 + g.n1) % g.n1;
-  if (ksub != nullptr && cb <= oz && (jr0 < g.ks1 || jr1 < g.ks1)) {
-    // P goes through shared memory and is read back afterwards, so the
-    // registers of the pair are free while the extraction runs.
-#pragma unroll
-    for (int u = 0; u < 8; ++u) *exr(u) = v[u];
-    __syncthreads();
-    if (c0 <= oz)
-      xcorr_pp_extract<L>(ex, t, p, c0, jr0, jr1, g.ks0, g.ks1, g.ks2, g.n1,
-                          ksub, ktab);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = *exr(u);
-    __syncthreads();
-  } else if constexpr (MODE == 1) {
-    // Every thread has read G from its slots before the inverse transform's
-    // first exchange writes over them.
-    __syncthreads();
-  }
-  // Rows x whose r-subgrid row (x + ro) mod L is below rs; when they all lie
-  // in the first and last TPC rows, only outputs u = 0 and 7 are computed.
-  const bool edges = g.ro <= Q::TPC && g.rs - g.ro <= Q::TPC;
-  reg_fft<L>(v, t, exf, exr, tabx, +1, 1, NoHook{}, edges);
-  if (edges) {
-#pragma unroll
-    for (int u = 0; u < 8; u += 7) {
-      const int ri = (t + Q::TPC * u + g.ro) & (L - 1);
-      if (ri < g.rs) cp.store(out, ri * stride, v[u]);
+    for (int u = 0; u < 8; ++u) {
+      const CPair gp = load_pair(reinterpret_cast<const float2 *>(exr(u)));
+      if constexpr (EVEN) v[u].x = __ffma2_rn(v[u].y, gp.y, __fmul2_rn(v[u].x, gp.x));
+      else v[u] = cmulc(v[u], gp);
     }
-    return;
   }
+  const int jr = (yy + g.ks1 / 2) % g.n1;
+  if (!SPLIT && ksub != nullptr && jr < g.ks1 && c0 <= g.ks2 / 2)
+    to_half_k<L, 2>(ksub, ktab, g, t, jr, c0, first != 0, [&](int u, int l) {
+      return (double)(l ? v[u].x.y : v[u].x.x);
+    });
+  // Every thread has read G from its slots before anything is written over
+  // them.
+  if constexpr (MODE == 1) __syncthreads();
+  if constexpr (EVEN) {
+    constexpr int H = Q::PB / 2;
+    using QH = PY<L, Q::B / 2>;
+    static_assert(QH::PB == H && 2 * QH::THREADS == Q::THREADS);
+    // A column that does not exist must not reach its neighbour's transform.
+    float2 *st = reinterpret_cast<float2 *>(smem_raw);
 #pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int x = t + Q::TPC * u;
-    for (int ri = (x + g.ro) & (L - 1); ri < g.rs; ri += L)
-      cp.store(out, ri * stride, v[u]);
+    for (int u = 0; u < 8; ++u)
+      st[(t + Q::TPC * u) * Q::PB + p] =
+          make_float2(cp.v0 ? v[u].x.x : 0.f, cp.v1 ? v[u].x.y : 0.f);
+    __syncthreads();
+    if (threadIdx.x >= QH::THREADS) return;
+    const int t2 = threadIdx.x / H, p2 = threadIdx.x % H;
+    CPair z[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      z[u] = load_pair(st + (t2 + Q::TPC * u) * Q::PB + 2 * p2);
+    __syncthreads();
+    const int rb2 = QH::rd_base(t2, p2);
+    auto zf = [&](int i) { return &ex[QH::row(i) * H + p2]; };
+    // Only rows |x| <= ro are stored: when they all lie in the first and last
+    // TPC rows, only outputs u = 0 and 7 are computed.
+    const bool edges = g.ro < Q::TPC;
+    reg_fft<L>(z, t2, zf, [&](int u) { return &ex[QH::rd(rb2, t2, p2, u)]; }, tabx, +1,
+               1, NoHook{}, edges);
+    if (edges) {
+      *zf(t2) = z[0];
+      *zf(t2 + 7 * Q::TPC) = z[7];
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) *zf(t2 + Q::TPC * u) = z[u];
+    }
+    __syncthreads();
+    for (int x = t2; x <= g.ro; x += Q::TPC) {
+      const CPair zp = *zf(x & (L - 1)), zm = *zf((L - x) & (L - 1));
+      float2 c[4];
+      split_pair(clane0(zp), clane0(zm), &c[0], &c[1]);
+      split_pair(clane1(zp), clane1(zm), &c[2], &c[3]);
+      float2 *o = out + x * stride;
+      if constexpr (SPLIT) {
+        const int pl = yy * Q::B + 4 * p2;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (pl + i < g.n1) o[(int64_t)(pl + i) * g.hp + g.h - 1] = c[i];
+      } else {
+        const int k = cb + 4 * p2;
+        o += (int64_t)yy * g.hp + k;
+        if (k + 3 < g.h) {
+          reinterpret_cast<float4 *>(o)[0] = make_float4(c[0].x, c[0].y, c[1].x, c[1].y);
+          reinterpret_cast<float4 *>(o)[1] = make_float4(c[2].x, c[2].y, c[3].x, c[3].y);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (k + i < g.h) o[i] = c[i];
+        }
+      }
+    }
+  } else {
+    // Rows x whose r-subgrid row (x + ro) mod L is below rs; when they all
+    // lie in the first and last TPC rows, only outputs u = 0 and 7 are
+    // computed.
+    const bool edges = g.ro <= Q::TPC && g.rs - g.ro <= Q::TPC;
+    reg_fft<L>(v, t, exf, exr, tabx, +1, 1, NoHook{}, edges);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (edges && u != 0 && u != 7) continue;
+      const int x = t + Q::TPC * u;
+      for (int ri = (x + g.ro) & (L - 1); ri < g.rs; ri += L)
+        cp.store(out, ri * stride, v[u]);
+    }
   }
 }
 
-template <int L, int MODE>
+template <int L, int MODE, bool EVEN>
 __global__ void __launch_bounds__(PY<L, kXB>::THREADS, 1024 / PY<L, kXB>::THREADS)
     k_xcorr_pp(const float2 *__restrict__ W, const float2 *__restrict__ G,
                float2 *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
                const float2 *__restrict__ tabx, const float *__restrict__ ktab,
-               float w00, int nyq) {
+               float w00, int nyq, int first) {
   // The last column split off (nyq) pays in the product mode only; the
   // ell = 0 mode compiles without it (with it: 215 vs 188 us).
   if constexpr (MODE == 1) {
     if (split_cta(nyq)) {
-      xcorr_pp_body<L, MODE, true>(W, G, out, ksub, g, tabx, ktab, w00);
+      xcorr_pp_body<L, MODE, true, EVEN>(W, G, out, ksub, g, tabx, ktab, w00, first);
       return;
     }
   }
-  xcorr_pp_body<L, MODE, false>(W, G, out, ksub, g, tabx, ktab, w00);
+  xcorr_pp_body<L, MODE, false, EVEN>(W, G, out, ksub, g, tabx, ktab, w00, first);
 }
 
 template <int L, bool SPLIT>
@@ -883,10 +924,10 @@ __device__ __forceinline__ void yinv_pp_body(const float2 *__restrict__ Wr,
   CPair *ex = reinterpret_cast<CPair *>(smem_raw);
   const int t = threadIdx.x / Q::PB;
   const int p = threadIdx.x - t * Q::PB;
-  // Planes are the r-subgrid's x rows ri: L * g.hp elements apart in Wr,
+  // Planes are the r-subgrid's x rows: L * g.hp elements apart in Wr,
   // rs * g.hp in Wry.
   ColPair<SPLIT> cp;
-  if (!col_pair<Q::B>(cp, p, blockIdx.y, (int64_t)L * g.hp, g.rs, g)) return;
+  if (!col_pair<Q::B>(cp, p, blockIdx.y, (int64_t)L * g.hp, g.nri, g)) return;
   CPair v[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) v[u] = cp.load(Wr, (int64_t)(t + Q::TPC * u) * g.hp);
@@ -896,7 +937,7 @@ __device__ __forceinline__ void yinv_pp_body(const float2 *__restrict__ Wr,
              [&](int u) { return &ex[Q::rd(rb, t, p, u)]; }, taby, +1, 1,
              NoHook{}, edges);
   ColPair<SPLIT> co;  // the same columns of the same planes in Wry
-  col_pair<Q::B>(co, p, blockIdx.y, (int64_t)g.rs * g.hp, g.rs, g);
+  col_pair<Q::B>(co, p, blockIdx.y, (int64_t)g.rs * g.hp, g.nri, g);
   if (edges) {
 #pragma unroll
     for (int u = 0; u < 8; u += 7) {
@@ -1192,15 +1233,16 @@ __global__ void k_rowpoly(float4 *__restrict__ tab, int64_t nrows, int n1,
 // normalisation (make_ylm, correlator.h:477-480), computed once per
 // correlator and multipole so the z inverse pass does a multiply-add.
 template <typename RT>
-__global__ void k_rtable(RT *__restrict__ tab, int rs,
+__global__ void k_rtable(RT *__restrict__ tab, FusedGeom g,
                          const double *__restrict__ raxis, YlmParams pr) {
-  const size_t n = (size_t)rs * rs * rs;
+  const size_t n = (size_t)g.nri * g.rs * g.rs;
+  const int x0 = g.rs - g.nri;  // the even form keeps the rows x >= 0
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
-    const int rk = (int)(i % rs);
-    const int rj = (int)((i / rs) % rs);
-    const int ri = (int)(i / ((size_t)rs * rs));
-    tab[i] = (RT)ylm_eval(pr, 1.0, raxis[ri], raxis[rj], raxis[rk]);
+    const int rk = (int)(i % g.rs);
+    const int rj = (int)((i / g.rs) % g.rs);
+    const int ri = (int)(i / ((size_t)g.rs * g.rs));
+    tab[i] = (RT)ylm_eval(pr, 1.0, raxis[x0 + ri], raxis[rj], raxis[rk]);
   }
 }
 
@@ -1209,21 +1251,20 @@ __global__ void k_rtable(RT *__restrict__ tab, int rs,
 // per correlator and multipole so the extraction in the x pass is a
 // multiply-add.
 template <typename KT>
-__global__ void k_ktable(KT *__restrict__ tab, int k0, int k1, int k2,
-                         const double *__restrict__ kx,
-                         const double *__restrict__ ky,
-                         const double *__restrict__ kz,
-                         const double *__restrict__ wx,
-                         const double *__restrict__ wy,
-                         const double *__restrict__ wz, YlmParams pk) {
-  const size_t n = (size_t)k0 * k1 * k2;
+__global__ void k_ktable(KT *__restrict__ tab, FusedGeom g, KAxes ax, YlmParams pk) {
+  const int oz = g.ks2 / 2;
+  const size_t n = (size_t)g.ks0 * g.ks1 * g.kp;
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
        c += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(c % k2);
-    const int j = (int)((c / k2) % k1);
-    const int i = (int)(c / ((size_t)k2 * k1));
-    const double inv_w = 1.0 / (wx[i] * wy[j] * wz[k]);
-    tab[c] = (KT)ylm_eval(pk, inv_w, kx[i], ky[j], kz[k]);
+    const int k = (int)(c % g.kp) + oz;
+    const int j = (int)((c / g.kp) % g.ks1);
+    const int i = (int)(c / ((size_t)g.kp * g.ks1));
+    if (k >= g.ks2) {  // padding of the row
+      tab[c] = (KT)0;
+      continue;
+    }
+    const double inv_w = 1.0 / (ax.wx[i] * ax.wy[j] * ax.wz[k]);
+    tab[c] = (KT)ylm_eval(pk, inv_w, ax.kx[i], ax.ky[j], ax.kz[k]);
   }
 }
 
@@ -1273,42 +1314,36 @@ void with_p2(int L, F &&f) {
   }
 }
 
+template <typename K>
+void big_smem(K kernel) {
+  FC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               200 * 1024));
+}
+
 template <typename T, int L>
 void p2_set_limits() {
-  const int big = 200 * 1024;
-  FC_CUDA(cudaFuncSetAttribute(k_yfwd_p2<T, L>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_yinv_p2<T, L>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_xcorr_p2<T, L, 0>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_xcorr_p2<T, L, 1>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_xcorr_p2<T, L, 2>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_zfwd_p2<T, L, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_zfwd_p2<T, L, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FC_CUDA(cudaFuncSetAttribute(k_zinv_p2<T, L>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  if constexpr (std::is_same_v<T, float>) {
-    FC_CUDA(cudaFuncSetAttribute(k_yfwd_pp<L>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    FC_CUDA(cudaFuncSetAttribute(k_yinv_pp<L>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    FC_CUDA(cudaFuncSetAttribute(k_xfwd_pp<L>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    FC_CUDA(cudaFuncSetAttribute(k_xcorr_pp<L, 1>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    FC_CUDA(cudaFuncSetAttribute(k_xcorr_pp<L, 2>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    FC_CUDA(cudaFuncSetAttribute(k_zfwd_pp<L, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    FC_CUDA(cudaFuncSetAttribute(k_zfwd_pp<L, false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    FC_CUDA(cudaFuncSetAttribute(k_zfwd_pp2<L>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  big_smem(k_zinv_p2<T, L>);
+  if constexpr (std::is_same_v<T, double>) {
+    big_smem(k_yfwd_p2<T, L>);
+    big_smem(k_yinv_p2<T, L>);
+    big_smem(k_xcorr_p2<L, 0, false>);
+    big_smem(k_xcorr_p2<L, 1, false>);
+    big_smem(k_xcorr_p2<L, 2, false>);
+    big_smem(k_xcorr_p2<L, 1, true>);
+    big_smem(k_xcorr_p2<L, 2, true>);
+    big_smem(k_zfwd_p2<T, L, true>);
+    big_smem(k_zfwd_p2<T, L, false>);
+  } else {
+    big_smem(k_yfwd_pp<L>);
+    big_smem(k_yinv_pp<L>);
+    big_smem(k_xfwd_pp<L>);
+    big_smem(k_xcorr_pp<L, 1, false>);
+    big_smem(k_xcorr_pp<L, 2, false>);
+    big_smem(k_xcorr_pp<L, 1, true>);
+    big_smem(k_xcorr_pp<L, 2, true>);
+    big_smem(k_zfwd_pp<L, true>);
+    big_smem(k_zfwd_pp<L, false>);
+    big_smem(k_zfwd_pp2<L>);
   }
 }
 
@@ -1320,7 +1355,7 @@ bool FusedSurvey::supported(const int shape[3], int rsize) {
 }
 
 FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
-                         bool fp64)
+                         bool fp64, bool even)
     : fp64_(fp64) {
   g.n0 = shape[0];
   g.n1 = shape[1];
@@ -1333,6 +1368,8 @@ FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
   g.ks0 = kshape[0];
   g.ks1 = kshape[1];
   g.ks2 = kshape[2];
+  g.kp = (g.ks2 / 2 + 1 + 3) / 4 * 4;
+  g.nri = even ? g.ro + 1 : g.rs;
   // Axes that the power-of-two passes do not take.
   if (!is_p2(g.n0)) gx.init(g.n0, false, fp64);
   if (!is_p2(g.n1)) gy.init(g.n1, false, fp64);
@@ -1350,8 +1387,8 @@ FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
   const size_t nc = (size_t)g.n0 * g.n1 * g.hp;
   W.resize(nc * eb);
   G.resize(nc * eb);
-  Wr.resize((size_t)g.rs * g.n1 * g.hp * eb);
-  Wry.resize((size_t)g.rs * g.rs * g.hp * eb);
+  Wr.resize((size_t)g.nri * g.n1 * g.hp * eb);
+  Wry.resize((size_t)g.nri * g.rs * g.hp * eb);
   if (!fp64) {
     rho32.resize((size_t)g.n0 * g.n1 * g.n2 * sizeof(float));
     rowtab.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
@@ -1458,63 +1495,60 @@ void FusedSurvey::yfwd(cudaStream_t s) {
 }
 
 template <typename T>
-void FusedSurvey::xcorr(bool product, double *ksub, const void *ktab_v,
-                        cudaStream_t s) {
-  const T *ktab = static_cast<const T *>(ktab_v);
-  if (is_p2(g.n0)) {
-    with_p2(g.n0, [&]<int L>() {
-      using Q = P2<T, L>;
-      dim3 grid((g.h + Q::B - 1) / Q::B, g.n1);
-      if (!product && std::is_same_v<T, float>) {
-        using Y = PY<L>;
-        dim3 gy((g.h + Y::B - 1) / Y::B, g.n1);
-        k_xfwd_pp<L><<<gy, Y::THREADS, Y::smem, s>>>(
-            W.as<float2>(), G.as<float2>(), g, tabx.as<float2>());
-      } else if (!product)
-        k_xcorr_p2<T, L, 0><<<grid, Q::THREADS, p2_col_smem<T, L>(), s>>>(
-            W.as<C2<T>>(), nullptr, G.as<C2<T>>(), nullptr, g, tabx.as<C2<T>>(),
-            nullptr, T(0));
-      else if constexpr (std::is_same_v<T, float>) {
-        using Y = PY<L, kXB>;
-        dim3 gy((g.h + Y::B - 1) / Y::B, g.n1);
-        k_xcorr_pp<L, 1><<<gy, Y::THREADS, Y::smem, s>>>(
-            W.as<float2>(), G.as<float2>(), Wr.as<float2>(), ksub, g,
-            tabx.as<float2>(), ktab, 0.f, nyq_group<Y::B>(ksub != nullptr));
-      } else
-        k_xcorr_p2<T, L, 1><<<grid, Q::THREADS, p2_col_smem<T, L>(), s>>>(
-            W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, g,
-            tabx.as<C2<T>>(), ktab, T(0));
-    });
-    FC_LAUNCH_CHECK();
-    return;
-  }
-  if (product)
-    gen_x<T>(gx, g, 1, W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, ktab, T(0), s);
-  else
-    gen_x<T>(gx, g, 0, W.as<C2<T>>(), nullptr, G.as<C2<T>>(), nullptr, nullptr, T(0), s);
-}
-
-template <typename T>
-void FusedSurvey::xcorr00(double *ksub, const void *ktab_v, double w00,
-                          cudaStream_t s) {
-  const T *ktab = static_cast<const T *>(ktab_v);
+void FusedSurvey::grid2_x(cudaStream_t s) {
   if (!is_p2(g.n0)) {
-    gen_x<T>(gx, g, 2, nullptr, G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, ktab, (T)w00, s);
+    gen_x<T>(gx, g, 0, W.as<C2<T>>(), nullptr, G.as<C2<T>>(), nullptr, nullptr, T(0), true, s);
     return;
   }
   with_p2(g.n0, [&]<int L>() {
-    using Q = P2<T, L>;
+    if constexpr (std::is_same_v<T, float>) {
+      using Y = PY<L>;
+      k_xfwd_pp<L><<<dim3((g.h + Y::B - 1) / Y::B, g.n1), Y::THREADS, Y::smem, s>>>(
+          W.as<float2>(), G.as<float2>(), g, tabx.as<float2>());
+    } else {
+      using Q = P2<T, L>;
+      k_xcorr_p2<L, 0, false>
+          <<<dim3((g.h + Q::B - 1) / Q::B, g.n1), Q::THREADS, p2_col_smem<T, L>(), s>>>(
+              W.as<C2<T>>(), nullptr, G.as<C2<T>>(), nullptr, g, tabx.as<C2<T>>(), nullptr,
+              T(0), 1);
+    }
+  });
+  FC_LAUNCH_CHECK();
+}
+
+template <typename T>
+void FusedSurvey::xcorr(bool from_g, double *ksub, const void *ktab_v, double w00,
+                        bool first, cudaStream_t s) {
+  const T *ktab = static_cast<const T *>(ktab_v);
+  if (!is_p2(g.n0)) {
+    gen_x<T>(gx, g, from_g ? 2 : 1, W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub,
+             ktab, (T)w00, first, s);
+    return;
+  }
+  with_p2(g.n0, [&]<int L>() {
     if constexpr (std::is_same_v<T, float>) {
       using Y = PY<L, kXB>;
-      dim3 gy((g.h + Y::B - 1) / Y::B, g.n1);
-      k_xcorr_pp<L, 2><<<gy, Y::THREADS, Y::smem, s>>>(
-          nullptr, G.as<float2>(), Wr.as<float2>(), ksub, g, tabx.as<float2>(),
-          ktab, (float)w00, 0);
+      auto go = [&](auto kernel, int nyq) {
+        kernel<<<dim3((g.h + Y::B - 1) / Y::B, g.n1), Y::THREADS, Y::smem, s>>>(
+            W.as<float2>(), G.as<float2>(), Wr.as<float2>(), ksub, g, tabx.as<float2>(),
+            ktab, (float)w00, nyq, first);
+      };
+      const int nyq = nyq_group<Y::B>(ksub != nullptr);
+      if (from_g && even()) go(k_xcorr_pp<L, 2, true>, 0);
+      else if (from_g) go(k_xcorr_pp<L, 2, false>, 0);
+      else if (even()) go(k_xcorr_pp<L, 1, true>, nyq);
+      else go(k_xcorr_pp<L, 1, false>, nyq);
     } else {
-      dim3 grid((g.h + Q::B - 1) / Q::B, g.n1);
-      k_xcorr_p2<T, L, 2><<<grid, Q::THREADS, p2_col_smem<T, L>(), s>>>(
-          nullptr, G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, g, tabx.as<C2<T>>(),
-          ktab, (T)w00);
+      using Q = P2<T, L>;
+      auto go = [&](auto kernel) {
+        kernel<<<dim3((g.h + Q::B - 1) / Q::B, g.n1), Q::THREADS, p2_col_smem<T, L>(), s>>>(
+            W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, g, tabx.as<C2<T>>(), ktab,
+            w00, first);
+      };
+      if (from_g && even()) go(k_xcorr_p2<L, 2, true>);
+      else if (from_g) go(k_xcorr_p2<L, 2, false>);
+      else if (even()) go(k_xcorr_p2<L, 1, true>);
+      else go(k_xcorr_p2<L, 1, false>);
     }
   });
   FC_LAUNCH_CHECK();
@@ -1527,12 +1561,12 @@ void FusedSurvey::yinv(cudaStream_t s) {
       using Q = P2<T, L>;
       if constexpr (std::is_same_v<T, float>) {
         using Y = PY<L>;
-        dim3 grid((g.h + Y::B - 1) / Y::B, g.rs);
+        dim3 grid((g.h + Y::B - 1) / Y::B, g.nri);
         k_yinv_pp<L><<<grid, Y::THREADS, Y::smem, s>>>(
             Wr.as<float2>(), Wry.as<float2>(), g, taby.as<float2>(),
             nyq_group<Y::B>(false));
       } else {
-        dim3 grid((g.h + Q::B - 1) / Q::B, g.rs);
+        dim3 grid((g.h + Q::B - 1) / Q::B, g.nri);
         k_yinv_p2<T, L><<<grid, Q::THREADS, p2_col_smem<T, L>(), s>>>(
             Wr.as<C2<T>>(), Wry.as<C2<T>>(), g, taby.as<C2<T>>());
       }
@@ -1544,20 +1578,20 @@ void FusedSurvey::yinv(cudaStream_t s) {
 }
 
 template <typename T>
-void FusedSurvey::zinv(double *rsub, const void *rtab_v, cudaStream_t s) {
+void FusedSurvey::zinv(double *rsub, const void *rtab_v, bool first, cudaStream_t s) {
   const T *rtab = static_cast<const T *>(rtab_v);
   if (p2_rows()) {
     with_p2(g.m, [&]<int L>() {
       using Q = P2<T, L>;
-      const int nrows = g.rs * g.rs;
+      const int nrows = g.nri * g.rs;
       const unsigned blocks = (unsigned)((nrows + Q::B - 1) / Q::B);
       k_zinv_p2<T, L><<<blocks, Q::THREADS, p2_row_smem<T, L>(), s>>>(
-          Wry.as<C2<T>>(), rsub, g, tabz.as<C2<T>>(), rtab);
+          Wry.as<C2<T>>(), rsub, g, tabz.as<C2<T>>(), rtab, first);
     });
     FC_LAUNCH_CHECK();
     return;
   }
-  gen_zinv<T>(gz, g, Wry.as<C2<T>>(), rsub, rtab, s);
+  gen_zinv<T>(gz, g, Wry.as<C2<T>>(), rsub, rtab, first, s);
 }
 
 const void *FusedSurvey::r_table(int ell, int m, const double *raxis,
@@ -1565,16 +1599,16 @@ const void *FusedSurvey::r_table(int ell, int m, const double *raxis,
   const int key = ell * 16 + (m + ell);
   auto it = rtabs.find(key);
   if (it != rtabs.end()) return it->second.get();
-  const size_t n = (size_t)g.rs * g.rs * g.rs;
+  const size_t n = (size_t)g.nri * g.rs * g.rs;
   DeviceBuffer &b = rtabs[key];
   // FP64 for the FP64 form, FP32 for the FP32-mixed form (the product with
   // the transform and the accumulation stay FP64).
   if (fp64_) {
     b.resize(std::max<size_t>(n, 1) * sizeof(double));
-    k_rtable<double><<<grid_for(n, 256), 256, 0, s>>>(b.as<double>(), g.rs, raxis, pr);
+    k_rtable<double><<<grid_for(n, 256), 256, 0, s>>>(b.as<double>(), g, raxis, pr);
   } else {
     b.resize(std::max<size_t>(n, 1) * sizeof(float));
-    k_rtable<float><<<grid_for(n, 256), 256, 0, s>>>(b.as<float>(), g.rs, raxis, pr);
+    k_rtable<float><<<grid_for(n, 256), 256, 0, s>>>(b.as<float>(), g, raxis, pr);
   }
   FC_LAUNCH_CHECK();
   return b.get();
@@ -1594,7 +1628,7 @@ const void *FusedSurvey::k_table(int ell, int m, const KAxes &ka,
   const int key = ell * 16 + (m + ell);
   auto it = ktabs.find(key);
   if (it != ktabs.end()) return it->second.get();
-  const size_t n = (size_t)g.ks0 * g.ks1 * g.ks2;
+  const size_t n = k_cells();
   DeviceBuffer &b = ktabs[key];
   const YlmParams pk = make_ylm_params(ell, m, 4.0 * M_PI);
   // FP64 weights for the FP64 form; the FP32 form keeps them in FP32 (a
@@ -1602,13 +1636,11 @@ const void *FusedSurvey::k_table(int ell, int m, const KAxes &ka,
   if (fp64_) {
     b.resize(std::max<size_t>(n, 1) * sizeof(double));
     k_ktable<double><<<grid_for(n, 256), 256, 0, s>>>(
-        b.as<double>(), g.ks0, g.ks1, g.ks2, ka.kx, ka.ky, ka.kz, ka.wx, ka.wy,
-        ka.wz, pk);
+        b.as<double>(), g, ka, pk);
   } else {
     b.resize(std::max<size_t>(n, 1) * sizeof(float));
     k_ktable<float><<<grid_for(n, 256), 256, 0, s>>>(
-        b.as<float>(), g.ks0, g.ks1, g.ks2, ka.kx, ka.ky, ka.kz, ka.wx, ka.wy,
-        ka.wz, pk);
+        b.as<float>(), g, ka, pk);
   }
   FC_LAUNCH_CHECK();
   return b.get();
@@ -1621,11 +1653,11 @@ void FusedSurvey::grid2(const void *rho_in, cudaStream_t s, const KAxes &ka) {
   if (fp64_) {
     zfwd<double>(rho_in, false, none, zero, s);
     yfwd<double>(s);
-    xcorr<double>(false, nullptr, nullptr, s);
+    grid2_x<double>(s);
   } else {
     zfwd<float>(rho_in, false, none, zero, s);
     yfwd<float>(s);
-    xcorr<float>(false, nullptr, nullptr, s);
+    grid2_x<float>(s);
   }
 }
 
@@ -1664,7 +1696,7 @@ void FusedSurvey::zfwd_pair(const void *rho_in, int ell_a, int m_a, int ell_b,
 int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
                        double ncells, double *ksub, double *rsub,
                        const double *raxis, const KAxes &ka, cudaStream_t s,
-                       PhaseHook *hook, bool g_of_input, bool z_done) {
+                       PhaseHook *hook, bool first, bool g_of_input, bool z_done) {
   const YlmParams pw = make_ylm_params(ell, m, 1.0);
   const YlmParams pr = make_ylm_params(ell, m, 4.0 * M_PI / ncells);
   const void *ktab = ksub ? k_table(ell, m, ka, s) : nullptr;
@@ -1676,7 +1708,7 @@ int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
       // The weight is the constant pw.value0, so the term's transform is
       // value0 * G (see k_xcorr_p2, MODE 2).
       if (hook) hook->begin("xcorr00");
-      xcorr00<T>(ksub, ktab, pw.value0, s);
+      xcorr<T>(true, ksub, ktab, pw.value0, first, s);
       if (hook) hook->end();
     } else {
       if (!z_done) {
@@ -1688,14 +1720,14 @@ int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
       yfwd<T>(s);
       if (hook) hook->end();
       if (hook) hook->begin("xcorr");
-      xcorr<T>(true, ksub, ktab, s);
+      xcorr<T>(false, ksub, ktab, 0.0, first, s);
       if (hook) hook->end();
     }
     if (hook) hook->begin("yinv");
     yinv<T>(s);
     if (hook) hook->end();
     if (hook) hook->begin("zinv");
-    zinv<T>(rsub, rtab, s);
+    zinv<T>(rsub, rtab, first, s);
     if (hook) hook->end();
   };
   if (fp64_)

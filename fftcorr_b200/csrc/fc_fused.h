@@ -29,7 +29,18 @@ class FusedSurvey {
   // fit.
   static bool supported(const int shape[3], int rsize);
 
-  FusedSurvey(const int shape[3], int rsize, const int kshape[3], bool fp64);
+  // even: the r-subgrid's bins are those of its mirror image, so the inverse
+  // transforms may take Re P (fc_fused.cu).
+  FusedSurvey(const int shape[3], int rsize, const int kshape[3], bool fp64,
+              bool even);
+  bool even() const { return g.nri != g.rs; }
+  // Cells of the stored subgrids (half_k_cell, half_r_cell).
+  size_t k_cells() const { return (size_t)g.ks0 * g.ks1 * g.kp; }
+  size_t r_cells() const { return (size_t)g.nri * g.rs * g.rs; }
+  // The stored cell of r = 0.
+  size_t zero_lag() const {
+    return half_r_cell(g, ((size_t)g.ro * g.rs + g.ro) * g.rs + g.ro);
+  }
 
   // The grid in the arithmetic of the passes: rho itself when its cells
   // already have the passes' type (f32: FP32 cells, in mixed precision
@@ -47,12 +58,12 @@ class FusedSurvey {
   void prepare_tables(int maxell, double ncells, const double *raxis,
                       const KAxes &ka, bool with_k, cudaStream_t s);
   // One (ell, m) term of Correlator::correlate_internal, accumulated into
-  // the FP64 subgrids.
+  // the FP64 subgrids, or (first) written over them.
   // Returns the number of full-grid transforms run (1 or 2).
   int term(const void *rho_in, int ell, int m, const double xyz0[3],
             double ncells, double *ksub, double *rsub, const double *raxis,
-            const KAxes &ka, cudaStream_t s, PhaseHook *hook,
-            bool g_of_input = false, bool z_done = false);
+            const KAxes &ka, cudaStream_t s, PhaseHook *hook, bool first,
+            bool g_of_input, bool z_done);
   // Whether two weighted terms can share one z pass (FP32, power-of-two
   // rows).  zfwd_pair runs the z pass of terms a and b (both ell > 0) in
   // one launch: term a's result lands in W, term b's in a second buffer
@@ -88,9 +99,10 @@ class FusedSurvey {
   template <typename T>
   void yfwd(cudaStream_t s);
   template <typename T>
-  void xcorr(bool product, double *ksub, const void *ktab, cudaStream_t s);
+  void grid2_x(cudaStream_t s);
   template <typename T>
-  void xcorr00(double *ksub, const void *ktab, double w00, cudaStream_t s);
+  void xcorr(bool from_g, double *ksub, const void *ktab, double w00, bool first,
+             cudaStream_t s);
   // Weights of the k-subgrid cells for (ell, m), built on first use.
   // (FP64 for the FP64 form, FP32 for the FP32-mixed form)
   const void *k_table(int ell, int m, const KAxes &ka, cudaStream_t s);
@@ -101,7 +113,7 @@ class FusedSurvey {
   template <typename T>
   void yinv(cudaStream_t s);
   template <typename T>
-  void zinv(double *rsub, const void *rtab, cudaStream_t s);
+  void zinv(double *rsub, const void *rtab, bool first, cudaStream_t s);
 
   bool fp64_;
   GenAxis gx, gy, gz;  // of the axes that are not powers of two

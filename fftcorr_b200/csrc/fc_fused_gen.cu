@@ -203,11 +203,16 @@ __global__ void __launch_bounds__(kYThreads, sizeof(T) == 4 ? 2 : 1)
 }
 
 // ------------------------------------------------------------------ x
-// The real parts of an element's values.
-__device__ __forceinline__ double real_part(const CPair &v, int l) {
-  return (double)(l ? v.x.y : v.x.x);
+// The W real parts of an element (n of them valid, the others zero) as they
+// are staged for the even form's inverse.
+__device__ __forceinline__ float2 real_parts(const CPair &v, int n) {
+  return make_float2(n > 0 ? v.x.x : 0.f, n > 1 ? v.x.y : 0.f);
 }
-__device__ __forceinline__ double real_part(const double2 &v, int) { return v.x; }
+__device__ __forceinline__ double real_parts(const double2 &v, int n) {
+  return n > 0 ? v.x : 0.0;
+}
+__device__ __forceinline__ double part(float2 r, int l) { return (double)(l ? r.y : r.x); }
+__device__ __forceinline__ double part(double r, int) { return r; }
 
 // w |q|^2 as an element.
 __device__ __forceinline__ CPair abs2_elem(const CPair &q, float w) {
@@ -220,17 +225,48 @@ __device__ __forceinline__ double2 abs2_elem(const double2 &q, double w) {
   return make_double2(w * (q.x * q.x + q.y * q.y), 0.0);
 }
 
+// Staged real parts of adjacent columns as elements: column pairs become the
+// real and imaginary parts of one complex column.
+__device__ __forceinline__ CPair from_staged(const CPair &raw) {
+  // in memory: (a0, b0, a1, b1), the pairs (a, b) of two complex columns
+  return cpack(raw.x, raw.y);
+}
+__device__ __forceinline__ double2 from_staged(const double2 &raw) { return raw; }
+
+// The columns A and B of Z = DFT(a + i b), a and b real, at x from Z at x
+// and -x: A = (Z(x) + conj Z(-x)) / 2, B = (Z(x) - conj Z(-x)) / 2i.  Of the
+// 2 W columns at p, n exist.
+template <typename C>
+__device__ __forceinline__ void split_store(C *p, C z, C m, int n) {
+  C a, b;
+  a.x = 0.5f * (z.x + m.x);
+  a.y = 0.5f * (z.y - m.y);
+  b.x = 0.5f * (z.y + m.y);
+  b.y = 0.5f * (m.x - z.x);
+  if (n > 0) p[0] = a;
+  if (n > 1) p[1] = b;
+}
+__device__ __forceinline__ void split_elem(float2 *p, const CPair &z, const CPair &m, int n) {
+  split_store(p, clane0(z), clane0(m), n);
+  split_store(p + 2, clane1(z), clane1(m), n - 2);
+}
+__device__ __forceinline__ void split_elem(double2 *p, const double2 &z, const double2 &m,
+                                           int n) {
+  split_store(p, z, m, n);
+}
+
 // MODE 0: G = DFT_x(W).  MODE 1: P = DFT_x(W) conj(G); MODE 2 (ell = 0 of an
 // autocorrelation): P = w00 |G|^2.  Then the k-subgrid extraction, straight
 // from the registers that hold P (every k-subgrid cell has one source
-// element, so the read-modify-writes never collide), and the inverse,
-// stored at the r-subgrid's rows.
-template <typename T, int B, int MODE>
+// element, so the read-modify-writes never collide; `first` overwrites), and
+// the inverse, stored at the r-subgrid's rows.  EVEN: the inverse of Re P
+// (fc_fused.h), two real columns to a complex one.
+template <typename T, int B, int MODE, bool EVEN>
 __global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
     k_gx(const C2<T> *__restrict__ W, const C2<T> *__restrict__ G,
          C2<T> *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
          const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw,
-         const T *__restrict__ ktab, T w00) {
+         const T *__restrict__ ktab, T w00, int first) {
   using GE = GElem<T>;
   using E = typename GE::E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -254,25 +290,30 @@ __global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
       GE::store(out + base + (int64_t)i * stride + GE::W * b, v, nb - GE::W * b);
     });
   } else {
-    const int ox = g.ks0 / 2, oy = g.ks1 / 2, oz = g.ks2 / 2;
-    int jr0 = yy + oy, jr1 = oy - yy;
-    if (jr0 >= g.n1) jr0 -= g.n1;
-    if (jr1 < 0) jr1 += g.n1;
-    const bool extract =
-        ksub != nullptr && kz0 <= oz && (jr0 < g.ks1 || jr1 < g.ks1);
-    auto to_ksub = [&](int x, int kz, double re) {
+    using RP = decltype(real_parts(E(), 0));
+    const int ox = g.ks0 / 2, oz = g.ks2 / 2;
+    int jr = yy + g.ks1 / 2;
+    if (jr >= g.n1) jr -= g.n1;
+    const bool extract = ksub != nullptr && kz0 <= oz && jr < g.ks1;
+    // Row x of P: to the k-subgrid, and to shared memory for the inverse.
+    auto take = [&](int x, int b, const E &v, E *dst) {
+      const int n = nb - GE::W * b;
+      const RP re = real_parts(v, n);
+      if constexpr (EVEN) reinterpret_cast<RP *>(dst)[x * B + b] = re;
+      else dst[x * BP + b] = v;
+      const int kz = kz0 + GE::W * b;
+      if (!extract || kz > oz) return;
+      int i = x + ox;
+      if (i >= g.n0) i -= g.n0;
+      for (; i < g.ks0; i += g.n0)
+        for (int j = jr; j < g.ks1; j += g.n1) {
+          // (The second cell of a pair may be the row's padding.)
+          const size_t cell = ((size_t)i * g.ks1 + j) * g.kp + kz;
 #pragma unroll
-      for (int refl = 0; refl < 2; ++refl) {
-        if (refl && kz == 0) continue;
-        int i = refl ? ox - x : x + ox;
-        i = i < 0 ? i + g.n0 : (i >= g.n0 ? i - g.n0 : i);
-        for (; i < g.ks0; i += g.n0)
-          for (int j = refl ? jr1 : jr0; j < g.ks1; j += g.n1) {
-            const size_t cell =
-                ((size_t)i * g.ks1 + j) * g.ks2 + (refl ? oz - kz : oz + kz);
-            ksub[cell] += (double)ktab[cell] * re;
-          }
-      }
+          for (int l = 0; l < GE::W; ++l)
+            ksub[cell + l] = (first ? 0.0 : ksub[cell + l]) +
+                             (double)ktab[cell + l] * part(re, l);
+        }
     };
     if constexpr (MODE == 1) {
       with_radix(last.R, [&]<int R>() {
@@ -288,20 +329,9 @@ __global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
           g_twiddle<R, -1>(v, tw + last.tw, last.Ns, j);
           GDft<R, -1, E>::run(v);
 #pragma unroll
-          for (int q = 0; q < R; ++q) {
-            v[q] = cmulc(v[q], gv[q]);
-            other[(j + q * last.LR) * BP + b] = v[q];
-          }
-          if (extract) {
+          for (int q = 0; q < R; ++q) v[q] = cmulc(v[q], gv[q]);
 #pragma unroll
-            for (int l = 0; l < GE::W; ++l) {
-              const int kz = kz0 + GE::W * b + l;
-              if (kz > oz) continue;
-#pragma unroll
-              for (int q = 0; q < R; ++q)
-                to_ksub(j + q * last.LR, kz, real_part(v[q], l));
-            }
-          }
+          for (int q = 0; q < R; ++q) take(j + q * last.LR, b, v[q], other);
         }
       });
       E *t = cur;
@@ -310,26 +340,50 @@ __global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
     } else {
       for (int idx = threadIdx.x; idx < g.n0 * B; idx += blockDim.x) {
         const int x = idx / B, b = idx % B;
-        const E p = abs2_elem(
-            GE::load(G + base + x * stride + GE::W * b, nb - GE::W * b), w00);
-        if (extract) {
-#pragma unroll
-          for (int l = 0; l < GE::W; ++l)
-            if (kz0 + GE::W * b + l <= oz)
-              to_ksub(x, kz0 + GE::W * b + l, real_part(p, l));
-        }
-        cur[x * BP + b] = p;
+        take(x, b,
+             abs2_elem(GE::load(G + base + x * stride + GE::W * b, nb - GE::W * b), w00),
+             cur);
       }
     }
     __syncthreads();
-    col_pass<1, B>(plan.p[0], tw, cur, other, true);
-    const E *res = col_middle<1, B>(plan, tw, other, cur);
-    col_last<1, B>(last, tw, res, [&](int x, int b, const E &v) {
-      int ri = x + g.ro;
-      if (ri >= g.n0) ri -= g.n0;
-      for (; ri < g.rs; ri += g.n0)
-        GE::store(out + base + ri * stride + GE::W * b, v, nb - GE::W * b);
-    });
+    if constexpr (EVEN) {
+      constexpr int H = B / 2, HP = pitch_of(H);
+      const GPass &f = plan.p[0];
+      with_radix(f.R, [&]<int R>() {
+        for (int bf = threadIdx.x; bf < f.LR * H; bf += blockDim.x) {
+          const int j = bf / H, b = bf % H;
+          E v[R];
+#pragma unroll
+          for (int q = 0; q < R; ++q) v[q] = from_staged(cur[(j + q * f.LR) * H + b]);
+          GDft<R, 1, E>::run(v);
+          E *o = other + j * R * HP + b;
+#pragma unroll
+          for (int q = 0; q < R; ++q) o[q * HP] = v[q];
+        }
+      });
+      __syncthreads();
+      const E *res = col_middle<1, H>(plan, tw, other, cur);
+      E *zb = res == cur ? other : cur;
+      col_last<1, H>(last, tw, res, [&](int x, int b, const E &v) {
+        if (x <= g.ro || x >= g.n0 - g.ro) zb[x * HP + b] = v;
+      });
+      __syncthreads();
+      for (int idx = threadIdx.x; idx < (g.ro + 1) * H; idx += blockDim.x) {
+        const int x = idx / H, b = idx % H;
+        const int xp = x == g.n0 ? 0 : x, xm = xp == 0 ? 0 : g.n0 - xp;
+        split_elem(out + base + x * stride + 2 * GE::W * b, zb[xp * HP + b],
+                   zb[xm * HP + b], nb - 2 * GE::W * b);
+      }
+    } else {
+      col_pass<1, B>(plan.p[0], tw, cur, other, true);
+      const E *res = col_middle<1, B>(plan, tw, other, cur);
+      col_last<1, B>(last, tw, res, [&](int x, int b, const E &v) {
+        int ri = x + g.ro;
+        if (ri >= g.n0) ri -= g.n0;
+        for (; ri < g.rs; ri += g.n0)
+          GE::store(out + base + ri * stride + GE::W * b, v, nb - GE::W * b);
+      });
+    }
   }
 }
 
@@ -491,7 +545,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
     k_gzinv(const C2<T> *__restrict__ Wry, double *__restrict__ rsub, FusedGeom g,
             const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw, int np,
-            const T *__restrict__ rtab) {
+            const T *__restrict__ rtab, int first) {
   using E = typename GElem<T>::E;
   constexpr int NR = 2 * GElem<T>::W;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -499,7 +553,7 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
   const int pitch = rpos(N - 1) + 1;
   E *buf = reinterpret_cast<E *>(smem_raw);
   E *other = buf + np * pitch;
-  const int nrows = g.rs * g.rs;
+  const int nrows = g.nri * g.rs;
   const int row0 = blockIdx.x * NR * np;
   const GPass &f = plan.p[0];
   with_radix(f.R, [&]<int R>() {
@@ -558,7 +612,8 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
           for (int c = 0; c < NR; ++c) {
             if (ra + c >= nrows) continue;
             const size_t cell = (size_t)(ra + c) * g.rs + rk;
-            rsub[cell] += (double)rtab[cell] * (double)comp(v[q], c);
+            rsub[cell] = (first ? 0.0 : rsub[cell]) +
+                         (double)rtab[cell] * (double)comp(v[q], c);
           }
         }
       }
@@ -606,9 +661,11 @@ template <typename T, int B>
 void col_limits() {
   big_smem(k_gyfwd<T, B>);
   big_smem(k_gyinv<T, B>);
-  big_smem(k_gx<T, B, 0>);
-  big_smem(k_gx<T, B, 1>);
-  big_smem(k_gx<T, B, 2>);
+  big_smem(k_gx<T, B, 0, false>);
+  big_smem(k_gx<T, B, 1, false>);
+  big_smem(k_gx<T, B, 2, false>);
+  big_smem(k_gx<T, B, 1, true>);
+  big_smem(k_gx<T, B, 2, true>);
 }
 template <typename T>
 void set_limits(int L, bool row) {
@@ -689,16 +746,19 @@ void gen_yfwd(const GenAxis &a, const FusedGeom &g, C2<T> *W, cudaStream_t s) {
 
 template <typename T>
 void gen_x(const GenAxis &a, const FusedGeom &g, int mode, const C2<T> *W, const C2<T> *G,
-           C2<T> *out, double *ksub, const T *ktab, T w00, cudaStream_t s) {
+           C2<T> *out, double *ksub, const T *ktab, T w00, bool first, cudaStream_t s) {
   with_width(a, [&]<int B>() {
     constexpr int NC = kCols<T, B>;
     auto go = [&](auto kernel) {
       kernel<<<dim3((g.h + NC - 1) / NC, g.n1), col_threads(a.plan, kXThreads), col_smem(g.n0), s>>>(
-          W, G, out, ksub, g, a.plan, a.tw.as<C2<T>>(), ktab, w00);
+          W, G, out, ksub, g, a.plan, a.tw.as<C2<T>>(), ktab, w00, first);
     };
-    if (mode == 0) go(k_gx<T, B, 0>);
-    else if (mode == 1) go(k_gx<T, B, 1>);
-    else go(k_gx<T, B, 2>);
+    const bool even = g.nri != g.rs;
+    if (mode == 0) go(k_gx<T, B, 0, false>);
+    else if (mode == 1 && even) go(k_gx<T, B, 1, true>);
+    else if (mode == 1) go(k_gx<T, B, 1, false>);
+    else if (even) go(k_gx<T, B, 2, true>);
+    else go(k_gx<T, B, 2, false>);
   });
   FC_LAUNCH_CHECK();
 }
@@ -708,7 +768,7 @@ void gen_yinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wr, C2<T> *Wry,
               cudaStream_t s) {
   with_width(a, [&]<int B>() {
     constexpr int NC = kCols<T, B>;
-    k_gyinv<T, B><<<dim3((g.h + NC - 1) / NC, g.rs), col_threads(a.plan, kYThreads),
+    k_gyinv<T, B><<<dim3((g.h + NC - 1) / NC, g.nri), col_threads(a.plan, kYThreads),
                     col_smem(g.n1), s>>>(Wr, Wry, g, a.plan, a.tw.as<C2<T>>());
   });
   FC_LAUNCH_CHECK();
@@ -716,12 +776,12 @@ void gen_yinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wr, C2<T> *Wry,
 
 template <typename T>
 void gen_zinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wry, double *rsub,
-              const T *rtab, cudaStream_t s) {
+              const T *rtab, bool first, cudaStream_t s) {
   constexpr int NR = 2 * GElem<T>::W;
-  const int nrows = g.rs * g.rs;
+  const int nrows = g.nri * g.rs;
   const int np = row_elems(a.plan, (nrows + NR - 1) / NR);
   k_gzinv<T><<<(nrows + NR * np - 1) / (NR * np), row_threads(a.plan, np), row_smem(g.n2, np), s>>>(
-      Wry, rsub, g, a.plan, a.tw.as<C2<T>>(), np, rtab);
+      Wry, rsub, g, a.plan, a.tw.as<C2<T>>(), np, rtab, first);
   FC_LAUNCH_CHECK();
 }
 
@@ -730,11 +790,12 @@ void gen_zinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wry, double *rs
                             bool, const YlmParams &, const double[3], cudaStream_t);   \
   template void gen_yfwd<T>(const GenAxis &, const FusedGeom &, C2<T> *, cudaStream_t); \
   template void gen_x<T>(const GenAxis &, const FusedGeom &, int, const C2<T> *,       \
-                         const C2<T> *, C2<T> *, double *, const T *, T, cudaStream_t); \
+                         const C2<T> *, C2<T> *, double *, const T *, T, bool,        \
+                         cudaStream_t); \
   template void gen_yinv<T>(const GenAxis &, const FusedGeom &, const C2<T> *,         \
                             C2<T> *, cudaStream_t);                                    \
   template void gen_zinv<T>(const GenAxis &, const FusedGeom &, const C2<T> *,         \
-                            double *, const T *, cudaStream_t);
+                            double *, const T *, bool, cudaStream_t);
 FC_GEN(float)
 FC_GEN(double)
 

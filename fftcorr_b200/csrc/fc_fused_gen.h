@@ -30,18 +30,19 @@ void gen_zfwd(const GenAxis &a, const FusedGeom &g, const T *rho,
 template <typename T>
 void gen_yfwd(const GenAxis &a, const FusedGeom &g, typename Vec2<T>::type *W,
               cudaStream_t s);
-// mode 0: out = G = DFT_x(W); 1: the product with G; 2: w00 |G|^2.
+// mode 0: out = G = DFT_x(W); 1: the product with G; 2: w00 |G|^2.  first:
+// the subgrid is overwritten, not added to.
 template <typename T>
 void gen_x(const GenAxis &a, const FusedGeom &g, int mode,
            const typename Vec2<T>::type *W, const typename Vec2<T>::type *G,
-           typename Vec2<T>::type *out, double *ksub, const T *ktab, T w00,
+           typename Vec2<T>::type *out, double *ksub, const T *ktab, T w00, bool first,
            cudaStream_t s);
 template <typename T>
 void gen_yinv(const GenAxis &a, const FusedGeom &g, const typename Vec2<T>::type *Wr,
               typename Vec2<T>::type *Wry, cudaStream_t s);
 template <typename T>
 void gen_zinv(const GenAxis &a, const FusedGeom &g, const typename Vec2<T>::type *Wry,
-              double *rsub, const T *rtab, cudaStream_t s);
+              double *rsub, const T *rtab, bool first, cudaStream_t s);
 
 // Coefficients of Y_lm r^ell (ell 2 or 4) as a polynomial in z with (x, y)
 // fixed, in FP64 with the normalisation folded in (spherical_harmonics.h:

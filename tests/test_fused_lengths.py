@@ -32,3 +32,23 @@ def test_survey_axis_lengths(shape, kmax, precision):
     c.cross_correlate(a, b)
     _compare_results(c.results(), O.survey_correlate(a, *args, grid2=b), FP64_RTOL,
                      "cross", fp32=precision == "fp32")
+
+
+@pytest.mark.parametrize("shape", [(64, 64, 64), (40, 64, 66)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_bins_that_differ_under_inversion(shape, precision):
+    """cell = 2.6 and dr = 7.8 put cells on bin edges whose rounded mirror
+    images lie on the other side, so the inverse may not drop the odd part of
+    the correlation: the counts of r and -r differ and every bin matches."""
+    cell, dr = 2.6, 7.8
+    r = -cell * 12 + np.arange(25) * cell
+    d = np.sqrt(r[:, None, None] ** 2 + r[None, :, None] ** 2 + r[None, None, :] ** 2)
+    bins = np.floor(d / dr)
+    assert np.any(bins != bins[::-1, ::-1, ::-1])
+    posmin = np.array([-30.0, 25.0, -35.0])
+    a = np.random.default_rng(6).standard_normal(shape)
+    args = (cell, posmin, TSC_ALIASED_CORRECTION, cell * 12, dr, 0.3, 0.05, 4)
+    c = fb.Correlator(shape, *args, precision=precision)
+    c.autocorrelate(a)
+    _compare_results(c.results(), O.survey_correlate(a, *args), FP64_RTOL, "auto",
+                     fp32=precision == "fp32")
