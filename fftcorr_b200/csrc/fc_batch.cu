@@ -4,13 +4,13 @@
 //
 // Per box (one lane stream of the graph):
 //   memset grid -> K-key -> radix sort -> K-tiles -> K-scatter colour passes
-//   (fc_assign.cu) -> k_norm_pad: (rho - mean) / mean into the FP32 or FP64
-//   padded work grid (fftcorr.cc:369-375 fused with array_ops.cc:35-53) ->
-//   r2c -> |F|^2 -> k-subgrids per ell -> c2r -> r-subgrids per ell
+//   (fc_assign.cu) -> k_norm_pad: (rho - mean) / mean in place, or into the
+//   padded work grid of a correlator on the cuFFT path (fftcorr.cc:369-375
+//   fused with array_ops.cc:35-53) -> the periodic correlation
 //   (correlator.h:273-357, fc_corr.cu)
 // and after all lanes join, one persistent chunk-reduction kernel and one
-// fold kernel produce every histogram of every box (the same sums, in the
-// same order, as the per-box BinIndex::reduce).
+// fold kernel (HistPlan) produce every histogram of every box (the same sums,
+// in the same order, as each correlator's own).
 //
 // Boxes are spread over the lanes by a greedy longest-first balance of their
 // estimated cost.  The launch shapes of the grid-stride kernels, the lane
@@ -34,11 +34,11 @@ namespace fc {
 namespace {
 
 // add_scalar(-mean) then multiply_by(1/mean) (fftcorr.cc:369-375), written
-// straight into the padded work grid in the transform precision.  mean =
-// totw / ncells from the assignor's device totals.
+// straight into the padded work grid in the transform precision, or in place
+// (work = rho, n2p = n2).  mean = totw / ncells from the assignor's device
+// totals.
 template <typename TI, typename T>
-__global__ void k_norm_pad(const TI *__restrict__ rho, T *__restrict__ work,
-                           int n0, int n1, int n2, int n2p,
+__global__ void k_norm_pad(const TI *rho, T *work, int n0, int n1, int n2, int n2p,
                            const double *__restrict__ totals, double ncells) {
   const double mean = totals[0] / ncells;
   const double shift = -mean;
@@ -51,34 +51,6 @@ __global__ void k_norm_pad(const TI *__restrict__ rho, T *__restrict__ work,
     // fc_grid_multiply_by round a grid's cells (a no-op for FP64 cells).
     for (int k = threadIdx.x; k < n2; k += blockDim.x)
       dst[k] = (T)((double)(TI)((double)src[k] + shift) * scale);
-  }
-}
-
-// Persistent chunk reductions over the work items of every box: item i is
-// summed exactly as k_chunk_sums sums chunk i of one BinIndex.
-__global__ void __launch_bounds__(kHistThreads)
-    k_batch_chunks(const HistItem *__restrict__ items, int n,
-                   double *__restrict__ partials) {
-  __shared__ double red[32];
-  for (int it = blockIdx.x; it < n; it += gridDim.x) {
-    const HistItem h = items[it];
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < h.len; i += blockDim.x)
-      acc += h.values[h.perm[h.start + i]];
-    acc = block_sum(acc, red);
-    if (threadIdx.x == 0) partials[it] = acc;
-  }
-}
-
-// One thread per bin of every box: its chunk partials folded in order.
-__global__ void k_batch_fold(const FoldItem *__restrict__ folds, int n,
-                             const double *__restrict__ partials) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gridDim.x * blockDim.x) {
-    const FoldItem f = folds[i];
-    double s = 0.0;
-    for (int c = f.first; c < f.first + f.count; ++c) s += partials[c];
-    *f.dest = s;
   }
 }
 
@@ -167,7 +139,7 @@ struct Batch {
   std::vector<cudaEvent_t> join_ev;
   std::vector<HistItem> items;
   std::vector<FoldItem> folds;
-  DeviceBuffer d_items, d_folds, d_partials;
+  HistPlan hist;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   size_t graph_nodes = 0, kernel_nodes = 0;
@@ -221,15 +193,7 @@ struct Batch {
       ls_norm.push_back(LaunchShape{256, 64});
     }
     for (auto *c : corrs) correlator_hist_work(c, items, folds);
-    d_items.resize(std::max<size_t>(items.size(), 1) * sizeof(HistItem));
-    d_folds.resize(std::max<size_t>(folds.size(), 1) * sizeof(FoldItem));
-    d_partials.resize(std::max<size_t>(items.size(), 1) * sizeof(double));
-    if (!items.empty())
-      FC_CUDA(cudaMemcpy(d_items.get(), items.data(),
-                         items.size() * sizeof(HistItem), cudaMemcpyHostToDevice));
-    if (!folds.empty())
-      FC_CUDA(cudaMemcpy(d_folds.get(), folds.data(),
-                         folds.size() * sizeof(FoldItem), cudaMemcpyHostToDevice));
+    hist.upload(items, folds);
     FC_CUDA(cudaDeviceSynchronize());
     tune_kernels();
     choose_lanes_and_capture();
@@ -258,12 +222,13 @@ struct Batch {
   void norm_pad(int i, cudaStream_t s) {
     const BatchBox &b = boxes[i];
     const size_t nrows = (size_t)b.shape[0] * b.shape[1];
-    const int n2p = 2 * (b.shape[2] / 2 + 1);
+    const bool in_place = correlator_fused(corrs[i]);
+    const int n2p = in_place ? b.shape[2] : 2 * (b.shape[2] / 2 + 1);
     const LaunchShape &ls = ls_norm[i];
     const unsigned blocks =
         (unsigned)std::min<size_t>(nrows, (size_t)sm_count() * ls.waves);
-    T *work = static_cast<T *>(correlator_work(corrs[i]));
     const Grid *g = grids[i].get();
+    T *work = static_cast<T *>(in_place ? g->raw() : correlator_work(corrs[i]));
     if (g->fp32())
       k_norm_pad<float, T><<<blocks, ls.threads, 0, s>>>(
           static_cast<const float *>(g->raw()), work, b.shape[0], b.shape[1],
@@ -284,21 +249,10 @@ struct Batch {
     else
       norm_pad<float>(i, s);
     correlator_set_stream(corrs[i], s);
-    correlator_enqueue_prepared(corrs[i]);
+    correlator_enqueue_prepared(corrs[i], g->raw());
   }
 
-  void enqueue_hist(cudaStream_t s) {
-    if (!items.empty()) {
-      k_batch_chunks<<<hist_blocks, kHistThreads, 0, s>>>(
-          d_items.as<HistItem>(), (int)items.size(), d_partials.as<double>());
-      FC_LAUNCH_CHECK();
-    }
-    if (!folds.empty()) {
-      k_batch_fold<<<grid_for(folds.size(), 128), 128, 0, s>>>(
-          d_folds.as<FoldItem>(), (int)folds.size(), d_partials.as<double>());
-      FC_LAUNCH_CHECK();
-    }
-  }
+  void enqueue_hist(cudaStream_t s) { hist.run(hist_blocks, s); }
 
   // ---------------------------------------------------------------- tuning
   // Grid-stride kernels, per distinct box shape: the fastest (threads,
@@ -316,6 +270,10 @@ struct Batch {
       for (int which = 0; which < 4; ++which) {
         const std::string key = tune::shape_key(names[which], fp64(), boxes[rep].shape);
         if (tune::get(key, &best[which])) continue;
+        if (which > 0 && correlator_fused(corrs[rep])) {
+          best[which] = {256, 8};  // (not launched)
+          continue;
+        }
         if (!prm.tune) {
           best[which] = which == 0 ? std::make_pair(256, 64) : std::make_pair(256, 8);
           continue;

@@ -6,11 +6,20 @@
 // layout and the centred subgrid extractions), spherical_harmonics.h:32-179,
 // window_correct.h:14-60, histogram_list.h:33-45.
 //
-// Layout in HBM (per correlator):
+// Grids whose sides are products of 2, 3, 5 and 7 run through the fused
+// passes (fc_fused.cu): a survey correlation term by term, a periodic one as
+// one chain z, y, x with |F|^2, the k-subgrid and the pruned inverse, whose
+// two subgrids every multipole reads with its own weights in the histogram
+// reduction.  Against cuFFT with copy, |F|^2 and extraction kernels around it
+// (one B200): 384^3 FP32 ell <= 2 1.54 -> 0.62 ms, 250 x 243 x 225 FP64
+// ell <= 4 0.87 -> 0.48 ms.
+//
+// Other sides, by cuFFT; layout in HBM (per correlator):
 //   work  [N0][N1][N2p] real == [N0][N1][N2p/2] complex, N2p = 2(N2/2+1),
 //         the FftGrid layout; FP64 or FP32 (mixed precision)
 //   g2    [N0][N1][N2/2+1] complex: FFT of grid2 (BaseCorrelator::grid2_fft_)
-//   rsub  [R][R][R] FP64, ksub [K0][K1][K2] FP64 subgrid accumulators
+//   rsub  [R][R][R] FP64, ksub [K0][K1][K2] FP64 subgrid accumulators, one
+//         pair per multipole
 //   BinIndex per subgrid: cells sorted by histogram bin
 // Per (ell, m) of a survey correlation:
 //   k_weight   work = Y_lm(cell) * rho        (make_ylm on the full grid)
@@ -19,7 +28,8 @@
 //   k_ksub     ksub += Y_lm(k)*W^-2*4pi*Re(work) on the k-subgrid
 //   cuFFT c2r  in place
 //   k_rsub     rsub += Y_lm(r)*4pi/N*work on the r-subgrid
-// then per ell the two deterministic histograms (fc_hist.cuh).
+// then the deterministic histograms of every multipole (fc_hist.cuh), two
+// launches.
 #include <cufft.h>
 
 #include <algorithm>
@@ -198,6 +208,27 @@ __global__ void k_bins_differ(const int *__restrict__ bins, size_t n, int *diffe
   for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n / 2;
        c += (size_t)gridDim.x * blockDim.x)
     if (bins[c] != bins[n - 1 - c]) *differ = 1;
+}
+
+// Weights of a periodic correlation's histogram of one multipole, in the
+// order of the bin index: y = Y_l0 coeff (/ the window on the k-subgrid, as
+// in k_ksub) of every cell.
+__global__ void k_bin_weights(double *__restrict__ w, const uint32_t *__restrict__ perm,
+                              size_t n, int n1, int n2, const double *__restrict__ ax,
+                              const double *__restrict__ ay,
+                              const double *__restrict__ az,
+                              const double *__restrict__ wx,
+                              const double *__restrict__ wy,
+                              const double *__restrict__ wz, YlmParams p) {
+  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n;
+       c += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t cell = perm[c];
+    const int k = (int)(cell % n2);
+    const int j = (int)((cell / n2) % n1);
+    const int i = (int)(cell / ((uint32_t)n2 * n1));
+    const double d = wx ? 1.0 / (wx[i] * wy[j] * wz[k]) : 1.0;
+    w[c] = ylm_eval(p, d, ax[i], ay[j], az[k]);
+  }
 }
 
 // Subgrid cells of a bin index to the cells the fused passes store.
@@ -407,17 +438,35 @@ struct Correlator {
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
 
-  DeviceBuffer work, g2, input, rsub, ksub;
+  DeviceBuffer work, g2, input;
+  // Subgrids: one of each per multipole, or in a fused periodic correlation
+  // the one of each that every multipole shares (its weights are in the
+  // histograms: rweights, kweights, per multipole in bin order).
+  std::vector<DeviceBuffer> rsub_l, ksub_l;
+  DeviceBuffer rweights, kweights;
   DeviceBuffer d_raxis, d_kaxes, d_kwin;
-  DeviceBuffer d_rhist, d_khist, d_zerolag;
+  DeviceBuffer d_out;  // r histograms | k histograms | zero lag
+  std::vector<HistItem> items;
+  std::vector<FoldItem> folds;
+  DeviceBuffer zero_cell;  // index of the subgrid cell r = 0
+  HistPlan hist, hist_cross;
   BinIndex rbins, kbins;
   bool have_g2 = false;
   bool have_result = false;
   double shift_value = 0.0;  // mean removed before FP32 transforms
 
   Profiler prof;
-  // Hand-written fused FFT passes for the survey loop (null: cuFFT path).
+  // Hand-written fused FFT passes (null: cuFFT path).
   std::unique_ptr<FusedSurvey> fused;
+  // A periodic cross correlation on a geometry whose r-subgrid bins differ
+  // under inversion takes the general inverse, made with its second grid,
+  // and the bin index's cells as they are.
+  std::unique_ptr<FusedSurvey> fused_cross;
+  DeviceBuffer rperm_full;
+  bool bins_even = true;
+  FusedSurvey *cross_passes() const {
+    return fused_cross ? fused_cross.get() : fused.get();
+  }
   cufftHandle plan_r2c = 0, plan_c2r = 0;
   DeviceBuffer fft_area;
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
@@ -431,11 +480,9 @@ struct Correlator {
   // Launch shapes of the grid-stride kernels; results do not depend on them
   // (every cell is computed independently), so the autotuner may change them.
   LaunchShape ls_abs2{256, 8}, ls_ksub{256, 8}, ls_rsub{256, 8};
-  // Deferred-histogram mode (batched form): each multipole keeps its own
-  // subgrids and the histograms are reduced later, for many correlators at
-  // once.
+  // Deferred-histogram mode (batched form): the histograms are reduced later,
+  // for many correlators at once.
   bool deferred = false;
-  std::vector<DeviceBuffer> rsub_l, ksub_l;
 
   Correlator(int kind_, const int shape[3], double cell, const double pmin[3],
              int window, double rmax, double dr, double kmax, double dk,
@@ -467,21 +514,22 @@ struct Correlator {
       const char *mode = std::getenv("FFTCORR_B200_FFT");
       const bool want_fused = !(mode && std::string(mode) == "cufft");
       upload_axes();
-      const bool even = build_bins();
-      if (kind == FC_SURVEY && want_fused &&
-          FusedSurvey::supported(geo.shape, geo.rsize)) {
-        fused.reset(
-            new FusedSurvey(geo.shape, geo.rsize, geo.kshape, fp64(), even));
-        half_cells();
-      }
+      bins_even = build_bins();
+      // (A periodic autocorrelation's P is even whatever the bins are.)
+      if (want_fused && FusedSurvey::supported(geo.shape, geo.rsize))
+        fused.reset(new FusedSurvey(geo.shape, geo.rsize, geo.kshape, fp64(),
+                                    bins_even || kind == FC_PERIODIC,
+                                    kind == FC_SURVEY));
       allocate();
+      if (fused) half_cells();
       if (!fused) make_plans();
+      build_hist();
       // Every (ell, m) weight table now: a correlation (a served job on a
       // resident correlator in particular) then allocates nothing.
-      if (fused)
+      if (fused && kind == FC_SURVEY)
         fused->prepare_tables(2 * (geo.nrows - 1), (double)geo.ncells(),
                               d_raxis.as<double>(), kaxes(),
-                              ksub.as<double>() != nullptr, stream);
+                              geo.kcells() > 0, stream);
     } catch (...) {
       // A failed construction leaves no stream, event or plan behind (the
       // buffers free themselves).
@@ -513,14 +561,66 @@ struct Correlator {
 
   void allocate() {
     if (!fused) work.resize(geo.nreal_padded() * real_bytes());
-    rsub.resize(rsub_cells() * sizeof(double));
-    ksub.resize(ksub_cells() * sizeof(double));
-    d_rhist.resize(std::max(1, geo.nrows * geo.nr) * sizeof(double));
-    d_khist.resize(std::max(1, geo.nrows * geo.nk) * sizeof(double));
-    d_zerolag.resize(sizeof(double));
-    FC_CUDA(cudaMemset(d_rhist.get(), 0, d_rhist.bytes()));
-    FC_CUDA(cudaMemset(d_khist.get(), 0, d_khist.bytes()));
-    FC_CUDA(cudaMemset(d_zerolag.get(), 0, d_zerolag.bytes()));
+    const int n = shared_subgrids() ? 1 : geo.nrows;
+    rsub_l.resize(n);
+    ksub_l.resize(n);
+    for (int r = 0; r < n; ++r) {
+      rsub_l[r].resize(rsub_cells() * sizeof(double));
+      ksub_l[r].resize(ksub_cells() * sizeof(double));
+    }
+    d_out.resize(out_len() * sizeof(double));
+    FC_CUDA(cudaMemset(d_out.get(), 0, d_out.bytes()));
+  }
+
+  // Whether every multipole reads the same subgrids.
+  bool shared_subgrids() const { return fused && kind == FC_PERIODIC; }
+  size_t out_len() const { return (size_t)geo.nrows * (geo.nr + geo.nk) + 1; }
+  double *rhist_row(int r) const { return d_out.as<double>() + (size_t)r * geo.nr; }
+  double *khist_row(int r) const {
+    return d_out.as<double>() + (size_t)geo.nrows * geo.nr + (size_t)r * geo.nk;
+  }
+  double *zerolag_out() const { return d_out.as<double>() + out_len() - 1; }
+  double *rsub(int ell) const { return rsub_l[ell / 2].as<double>(); }
+  double *ksub(int ell) const { return ksub_l[ell / 2].as<double>(); }
+  // Periodic weights (correlator.h:304-349): sqrt(4 pi (2 ell + 1)) times the
+  // normalisations of P and of xi.
+  double k_coeff(int ell) const {
+    return sqrt((4.0 * M_PI) * (2 * ell + 1)) *
+           (geo.cell * geo.cell * geo.cell / (double)geo.ncells());
+  }
+  double r_coeff(int ell) const {
+    return sqrt((4.0 * M_PI) * (2 * ell + 1)) * (1.0 / geo.ncells() / geo.ncells());
+  }
+
+  // The reductions of every histogram and the zero lag, over rcells (the r bin
+  // index's cells as rsub_l holds them; r0 the one of r = 0).
+  void hist_items(const uint32_t *rcells, std::vector<HistItem> &it,
+                  std::vector<FoldItem> &fo) const {
+    const bool sh = shared_subgrids();
+    for (int r = 0; r < geo.nrows; ++r) {
+      rbins.append_work(rsub_l[sh ? 0 : r].as<double>(), rcells,
+                        sh ? rweights.as<double>() + r * rbins.ninrange : nullptr, 1.0,
+                        rhist_row(r), it, fo);
+      kbins.append_work(ksub_l[sh ? 0 : r].as<double>(), kbins.perm.as<uint32_t>(),
+                        sh ? kweights.as<double>() + r * kbins.ninrange : nullptr, 1.0,
+                        khist_row(r), it, fo);
+    }
+    const uint32_t *zero = zero_cell.as<uint32_t>();
+    fo.push_back(FoldItem{(int)it.size(), 1, zerolag_out()});
+    it.push_back(HistItem{rsub_l[0].as<double>(), zero, nullptr,
+                          sh ? make_ylm_params(0, 0, r_coeff(0)).value0 : 1.0,
+                          rcells == rbins.perm.as<uint32_t>() ? 0u : 1u, 1});
+  }
+
+  void build_hist() {
+    // r = 0 in the stored subgrid, and in the whole one.
+    const uint32_t centre = (uint32_t)(geo.rcells() / 2);
+    const uint32_t zero[2] = {fused ? (uint32_t)half_r_cell(fused->g, centre) : centre,
+                              centre};
+    zero_cell.resize(sizeof(zero));
+    FC_CUDA(cudaMemcpy(zero_cell.get(), zero, sizeof(zero), cudaMemcpyHostToDevice));
+    hist_items(rbins.perm.as<uint32_t>(), items, folds);
+    hist.upload(items, folds);
   }
 
   void upload_axes() {
@@ -615,8 +715,38 @@ struct Correlator {
     return differ == 0;
   }
 
-  // The bin indices' cells as the fused passes store them.
+  // The bin indices' cells as the fused passes store them, and before that
+  // the periodic weights of the whole cells.
   void half_cells() {
+    if (kind == FC_PERIODIC) {
+      const size_t nr = (size_t)rbins.ninrange, nk = (size_t)kbins.ninrange;
+      rweights.resize(geo.nrows * nr * sizeof(double));
+      kweights.resize(geo.nrows * nk * sizeof(double));
+      const KAxes k = kaxes();
+      const double *r = d_raxis.as<double>();
+      for (int row = 0; row < geo.nrows; ++row) {
+        const int ell = 2 * row;
+        if (nr) {
+          k_bin_weights<<<grid_for(nr, 256), 256, 0, stream>>>(
+              rweights.as<double>() + row * nr, rbins.perm.as<uint32_t>(), nr, geo.rsize,
+              geo.rsize, r, r, r, nullptr, nullptr, nullptr,
+              make_ylm_params(ell, 0, r_coeff(ell)));
+          FC_LAUNCH_CHECK();
+        }
+        if (nk) {
+          k_bin_weights<<<grid_for(nk, 256), 256, 0, stream>>>(
+              kweights.as<double>() + row * nk, kbins.perm.as<uint32_t>(), nk,
+              geo.kshape[1], geo.kshape[2], k.kx, k.ky, k.kz, k.wx, k.wy, k.wz,
+              make_ylm_params(ell, 0, k_coeff(ell)));
+          FC_LAUNCH_CHECK();
+        }
+      }
+      if (!bins_even && nr) {
+        rperm_full.resize(nr * sizeof(uint32_t));
+        FC_CUDA(cudaMemcpyAsync(rperm_full.get(), rbins.perm.get(), nr * sizeof(uint32_t),
+                                cudaMemcpyDeviceToDevice, stream));
+      }
+    }
     for (int k = 0; k < 2; ++k) {
       BinIndex &b = k ? kbins : rbins;
       const size_t n = (size_t)b.ninrange;
@@ -725,47 +855,41 @@ struct Correlator {
   }
 
   template <typename T>
-  void ksub_acc(int ell, int m, double coeff, double *dst = nullptr) {
+  void ksub_acc(int ell, int m, double coeff) {
     Profiler::Scope ps(&prof, stream, "ksub");
     using C = typename Cplx<T>::type;
     const double *ax = d_kaxes.as<double>();
     const double *wn = d_kwin.as<double>();
     const int a = geo.kshape[0], b = geo.kshape[1];
     k_ksub<C><<<ls_ksub.grid(geo.kcells()), ls_ksub.threads, 0, stream>>>(
-        work.as<C>(), dst ? dst : ksub.as<double>(), geo.kshape[0], geo.kshape[1],
+        work.as<C>(), ksub(ell), geo.kshape[0], geo.kshape[1],
         geo.kshape[2], geo.shape[0], geo.shape[1], geo.n2p() / 2, ax, ax + a,
         ax + a + b, wn, wn + a, wn + a + b, make_ylm_params(ell, m, coeff));
     FC_LAUNCH_CHECK();
   }
 
   template <typename T>
-  void rsub_acc(int ell, int m, double coeff, double *dst = nullptr) {
+  void rsub_acc(int ell, int m, double coeff) {
     Profiler::Scope ps(&prof, stream, "rsub");
     k_rsub<T><<<ls_rsub.grid(geo.rcells()), ls_rsub.threads, 0, stream>>>(
-        work.as<T>(), dst ? dst : rsub.as<double>(), geo.rsize, geo.shape[0], geo.shape[1],
+        work.as<T>(), rsub(ell), geo.rsize, geo.shape[0], geo.shape[1],
         geo.shape[2], geo.n2p(), d_raxis.as<double>(),
         make_ylm_params(ell, m, coeff));
     FC_LAUNCH_CHECK();
   }
 
-  void hist_rows(int ell, bool do_r, bool do_k) {
+  // Every histogram and the zero lag, unless the caller reduces them.
+  void reduce_hist(const HistPlan &h) {
+    have_result = true;
+    if (deferred) return;
     Profiler::Scope ps(&prof, stream, "hist");
-    const int ih = ell / 2;
-    if (do_r) rbins.reduce(rsub.as<double>(), d_rhist.as<double>() + ih * geo.nr, stream);
-    if (do_k) kbins.reduce(ksub.as<double>(), d_khist.as<double>() + ih * geo.nk, stream);
+    h.run(stream);
   }
 
-  void zero_sub(bool r, bool k) {
-    if (r) FC_CUDA(cudaMemsetAsync(rsub.get(), 0, rsub_cells() * sizeof(double), stream));
-    if (k) FC_CUDA(cudaMemsetAsync(ksub.get(), 0, ksub_cells() * sizeof(double), stream));
-  }
-
-  void save_zerolag() {
-    const size_t rz = fused ? fused->zero_lag()
-                            : ((size_t)geo.rmax_cells * geo.rsize + geo.rmax_cells) *
-                                      geo.rsize + geo.rmax_cells;
-    FC_CUDA(cudaMemcpyAsync(d_zerolag.get(), rsub.as<double>() + rz,
-                            sizeof(double), cudaMemcpyDeviceToDevice, stream));
+  void zero_sub(int ell) {
+    DeviceBuffer &r = rsub_l[ell / 2], &k = ksub_l[ell / 2];
+    FC_CUDA(cudaMemsetAsync(r.get(), 0, r.bytes(), stream));
+    FC_CUDA(cudaMemsetAsync(k.get(), 0, k.bytes(), stream));
   }
 
   // ----------------------------------------------------------- grid2
@@ -774,9 +898,11 @@ struct Correlator {
   void set_grid2_dev(Density d) {
     using C = typename Cplx<T>::type;
     if (fused) {
+      make_cross_passes();
+      FusedSurvey *f = cross_passes();
       ProfHook hook(&prof, stream);
       hook.begin("grid2");
-      fused->grid2(fused->prepare_input(d.p, d.f32, stream), stream, kaxes());
+      f->grid2(f->prepare_input(d.p, d.f32, stream), stream, kaxes());
       hook.end();
       ++n_fft;
       have_g2 = true;
@@ -786,6 +912,23 @@ struct Correlator {
     copy_pad<T>(d, shift_for(d));
     exec_r2c(work.get(), g2.get());
     have_g2 = true;
+  }
+
+  void make_cross_passes() {
+    if (kind != FC_PERIODIC || bins_even || fused_cross) return;
+    std::unique_ptr<FusedSurvey> f(new FusedSurvey(geo.shape, geo.rsize, geo.kshape,
+                                                   fp64(), false, true));
+    rsub_l[0].resize(geo.rcells() * sizeof(double));
+    std::vector<HistItem> it;
+    std::vector<FoldItem> fo;
+    hist_items(rperm_full.as<uint32_t>(), it, fo);
+    hist_cross.upload(it, fo);
+    // The r-subgrid may have moved.
+    items.clear();
+    folds.clear();
+    hist_items(rbins.perm.as<uint32_t>(), items, folds);
+    hist.upload(items, folds);
+    fused_cross = std::move(f);
   }
 
   // The FP64 cells of a density that accept() has passed through.
@@ -814,9 +957,11 @@ struct Correlator {
   void set_grid2_fft_host(const double *host_complex) {
     const size_t nc = geo.ncomplex();
     if (fused) {
-      const int h = fused->g.h, hp = fused->g.hp;
+      make_cross_passes();
+      FusedSurvey *f = cross_passes();
+      const int h = f->g.h, hp = f->g.hp;
       if (fp64()) {
-        FC_CUDA(cudaMemcpy2DAsync(fused->g_data(), hp * sizeof(double2),
+        FC_CUDA(cudaMemcpy2DAsync(f->g_data(), hp * sizeof(double2),
                                   host_complex, h * sizeof(double2),
                                   h * sizeof(double2), nc / h,
                                   cudaMemcpyHostToDevice, stream));
@@ -825,7 +970,7 @@ struct Correlator {
         FC_CUDA(cudaMemcpyAsync(tmp.get(), host_complex, nc * sizeof(double2),
                                 cudaMemcpyHostToDevice, stream));
         k_z2c<<<grid_for(nc, 256), 256, 0, stream>>>(
-            tmp.as<double2>(), static_cast<float2 *>(fused->g_data()), nc, h,
+            tmp.as<double2>(), static_cast<float2 *>(f->g_data()), nc, h,
             hp);
         FC_LAUNCH_CHECK();
         FC_CUDA(cudaStreamSynchronize(stream));
@@ -856,82 +1001,60 @@ struct Correlator {
   // PeriodicCorrelator::correlate_internal (correlator.h:273-357).
   template <typename T>
   void periodic_run(Density d, bool cross) {
-    const size_t ncells = geo.ncells();
+    if (fused) {
+      FusedSurvey *f = cross ? cross_passes() : fused.get();
+      ProfHook hook(&prof, stream);
+      f->periodic(f->prepare_input(d.p, d.f32, stream), cross, ksub(0), rsub(0), stream,
+                  prof.on ? &hook : nullptr);
+      n_fft += 2;
+      reduce_hist(cross && fused_cross ? hist_cross : hist);
+      return;
+    }
     copy_pad<T>(d, 0.0);
+    periodic_prepared<T>(cross);
+  }
+
+  // The same on a density already in the padded work grid.  In deferred mode
+  // the histograms are the caller's (hist_work): enqueue only, no allocation,
+  // no host synchronisation, so it can be captured into a CUDA graph.
+  template <typename T>
+  void periodic_prepared(bool cross) {
     exec_r2c(work.get(), work.get());
     conj_mul<T>(!cross);
-    const double k_rescale = geo.cell * geo.cell * geo.cell / (double)ncells;
     const int maxell = 2 * (geo.nrows - 1);
     for (int ell = 0; ell <= maxell; ell += 2) {
-      zero_sub(false, true);
-      const double coeff = sqrt((4.0 * M_PI) * (2 * ell + 1)) * k_rescale;
-      ksub_acc<T>(ell, 0, coeff);
-      hist_rows(ell, false, true);
+      zero_sub(ell);
+      ksub_acc<T>(ell, 0, k_coeff(ell));
     }
     exec_c2r(work.get(), work.get());
-    const double r_rescale = (1.0 / ncells / ncells);
-    for (int ell = 0; ell <= maxell; ell += 2) {
-      zero_sub(true, false);
-      const double coeff = sqrt((4.0 * M_PI) * (2 * ell + 1)) * r_rescale;
-      rsub_acc<T>(ell, 0, coeff);
-      hist_rows(ell, true, false);
-      if (ell == 0) save_zerolag();
-    }
+    for (int ell = 0; ell <= maxell; ell += 2) rsub_acc<T>(ell, 0, r_coeff(ell));
+    reduce_hist(hist);
   }
 
-  // Deferred-histogram mode: one r- and one k-subgrid per multipole.
+  // Deferred mode on the cells of a grid of this correlator's precision.
+  void enqueue_prepared(const void *cells) {
+    if (fused)
+      periodic_run<float>({cells, !fp64()}, false);
+    else if (fp64())
+      periodic_prepared<double>(false);
+    else
+      periodic_prepared<float>(false);
+  }
+
   void make_deferred() {
-    FC_REQUIRE(kind == FC_PERIODIC && !fused, FC_ERR_UNSUPPORTED,
+    FC_REQUIRE(kind == FC_PERIODIC, FC_ERR_UNSUPPORTED,
                "deferred histograms are built for the periodic correlator");
     deferred = true;
-    rsub_l.resize(geo.nrows);
-    ksub_l.resize(geo.nrows);
-    for (int r = 0; r < geo.nrows; ++r) {
-      rsub_l[r].resize(geo.rcells() * sizeof(double));
-      ksub_l[r].resize(geo.kcells() * sizeof(double));
-    }
-  }
-
-  // PeriodicCorrelator::correlate_internal (correlator.h:273-357) on a
-  // density the caller has already written into the padded work grid, with
-  // the histograms deferred (hist_work).  Enqueue only: no allocation, no
-  // host synchronisation, so it can be captured into a CUDA graph.
-  template <typename T>
-  void periodic_prepared() {
-    const size_t ncells = geo.ncells();
-    exec_r2c(work.get(), work.get());
-    conj_mul<T>(true);
-    const double k_rescale = geo.cell * geo.cell * geo.cell / (double)ncells;
-    const int maxell = 2 * (geo.nrows - 1);
-    for (int ell = 0; ell <= maxell; ell += 2) {
-      double *dst = ksub_l[ell / 2].as<double>();
-      FC_CUDA(cudaMemsetAsync(dst, 0, geo.kcells() * sizeof(double), stream));
-      const double coeff = sqrt((4.0 * M_PI) * (2 * ell + 1)) * k_rescale;
-      ksub_acc<T>(ell, 0, coeff, dst);
-    }
-    exec_c2r(work.get(), work.get());
-    const double r_rescale = (1.0 / ncells / ncells);
-    for (int ell = 0; ell <= maxell; ell += 2) {
-      double *dst = rsub_l[ell / 2].as<double>();
-      FC_CUDA(cudaMemsetAsync(dst, 0, geo.rcells() * sizeof(double), stream));
-      const double coeff = sqrt((4.0 * M_PI) * (2 * ell + 1)) * r_rescale;
-      rsub_acc<T>(ell, 0, coeff, dst);
-    }
-    const size_t rz = ((size_t)geo.rmax_cells * geo.rsize + geo.rmax_cells) *
-                          geo.rsize + geo.rmax_cells;
-    FC_CUDA(cudaMemcpyAsync(d_zerolag.get(), rsub_l[0].as<double>() + rz,
-                            sizeof(double), cudaMemcpyDeviceToDevice, stream));
-    have_result = true;
   }
 
   // The histogram reductions of the deferred subgrids as work items.
-  void hist_work(std::vector<HistItem> &items, std::vector<FoldItem> &folds) {
+  void hist_work(std::vector<HistItem> &it, std::vector<FoldItem> &fo) {
     FC_REQUIRE(deferred, FC_ERR_STATE, "correlator is not in deferred mode");
-    for (int r = 0; r < geo.nrows; ++r) {
-      rbins.append_work(rsub_l[r].as<double>(), d_rhist.as<double>() + r * geo.nr,
-                        items, folds);
-      kbins.append_work(ksub_l[r].as<double>(), d_khist.as<double>() + r * geo.nk,
-                        items, folds);
+    const int base = (int)it.size();
+    it.insert(it.end(), items.begin(), items.end());
+    for (FoldItem f : folds) {
+      f.first += base;
+      fo.push_back(f);
     }
   }
 
@@ -979,21 +1102,19 @@ struct Correlator {
           // One forward and one (pruned) inverse transform, or the inverse
           // alone for the ell = 0 term of an autocorrelation.
           n_fft += fused->term(in, ell, m, xyz0, (double)ncells,
-                               ksub.as<double>(), rsub.as<double>(),
-                               d_raxis.as<double>(), ka, stream, ph, first,
+                               ksub(ell), rsub(ell), d_raxis.as<double>(), ka, stream, ph, first,
                                prepared, z_done);
           first = false;
         }
-        if (first) zero_sub(true, true);
-        hist_rows(ell, true, true);
-        if (ell == 0) save_zerolag();
+        if (first) zero_sub(ell);
       }
+      reduce_hist(hist);
       return;
     }
     const double *rho = fp64_cells(d);
     int term = 0;
     for (int ell = 0; ell <= maxell; ell += 2) {
-      zero_sub(true, true);
+      zero_sub(ell);
       for (int m = -ell; m <= ell; ++m) {
         if (!owns_term(term++)) continue;
         weight<T>(rho, ell, m, 0.0);
@@ -1003,9 +1124,8 @@ struct Correlator {
         exec_c2r(work.get(), work.get());
         rsub_acc<T>(ell, m, 4.0 * M_PI / ncells);
       }
-      hist_rows(ell, true, true);
-      if (ell == 0) save_zerolag();
     }
+    reduce_hist(hist);
   }
 
   template <typename T>
@@ -1074,15 +1194,14 @@ struct Correlator {
       for (int r = 0; r < nrows; ++r)
         for (int i = 0; i < nk; ++i)
           kcounts[r * nk + i] = have_result ? kbins.counts[i] : 0;
-    if (rhist)
-      FC_CUDA(cudaMemcpy(rhist, d_rhist.get(), (size_t)nrows * nr * sizeof(double),
+    std::vector<double> out(out_len());
+    if (rhist || khist || zerolag)
+      FC_CUDA(cudaMemcpy(out.data(), d_out.get(), out.size() * sizeof(double),
                          cudaMemcpyDeviceToHost));
-    if (khist)
-      FC_CUDA(cudaMemcpy(khist, d_khist.get(), (size_t)nrows * nk * sizeof(double),
-                         cudaMemcpyDeviceToHost));
-    if (zerolag)
-      FC_CUDA(cudaMemcpy(zerolag, d_zerolag.get(), sizeof(double),
-                         cudaMemcpyDeviceToHost));
+    const double *o = out.data();
+    if (rhist) std::copy(o, o + (size_t)nrows * nr, rhist);
+    if (khist) std::copy(o + (size_t)nrows * nr, o + (size_t)nrows * (nr + nk), khist);
+    if (zerolag) *zerolag = out.back();
   }
 };
 
@@ -1112,11 +1231,9 @@ void correlator_autocorrelate(Correlator *c, const Grid *g) {
 void correlator_make_deferred(Correlator *c) { c->make_deferred(); }
 void *correlator_work(Correlator *c) { return c->work.get(); }
 void correlator_set_stream(Correlator *c, cudaStream_t s) { c->set_stream(s); }
-void correlator_enqueue_prepared(Correlator *c) {
-  if (c->fp64())
-    c->periodic_prepared<double>();
-  else
-    c->periodic_prepared<float>();
+bool correlator_fused(const Correlator *c) { return c->fused != nullptr; }
+void correlator_enqueue_prepared(Correlator *c, const void *cells) {
+  c->enqueue_prepared(cells);
 }
 void correlator_hist_work(Correlator *c, std::vector<HistItem> &items,
                           std::vector<FoldItem> &folds) {
@@ -1138,16 +1255,14 @@ CorrShapes correlator_shapes(Correlator *c) {
 void correlator_time_kernels(Correlator *c, int which, cudaStream_t s) {
   c->set_stream(s);
   const int ell = c->geo.nrows > 1 ? 2 : 0;
-  double *k = c->deferred ? c->ksub_l[0].as<double>() : c->ksub.as<double>();
-  double *r = c->deferred ? c->rsub_l[0].as<double>() : c->rsub.as<double>();
   if (c->fp64()) {
     if (which == 0) c->conj_mul<double>(true);
-    if (which == 1) c->ksub_acc<double>(ell, 0, 1.0, k);
-    if (which == 2) c->rsub_acc<double>(ell, 0, 1.0, r);
+    if (which == 1) c->ksub_acc<double>(ell, 0, 1.0);
+    if (which == 2) c->rsub_acc<double>(ell, 0, 1.0);
   } else {
     if (which == 0) c->conj_mul<float>(true);
-    if (which == 1) c->ksub_acc<float>(ell, 0, 1.0, k);
-    if (which == 2) c->rsub_acc<float>(ell, 0, 1.0, r);
+    if (which == 1) c->ksub_acc<float>(ell, 0, 1.0);
+    if (which == 2) c->rsub_acc<float>(ell, 0, 1.0);
   }
 }
 
@@ -1162,27 +1277,33 @@ size_t correlator_footprint(int kind, const int shape[3], double cell,
   size_t bytes = 0;
   const char *mode = std::getenv("FFTCORR_B200_FFT");
   const bool want_fused = !(mode && std::string(mode) == "cufft");
-  if (kind == FC_SURVEY && want_fused && FusedSurvey::supported(g.shape, g.rsize)) {
+  if (want_fused && FusedSurvey::supported(g.shape, g.rsize)) {
     const size_t h = (g.shape[2] / 2 + 1 + 15) / 16 * 16;   // row pitch
-    bytes += 2 * (size_t)g.shape[0] * g.shape[1] * h * eb;   // W, G
+    // W, and G with a survey
+    bytes += (kind == FC_SURVEY ? 2 : 1) * (size_t)g.shape[0] * g.shape[1] * h * eb;
     // Wr and Wry, and below the r-subgrid, whole: the even form keeps half.
     bytes += (size_t)g.rsize * g.shape[1] * h * eb;
     bytes += (size_t)g.rsize * g.rsize * h * eb;
     if (precision != FC_FP64) {                              // FP32 density,
-      bytes += g.ncells() * 4 + (size_t)g.shape[0] * g.shape[1] * 32;  // row table
+      bytes += g.ncells() * 4;
+      if (kind == FC_SURVEY) bytes += (size_t)g.shape[0] * g.shape[1] * 32;  // row table
       const int m = g.shape[2] / 2;
-      if (m >= 32 && m <= 2048 && (m & (m - 1)) == 0)        // paired z pass:
+      if (kind == FC_SURVEY && m >= 32 && m <= 2048 && (m & (m - 1)) == 0)        // paired z pass:
         bytes += (size_t)g.shape[0] * g.shape[1] * (h * eb + 32);  // W2, table
     }
-    const int nlm = maxell == 0 ? 1 : maxell == 2 ? 6 : 15;
-    bytes += (size_t)nlm * g.kcells() * rb;                  // k weights
-    bytes += (size_t)nlm * g.rsize * g.rsize * g.rsize * rb; // r weights
+    if (kind == FC_SURVEY) {
+      const int nlm = maxell == 0 ? 1 : maxell == 2 ? 6 : 15;
+      bytes += (size_t)nlm * (g.kcells() + g.rcells()) * rb;   // weight tables
+    } else {
+      bytes += (size_t)g.nrows * (g.kcells() + g.rcells()) * 8;  // bin weights
+    }
   } else {
     bytes += g.nreal_padded() * rb;                          // work
     if (kind == FC_SURVEY) bytes += g.ncomplex() * eb;       // grid2 FFT
     bytes += g.ncomplex() * eb;                              // cuFFT work area
   }
-  bytes += g.rcells() * (8 + 4) + g.kcells() * (8 + 4);    // subgrids + perms
+  // Subgrids per multipole and bin indices.
+  bytes += (g.rcells() + g.kcells()) * (size_t)(8 * g.nrows + 4);
   return bytes + (4 << 20);
 }
 

@@ -292,7 +292,7 @@ __device__ __forceinline__ void to_half_k(double *__restrict__ ksub,
         for (int l = 0; l < W; ++l) {
           w[s][l] = acc[s][l] = 0.0;
           if (on[s]) {
-            w[s][l] = (double)ktab[cell[s] + l];
+            w[s][l] = ktab ? (double)ktab[cell[s] + l] : 1.0;
             if (!first) acc[s][l] = ksub[cell[s] + l];
           }
         }
@@ -309,7 +309,7 @@ __device__ __forceinline__ void to_half_k(double *__restrict__ ksub,
       const size_t c = ((size_t)L * g.ks1 + j) * g.kp + kz;
       for (int l = 0; l < W; ++l)
         ksub[c + l] = (first ? 0.0 : ksub[c + l]) +
-                      (double)ktab[c + l] * re(L / 2 / TPC, l);
+                      (ktab ? (double)ktab[c + l] : 1.0) * re(L / 2 / TPC, l);
     }
 }
 
@@ -327,9 +327,11 @@ __device__ __forceinline__ void split_pair(const C &z, const C &m, C *a, C *b) {
 // FP64.  MODE 0: out = G = DFT_x(W).  MODE 1: the product, extraction and
 // inverse described at the top; MODE 2 (ell = 0 of an autocorrelation): the
 // weighted field is w00 * rho, whose transform is w00 * G, so P = w00 |G|^2
-// and neither W nor a forward transform is needed.  EVEN: the inverse of
-// Re P, two real columns to a complex one: half of the CTA's threads
-// transform half as many columns, the others leave.
+// and neither W nor a forward transform is needed; MODE 3 (periodic
+// autocorrelation): P = |DFT_x(W)|^2.  Without ktab the k-subgrid's weights
+// are 1.  EVEN: the inverse of Re P, two real columns to a complex one:
+// half of the CTA's threads transform half as many columns, the others
+// leave.
 template <int L, int MODE, bool EVEN>
 __global__ void __launch_bounds__(P2<double, L>::THREADS)
     k_xcorr_p2(const double2 *__restrict__ W, const double2 *__restrict__ G,
@@ -379,6 +381,9 @@ __global__ void __launch_bounds__(P2<double, L>::THREADS)
     if constexpr (MODE == 1) {
 #pragma unroll
       for (int u = 0; u < 8; ++u) v[u] = cmulc(v[u], gv[u]);
+    } else if constexpr (MODE == 3) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u].x = v[u].x * v[u].x + v[u].y * v[u].y;
     }
     const int jr = (yy + g.ks1 / 2) % g.n1;
     if (ksub != nullptr && jr < g.ks1 && kzi <= g.ks2 / 2)
@@ -549,7 +554,8 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
       const double val = (double)(h ? v[u].y : v[u].x);
       for (int rk = (z + g.ro) % g.n2; rk < g.rs; rk += g.n2) {
         const size_t cell = (size_t)row * g.rs + rk;
-        rsub[cell] = (first ? 0.0 : rsub[cell]) + (double)rtab[cell] * val;
+        rsub[cell] = rtab == nullptr ? val
+                                     : (first ? 0.0 : rsub[cell]) + (double)rtab[cell] * val;
       }
     }
   }
@@ -756,7 +762,8 @@ __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
 
 // The FP32 x pass of one (ell, m) term with the same column pairing.
 // MODE 1: P = DFT_x(W) conj(G); MODE 2 (ell = 0 of an autocorrelation):
-// P = w00 |G|^2 with no forward transform (see k_xcorr_p2).  Then the
+// P = w00 |G|^2 with no forward transform; MODE 3 (periodic
+// autocorrelation): P = |DFT_x(W)|^2 (see k_xcorr_p2).  Then the
 // k-subgrid extraction and the inverse transform, stored only at the
 // r-subgrid's rows.  G is read after the forward transform, so a thread
 // holds one pair of columns at a time and two CTAs fit an SM; the other
@@ -796,6 +803,12 @@ __device__ __forceinline__ void xcorr_pp_body(
       v[u].x = w * __ffma2_rn(q.x, q.x, q.y * q.y);
       v[u].y = f2splat(0.f);
     }
+  } else if constexpr (MODE == 3) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = cp.load(W, (t + Q::TPC * u) * stride);
+    reg_fft<L>(v, t, exf, exr, tabx, -1);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u].x = __ffma2_rn(v[u].x, v[u].x, v[u].y * v[u].y);
   } else {
 #pragma unroll
     for (int u = 0; u < 8; ++u) v[u] = cp.load(W, (t + Q::TPC * u) * stride);
@@ -1331,6 +1344,7 @@ void p2_set_limits() {
     big_smem(k_xcorr_p2<L, 2, false>);
     big_smem(k_xcorr_p2<L, 1, true>);
     big_smem(k_xcorr_p2<L, 2, true>);
+    big_smem(k_xcorr_p2<L, 3, true>);
     big_smem(k_zfwd_p2<T, L, true>);
     big_smem(k_zfwd_p2<T, L, false>);
   } else {
@@ -1341,6 +1355,7 @@ void p2_set_limits() {
     big_smem(k_xcorr_pp<L, 2, false>);
     big_smem(k_xcorr_pp<L, 1, true>);
     big_smem(k_xcorr_pp<L, 2, true>);
+    big_smem(k_xcorr_pp<L, 3, true>);
     big_smem(k_zfwd_pp<L, true>);
     big_smem(k_zfwd_pp<L, false>);
     big_smem(k_zfwd_pp2<L>);
@@ -1355,8 +1370,10 @@ bool FusedSurvey::supported(const int shape[3], int rsize) {
 }
 
 FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
-                         bool fp64, bool even)
+                         bool fp64, bool even, bool survey)
     : fp64_(fp64) {
+  if (fault_fires(kFaultFftPlan))
+    FC_THROW(FC_ERR_CUFFT, "injected FFT plan creation failure");
   g.n0 = shape[0];
   g.n1 = shape[1];
   g.n2 = shape[2];
@@ -1386,13 +1403,13 @@ FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
   }
   const size_t nc = (size_t)g.n0 * g.n1 * g.hp;
   W.resize(nc * eb);
-  G.resize(nc * eb);
+  if (survey) G.resize(nc * eb);
   Wr.resize((size_t)g.nri * g.n1 * g.hp * eb);
   Wry.resize((size_t)g.nri * g.rs * g.hp * eb);
   if (!fp64) {
     rho32.resize((size_t)g.n0 * g.n1 * g.n2 * sizeof(float));
-    rowtab.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
-    if (pairs()) {
+    if (survey) rowtab.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
+    if (survey && pairs()) {
       W2.resize(nc * eb);
       rowtab2.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
     }
@@ -1517,11 +1534,11 @@ void FusedSurvey::grid2_x(cudaStream_t s) {
 }
 
 template <typename T>
-void FusedSurvey::xcorr(bool from_g, double *ksub, const void *ktab_v, double w00,
+void FusedSurvey::xcorr(int mode, double *ksub, const void *ktab_v, double w00,
                         bool first, cudaStream_t s) {
   const T *ktab = static_cast<const T *>(ktab_v);
   if (!is_p2(g.n0)) {
-    gen_x<T>(gx, g, from_g ? 2 : 1, W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub,
+    gen_x<T>(gx, g, mode, W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub,
              ktab, (T)w00, first, s);
     return;
   }
@@ -1534,8 +1551,9 @@ void FusedSurvey::xcorr(bool from_g, double *ksub, const void *ktab_v, double w0
             ktab, (float)w00, nyq, first);
       };
       const int nyq = nyq_group<Y::B>(ksub != nullptr);
-      if (from_g && even()) go(k_xcorr_pp<L, 2, true>, 0);
-      else if (from_g) go(k_xcorr_pp<L, 2, false>, 0);
+      if (mode == 3) go(k_xcorr_pp<L, 3, true>, 0);
+      else if (mode == 2 && even()) go(k_xcorr_pp<L, 2, true>, 0);
+      else if (mode == 2) go(k_xcorr_pp<L, 2, false>, 0);
       else if (even()) go(k_xcorr_pp<L, 1, true>, nyq);
       else go(k_xcorr_pp<L, 1, false>, nyq);
     } else {
@@ -1545,8 +1563,9 @@ void FusedSurvey::xcorr(bool from_g, double *ksub, const void *ktab_v, double w0
             W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, g, tabx.as<C2<T>>(), ktab,
             w00, first);
       };
-      if (from_g && even()) go(k_xcorr_p2<L, 2, true>);
-      else if (from_g) go(k_xcorr_p2<L, 2, false>);
+      if (mode == 3) go(k_xcorr_p2<L, 3, true>);
+      else if (mode == 2 && even()) go(k_xcorr_p2<L, 2, true>);
+      else if (mode == 2) go(k_xcorr_p2<L, 2, false>);
       else if (even()) go(k_xcorr_p2<L, 1, true>);
       else go(k_xcorr_p2<L, 1, false>);
     }
@@ -1648,6 +1667,7 @@ const void *FusedSurvey::k_table(int ell, int m, const KAxes &ka,
 
 void FusedSurvey::grid2(const void *rho_in, cudaStream_t s, const KAxes &ka) {
   (void)ka;
+  G.resize(W.bytes());
   YlmParams none = make_ylm_params(0, 0, 1.0);
   const double zero[3] = {0, 0, 0};
   if (fp64_) {
@@ -1708,7 +1728,7 @@ int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
       // The weight is the constant pw.value0, so the term's transform is
       // value0 * G (see k_xcorr_p2, MODE 2).
       if (hook) hook->begin("xcorr00");
-      xcorr<T>(true, ksub, ktab, pw.value0, first, s);
+      xcorr<T>(2, ksub, ktab, pw.value0, first, s);
       if (hook) hook->end();
     } else {
       if (!z_done) {
@@ -1720,7 +1740,7 @@ int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
       yfwd<T>(s);
       if (hook) hook->end();
       if (hook) hook->begin("xcorr");
-      xcorr<T>(false, ksub, ktab, 0.0, first, s);
+      xcorr<T>(1, ksub, ktab, 0.0, first, s);
       if (hook) hook->end();
     }
     if (hook) hook->begin("yinv");
@@ -1735,6 +1755,29 @@ int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
   else
     run(float());
   return from_g ? 1 : 2;
+}
+
+void FusedSurvey::periodic(const void *rho_in, bool cross, double *ksub, double *rsub,
+                           cudaStream_t s, PhaseHook *hook) {
+  const YlmParams none = make_ylm_params(0, 0, 1.0);
+  const double zero[3] = {0, 0, 0};
+  auto phase = [&](const char *name, auto f) {
+    if (hook) hook->begin(name);
+    f();
+    if (hook) hook->end();
+  };
+  auto run = [&](auto tag) {
+    using T = decltype(tag);
+    phase("zfwd", [&] { zfwd<T>(rho_in, false, none, zero, s); });
+    phase("yfwd", [&] { yfwd<T>(s); });
+    phase("xcorr", [&] { xcorr<T>(cross ? 1 : 3, ksub, nullptr, 0.0, true, s); });
+    phase("yinv", [&] { yinv<T>(s); });
+    phase("zinv", [&] { zinv<T>(rsub, nullptr, true, s); });
+  };
+  if (fp64_)
+    run(double());
+  else
+    run(float());
 }
 
 }  // namespace fc

@@ -31,8 +31,9 @@ class FusedSurvey {
 
   // even: the r-subgrid's bins are those of its mirror image, so the inverse
   // transforms may take Re P (fc_fused.cu).
+  // survey: the buffers of weighted terms and of G are allocated now.
   FusedSurvey(const int shape[3], int rsize, const int kshape[3], bool fp64,
-              bool even);
+              bool even, bool survey);
   bool even() const { return g.nri != g.rs; }
   // Cells of the stored subgrids (half_k_cell, half_r_cell).
   size_t k_cells() const { return (size_t)g.ks0 * g.ks1 * g.kp; }
@@ -64,6 +65,12 @@ class FusedSurvey {
             double ncells, double *ksub, double *rsub, const double *raxis,
             const KAxes &ka, cudaStream_t s, PhaseHook *hook, bool first,
             bool g_of_input, bool z_done);
+  // PeriodicCorrelator::correlate_internal (correlator.h:273-357): the one P
+  // of every multipole, |F|^2 or (cross) F conj(G), left unweighted in the
+  // stored subgrids, P itself in ksub and its inverse transform in rsub.
+  // The autocorrelation needs the even form.
+  void periodic(const void *rho_in, bool cross, double *ksub, double *rsub,
+                cudaStream_t s, PhaseHook *hook);
   // Whether two weighted terms can share one z pass (FP32, power-of-two
   // rows).  zfwd_pair runs the z pass of terms a and b (both ell > 0) in
   // one launch: term a's result lands in W, term b's in a second buffer
@@ -82,7 +89,10 @@ class FusedSurvey {
 
   // G in the half-complex layout [N0][N1][N2/2+1] with rows g.hp elements
   // apart (FP64 or FP32 complex).
-  void *g_data() const { return G.get(); }
+  void *g_data() {
+    G.resize(W.bytes());
+    return G.get();
+  }
   bool fp64() const { return fp64_; }
 
   FusedGeom g;
@@ -101,7 +111,7 @@ class FusedSurvey {
   template <typename T>
   void grid2_x(cudaStream_t s);
   template <typename T>
-  void xcorr(bool from_g, double *ksub, const void *ktab, double w00, bool first,
+  void xcorr(int mode, double *ksub, const void *ktab, double w00, bool first,
              cudaStream_t s);
   // Weights of the k-subgrid cells for (ell, m), built on first use.
   // (FP64 for the FP64 form, FP32 for the FP32-mixed form)

@@ -256,7 +256,8 @@ __device__ __forceinline__ void split_elem(double2 *p, const double2 &z, const d
 }
 
 // MODE 0: G = DFT_x(W).  MODE 1: P = DFT_x(W) conj(G); MODE 2 (ell = 0 of an
-// autocorrelation): P = w00 |G|^2.  Then the k-subgrid extraction, straight
+// autocorrelation): P = w00 |G|^2; MODE 3 (periodic autocorrelation): P =
+// |DFT_x(W)|^2.  Then the k-subgrid extraction (weights 1 without ktab), straight
 // from the registers that hold P (every k-subgrid cell has one source
 // element, so the read-modify-writes never collide; `first` overwrites), and
 // the inverse, stored at the r-subgrid's rows.  EVEN: the inverse of Re P
@@ -312,24 +313,25 @@ __global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
 #pragma unroll
           for (int l = 0; l < GE::W; ++l)
             ksub[cell + l] = (first ? 0.0 : ksub[cell + l]) +
-                             (double)ktab[cell + l] * part(re, l);
+                             (ktab ? (double)ktab[cell + l] : 1.0) * part(re, l);
         }
     };
-    if constexpr (MODE == 1) {
+    if constexpr (MODE == 1 || MODE == 3) {
       with_radix(last.R, [&]<int R>() {
         for (int bf = threadIdx.x; bf < last.LR * B; bf += blockDim.x) {
           const int j = bf / B, b = bf % B;
           const C2<T> *gp = G + base + j * stride + GE::W * b;
           E gv[R], v[R];
 #pragma unroll
-          for (int q = 0; q < R; ++q)
+          for (int q = 0; q < (MODE == 1 ? R : 0); ++q)
             gv[q] = GE::load(gp + (int64_t)(q * last.LR) * stride, nb - GE::W * b);
 #pragma unroll
           for (int q = 0; q < R; ++q) v[q] = cur[(j + q * last.LR) * BP + b];
           g_twiddle<R, -1>(v, tw + last.tw, last.Ns, j);
           GDft<R, -1, E>::run(v);
 #pragma unroll
-          for (int q = 0; q < R; ++q) v[q] = cmulc(v[q], gv[q]);
+          for (int q = 0; q < R; ++q)
+            v[q] = MODE == 1 ? cmulc(v[q], gv[q]) : abs2_elem(v[q], (T)1);
 #pragma unroll
           for (int q = 0; q < R; ++q) take(j + q * last.LR, b, v[q], other);
         }
@@ -612,8 +614,10 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
           for (int c = 0; c < NR; ++c) {
             if (ra + c >= nrows) continue;
             const size_t cell = (size_t)(ra + c) * g.rs + rk;
-            rsub[cell] = (first ? 0.0 : rsub[cell]) +
-                         (double)rtab[cell] * (double)comp(v[q], c);
+            const double val = (double)comp(v[q], c);
+            rsub[cell] = rtab == nullptr ? val
+                                         : (first ? 0.0 : rsub[cell]) +
+                                               (double)rtab[cell] * val;
           }
         }
       }
@@ -666,6 +670,7 @@ void col_limits() {
   big_smem(k_gx<T, B, 2, false>);
   big_smem(k_gx<T, B, 1, true>);
   big_smem(k_gx<T, B, 2, true>);
+  big_smem(k_gx<T, B, 3, true>);
 }
 template <typename T>
 void set_limits(int L, bool row) {
@@ -755,6 +760,7 @@ void gen_x(const GenAxis &a, const FusedGeom &g, int mode, const C2<T> *W, const
     };
     const bool even = g.nri != g.rs;
     if (mode == 0) go(k_gx<T, B, 0, false>);
+    else if (mode == 3) go(k_gx<T, B, 3, true>);
     else if (mode == 1 && even) go(k_gx<T, B, 1, true>);
     else if (mode == 1) go(k_gx<T, B, 1, false>);
     else if (even) go(k_gx<T, B, 2, true>);

@@ -30,7 +30,8 @@ void gen_zfwd(const GenAxis &a, const FusedGeom &g, const T *rho,
 template <typename T>
 void gen_yfwd(const GenAxis &a, const FusedGeom &g, typename Vec2<T>::type *W,
               cudaStream_t s);
-// mode 0: out = G = DFT_x(W); 1: the product with G; 2: w00 |G|^2.  first:
+// mode 0: out = G = DFT_x(W); 1: the product with G; 2: w00 |G|^2;
+// 3: |DFT_x(W)|^2.  first:
 // the subgrid is overwritten, not added to.
 template <typename T>
 void gen_x(const GenAxis &a, const FusedGeom &g, int mode,

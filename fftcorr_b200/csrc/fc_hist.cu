@@ -2,6 +2,7 @@
 // the HistogramList C entry points (cc/histogram/histogram_list.h:10-68).
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <cmath>
 
 #include "fc_hist.cuh"
@@ -54,12 +55,45 @@ __global__ void __launch_bounds__(256)
 
 // One thread per bin: chunk partials folded in chunk order.
 __global__ void k_bin_fold(const double *partials, const int *chunk_first,
-                           int nbins, double *hist_row, int add) {
+                           int nbins, double *hist_row) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nbins;
        b += gridDim.x * blockDim.x) {
     double s = 0.0;
     for (int c = chunk_first[b]; c < chunk_first[b + 1]; ++c) s += partials[c];
-    hist_row[b] = add ? hist_row[b] + s : s;
+    hist_row[b] += s;
+  }
+}
+
+// Persistent chunk reductions over the work items of any number of
+// histograms.
+__global__ void __launch_bounds__(kHistThreads)
+    k_hist_items(const HistItem *__restrict__ items, int n,
+                 double *__restrict__ partials) {
+  __shared__ double red[32];
+  for (int it = blockIdx.x; it < n; it += gridDim.x) {
+    const HistItem h = items[it];
+    double acc = 0.0;
+    if (h.weights) {
+      for (int i = threadIdx.x; i < h.len; i += blockDim.x)
+        acc += h.weights[h.start + i] * h.values[h.perm[h.start + i]];
+    } else {
+      for (int i = threadIdx.x; i < h.len; i += blockDim.x)
+        acc += h.scale * h.values[h.perm[h.start + i]];
+    }
+    acc = block_sum(acc, red);
+    if (threadIdx.x == 0) partials[it] = acc;
+  }
+}
+
+// One thread per bin: its chunk partials folded in order.
+__global__ void k_hist_folds(const FoldItem *__restrict__ folds, int n,
+                             const double *__restrict__ partials) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += gridDim.x * blockDim.x) {
+    const FoldItem f = folds[i];
+    double s = 0.0;
+    for (int c = f.first; c < f.first + f.count; ++c) s += partials[c];
+    *f.dest = s;
   }
 }
 
@@ -148,22 +182,6 @@ void BinIndex::build(int *bins_dev, int64_t n, int nbins_, cudaStream_t s) {
   FC_CUDA(cudaStreamSynchronize(s));
 }
 
-void BinIndex::reduce(const double *values, double *hist_row,
-                      cudaStream_t s) const {
-  if (nchunks > 0) {
-    k_chunk_sums<<<nchunks, kHistThreads, 0, s>>>(values, perm.as<uint32_t>(),
-                                         chunk_start.as<uint32_t>(),
-                                         chunk_len.as<int>(),
-                                         partials.as<double>());
-    FC_LAUNCH_CHECK();
-  }
-  if (nbins > 0) {
-    k_bin_fold<<<grid_for(nbins, 128), 128, 0, s>>>(
-        partials.as<double>(), chunk_first.as<int>(), nbins, hist_row, 0);
-    FC_LAUNCH_CHECK();
-  }
-}
-
 void BinIndex::reduce_add(const double *values, double *hist_row,
                           cudaStream_t s) const {
   if (nchunks > 0) {
@@ -175,22 +193,54 @@ void BinIndex::reduce_add(const double *values, double *hist_row,
   }
   if (nbins > 0) {
     k_bin_fold<<<grid_for(nbins, 128), 128, 0, s>>>(
-        partials.as<double>(), chunk_first.as<int>(), nbins, hist_row, 1);
+        partials.as<double>(), chunk_first.as<int>(), nbins, hist_row);
     FC_LAUNCH_CHECK();
   }
 }
 
-void BinIndex::append_work(const double *values, double *hist_row,
+void BinIndex::append_work(const double *values, const uint32_t *cells,
+                           const double *weights, double scale, double *hist_row,
                            std::vector<HistItem> &items,
                            std::vector<FoldItem> &folds) const {
   const int base = (int)items.size();
   for (int c = 0; c < nchunks; ++c)
-    items.push_back(HistItem{values, perm.as<uint32_t>(), h_chunk_start[c],
+    items.push_back(HistItem{values, cells, weights, scale, h_chunk_start[c],
                              h_chunk_len[c]});
   for (int b = 0; b < nbins; ++b)
     folds.push_back(FoldItem{base + h_chunk_first[b],
                              h_chunk_first[b + 1] - h_chunk_first[b],
                              hist_row + b});
+}
+
+void HistPlan::upload(const std::vector<HistItem> &it, const std::vector<FoldItem> &fo) {
+  nitems = (int)it.size();
+  nfolds = (int)fo.size();
+  items.resize(std::max<size_t>(it.size(), 1) * sizeof(HistItem));
+  folds.resize(std::max<size_t>(fo.size(), 1) * sizeof(FoldItem));
+  partials.resize(std::max<size_t>(it.size(), 1) * sizeof(double));
+  if (nitems)
+    FC_CUDA(cudaMemcpy(items.get(), it.data(), it.size() * sizeof(HistItem),
+                       cudaMemcpyHostToDevice));
+  if (nfolds)
+    FC_CUDA(cudaMemcpy(folds.get(), fo.data(), fo.size() * sizeof(FoldItem),
+                       cudaMemcpyHostToDevice));
+}
+
+void HistPlan::run(int blocks, cudaStream_t s) const {
+  if (nitems) {
+    k_hist_items<<<blocks, kHistThreads, 0, s>>>(items.as<HistItem>(), nitems,
+                                                 partials.as<double>());
+    FC_LAUNCH_CHECK();
+  }
+  if (nfolds) {
+    k_hist_folds<<<grid_for(nfolds, 32), 32, 0, s>>>(folds.as<FoldItem>(), nfolds,
+                                                     partials.as<double>());
+    FC_LAUNCH_CHECK();
+  }
+}
+
+void HistPlan::run(cudaStream_t s) const {
+  run(std::max(1, std::min(nitems, sm_count() * 8)), s);
 }
 
 // HistogramList with its counts and sums in device memory.

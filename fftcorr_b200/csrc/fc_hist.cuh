@@ -22,11 +22,14 @@ constexpr int kHistChunk = 2048;
 // Threads of a chunk reduction: part of the summation order, so fixed.
 constexpr int kHistThreads = 256;
 
-// One chunk of a histogram reduction: the sum of values[perm[start ..
-// start + len)] (k_chunk_sums' fixed tree) goes to partials[item index].
+// One chunk of a histogram reduction: the sum over [start, start + len) of
+// w[i] values[perm[i]] in a fixed tree, w[i] = weights[i] or, without
+// weights, scale.
 struct HistItem {
   const double *values;
   const uint32_t *perm;
+  const double *weights;
+  double scale;
   uint32_t start;
   int len;
 };
@@ -55,16 +58,26 @@ struct BinIndex {
   // excluded).  bins_dev is clobbered.  Synchronises the stream.
   void build(int *bins_dev, int64_t n, int nbins_, cudaStream_t s);
 
-  // hist_row[b] = sum over elements e of bin b of values[e] (overwrites).
-  void reduce(const double *values, double *hist_row, cudaStream_t s) const;
-  // hist_row[b] += that sum.
+  // hist_row[b] += sum over elements e of bin b of values[e].
   void reduce_add(const double *values, double *hist_row,
                   cudaStream_t s) const;
-  // Appends the work of reduce(values, hist_row) as chunk and fold items
-  // (the same sums in the same order).
-  void append_work(const double *values, double *hist_row,
+  // Appends the reduction hist_row[b] = sum over elements i of bin b of
+  // w[i] values[cells[i]] as chunk and fold items; cells is perm, or the same
+  // elements by another numbering.
+  void append_work(const double *values, const uint32_t *cells,
+                   const double *weights, double scale, double *hist_row,
                    std::vector<HistItem> &items,
                    std::vector<FoldItem> &folds) const;
+};
+
+// Work items and folds on the device, and the two launches that run them
+// (k_hist_items on `blocks` persistent CTAs, then k_hist_folds).
+struct HistPlan {
+  int nitems = 0, nfolds = 0;
+  DeviceBuffer items, folds, partials;
+  void upload(const std::vector<HistItem> &it, const std::vector<FoldItem> &fo);
+  void run(int blocks, cudaStream_t s) const;
+  void run(cudaStream_t s) const;
 };
 
 // Bin index of value v for HistogramList(minval, binsize, nbins); -1 when

@@ -159,16 +159,19 @@ void correlator_delete(Correlator *c);
 void correlator_autocorrelate(Correlator *c, const Grid *g);
 size_t correlator_footprint(int kind, const int shape[3], double cell,
                             double rmax, double kmax, int maxell, int precision);
-// Periodic correlators only: every multipole keeps its own subgrids and the
-// histograms are left to the caller (correlator_hist_work).
+// Periodic correlators only: the histograms are left to the caller
+// (correlator_hist_work).
 void correlator_make_deferred(Correlator *c);
-// The padded real work grid [N0][N1][2(N2/2+1)] in the correlator's
-// precision.
+// Whether the correlator runs the fused passes, which read a grid's cells.
+bool correlator_fused(const Correlator *c);
+// Otherwise: the padded real work grid [N0][N1][2(N2/2+1)] in the
+// correlator's precision.
 void *correlator_work(Correlator *c);
 void correlator_set_stream(Correlator *c, cudaStream_t s);
-// Enqueues a periodic autocorrelation of the density already in the work
-// grid (deferred mode; no allocation or host synchronisation).
-void correlator_enqueue_prepared(Correlator *c);
+// Enqueues a periodic autocorrelation (deferred mode; no allocation or host
+// synchronisation) of a grid's cells, in the correlator's precision, or of
+// the density already in the work grid.
+void correlator_enqueue_prepared(Correlator *c, const void *cells);
 // Appends the histogram reductions of the last deferred run.
 void correlator_hist_work(Correlator *c, std::vector<HistItem> &items,
                           std::vector<FoldItem> &folds);

@@ -34,6 +34,33 @@ def test_survey_axis_lengths(shape, kmax, precision):
                      "cross", fp32=precision == "fp32")
 
 
+@pytest.mark.parametrize("shape", [(7, 450, 9), (486, 5, 14), (1, 30, 21), (64, 64, 64),
+                                   (128, 64, 35), (11, 16, 20)])
+@pytest.mark.parametrize("kmax", [0.15, 0.35])
+@pytest.mark.parametrize("cell,dr", [(10.0, 6.0), (2.6, 5.2)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_periodic_axis_lengths(shape, kmax, cell, dr, precision):
+    """Periodic correlations through the fused passes (11 cells: cuFFT), with
+    bins that are the same under inversion (10, 6) and that are not (2.6,
+    5.2), where a cross correlation takes the general inverse."""
+    rng = np.random.default_rng(7)
+    a, b = rng.standard_normal(shape), rng.standard_normal(shape)
+    rmax = cell * min(9, min(shape))
+    args = (cell, TSC_ALIASED_CORRECTION, rmax, dr, kmax, 0.03, 4)
+    fp32 = precision == "fp32"
+    if rmax < dr and fp32:
+        pytest.skip("no separation bin to take an rms over")
+    c = fb.PeriodicCorrelator(shape, *args, precision=precision)
+    ref = O.periodic_correlate(a, *args)
+    c.autocorrelate(a)
+    _compare_results(c.results(), ref, FP64_RTOL, "auto", fp32=fp32)
+    c.cross_correlate(a, b)
+    _compare_results(c.results(), O.periodic_correlate(a, *args, grid2=b), FP64_RTOL,
+                     "cross", fp32=fp32)
+    c.autocorrelate(a)
+    _compare_results(c.results(), ref, FP64_RTOL, "auto again", fp32=fp32)
+
+
 @pytest.mark.parametrize("shape", [(64, 64, 64), (40, 64, 66)])
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_bins_that_differ_under_inversion(shape, precision):
