@@ -12,8 +12,9 @@
 //             of particles inside a cell is their input order
 //   K-units   first sorted position of every scatter unit (binary search)
 //             and, per colour, the list of non-empty units
-//   K-scatter NGP/CIC/TSC: persistent CTAs per colour pass draw 2x8x8-cell
-//             units; a thread per home cell sums its particles' stencil
+//   K-scatter NGP/CIC/TSC, per colour pass: 2x8x8-cell units of a few
+//             particles go to a warp each (k_scatter_w); persistent CTAs draw
+//             the larger ones: a thread per home cell sums its particles' stencil
 //             products in registers, and the footprint (unit + stencil
 //             halo) takes the home cells' sums in W^3 ordered rounds.  D12
 //             (8^3 taps): one CTA per 8^3 tile; particles are staged in
@@ -46,9 +47,12 @@ namespace {
 
 constexpr int kTile = 8;         // tile edge in cells
 constexpr int kTileCells = 512;  // cells per tile
-// A scatter unit with more particles than this is drawn before the others
-// of its colour pass (a quarter of the narrow stencils' staging chunk).
-constexpr uint32_t kHeavyUnit = 128;
+// A scatter unit of at most this many particles, one per lane, is taken by
+// one warp (k_scatter_w), a larger one by a CTA (k_scatter_p).  With two or
+// four rounds of lanes (64, 128) a batch of clustered boxes gained 1% and 0%,
+// 8M clustered points in 384^3 lost 1% and 14%, and 100M randoms, whose few
+// small units then hold up each pass, 0.6% and 1.8%.
+constexpr uint32_t kWarpUnit = 32;
 constexpr int kScatterThreads = 256;
 constexpr int kChunk = 256;      // particles staged per shared-memory chunk
 
@@ -281,10 +285,8 @@ __global__ void k_unit_ranges(const uint32_t *__restrict__ units, int64_t nu,
                               uint4 *__restrict__ ranges) {
   // The loop is warp-uniform so that the lanes of a warp that hold
   // non-empty units of the same colour and class take their slots with one
-  // atomic.  Units of more than kHeavyUnit particles fill the colour's slice
-  // from its end (counter cnt[2 ncolors + c]), the others from its start
-  // (cnt[c]); the scatter draws the heavy ones first, so that no long unit
-  // starts near the end of a pass.
+  // atomic.  The CTAs' units fill the colour's slice from its end (counter
+  // cnt[2 ncolors + c]), the warps' from its start (cnt[c]).
   for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x; i0 < nu;
        i0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = i0 + threadIdx.x;
@@ -299,7 +301,7 @@ __global__ void k_unit_ranges(const uint32_t *__restrict__ units, int64_t nu,
     const bool ne = i < nu && ts < te;
     const unsigned act = __ballot_sync(0xffffffffu, ne);
     if (!ne) continue;
-    const bool heavy = te - ts > kHeavyUnit;
+    const bool heavy = te - ts > kWarpUnit;
     const unsigned grp = __match_any_sync(act, 2 * c + (heavy ? 1 : 0));
     const int lane = threadIdx.x & 31;
     const int leader = __ffs(grp) - 1;
@@ -311,14 +313,6 @@ __global__ void k_unit_ranges(const uint32_t *__restrict__ units, int64_t nu,
     const int64_t at = heavy ? coff[c + 1] - 1 - (int64_t)slot : coff[c] + slot;
     ranges[at] = make_uint4(u, ts, te, 0u);
   }
-}
-
-// Unit i of a colour pass: the heavy units (nh of them, stored from the
-// slice's end backwards) first, then the others from the slice's start.
-__device__ __forceinline__ uint4 pass_unit(const uint4 *__restrict__ front,
-                                           const uint4 *__restrict__ back,
-                                           unsigned nh, unsigned i) {
-  return i < nh ? back[-1 - (int64_t)i] : front[i - nh];
 }
 
 // Exclusive prefix sum over the block (blockDim.x a multiple of 32, at most
@@ -511,19 +505,28 @@ __device__ __forceinline__ size_t foot_cell(int fx, int fy, int fz, int o0,
   return ((size_t)gx * g.n[1] + gy) * g.n[2] + gz;
 }
 
-// [ranges, ranges_end): this colour's slice of (unit, first, end) records,
-// `count` non-empty units from its start and `count_heavy` heavy ones from
-// its end; `next` is this colour's work counter (zero before the pass).
+// Programmatic dependent launch: a kernel lets the next one of its stream
+// start when every CTA of it has called launch_dependents (or left), and a
+// kernel so started waits for the whole of the one before with
+// grid_dependency_wait.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The `count` (unit, first, end) records before ranges_end, from the last
+// backwards, are this colour's large units; `next` is their work counter
+// (zero before the pass).
 // GT is the grid's cell type: each footprint cell's FP64 sum for the unit is
 // added to the cell in FP64 and rounded to GT once.
 template <int S, typename KeyT, int TX, typename GT>
 __global__ void __launch_bounds__(TX * 64, ScatterP<S, TX>::MIN_BLOCKS)
     k_scatter_p(const double *__restrict__ posw, const KeyT *__restrict__ keys,
                 const uint32_t *__restrict__ vals,
-                const uint4 *__restrict__ ranges,
                 const uint4 *__restrict__ ranges_end,
-                const unsigned *__restrict__ count,
-                const unsigned *__restrict__ count_heavy, unsigned *next,
+                const unsigned *__restrict__ count, unsigned *next,
                 AssignGeom g, GT *__restrict__ grid) {
   using Q = ScatterP<S, TX>;
   constexpr int W = Q::W;
@@ -553,12 +556,14 @@ __global__ void __launch_bounds__(TX * 64, ScatterP<S, TX>::MIN_BLOCKS)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
 
-  const unsigned nh = *count_heavy;
-  const unsigned n = *count + nh;
+  // The small units' kernel touches other cells and may run beside this one.
+  grid_launch_dependents();
+  const unsigned n = *count;
+  if (n <= blockIdx.x) return;  // (each CTA draws at least one unit)
   if (threadIdx.x == 0) {
     const unsigned i0 = atomicAdd(next, 1u);
     s_next = atomicAdd(next, 1u);
-    s_rg = i0 < n ? pass_unit(ranges, ranges_end, nh, i0) : make_uint4(0u, 0u, 0u, 0u);
+    s_rg = i0 < n ? ranges_end[-1 - (int64_t)i0] : make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
   uint4 rg = s_rg;
@@ -573,7 +578,7 @@ __global__ void __launch_bounds__(TX * 64, ScatterP<S, TX>::MIN_BLOCKS)
     unsigned inn = 0;
     if (threadIdx.x == 0) {
       inn = atomicAdd(next, 1u);
-      if (inext < n) rgn = pass_unit(ranges, ranges_end, nh, inext);
+      if (inext < n) rgn = ranges_end[-1 - (int64_t)inext];
     }
     const uint32_t unit = rg.x, ts = rg.y, te = rg.z;
     const uint32_t tile = unit / NS;
@@ -763,6 +768,198 @@ __global__ void __launch_bounds__(TX * 64, ScatterP<S, TX>::MIN_BLOCKS)
   }
 }
 
+// The small units of a colour pass (the first `count` of the colour's slice
+// of ranges): one warp each, at most 32 particles.  A CTA's fixed cost per
+// unit -- the barriers of ranking, staging and footprint rounds, about 4 us --
+// is what a unit of a few particles costs in k_scatter_p; here each lane
+// computes one particle's 1-D weights, and then the lanes are the W^3 taps of
+// one particle after another, added to the warp's footprint in shared memory
+// in sorted (input) order.  Bound by its instructions (1100 a unit at 18
+// particles, CIC: weights, sums and addresses in equal parts).  Measured: 8M
+// clustered points, CIC, 384^3 FP64 2.79 -> 1.64 ms (a colour pass 298 -> 125
+// us plus 26 us for the large units), a batch of 12 boxes 17.1 -> 11.2 ms,
+// 100k points in 128^3 a pass 16 -> 10 us.
+constexpr int kWarpsPerCta = 4;
+template <int S>
+struct ScatterW {
+  static constexpr int W = Stencil<S>::W;
+  static constexpr int FX = kUnitX + W - 1;
+  static constexpr int FY = kTile + W - 1;
+  static constexpr int F3 = FX * FY * FY;
+  static constexpr int WT = 3 * W + 1;  // a particle's weights, and a pad
+  // The footprint is NR rows of FY cells along z; G rows at a time are the
+  // warp's lanes, lane = (row, z).
+  static constexpr int NR = FX * FY, G = 32 / FY, STEPS = (NR + G - 1) / G;
+  // per warp: acc[F3] | gfoot[F3] | wts[32][WT] doubles, row[NR] int64,
+  // base[32] ints
+  static constexpr int DOUBLES = 2 * F3 + 32 * WT + NR + 16;
+};
+
+// Particles of a small unit's range record (bounded by the lanes).
+__device__ __forceinline__ int unit_particles(const uint4 &r) {
+  return (int)min(r.z - r.y, 32u);
+}
+
+template <int S, typename KeyT, typename GT>
+__global__ void __launch_bounds__(32 * kWarpsPerCta, 8)
+    k_scatter_w(const double *__restrict__ posw, const KeyT *__restrict__ keys,
+                const uint32_t *__restrict__ vals,
+                const uint4 *__restrict__ ranges,
+                const unsigned *__restrict__ count, AssignGeom g,
+                GT *__restrict__ grid) {
+  using Q = ScatterW<S>;
+  constexpr int W = Q::W, W3 = W * W * W, FX = Q::FX, FY = Q::FY, F3 = Q::F3;
+  constexpr int NR = Q::NR, G = Q::G;
+  constexpr int OMIN = Stencil<S>::OMIN, NS = kTile / kUnitX;
+  constexpr int T = kUnitX * kTile * kTile;
+  extern __shared__ __align__(16) double smem[];
+  const int lane = threadIdx.x & 31;
+  double *acc = smem + (threadIdx.x >> 5) * Q::DOUBLES;
+  GT *gfoot = reinterpret_cast<GT *>(acc + F3);
+  double *wts = acc + 2 * F3;
+  int64_t *rows = reinterpret_cast<int64_t *>(wts + 32 * Q::WT);
+  int *base = reinterpret_cast<int *>(rows + NR);
+  const int lr = lane / FY, lz = lane % FY;  // this lane's footprint row and z
+  auto on_row = [&](int step) { return lr < G && step * G + lr < NR; };
+  const unsigned n = *count;
+  const bool direct = g.n[0] >= FX && g.n[1] >= FY && g.n[2] >= FY;
+  const bool a16 = (reinterpret_cast<uintptr_t>(posw) & 15) == 0;
+  // This lane's tap.
+  const int ta = lane / (W * W), tb = (lane / W) % W, tc = lane % W;
+  const int toff = (ta * FY + tb) * FY + tc;
+
+  // A unit's loads form a chain (range, keys and indices, rows), so the next
+  // unit's range is fetched at the start of this one and its first keys and
+  // indices before this one's particles are summed.
+  // (Units are dealt out in turn: they are all small, and a counter that
+  // every warp draws from would be the bound.)
+  const unsigned nwarps = gridDim.x * kWarpsPerCta;
+  const unsigned i0 = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
+  unsigned i1 = i0 + nwarps;
+  if (i0 >= n) {
+    grid_dependency_wait();
+    return;
+  }
+  uint4 rg = ranges[i0];
+  KeyT key = 0;
+  uint32_t idx = 0;
+  if (lane < unit_particles(rg)) {
+    key = keys[rg.y + lane];
+    idx = vals[rg.y + lane];
+  }
+  for (;;) {
+    const uint4 rgn = i1 < n ? ranges[i1] : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t unit = rg.x;
+    const uint32_t tile = unit / NS;
+    const int tz = tile % g.nt[2];
+    const int ty = (tile / g.nt[2]) % g.nt[1];
+    const int tx = tile / (g.nt[2] * g.nt[1]);
+    const int o0 = tx * kTile + (int)(unit % NS) * kUnitX;
+    const int o1 = ty * kTile, o2 = tz * kTile;
+    const int m = unit_particles(rg);
+    double p[4] = {0.0, 0.0, 0.0, 0.0};
+    if (lane < m) {
+      const double *src = posw + 4 * (size_t)idx;
+      if (a16) {
+        const double2 u = reinterpret_cast<const double2 *>(src)[0];
+        const double2 v = reinterpret_cast<const double2 *>(src)[1];
+        p[0] = u.x;
+        p[1] = u.y;
+        p[2] = v.x;
+        p[3] = v.y;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) p[k] = src[k];
+      }
+    }
+    // While the rows are under way: the grid's cells (no other unit of this
+    // pass touches them), the empty footprint, the next unit's keys.
+    int64_t zoff = 0;
+    if (direct) {
+      // First cell of every footprint row in the grid; this lane's z.
+      for (int r = lane; r < NR; r += 32)
+        rows[r] = (int64_t)foot_cell<OMIN>(r / FY, r % FY, -OMIN - o2, o0, o1, o2, g);
+      const int gz = o2 + lz + OMIN;
+      zoff = gz < 0 ? gz + g.n[2] : (gz >= g.n[2] ? gz - g.n[2] : gz);
+      __syncwarp();
+    }
+#pragma unroll
+    for (int st = 0; st < Q::STEPS; ++st)
+      if (on_row(st)) {
+        const int f = st * (G * FY) + lane;
+        if (direct) cp_async_cell(gfoot + f, grid + rows[st * G + lr] + zoff);
+        acc[f] = 0.0;
+      }
+    KeyT keyn = 0;
+    uint32_t idxn = 0;
+    if (lane < unit_particles(rgn)) {
+      keyn = keys[rgn.y + lane];
+      idxn = vals[rgn.y + lane];
+    }
+    if (lane < m) {
+      double x[3];
+      dev_grid_coords(p, g, x);
+      double *w = wts + lane * Q::WT;
+      Stencil<S>::weights(x[0] - floor(x[0]), x[1] - floor(x[1]), x[2] - floor(x[2]),
+                          p[3], w, w + W, w + 2 * W);
+      // (A key outside this unit cannot occur in a correct sort; it is
+      // dropped rather than indexing outside the footprint.)
+      const KeyT kd = key - (KeyT)unit * (KeyT)T;
+      const int h = (int)kd;
+      base[lane] = kd < (KeyT)T ? ((h >> 6) * FY + ((h >> 3) & 7)) * FY + (h & 7) : -1;
+    }
+    __syncwarp();
+    for (int q = 0; q < m; ++q) {
+      const int b = base[q];
+      if (lane < W3 && b >= 0) {
+        const double *w = wts + q * Q::WT;
+        double *a = acc + b + toff;
+        *a = fma(w[ta] * w[W + tb], w[2 * W + tc], *a);
+      }
+      __syncwarp();
+    }
+    if (direct) {
+      cp_async_wait_all();  // this lane reads the cells it copied
+#pragma unroll
+      for (int st = 0; st < Q::STEPS; ++st)
+        if (on_row(st)) {
+          const int f = st * (G * FY) + lane;
+          const double v = acc[f];
+          if (v != 0.0) grid[rows[st * G + lr] + zoff] = (GT)((double)gfoot[f] + v);
+        }
+    } else {
+      // Each global cell is written by one footprint cell (its smallest
+      // alias when the footprint wraps onto itself on narrow grids).
+      for (int f = lane; f < F3; f += 32) {
+        const int fx = f / (FY * FY), fy = (f / FY) % FY, fz = f % FY;
+        if (fx >= g.n[0] || fy >= g.n[1] || fz >= g.n[2]) continue;
+        double v = 0.0;
+        for (int ax = fx; ax < FX; ax += g.n[0])
+          for (int ay = fy; ay < FY; ay += g.n[1])
+            for (int az = fz; az < FY; az += g.n[2]) v += acc[(ax * FY + ay) * FY + az];
+        if (v == 0.0) continue;
+        int gx = (o0 + fx + OMIN) % g.n[0];
+        int gy = (o1 + fy + OMIN) % g.n[1];
+        int gz = (o2 + fz + OMIN) % g.n[2];
+        if (gx < 0) gx += g.n[0];
+        if (gy < 0) gy += g.n[1];
+        if (gz < 0) gz += g.n[2];
+        GT &cell = grid[((size_t)gx * g.n[1] + gy) * g.n[2] + gz];
+        cell = (GT)((double)cell + v);
+      }
+    }
+    __syncwarp();
+    if (i1 >= n) break;
+    rg = rgn;
+    key = keyn;
+    idx = idxn;
+    i1 += nwarps;
+  }
+  // The next pass may start when this one has finished, not before the large
+  // units' kernel, beside which this one runs, has too.
+  grid_dependency_wait();
+}
+
 template <int S>
 size_t scatter_smem() {
   constexpr int W = Stencil<S>::W;
@@ -815,22 +1012,27 @@ int stencil_width(int scheme, int *omin) {
   }
 }
 
-// Scatter kernel for scheme 0, 1 or 3, a key type and a cell type.
+// Scatter kernels for scheme 0, 1 or 3, a key type and a cell type.
+struct ScatterFns {
+  const void *cta = nullptr, *warp = nullptr;
+  size_t smem = 0, warp_smem = 0;  // of their CTAs
+};
 template <typename KeyT, typename GT>
-void scatter_p_kernel(int scheme, const void **fn, size_t *smem) {
+ScatterFns scatter_fns(int scheme) {
+  auto of = [](auto cta, auto warp, size_t smem, int doubles) {
+    return ScatterFns{(const void *)cta, (const void *)warp, smem,
+                      kWarpsPerCta * doubles * sizeof(double)};
+  };
   switch (scheme) {
     case 0:
-      *fn = (const void *)k_scatter_p<0, KeyT, kUnitX, GT>;
-      *smem = ScatterP<0, kUnitX>::smem;
-      break;
+      return of(k_scatter_p<0, KeyT, kUnitX, GT>, k_scatter_w<0, KeyT, GT>,
+                ScatterP<0, kUnitX>::smem, ScatterW<0>::DOUBLES);
     case 1:
-      *fn = (const void *)k_scatter_p<1, KeyT, kUnitX, GT>;
-      *smem = ScatterP<1, kUnitX>::smem;
-      break;
+      return of(k_scatter_p<1, KeyT, kUnitX, GT>, k_scatter_w<1, KeyT, GT>,
+                ScatterP<1, kUnitX>::smem, ScatterW<1>::DOUBLES);
     default:
-      *fn = (const void *)k_scatter_p<3, KeyT, kUnitX, GT>;
-      *smem = ScatterP<3, kUnitX>::smem;
-      break;
+      return of(k_scatter_p<3, KeyT, kUnitX, GT>, k_scatter_w<3, KeyT, GT>,
+                ScatterP<3, kUnitX>::smem, ScatterW<3>::DOUBLES);
   }
 }
 
@@ -861,12 +1063,11 @@ struct Assignor {
   DeviceBuffer color_units;            // units in colour order
   DeviceBuffer unit_ranges;            // uint4 per unit, colour slices
   DeviceBuffer color_off_dev;          // color_offsets on the device
-  DeviceBuffer pass_counters;          // per colour: light units, work, heavy units
+  DeviceBuffer pass_counters;          // per colour: the warps' units, CTAs'
+                                       // units drawn, the CTAs' units
   std::vector<int64_t> color_offsets;  // per colour, into color_units
-  const void *scatter_fn = nullptr;    // k_scatter_p for this scheme / keys
-  size_t scatter_smem_bytes = 0;
-  int scatter_threads = 0;
-  unsigned scatter_ctas = 0;           // persistent CTAs per colour pass
+  ScatterFns scatter;                  // for this scheme, keys and cells
+  unsigned scatter_ctas = 0, scatter_w_ctas = 0;  // persistent CTAs of each
   DeviceBuffer partials;               // K-key block partials
   DeviceBuffer totals;                 // [totw, totwsq]
   DeviceBuffer counts;                 // [num_added]
@@ -917,22 +1118,25 @@ struct Assignor {
     FC_CUDA(cudaMemsetAsync(counts.get(), 0, counts.bytes(), grid->stream));
     if (scheme != 2) {
       while ((1 << unit_shift) < unit_x * kTile * kTile) ++unit_shift;
-      if (wide_keys && grid->fp32())
-        scatter_p_kernel<uint64_t, float>(scheme, &scatter_fn, &scatter_smem_bytes);
-      else if (wide_keys)
-        scatter_p_kernel<uint64_t, double>(scheme, &scatter_fn, &scatter_smem_bytes);
-      else if (grid->fp32())
-        scatter_p_kernel<uint32_t, float>(scheme, &scatter_fn, &scatter_smem_bytes);
+      if (wide_keys)
+        scatter = grid->fp32() ? scatter_fns<uint64_t, float>(scheme)
+                               : scatter_fns<uint64_t, double>(scheme);
       else
-        scatter_p_kernel<uint32_t, double>(scheme, &scatter_fn, &scatter_smem_bytes);
-      scatter_threads = unit_x * 64;
-      FC_CUDA(cudaFuncSetAttribute(scatter_fn,
+        scatter = grid->fp32() ? scatter_fns<uint32_t, float>(scheme)
+                               : scatter_fns<uint32_t, double>(scheme);
+      FC_CUDA(cudaFuncSetAttribute(scatter.cta,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)scatter_smem_bytes));
+                                   (int)scatter.smem));
       int per_sm = 0;
       FC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, scatter_fn, scatter_threads, scatter_smem_bytes));
+          &per_sm, scatter.cta, unit_x * 64, scatter.smem));
       scatter_ctas = (unsigned)std::max(1, per_sm) * (unsigned)sm_count();
+      FC_CUDA(cudaFuncSetAttribute(scatter.warp,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)scatter.warp_smem));
+      FC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+          &per_sm, scatter.warp, 32 * kWarpsPerCta, scatter.warp_smem));
+      scatter_w_ctas = (unsigned)std::max(1, per_sm) * (unsigned)sm_count();
     }
     for (int b = 1; b <= radix::kMaxBits; ++b)
       FC_CUDA(cudaFuncSetAttribute(radix::downsweep_kernel(b),
@@ -1304,15 +1508,34 @@ struct Assignor {
       if (nu == 0) continue;
       const uint4 *cr = unit_ranges.as<uint4>() + color_offsets[c];
       const uint4 *cre = unit_ranges.as<uint4>() + color_offsets[c + 1];
-      const unsigned *cnt = counters + c;
-      const unsigned *cnth = counters + 2 * ncolors + c;
+      // The large units first: their tail is the longer one.
+      const unsigned *cnt = counters + 2 * ncolors + c;
       unsigned *nxt = counters + ncolors + c;
-      void *args[] = {(void *)&pw, (void *)&sk,  (void *)&sv,  (void *)&cr,
-                      (void *)&cre, (void *)&cnt, (void *)&cnth, (void *)&nxt,
-                      (void *)&ga, (void *)&gp};
-      const unsigned ctas = (unsigned)std::min<int64_t>(nu, scatter_ctas);
-      FC_CUDA(cudaLaunchKernel(scatter_fn, dim3(ctas), dim3(scatter_threads),
-                               args, scatter_smem_bytes, st));
+      void *cta_args[] = {(void *)&pw,  (void *)&sk,  (void *)&sv, (void *)&cre,
+                          (void *)&cnt, (void *)&nxt, (void *)&ga, (void *)&gp};
+      if (n > kWarpUnit) {
+        FC_CUDA(cudaLaunchKernel(scatter.cta,
+                                 dim3((unsigned)std::min<int64_t>(nu, scatter_ctas)),
+                                 dim3(unit_x * 64), cta_args, scatter.smem, st));
+        FC_LAUNCH_CHECK();
+      }
+      const unsigned *wcnt = counters + c;
+      void *warp_args[] = {(void *)&pw,   (void *)&sk,   (void *)&sv, (void *)&cr,
+                           (void *)&wcnt, (void *)&ga,   (void *)&gp};
+      const int64_t wctas = (nu + kWarpsPerCta - 1) / kWarpsPerCta;
+      // It needs nothing of the large units' kernel, so it starts as that
+      // one's CTAs leave room, and fills its tail.
+      cudaLaunchAttribute beside{};
+      beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      beside.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((unsigned)std::min<int64_t>(wctas, scatter_w_ctas));
+      cfg.blockDim = dim3(32 * kWarpsPerCta);
+      cfg.dynamicSmemBytes = scatter.warp_smem;
+      cfg.stream = st;
+      cfg.attrs = &beside;
+      cfg.numAttrs = n > kWarpUnit ? 1 : 0;
+      FC_CUDA(cudaLaunchKernelExC(&cfg, scatter.warp, warp_args));
       FC_LAUNCH_CHECK();
     }
     if (!graph_mode) window_timer.stop(st);
