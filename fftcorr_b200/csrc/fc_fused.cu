@@ -52,25 +52,6 @@ struct Tile {
   static constexpr int B = 64 / (2 * sizeof(T));  // 8 for FP32, 4 for FP64
 };
 
-// Y_lm * D in the arithmetic of the pass: the reference's FP64 evaluation
-// for the FP64 form, the FP32 evaluator (FP64 coordinates and
-// normalisation) for the FP32-mixed form.
-template <typename T>
-__device__ __forceinline__ T weight_value(const YlmParams &p, T D, double x,
-                                          double y, double z);
-template <>
-__device__ __forceinline__ double weight_value<double>(const YlmParams &p,
-                                                       double D, double x,
-                                                       double y, double z) {
-  return ylm_eval(p, D, x, y, z);
-}
-template <>
-__device__ __forceinline__ float weight_value<float>(const YlmParams &p,
-                                                     float D, double x,
-                                                     double y, double z) {
-  return ylm_eval_f32(p, D, x, y, z);
-}
-
 // FP32-mixed weighting of one grid row: with (x, y) fixed, Y_lm * r^ell is
 // a polynomial in z, so the row's coefficients (normalisation folded in)
 // are formed once in FP64 and each cell costs a Horner evaluation and one
@@ -92,19 +73,6 @@ __device__ __forceinline__ RowPoly row_poly(const YlmParams &p, double x,
   for (int i = 0; i < 5; ++i) r.c[i] = (float)c[i];
   r.rxy2 = (float)(x * x + y * y);
   return r;
-}
-
-// z is the cell's z coordinate rounded to FP32 (the polynomial is FP32).
-// 1/r^2 uses the fast reciprocal-divide intrinsic: r^2 lies between 1e-20
-// and 1e10 here, where its error is 2 ulp, far inside the FP32 budget.
-__device__ __forceinline__ float row_weight(const RowPoly &r, float D,
-                                            float z) {
-  if (r.ell == 0) return D * r.value0;
-  const float z2 = z * z;
-  const float poly =
-      (((r.c[4] * z + r.c[3]) * z + r.c[2]) * z + r.c[1]) * z + r.c[0];
-  const float ir2 = __fdividef(1.0f, r.rxy2 + z2 + 1e-20f);
-  return r.ell == 2 ? D * poly * ir2 : D * poly * (ir2 * ir2);
 }
 
 // The row polynomial of an (ell, m) term has only the powers of z of one
@@ -433,14 +401,17 @@ __global__ void __launch_bounds__(P2<double, L>::THREADS)
   }
 }
 
-// Rows of the z transform: thread t of row b holds z[t + TPC u].
-template <typename T, int L, bool WEIGHT>
-__global__ void __launch_bounds__(P2<T, L>::THREADS)
-    k_zfwd_p2(const T *__restrict__ rho, C2<T> *__restrict__ W, FusedGeom g,
+// FP64 rows of the z transform: thread t of row b holds z[t + TPC u].  The
+// weight of a cell is its row's polynomial in z over r^ell (row_poly_coefs),
+// formed per thread: with the evaluation of Y_lm from (x, y, z) at every cell
+// the pass took 108 us at 256^3 against 66, bound by FP64 instructions.
+template <int L, bool WEIGHT>
+__global__ void __launch_bounds__(P2<double, L>::THREADS)
+    k_zfwd_p2(const double *__restrict__ rho, double2 *__restrict__ W, FusedGeom g,
               YlmParams p, double x0, double y0, double z0,
-              const C2<T> *__restrict__ tabz) {
-  using C = C2<T>;
-  using Q = P2<T, L>;
+              const double2 *__restrict__ tabz) {
+  using C = double2;
+  using Q = P2<double, L>;
   // Row pitch in shared memory, with one pad slot every 8 elements so the
   // strided Stockham writes spread over the banks.
   constexpr int RP = L + L / 8 + 1;
@@ -451,39 +422,42 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
   const int64_t nrows = (int64_t)g.n0 * g.n1;
   const int64_t row = (int64_t)blockIdx.x * Q::B + b;
   const bool valid = row < nrows;
+  const C *src = reinterpret_cast<const C *>(rho + (valid ? row : 0) * g.n2);
   C v[8];
-  int x = 0, y = 0;
-  if (valid) {
-    x = (int)(row / g.n1);
-    y = (int)(row - (int64_t)x * g.n1);
-  }
-  const double cx = x0 + x * 1.0;
-  const double cy = y0 + y * 1.0;
-  const C *src = reinterpret_cast<const C *>(rho + row * g.n2);
-  RowPoly rp;
-  // z of this thread's first element in FP64; the elements u step by the
-  // exact integer 2 TPC, added in FP32.
-  float zt = 0.f;
-  if constexpr (WEIGHT && sizeof(T) == 4) {
-    rp = row_poly(p, cx, cy);
-    zt = (float)(z0 + (2 * t) * 1.0);
-  }
 #pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    v[u].x = 0;
-    v[u].y = 0;
-    if (valid) {
-      const int jj = t + Q::TPC * u;
-      const C pr = src[jj];
-      v[u] = pr;
-      if constexpr (WEIGHT && sizeof(T) == 4) {
-        const float zu = zt + (float)(2 * Q::TPC * u);
-        v[u].x = row_weight(rp, pr.x, zu);
-        v[u].y = row_weight(rp, pr.y, zu + 1.0f);
-      } else if constexpr (WEIGHT) {
-        v[u].x = weight_value<T>(p, pr.x, cx, cy, z0 + (2 * jj) * 1.0);
-        v[u].y = weight_value<T>(p, pr.y, cx, cy, z0 + (2 * jj + 1) * 1.0);
+  for (int u = 0; u < 8; ++u) v[u] = valid ? src[t + Q::TPC * u] : make_double2(0, 0);
+  if constexpr (WEIGHT) {
+    if (p.ell == 0) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        v[u].x *= p.value0;
+        v[u].y *= p.value0;
       }
+    } else {
+      const int x = (int)((unsigned)row / (unsigned)g.n1);
+      const int y = (int)row - x * g.n1;
+      const double cx = x0 + x * 1.0, cy = y0 + y * 1.0;
+      const double rxy2 = cx * cx + cy * cy;
+      double c[5];
+      row_poly_coefs(p, cx, cy, c);
+      auto weigh = [&](auto ell, double d, double z) {
+        const double z2 = z * z;
+        const double ir2 = 1.0 / (rxy2 + z2 + 1e-20);
+        if constexpr (decltype(ell)::value == 2)
+          return d * ((c[2] * z + c[1]) * z + c[0]) * ir2;
+        else
+          return d * ((((c[4] * z + c[3]) * z + c[2]) * z + c[1]) * z + c[0]) * ir2 * ir2;
+      };
+      auto row_of = [&](auto ell) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const double z = z0 + (2 * (t + Q::TPC * u)) * 1.0;
+          v[u].x = weigh(ell, v[u].x, z);
+          v[u].y = weigh(ell, v[u].y, z + 1.0);
+        }
+      };
+      if (p.ell == 2) row_of(std::integral_constant<int, 2>());
+      else row_of(std::integral_constant<int, 4>());
     }
   }
   auto exf = [&](int i) { return &ex[b * RP + i + (i >> 3)]; };
@@ -497,12 +471,12 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
   for (int k = t; k <= L; k += Q::TPC) {
     const C a = *exf(k == L ? 0 : k);
     const C c = cconj(*exf(k == 0 ? 0 : L - k));
-    C e, d, o;
-    e.x = (T)0.5 * (a.x + c.x);
-    e.y = (T)0.5 * (a.y + c.y);
-    d = csub(a, c);
-    o.x = (T)0.5 * d.y;
-    o.y = (T)-0.5 * d.x;
+    C e, o;
+    e.x = 0.5 * (a.x + c.x);
+    e.y = 0.5 * (a.y + c.y);
+    const C d = csub(a, c);
+    o.x = 0.5 * d.y;
+    o.y = -0.5 * d.x;
     dst[k] = cadd(e, cmul(__ldg(&tabz[k]), o));
   }
 }
@@ -1345,8 +1319,8 @@ void p2_set_limits() {
     big_smem(k_xcorr_p2<L, 1, true>);
     big_smem(k_xcorr_p2<L, 2, true>);
     big_smem(k_xcorr_p2<L, 3, true>);
-    big_smem(k_zfwd_p2<T, L, true>);
-    big_smem(k_zfwd_p2<T, L, false>);
+    big_smem(k_zfwd_p2<L, true>);
+    big_smem(k_zfwd_p2<L, false>);
   } else {
     big_smem(k_yfwd_pp<L>);
     big_smem(k_yinv_pp<L>);
@@ -1474,14 +1448,15 @@ void FusedSurvey::zfwd(const void *rho, bool weight, const YlmParams &p,
               xyz0[2], tabz.as<float2>(), nullptr);
         return;
       }
-      if (weight)
-        k_zfwd_p2<T, L, true><<<blocks, Q::THREADS, p2_row_smem<T, L>(), s>>>(
-            (const T *)rho, W.as<C2<T>>(), g, p, xyz0[0], xyz0[1], xyz0[2],
-            tabz.as<C2<T>>());
-      else
-        k_zfwd_p2<T, L, false><<<blocks, Q::THREADS, p2_row_smem<T, L>(), s>>>(
-            (const T *)rho, W.as<C2<T>>(), g, p, xyz0[0], xyz0[1], xyz0[2],
-            tabz.as<C2<T>>());
+      if constexpr (std::is_same_v<T, double>) {
+        auto go = [&](auto kernel) {
+          kernel<<<blocks, Q::THREADS, p2_row_smem<T, L>(), s>>>(
+              (const T *)rho, W.as<C2<T>>(), g, p, xyz0[0], xyz0[1], xyz0[2],
+              tabz.as<C2<T>>());
+        };
+        if (weight) go(k_zfwd_p2<L, true>);
+        else go(k_zfwd_p2<L, false>);
+      }
     });
     FC_LAUNCH_CHECK();
     return;
