@@ -473,7 +473,10 @@ struct ScatterP {
   static constexpr int W = Stencil<S>::W;
   static constexpr int W3 = W * W * W;
   static constexpr int THREADS = TX * 64;
-  static constexpr int MIN_BLOCKS = TX == 2 ? 5 : kTile / TX;
+  // CTAs per SM: TSC's table and its 27 sums a thread leave room for five,
+  // the narrower stencils for eight (8M clustered points, CIC, 384^3 1.61 ->
+  // 1.51 ms; a batch of 12 boxes 11.1 -> 10.7 ms).
+  static constexpr int MIN_BLOCKS = TX == 2 ? (W == 3 ? 5 : 8) : kTile / TX;
   static constexpr int FX = TX + W - 1;     // footprint extent along x
   static constexpr int FY = kTile + W - 1;  // ... along y and z
   static constexpr int F3 = FX * FY * FY;
