@@ -508,17 +508,6 @@ __device__ __forceinline__ size_t foot_cell(int fx, int fy, int fz, int o0,
   return ((size_t)gx * g.n[1] + gy) * g.n[2] + gz;
 }
 
-// Programmatic dependent launch: a kernel lets the next one of its stream
-// start when every CTA of it has called launch_dependents (or left), and a
-// kernel so started waits for the whole of the one before with
-// grid_dependency_wait.
-__device__ __forceinline__ void grid_dependency_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void grid_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // The `count` (unit, first, end) records before ranges_end, from the last
 // backwards, are this colour's large units; `next` is their work counter
 // (zero before the pass).

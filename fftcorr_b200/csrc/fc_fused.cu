@@ -174,6 +174,7 @@ template <typename T, int L>
 __global__ void __launch_bounds__(P2<T, L>::THREADS)
     k_yfwd_p2(C2<T> *__restrict__ W, FusedGeom g,
               const C2<T> *__restrict__ taby) {
+  grid_chain();
   using C = C2<T>;
   using Q = P2<T, L>;
   extern __shared__ unsigned char smem_raw[];
@@ -203,6 +204,7 @@ template <typename T, int L>
 __global__ void __launch_bounds__(P2<T, L>::THREADS)
     k_yinv_p2(const C2<T> *__restrict__ Wr, C2<T> *__restrict__ Wry,
               FusedGeom g, const C2<T> *__restrict__ taby) {
+  grid_chain();
   using C = C2<T>;
   using Q = P2<T, L>;
   extern __shared__ unsigned char smem_raw[];
@@ -306,6 +308,7 @@ __global__ void __launch_bounds__(P2<double, L>::THREADS)
                double2 *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
                const double2 *__restrict__ tabx, const double *__restrict__ ktab,
                double w00, int first) {
+  grid_chain();
   using C = double2;
   using Q = P2<double, L>;
   extern __shared__ unsigned char smem_raw[];
@@ -410,6 +413,7 @@ __global__ void __launch_bounds__(P2<double, L>::THREADS)
     k_zfwd_p2(const double *__restrict__ rho, double2 *__restrict__ W, FusedGeom g,
               YlmParams p, double x0, double y0, double z0,
               const double2 *__restrict__ tabz) {
+  grid_chain();
   using C = double2;
   using Q = P2<double, L>;
   // Row pitch in shared memory, with one pad slot every 8 elements so the
@@ -486,6 +490,7 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
     k_zinv_p2(const C2<T> *__restrict__ Wry, double *__restrict__ rsub,
               FusedGeom g, const C2<T> *__restrict__ tabz,
               const T *__restrict__ rtab, int first) {
+  grid_chain();
   using C = C2<T>;
   using Q = P2<T, L>;
   constexpr int RP = L + L / 8 + 1;
@@ -697,6 +702,7 @@ template <int L>
 __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
     k_yfwd_pp(float2 *__restrict__ W, FusedGeom g,
               const float2 *__restrict__ taby) {
+  grid_chain();
   // (Splitting off the last column measured slower here: 194 vs 183 us.)
   yfwd_pp_body<L, false>(W, g, taby);
 }
@@ -731,6 +737,7 @@ template <int L>
 __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
     k_xfwd_pp(const float2 *__restrict__ W, float2 *__restrict__ G, FusedGeom g,
               const float2 *__restrict__ tabx) {
+  grid_chain();
   xfwd_pp_body<L, false>(W, G, g, tabx);
 }
 
@@ -890,6 +897,7 @@ __global__ void __launch_bounds__(PY<L, kXB>::THREADS, 1024 / PY<L, kXB>::THREAD
                float2 *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
                const float2 *__restrict__ tabx, const float *__restrict__ ktab,
                float w00, int nyq, int first) {
+  grid_chain();
   // The last column split off (nyq) pays in the product mode only; the
   // ell = 0 mode compiles without it (with it: 215 vs 188 us).
   if constexpr (MODE == 1) {
@@ -945,6 +953,7 @@ template <int L>
 __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
     k_yinv_pp(const float2 *__restrict__ Wr, float2 *__restrict__ Wry,
               FusedGeom g, const float2 *__restrict__ taby, int nyq) {
+  grid_chain();
   if (split_cta(nyq))
     yinv_pp_body<L, true>(Wr, Wry, g, taby);
   else
@@ -959,6 +968,7 @@ __global__ void __launch_bounds__(PP<L>::THREADS)
               YlmParams p, double x0, double y0, double z0,
               const float2 *__restrict__ tabz,
               const float4 *__restrict__ rowtab) {
+  grid_chain();
   using Q = PP<L>;
   constexpr int RP = L + L / 8 + 1;
   extern __shared__ unsigned char smem_raw[];
@@ -1148,6 +1158,7 @@ __global__ void __launch_bounds__(PP<L>::THREADS, 1024 / PP<L>::THREADS)
                double z0, const float2 *__restrict__ tabz,
                const float4 *__restrict__ rowtab_a,
                const float4 *__restrict__ rowtab_b) {
+  grid_chain();
   using Q = PP<L>;
   constexpr int RP = L + L / 8 + 1;
   extern __shared__ unsigned char smem_raw[];
@@ -1206,6 +1217,7 @@ __global__ void __launch_bounds__(PP<L>::THREADS, 1024 / PP<L>::THREADS)
 // row, so the z pass does no FP64 work per row.
 __global__ void k_rowpoly(float4 *__restrict__ tab, int64_t nrows, int n1,
                           YlmParams p, double x0, double y0) {
+  grid_chain();
   for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
        row < nrows; row += (int64_t)gridDim.x * blockDim.x) {
     const int x = (int)(row / n1);
@@ -1433,24 +1445,24 @@ void FusedSurvey::zfwd(const void *rho, bool weight, const YlmParams &p,
         const float4 *rt = nullptr;
         if (weight && p.ell != 0) {
           rowtab.resize((size_t)nrows * 2 * sizeof(float4));
-          k_rowpoly<<<grid_for(nrows, 256), 256, 0, s>>>(
+          launch_after(k_rowpoly, grid_for(nrows, 256), 256, 0, s, 
               rowtab.as<float4>(), nrows, g.n1, p, xyz0[0], xyz0[1]);
           FC_LAUNCH_CHECK();
           rt = rowtab.as<float4>();
         }
         if (weight)
-          k_zfwd_pp<L, true><<<blocks, PQ::THREADS, p2_row_smem<T, L>(), s>>>(
+          launch_after(k_zfwd_pp<L, true>, blocks, PQ::THREADS, p2_row_smem<T, L>(), s, 
               (const float *)rho, W.as<float2>(), g, p, xyz0[0], xyz0[1],
               xyz0[2], tabz.as<float2>(), rt);
         else
-          k_zfwd_pp<L, false><<<blocks, PQ::THREADS, p2_row_smem<T, L>(), s>>>(
+          launch_after(k_zfwd_pp<L, false>, blocks, PQ::THREADS, p2_row_smem<T, L>(), s, 
               (const float *)rho, W.as<float2>(), g, p, xyz0[0], xyz0[1],
               xyz0[2], tabz.as<float2>(), nullptr);
         return;
       }
       if constexpr (std::is_same_v<T, double>) {
         auto go = [&](auto kernel) {
-          kernel<<<blocks, Q::THREADS, p2_row_smem<T, L>(), s>>>(
+          launch_small(kernel, blocks, Q::THREADS, p2_row_smem<T, L>(), s, 
               (const T *)rho, W.as<C2<T>>(), g, p, xyz0[0], xyz0[1], xyz0[2],
               tabz.as<C2<T>>());
         };
@@ -1472,11 +1484,11 @@ void FusedSurvey::yfwd(cudaStream_t s) {
       if constexpr (std::is_same_v<T, float>) {
         using Y = PY<L>;
         dim3 grid((g.h + Y::B - 1) / Y::B, g.n0);
-        k_yfwd_pp<L><<<grid, Y::THREADS, Y::smem, s>>>(W.as<float2>(), g,
+        launch_after(k_yfwd_pp<L>, grid, Y::THREADS, Y::smem, s, W.as<float2>(), g,
                                                         taby.as<float2>());
       } else {
         dim3 grid((g.h + Q::B - 1) / Q::B, g.n0);
-        k_yfwd_p2<T, L><<<grid, Q::THREADS, p2_col_smem<T, L>(), s>>>(
+        launch_small(k_yfwd_p2<T, L>, grid, Q::THREADS, p2_col_smem<T, L>(), s, 
             W.as<C2<T>>(), g, taby.as<C2<T>>());
       }
     });
@@ -1495,12 +1507,11 @@ void FusedSurvey::grid2_x(cudaStream_t s) {
   with_p2(g.n0, [&]<int L>() {
     if constexpr (std::is_same_v<T, float>) {
       using Y = PY<L>;
-      k_xfwd_pp<L><<<dim3((g.h + Y::B - 1) / Y::B, g.n1), Y::THREADS, Y::smem, s>>>(
+      launch_after(k_xfwd_pp<L>, dim3((g.h + Y::B - 1) / Y::B, g.n1), Y::THREADS, Y::smem, s, 
           W.as<float2>(), G.as<float2>(), g, tabx.as<float2>());
     } else {
       using Q = P2<T, L>;
-      k_xcorr_p2<L, 0, false>
-          <<<dim3((g.h + Q::B - 1) / Q::B, g.n1), Q::THREADS, p2_col_smem<T, L>(), s>>>(
+      launch_small(k_xcorr_p2<L, 0, false>, dim3((g.h + Q::B - 1) / Q::B, g.n1), Q::THREADS, p2_col_smem<T, L>(), s, 
               W.as<C2<T>>(), nullptr, G.as<C2<T>>(), nullptr, g, tabx.as<C2<T>>(), nullptr,
               T(0), 1);
     }
@@ -1521,7 +1532,7 @@ void FusedSurvey::xcorr(int mode, double *ksub, const void *ktab_v, double w00,
     if constexpr (std::is_same_v<T, float>) {
       using Y = PY<L, kXB>;
       auto go = [&](auto kernel, int nyq) {
-        kernel<<<dim3((g.h + Y::B - 1) / Y::B, g.n1), Y::THREADS, Y::smem, s>>>(
+        launch_after(kernel, dim3((g.h + Y::B - 1) / Y::B, g.n1), Y::THREADS, Y::smem, s, 
             W.as<float2>(), G.as<float2>(), Wr.as<float2>(), ksub, g, tabx.as<float2>(),
             ktab, (float)w00, nyq, first);
       };
@@ -1534,7 +1545,7 @@ void FusedSurvey::xcorr(int mode, double *ksub, const void *ktab_v, double w00,
     } else {
       using Q = P2<T, L>;
       auto go = [&](auto kernel) {
-        kernel<<<dim3((g.h + Q::B - 1) / Q::B, g.n1), Q::THREADS, p2_col_smem<T, L>(), s>>>(
+        launch_small(kernel, dim3((g.h + Q::B - 1) / Q::B, g.n1), Q::THREADS, p2_col_smem<T, L>(), s, 
             W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, g, tabx.as<C2<T>>(), ktab,
             w00, first);
       };
@@ -1556,12 +1567,12 @@ void FusedSurvey::yinv(cudaStream_t s) {
       if constexpr (std::is_same_v<T, float>) {
         using Y = PY<L>;
         dim3 grid((g.h + Y::B - 1) / Y::B, g.nri);
-        k_yinv_pp<L><<<grid, Y::THREADS, Y::smem, s>>>(
+        launch_after(k_yinv_pp<L>, grid, Y::THREADS, Y::smem, s, 
             Wr.as<float2>(), Wry.as<float2>(), g, taby.as<float2>(),
             nyq_group<Y::B>(false));
       } else {
         dim3 grid((g.h + Q::B - 1) / Q::B, g.nri);
-        k_yinv_p2<T, L><<<grid, Q::THREADS, p2_col_smem<T, L>(), s>>>(
+        launch_small(k_yinv_p2<T, L>, grid, Q::THREADS, p2_col_smem<T, L>(), s, 
             Wr.as<C2<T>>(), Wry.as<C2<T>>(), g, taby.as<C2<T>>());
       }
     });
@@ -1579,7 +1590,7 @@ void FusedSurvey::zinv(double *rsub, const void *rtab_v, bool first, cudaStream_
       using Q = P2<T, L>;
       const int nrows = g.nri * g.rs;
       const unsigned blocks = (unsigned)((nrows + Q::B - 1) / Q::B);
-      k_zinv_p2<T, L><<<blocks, Q::THREADS, p2_row_smem<T, L>(), s>>>(
+      launch_chain(!fp64_ || blocks <= 4u * sm_count(), k_zinv_p2<T, L>, blocks, Q::THREADS, p2_row_smem<T, L>(), s, 
           Wry.as<C2<T>>(), rsub, g, tabz.as<C2<T>>(), rtab, first);
     });
     FC_LAUNCH_CHECK();
@@ -1669,17 +1680,17 @@ void FusedSurvey::zfwd_pair(const void *rho_in, int ell_a, int m_a, int ell_b,
   const YlmParams pa = make_ylm_params(ell_a, m_a, 1.0);
   const YlmParams pb = make_ylm_params(ell_b, m_b, 1.0);
   const int64_t nrows = (int64_t)g.n0 * g.n1;
-  k_rowpoly<<<grid_for(nrows, 256), 256, 0, s>>>(rowtab.as<float4>(), nrows,
+  launch_after(k_rowpoly, grid_for(nrows, 256), 256, 0, s, rowtab.as<float4>(), nrows,
                                                  g.n1, pa, xyz0[0], xyz0[1]);
   FC_LAUNCH_CHECK();
-  k_rowpoly<<<grid_for(nrows, 256), 256, 0, s>>>(rowtab2.as<float4>(), nrows,
+  launch_after(k_rowpoly, grid_for(nrows, 256), 256, 0, s, rowtab2.as<float4>(), nrows,
                                                  g.n1, pb, xyz0[0], xyz0[1]);
   FC_LAUNCH_CHECK();
   if (hook) hook->begin("zfwd2");
   with_p2(g.m, [&]<int L>() {
     using PQ = PP<L>;
     const unsigned blocks = (unsigned)((nrows + PQ::PB - 1) / PQ::PB);
-    k_zfwd_pp2<L><<<blocks, PQ::THREADS, p2_row_smem<float, L>(), s>>>(
+    launch_after(k_zfwd_pp2<L>, blocks, PQ::THREADS, p2_row_smem<float, L>(), s, 
         static_cast<const float *>(rho_in), W.as<float2>(), W2.as<float2>(), g,
         pa, pb, xyz0[2], tabz.as<float2>(), rowtab.as<float4>(),
         rowtab2.as<float4>());

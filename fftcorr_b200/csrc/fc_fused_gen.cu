@@ -166,6 +166,7 @@ template <typename T, int B>
 __global__ void __launch_bounds__(kYThreads, sizeof(T) == 4 ? 2 : 1)
     k_gyfwd(C2<T> *W, FusedGeom g, const __grid_constant__ GPlan plan,
             const C2<T> *__restrict__ tw) {
+  grid_chain();
   using GE = GElem<T>;
   using E = typename GE::E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -184,6 +185,7 @@ template <typename T, int B>
 __global__ void __launch_bounds__(kYThreads, sizeof(T) == 4 ? 2 : 1)
     k_gyinv(const C2<T> *__restrict__ Wr, C2<T> *__restrict__ Wry, FusedGeom g,
             const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw) {
+  grid_chain();
   using GE = GElem<T>;
   using E = typename GE::E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -268,6 +270,7 @@ __global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
          C2<T> *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
          const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw,
          const T *__restrict__ ktab, T w00, int first) {
+  grid_chain();
   using GE = GElem<T>;
   using E = typename GE::E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -453,6 +456,7 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
     k_gzfwd(const T *__restrict__ rho, C2<T> *__restrict__ W, FusedGeom g,
             const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw, int np,
             YlmParams p, double x0, double y0, double z0) {
+  grid_chain();
   using E = typename GElem<T>::E;
   constexpr int NR = 2 * GElem<T>::W;  // grid rows per element
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -548,6 +552,7 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
     k_gzinv(const C2<T> *__restrict__ Wry, double *__restrict__ rsub, FusedGeom g,
             const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw, int np,
             const T *__restrict__ rtab, int first) {
+  grid_chain();
   using E = typename GElem<T>::E;
   constexpr int NR = 2 * GElem<T>::W;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -722,7 +727,7 @@ void gen_zfwd(const GenAxis &a, const FusedGeom &g, const T *rho, C2<T> *W, bool
   const unsigned blocks = (unsigned)((nrows + NR * np - 1) / (NR * np));
   const size_t sm = row_smem(g.n2, np);
   auto go = [&](auto kernel) {
-    kernel<<<blocks, row_threads(a.plan, np), sm, s>>>(rho, W, g, a.plan, a.tw.as<C2<T>>(), np, p,
+    launch_small(kernel, blocks, row_threads(a.plan, np), sm, s, rho, W, g, a.plan, a.tw.as<C2<T>>(), np, p,
                                            xyz0[0], xyz0[1], xyz0[2]);
   };
   if (!weight) go(k_gzfwd<T, -1>);
@@ -743,8 +748,7 @@ template <typename T>
 void gen_yfwd(const GenAxis &a, const FusedGeom &g, C2<T> *W, cudaStream_t s) {
   with_width(a, [&]<int B>() {
     constexpr int NC = kCols<T, B>;
-    k_gyfwd<T, B><<<dim3((g.h + NC - 1) / NC, g.n0), col_threads(a.plan, kYThreads),
-                    col_smem(g.n1), s>>>(W, g, a.plan, a.tw.as<C2<T>>());
+    launch_small(k_gyfwd<T, B>, dim3((g.h + NC - 1) / NC, g.n0), col_threads(a.plan, kYThreads), col_smem(g.n1), s, W, g, a.plan, a.tw.as<C2<T>>());
   });
   FC_LAUNCH_CHECK();
 }
@@ -755,7 +759,7 @@ void gen_x(const GenAxis &a, const FusedGeom &g, int mode, const C2<T> *W, const
   with_width(a, [&]<int B>() {
     constexpr int NC = kCols<T, B>;
     auto go = [&](auto kernel) {
-      kernel<<<dim3((g.h + NC - 1) / NC, g.n1), col_threads(a.plan, kXThreads), col_smem(g.n0), s>>>(
+      launch_small(kernel, dim3((g.h + NC - 1) / NC, g.n1), col_threads(a.plan, kXThreads), col_smem(g.n0), s, 
           W, G, out, ksub, g, a.plan, a.tw.as<C2<T>>(), ktab, w00, first);
     };
     const bool even = g.nri != g.rs;
@@ -774,8 +778,7 @@ void gen_yinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wr, C2<T> *Wry,
               cudaStream_t s) {
   with_width(a, [&]<int B>() {
     constexpr int NC = kCols<T, B>;
-    k_gyinv<T, B><<<dim3((g.h + NC - 1) / NC, g.nri), col_threads(a.plan, kYThreads),
-                    col_smem(g.n1), s>>>(Wr, Wry, g, a.plan, a.tw.as<C2<T>>());
+    launch_small(k_gyinv<T, B>, dim3((g.h + NC - 1) / NC, g.nri), col_threads(a.plan, kYThreads), col_smem(g.n1), s, Wr, Wry, g, a.plan, a.tw.as<C2<T>>());
   });
   FC_LAUNCH_CHECK();
 }
@@ -786,7 +789,7 @@ void gen_zinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wry, double *rs
   constexpr int NR = 2 * GElem<T>::W;
   const int nrows = g.nri * g.rs;
   const int np = row_elems(a.plan, (nrows + NR - 1) / NR);
-  k_gzinv<T><<<(nrows + NR * np - 1) / (NR * np), row_threads(a.plan, np), row_smem(g.n2, np), s>>>(
+  launch_small(k_gzinv<T>, (nrows + NR * np - 1) / (NR * np), row_threads(a.plan, np), row_smem(g.n2, np), s, 
       Wry, rsub, g, a.plan, a.tw.as<C2<T>>(), np, rtab, first);
   FC_LAUNCH_CHECK();
 }

@@ -69,6 +69,7 @@ __global__ void k_bin_fold(const double *partials, const int *chunk_first,
 __global__ void __launch_bounds__(kHistThreads)
     k_hist_items(const HistItem *__restrict__ items, int n,
                  double *__restrict__ partials) {
+  grid_chain();
   __shared__ double red[32];
   for (int it = blockIdx.x; it < n; it += gridDim.x) {
     const HistItem h = items[it];
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(kHistThreads)
 // One thread per bin: its chunk partials folded in order.
 __global__ void k_hist_folds(const FoldItem *__restrict__ folds, int n,
                              const double *__restrict__ partials) {
+  grid_chain();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += gridDim.x * blockDim.x) {
     const FoldItem f = folds[i];
@@ -228,12 +230,12 @@ void HistPlan::upload(const std::vector<HistItem> &it, const std::vector<FoldIte
 
 void HistPlan::run(int blocks, cudaStream_t s) const {
   if (nitems) {
-    k_hist_items<<<blocks, kHistThreads, 0, s>>>(items.as<HistItem>(), nitems,
+    launch_after(k_hist_items, blocks, kHistThreads, 0, s, items.as<HistItem>(), nitems,
                                                  partials.as<double>());
     FC_LAUNCH_CHECK();
   }
   if (nfolds) {
-    k_hist_folds<<<grid_for(nfolds, 32), 32, 0, s>>>(folds.as<FoldItem>(), nfolds,
+    launch_after(k_hist_folds, grid_for(nfolds, 32), 32, 0, s, folds.as<FoldItem>(), nfolds,
                                                      partials.as<double>());
     FC_LAUNCH_CHECK();
   }
