@@ -53,6 +53,10 @@ constexpr int kTileCells = 512;  // cells per tile
 // 8M clustered points in 384^3 lost 1% and 14%, and 100M randoms, whose few
 // small units then hold up each pass, 0.6% and 1.8%.
 constexpr uint32_t kWarpUnit = 32;
+// With more particles than this per unit of the grid on average (a Poisson
+// catalog then has 32 or fewer in a tenth of its units) every unit goes to a
+// CTA, and the warps' launches, 2 us a colour pass, are left out.
+constexpr int64_t kDenseUnit = 40;
 constexpr int kScatterThreads = 256;
 constexpr int kChunk = 256;      // particles staged per shared-memory chunk
 
@@ -281,7 +285,7 @@ __global__ void k_unit_starts(const KeyT *keys, int64_t n, int64_t nunits,
 __global__ void k_unit_ranges(const uint32_t *__restrict__ units, int64_t nu,
                               const uint32_t *__restrict__ start,
                               const int64_t *__restrict__ coff, int ncolors,
-                              unsigned *__restrict__ cnt,
+                              uint32_t warp_unit, unsigned *__restrict__ cnt,
                               uint4 *__restrict__ ranges) {
   // The loop is warp-uniform so that the lanes of a warp that hold
   // non-empty units of the same colour and class take their slots with one
@@ -301,7 +305,7 @@ __global__ void k_unit_ranges(const uint32_t *__restrict__ units, int64_t nu,
     const bool ne = i < nu && ts < te;
     const unsigned act = __ballot_sync(0xffffffffu, ne);
     if (!ne) continue;
-    const bool heavy = te - ts > kWarpUnit;
+    const bool heavy = te - ts > warp_unit;
     const unsigned grp = __match_any_sync(act, 2 * c + (heavy ? 1 : 0));
     const int lane = threadIdx.x & 31;
     const int leader = __ffs(grp) - 1;
@@ -1480,6 +1484,7 @@ struct Assignor {
     sort_keys<KeyT>(unit_shift, &sk, &sv);
     cudaStream_t st = stream();
     if (!graph_mode) window_timer.start(st);
+    const uint32_t warp_unit = n > kDenseUnit * nunits ? 0u : kWarpUnit;
     const int unit_cells = unit_x * kTile * kTile;
     k_unit_starts<KeyT><<<grid_for(nunits + 1, 256), 256, 0, st>>>(
         sk, n, nunits, unit_cells, unit_start.as<uint32_t>());
@@ -1490,7 +1495,7 @@ struct Assignor {
     FC_CUDA(cudaMemsetAsync(counters, 0, pass_counters.bytes(), st));
     k_unit_ranges<<<grid_for(nunits, 256), 256, 0, st>>>(
         units, nunits, unit_start.as<uint32_t>(), color_off_dev.as<int64_t>(),
-        ncolors, counters, unit_ranges.as<uint4>());
+        ncolors, warp_unit, counters, unit_ranges.as<uint4>());
     FC_LAUNCH_CHECK();
     void *gp = grid->raw();
     AssignGeom ga = geom;
@@ -1505,12 +1510,13 @@ struct Assignor {
       unsigned *nxt = counters + ncolors + c;
       void *cta_args[] = {(void *)&pw,  (void *)&sk,  (void *)&sv, (void *)&cre,
                           (void *)&cnt, (void *)&nxt, (void *)&ga, (void *)&gp};
-      if (n > kWarpUnit) {
+      if (n > warp_unit) {
         FC_CUDA(cudaLaunchKernel(scatter.cta,
                                  dim3((unsigned)std::min<int64_t>(nu, scatter_ctas)),
                                  dim3(unit_x * 64), cta_args, scatter.smem, st));
         FC_LAUNCH_CHECK();
       }
+      if (warp_unit == 0) continue;
       const unsigned *wcnt = counters + c;
       void *warp_args[] = {(void *)&pw,   (void *)&sk,   (void *)&sv, (void *)&cr,
                            (void *)&wcnt, (void *)&ga,   (void *)&gp};
@@ -1526,7 +1532,7 @@ struct Assignor {
       cfg.dynamicSmemBytes = scatter.warp_smem;
       cfg.stream = st;
       cfg.attrs = &beside;
-      cfg.numAttrs = n > kWarpUnit ? 1 : 0;
+      cfg.numAttrs = n > warp_unit ? 1 : 0;
       FC_CUDA(cudaLaunchKernelExC(&cfg, scatter.warp, warp_args));
       FC_LAUNCH_CHECK();
     }

@@ -50,3 +50,14 @@ def test_units_around_one_warp(scheme, periodic, precision, shift):
     tol = 1e-12 if precision == "fp64" else 12 * 6e-8
     assert np.max(np.abs(np.asarray(grid) - ref)) <= tol * np.max(np.abs(ref))
     assert ma.num_added == n
+
+
+def test_dense_catalog_leaves_the_warps_out():
+    """More than 40 particles per unit on average: every unit, the nearly empty
+    ones too, goes to a CTA."""
+    shape = (16, 24, 32)
+    posw = _unit_points(np.random.default_rng(4), shape, [4000, 1, 31, 32, 33, 200])
+    ref, _ = O.mass_assign(posw, shape, [0.0] * 3, 1.0, 1, True)
+    grid = fb.ConfigSpaceGrid.from_geometry(shape, [0.0] * 3, 1.0)
+    fb.MassAssignor(grid, 1, True, 0).add_particles(posw)
+    assert np.max(np.abs(np.asarray(grid) - ref)) <= 1e-12 * np.max(np.abs(ref))
