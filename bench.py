@@ -311,10 +311,10 @@ TRAFFIC_PER_LAUNCH_512 = {
     "zfwd": 1048.8e6,
     "zfwd2": 1603.7e6,
     "yfwd": 1063.2e6,
-    "xcorr": 1375.7e6,
-    "xcorr00": 801.0e6,
-    "yinv": 144.4e6,
-    "zinv": 49.1e6,
+    "xcorr": 1227.3e6,
+    "xcorr00": 652.7e6,
+    "yinv": 66.0e6,
+    "zinv": 18.3e6,
 }
 
 
@@ -335,29 +335,31 @@ def algorithmic_bytes(family, w, precision, rs, ks):
       zfwd2  the z pass of two terms at once: density in (N * s) + two W
              out (2 Nc e)
       yfwd   W in and out (2 Nc e)
-      xcorr  W and G in (2 Nc e) + x-pruned Wr out (rs N1 h e)
-             + k-subgrid weight read (s bytes a cell) and FP64
-             read-modify-write (K0 K1 K2 * (16 + s))
+      xcorr  W and G in (2 Nc e) + x-pruned Wr out (R N1 h e, the R =
+             rs/2 + 1 rows x >= 0 of the r-subgrid) + weight read (s bytes a
+             cell) and FP64 read-modify-write of the k-subgrid's half with
+             kz >= 0 (K0 K1 (K2/2 + 1) * (16 + s))
       xcorr00  the ell = 0 term of an autocorrelation: G in (Nc e) + Wr out
              + k-subgrid as xcorr (its transform is a multiple of G)
-      yinv   Wr in (rs N1 h e) + Wry out (rs rs h e)
-      zinv   Wry in (rs rs h e) + r-subgrid weight read (s bytes a cell)
-             and FP64 read-modify-write (rs^3 * (16 + s))"""
+      yinv   Wr in (R N1 h e) + Wry out (R rs h e)
+      zinv   Wry in (R rs h e) + r-subgrid weight read (s bytes a cell)
+             and FP64 read-modify-write (R rs^2 * (16 + s))"""
     s = 8 if precision == "fp64" else 4
     e = 2 * s
     n0, n1, n2 = w.ngrid
     n = n0 * n1 * n2
     h = n2 // 2 + 1
     nc = n0 * n1 * h
-    kc = ks[0] * ks[1] * ks[2]
+    kc = ks[0] * ks[1] * (ks[2] // 2 + 1)
+    r = rs // 2 + 1
     table = {
         "zfwd": n * s + nc * e,
         "zfwd2": n * s + 2 * nc * e,
         "yfwd": 2 * nc * e,
-        "xcorr": 2 * nc * e + rs * n1 * h * e + kc * (16 + s),
-        "xcorr00": nc * e + rs * n1 * h * e + kc * (16 + s),
-        "yinv": rs * n1 * h * e + rs * rs * h * e,
-        "zinv": rs * rs * h * e + rs ** 3 * (16 + s),
+        "xcorr": 2 * nc * e + r * n1 * h * e + kc * (16 + s),
+        "xcorr00": nc * e + r * n1 * h * e + kc * (16 + s),
+        "yinv": r * n1 * h * e + r * rs * h * e,
+        "zinv": r * rs * h * e + r * rs * rs * (16 + s),
         "weight": n * 8 + n * s,
         "copy_pad": n * 8 + n * s,
         "conj_mul": 3 * nc * e,
