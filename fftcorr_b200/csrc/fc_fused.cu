@@ -98,8 +98,10 @@ __device__ __forceinline__ float row_weight_form(const RowPoly &r, float D,
   else if constexpr (POLY == 3) poly = (r.c[3] * z2 + r.c[1]) * z;
   else poly = (r.c[4] * z2 + r.c[2]) * z2 + r.c[0];
   const float ir2 = __fdividef(1.0f, r.rxy2 + z2 + 1e-20f);
+  // (1 / r^2 twice: its square is infinite in FP32 at the observer, r = 0,
+  // where poly is 0 and the weight must be.)
   if constexpr (ELL == 2) return D * poly * ir2;
-  else return D * poly * (ir2 * ir2);
+  else return D * poly * ir2 * ir2;
 }
 
 __device__ __forceinline__ RowPoly load_row_poly(const float4 *__restrict__ tab,
@@ -1130,10 +1132,10 @@ __device__ __forceinline__ void weigh_row_pair(const RowPoly &ra,
       auto one = [&](float d, float z, float &wa, float &wq) {
         const float z2 = z * z;
         const float ir2 = __fdividef(1.0f, ra.rxy2 + z2 + 1e-20f);
-        const float fa = EA == 2 ? ir2 : ir2 * ir2;
-        const float fq = EQ == 2 ? ir2 : ir2 * ir2;
-        wq = d * row_poly_at<PQ>(rq, z, z2) * fq;
-        wa = d * row_poly_at<PA>(ra, z, z2) * fa;
+        wq = d * row_poly_at<PQ>(rq, z, z2) * ir2;
+        wa = d * row_poly_at<PA>(ra, z, z2) * ir2;
+        if constexpr (EQ == 4) wq *= ir2;
+        if constexpr (EA == 4) wa *= ir2;
       };
 #pragma unroll
       for (int u = 0; u < 8; ++u) {

@@ -407,8 +407,9 @@ __device__ __forceinline__ T row_value(const RowCoef<T> &r, T D, T z) {
   if constexpr (sizeof(T) == 4) {
     const float ir2 = __fdividef(1.0f, r.rxy2 + z2 + 1e-20f);
     if constexpr (ELL == 2) return D * ((r.c[2] * z + r.c[1]) * z + r.c[0]) * ir2;
-    return D * ((((r.c[4] * z + r.c[3]) * z + r.c[2]) * z + r.c[1]) * z + r.c[0]) *
-           (ir2 * ir2);
+    // (1 / r^2 twice: its square is infinite in FP32 at the observer, r = 0.)
+    return D * ((((r.c[4] * z + r.c[3]) * z + r.c[2]) * z + r.c[1]) * z + r.c[0]) * ir2 *
+           ir2;
   } else {
     const double ir2 = 1.0 / (r.rxy2 + z2 + 1e-20);
     if constexpr (ELL == 2) return D * ((r.c[2] * z + r.c[1]) * z + r.c[0]) * ir2;
