@@ -469,8 +469,9 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
   const int64_t nrows = (int64_t)g.n0 * g.n1;
   const int64_t row0 = (int64_t)blockIdx.x * NR * np;
   if constexpr (ELL > 0) {
-    if ((int)threadIdx.x < NR * np) {
-      const int64_t row = min(row0 + threadIdx.x, nrows - 1);
+    // (Short rows leave the CTA with fewer threads than table entries.)
+    for (int e = threadIdx.x; e < NR * np; e += blockDim.x) {
+      const int64_t row = min(row0 + e, nrows - 1);
       const int x = (int)(row / g.n1);
       const int y = (int)(row - (int64_t)x * g.n1);
       double c[5];
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
       RowCoef<T> r;
       for (int i = 0; i < 5; ++i) r.c[i] = (T)c[i];
       r.rxy2 = (T)((x0 + x) * (x0 + x) + (y0 + y) * (y0 + y));
-      rc[threadIdx.x] = r;
+      rc[e] = r;
     }
     __syncthreads();
   }

@@ -1,5 +1,5 @@
 """Survey correlations at the edges of what they accept, against the oracle: an
-observer at the centre of a cell."""
+observer at the centre of a cell, many short rows."""
 import numpy as np
 import pytest
 
@@ -30,3 +30,12 @@ def test_observer_at_the_centre_of_a_cell(n, precision):
     """1 / r^4 overflows FP32 in that cell, whose weight is 0."""
     posmin = np.full(3, -CELL * (n // 2 + 0.5))
     _survey((n, n, n), posmin, precision, f"observer in cell {n // 2}")
+
+
+# Rows of which a CTA of the z pass takes more than it has threads (on 148 SMs
+# from about 10700 rows).
+@pytest.mark.parametrize("shape", [(128, 128, 4), (108, 108, 6), (128, 128, 5),
+                                   (128, 128, 7), (120, 90, 9)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_many_short_rows(shape, precision):
+    _survey(shape, np.array([-400.0, 250.0, -30.0]), precision, "short rows")
