@@ -459,10 +459,10 @@ struct Correlator {
   // Hand-written fused FFT passes (null: cuFFT path).
   std::unique_ptr<FusedSurvey> fused;
   // A periodic cross correlation on a geometry whose r-subgrid bins differ
-  // under inversion takes the general inverse, made with its second grid,
-  // and the bin index's cells as they are.
+  // under inversion takes the general inverse, made with its second grid, a
+  // whole r-subgrid and the bin index's cells as they are.
   std::unique_ptr<FusedSurvey> fused_cross;
-  DeviceBuffer rperm_full;
+  DeviceBuffer rsub_cross, rperm_full;
   bool bins_even = true;
   FusedSurvey *cross_passes() const {
     return fused_cross ? fused_cross.get() : fused.get();
@@ -592,13 +592,15 @@ struct Correlator {
     return sqrt((4.0 * M_PI) * (2 * ell + 1)) * (1.0 / geo.ncells() / geo.ncells());
   }
 
-  // The reductions of every histogram and the zero lag, over rcells (the r bin
-  // index's cells as rsub_l holds them; r0 the one of r = 0).
-  void hist_items(const uint32_t *rcells, std::vector<HistItem> &it,
+  // The reductions of every histogram and the zero lag, over the r-subgrids
+  // that rsub_of(row) gives and rcells, the r bin index's cells as those hold
+  // them.
+  template <typename RsubOf>
+  void hist_items(RsubOf rsub_of, const uint32_t *rcells, std::vector<HistItem> &it,
                   std::vector<FoldItem> &fo) const {
     const bool sh = shared_subgrids();
     for (int r = 0; r < geo.nrows; ++r) {
-      rbins.append_work(rsub_l[sh ? 0 : r].as<double>(), rcells,
+      rbins.append_work(rsub_of(r), rcells,
                         sh ? rweights.as<double>() + r * rbins.ninrange : nullptr, 1.0,
                         rhist_row(r), it, fo);
       kbins.append_work(ksub_l[sh ? 0 : r].as<double>(), kbins.perm.as<uint32_t>(),
@@ -607,7 +609,7 @@ struct Correlator {
     }
     const uint32_t *zero = zero_cell.as<uint32_t>();
     fo.push_back(FoldItem{(int)it.size(), 1, zerolag_out()});
-    it.push_back(HistItem{rsub_l[0].as<double>(), zero, nullptr,
+    it.push_back(HistItem{rsub_of(0), zero, nullptr,
                           sh ? make_ylm_params(0, 0, r_coeff(0)).value0 : 1.0,
                           rcells == rbins.perm.as<uint32_t>() ? 0u : 1u, 1});
   }
@@ -619,7 +621,9 @@ struct Correlator {
                               centre};
     zero_cell.resize(sizeof(zero));
     FC_CUDA(cudaMemcpy(zero_cell.get(), zero, sizeof(zero), cudaMemcpyHostToDevice));
-    hist_items(rbins.perm.as<uint32_t>(), items, folds);
+    const bool sh = shared_subgrids();
+    hist_items([&](int r) { return rsub_l[sh ? 0 : r].as<double>(); },
+               rbins.perm.as<uint32_t>(), items, folds);
     hist.upload(items, folds);
   }
 
@@ -914,20 +918,20 @@ struct Correlator {
     have_g2 = true;
   }
 
+  // Everything is made before any member changes: where an allocation fails,
+  // the correlator is what it was.
   void make_cross_passes() {
     if (kind != FC_PERIODIC || bins_even || fused_cross) return;
     std::unique_ptr<FusedSurvey> f(new FusedSurvey(geo.shape, geo.rsize, geo.kshape,
                                                    fp64(), false, true));
-    rsub_l[0].resize(geo.rcells() * sizeof(double));
+    DeviceBuffer r(geo.rcells() * sizeof(double));
     std::vector<HistItem> it;
     std::vector<FoldItem> fo;
-    hist_items(rperm_full.as<uint32_t>(), it, fo);
-    hist_cross.upload(it, fo);
-    // The r-subgrid may have moved.
-    items.clear();
-    folds.clear();
-    hist_items(rbins.perm.as<uint32_t>(), items, folds);
-    hist.upload(items, folds);
+    hist_items([&](int) { return r.as<double>(); }, rperm_full.as<uint32_t>(), it, fo);
+    HistPlan h;
+    h.upload(it, fo);
+    rsub_cross = std::move(r);
+    hist_cross = std::move(h);
     fused_cross = std::move(f);
   }
 
@@ -1002,12 +1006,14 @@ struct Correlator {
   template <typename T>
   void periodic_run(Density d, bool cross) {
     if (fused) {
-      FusedSurvey *f = cross ? cross_passes() : fused.get();
+      const bool whole = cross && fused_cross;
+      FusedSurvey *f = whole ? fused_cross.get() : fused.get();
       ProfHook hook(&prof, stream);
-      f->periodic(f->prepare_input(d.p, d.f32, stream), cross, ksub(0), rsub(0), stream,
+      f->periodic(f->prepare_input(d.p, d.f32, stream), cross, ksub(0),
+                  whole ? rsub_cross.as<double>() : rsub(0), stream,
                   prof.on ? &hook : nullptr);
       n_fft += 2;
-      reduce_hist(cross && fused_cross ? hist_cross : hist);
+      reduce_hist(whole ? hist_cross : hist);
       return;
     }
     copy_pad<T>(d, 0.0);
