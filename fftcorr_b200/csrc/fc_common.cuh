@@ -232,7 +232,13 @@ __device__ __forceinline__ void grid_dependency_wait() {
 __device__ __forceinline__ void grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// First statement of a kernel of such a chain.
+// First statement of a kernel of such a chain.  The kernel before it may still
+// be writing when this one starts, so what that one or any other kernel of the
+// chain writes is read by plain loads, through pointers without __restrict__:
+// a load by __ldg, or one that the compiler turns into it for a const
+// __restrict__ pointer, is only defined for memory that nothing writes while
+// the kernel lives, and may be moved above the wait.  Tables made with the
+// correlator may be read either way.
 __device__ __forceinline__ void grid_chain() {
   grid_launch_dependents();
   grid_dependency_wait();

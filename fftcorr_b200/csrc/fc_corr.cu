@@ -530,6 +530,8 @@ struct Correlator {
         fused->prepare_tables(2 * (geo.nrows - 1), (double)geo.ncells(),
                               d_raxis.as<double>(), kaxes(),
                               geo.kcells() > 0, stream);
+      // The tables are complete before any stream reads them.
+      FC_CUDA(cudaStreamSynchronize(stream));
     } catch (...) {
       // A failed construction leaves no stream, event or plan behind (the
       // buffers free themselves).

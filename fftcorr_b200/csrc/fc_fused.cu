@@ -104,11 +104,11 @@ __device__ __forceinline__ float row_weight_form(const RowPoly &r, float D,
   else return D * poly * ir2 * ir2;
 }
 
-__device__ __forceinline__ RowPoly load_row_poly(const float4 *__restrict__ tab,
-                                                 int64_t row,
+// (Plain loads: k_rowpoly writes the table just before, see grid_chain.)
+__device__ __forceinline__ RowPoly load_row_poly(const float4 *tab, int64_t row,
                                                  const YlmParams &p) {
-  const float4 a = __ldg(&tab[2 * row]);
-  const float4 b = __ldg(&tab[2 * row + 1]);
+  const float4 a = tab[2 * row];
+  const float4 b = tab[2 * row + 1];
   RowPoly r;
   r.c[0] = a.x;
   r.c[1] = a.y;
@@ -174,8 +174,7 @@ struct P2B {
 
 template <typename T, int L>
 __global__ void __launch_bounds__(P2<T, L>::THREADS)
-    k_yfwd_p2(C2<T> *__restrict__ W, FusedGeom g,
-              const C2<T> *__restrict__ taby) {
+    k_yfwd_p2(C2<T> *W, FusedGeom g, const C2<T> *__restrict__ taby) {
   grid_chain();
   using C = C2<T>;
   using Q = P2<T, L>;
@@ -204,8 +203,8 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
 
 template <typename T, int L>
 __global__ void __launch_bounds__(P2<T, L>::THREADS)
-    k_yinv_p2(const C2<T> *__restrict__ Wr, C2<T> *__restrict__ Wry,
-              FusedGeom g, const C2<T> *__restrict__ taby) {
+    k_yinv_p2(const C2<T> *Wr, C2<T> *Wry, FusedGeom g,
+              const C2<T> *__restrict__ taby) {
   grid_chain();
   using C = C2<T>;
   using Q = P2<T, L>;
@@ -242,8 +241,7 @@ __global__ void __launch_bounds__(P2<T, L>::THREADS)
 // may be the row's padding), or overwrites it when `first`.  A cell has one
 // source element, so nothing collides.
 template <int L, int W, typename KT, typename Re>
-__device__ __forceinline__ void to_half_k(double *__restrict__ ksub,
-                                          const KT *__restrict__ ktab,
+__device__ __forceinline__ void to_half_k(double *ksub, const KT *__restrict__ ktab,
                                           const FusedGeom &g, int t, int jr, int kz,
                                           bool first, Re re) {
   constexpr int TPC = L / 8;
@@ -306,8 +304,7 @@ __device__ __forceinline__ void split_pair(const C &z, const C &m, C *a, C *b) {
 // leave.
 template <int L, int MODE, bool EVEN>
 __global__ void __launch_bounds__(P2<double, L>::THREADS)
-    k_xcorr_p2(const double2 *__restrict__ W, const double2 *__restrict__ G,
-               double2 *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
+    k_xcorr_p2(const double2 *W, const double2 *G, double2 *out, double *ksub, FusedGeom g,
                const double2 *__restrict__ tabx, const double *__restrict__ ktab,
                double w00, int first) {
   grid_chain();
@@ -412,7 +409,7 @@ __global__ void __launch_bounds__(P2<double, L>::THREADS)
 // the pass took 108 us at 256^3 against 66, bound by FP64 instructions.
 template <int L, bool WEIGHT>
 __global__ void __launch_bounds__(P2<double, L>::THREADS)
-    k_zfwd_p2(const double *__restrict__ rho, double2 *__restrict__ W, FusedGeom g,
+    k_zfwd_p2(const double *rho, double2 *W, FusedGeom g,
               YlmParams p, double x0, double y0, double z0,
               const double2 *__restrict__ tabz) {
   grid_chain();
@@ -489,8 +486,8 @@ __global__ void __launch_bounds__(P2<double, L>::THREADS)
 
 template <typename T, int L>
 __global__ void __launch_bounds__(P2<T, L>::THREADS)
-    k_zinv_p2(const C2<T> *__restrict__ Wry, double *__restrict__ rsub,
-              FusedGeom g, const C2<T> *__restrict__ tabz,
+    k_zinv_p2(const C2<T> *Wry, double *rsub, FusedGeom g,
+              const C2<T> *__restrict__ tabz,
               const T *__restrict__ rtab, int first) {
   grid_chain();
   using C = C2<T>;
@@ -679,8 +676,7 @@ __device__ __forceinline__ bool split_cta(int nyq) {
 }
 
 template <int L, bool SPLIT>
-__device__ __forceinline__ void yfwd_pp_body(float2 *__restrict__ W,
-                                             const FusedGeom &g,
+__device__ __forceinline__ void yfwd_pp_body(float2 *W, const FusedGeom &g,
                                              const float2 *__restrict__ taby) {
   using Q = PY<L>;
   extern __shared__ unsigned char smem_raw[];
@@ -702,8 +698,7 @@ __device__ __forceinline__ void yfwd_pp_body(float2 *__restrict__ W,
 
 template <int L>
 __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
-    k_yfwd_pp(float2 *__restrict__ W, FusedGeom g,
-              const float2 *__restrict__ taby) {
+    k_yfwd_pp(float2 *W, FusedGeom g, const float2 *__restrict__ taby) {
   grid_chain();
   // (Splitting off the last column measured slower here: 194 vs 183 us.)
   yfwd_pp_body<L, false>(W, g, taby);
@@ -712,8 +707,7 @@ __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
 // grid2's x transform in the FP32 form: G = DFT_x(W), the same column
 // pairing as the y passes, with rows N1 * hp elements apart.
 template <int L, bool SPLIT>
-__device__ __forceinline__ void xfwd_pp_body(const float2 *__restrict__ W,
-                                             float2 *__restrict__ G,
+__device__ __forceinline__ void xfwd_pp_body(const float2 *W, float2 *G,
                                              const FusedGeom &g,
                                              const float2 *__restrict__ tabx) {
   using Q = PY<L>;
@@ -737,7 +731,7 @@ __device__ __forceinline__ void xfwd_pp_body(const float2 *__restrict__ W,
 
 template <int L>
 __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
-    k_xfwd_pp(const float2 *__restrict__ W, float2 *__restrict__ G, FusedGeom g,
+    k_xfwd_pp(const float2 *W, float2 *G, FusedGeom g,
               const float2 *__restrict__ tabx) {
   grid_chain();
   xfwd_pp_body<L, false>(W, G, g, tabx);
@@ -757,8 +751,7 @@ constexpr int kXB = 16;  // columns per CTA of the FP32 x passes
 
 template <int L, int MODE, bool SPLIT, bool EVEN>
 __device__ __forceinline__ void xcorr_pp_body(
-    const float2 *__restrict__ W, const float2 *__restrict__ G,
-    float2 *__restrict__ out, double *__restrict__ ksub, const FusedGeom &g,
+    const float2 *W, const float2 *G, float2 *out, double *ksub, const FusedGeom &g,
     const float2 *__restrict__ tabx, const float *__restrict__ ktab, float w00,
     int first) {
   using Q = PY<L, kXB>;
@@ -895,8 +888,7 @@ __device__ __forceinline__ void xcorr_pp_body(
 
 template <int L, int MODE, bool EVEN>
 __global__ void __launch_bounds__(PY<L, kXB>::THREADS, 1024 / PY<L, kXB>::THREADS)
-    k_xcorr_pp(const float2 *__restrict__ W, const float2 *__restrict__ G,
-               float2 *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
+    k_xcorr_pp(const float2 *W, const float2 *G, float2 *out, double *ksub, FusedGeom g,
                const float2 *__restrict__ tabx, const float *__restrict__ ktab,
                float w00, int nyq, int first) {
   grid_chain();
@@ -912,8 +904,7 @@ __global__ void __launch_bounds__(PY<L, kXB>::THREADS, 1024 / PY<L, kXB>::THREAD
 }
 
 template <int L, bool SPLIT>
-__device__ __forceinline__ void yinv_pp_body(const float2 *__restrict__ Wr,
-                                             float2 *__restrict__ Wry,
+__device__ __forceinline__ void yinv_pp_body(const float2 *Wr, float2 *Wry,
                                              const FusedGeom &g,
                                              const float2 *__restrict__ taby) {
   using Q = PY<L>;
@@ -953,8 +944,8 @@ __device__ __forceinline__ void yinv_pp_body(const float2 *__restrict__ Wr,
 
 template <int L>
 __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
-    k_yinv_pp(const float2 *__restrict__ Wr, float2 *__restrict__ Wry,
-              FusedGeom g, const float2 *__restrict__ taby, int nyq) {
+    k_yinv_pp(const float2 *Wr, float2 *Wry, FusedGeom g,
+              const float2 *__restrict__ taby, int nyq) {
   grid_chain();
   if (split_cta(nyq))
     yinv_pp_body<L, true>(Wr, Wry, g, taby);
@@ -966,10 +957,9 @@ __global__ void __launch_bounds__(PY<L>::THREADS, 1024 / PY<L>::THREADS)
 // CTA's B, thread t of a row pair holding z[t + TPC u] of both.
 template <int L, bool WEIGHT>
 __global__ void __launch_bounds__(PP<L>::THREADS)
-    k_zfwd_pp(const float *__restrict__ rho, float2 *__restrict__ W, FusedGeom g,
+    k_zfwd_pp(const float *rho, float2 *W, FusedGeom g,
               YlmParams p, double x0, double y0, double z0,
-              const float2 *__restrict__ tabz,
-              const float4 *__restrict__ rowtab) {
+              const float2 *__restrict__ tabz, const float4 *rowtab) {
   grid_chain();
   using Q = PP<L>;
   constexpr int RP = L + L / 8 + 1;
@@ -1155,11 +1145,10 @@ __device__ __forceinline__ void weigh_row_pair(const RowPoly &ra,
 // split are those of k_zfwd_pp.
 template <int L>
 __global__ void __launch_bounds__(PP<L>::THREADS, 1024 / PP<L>::THREADS)
-    k_zfwd_pp2(const float *__restrict__ rho, float2 *__restrict__ Wa,
-               float2 *__restrict__ Wb, FusedGeom g, YlmParams pa, YlmParams pq,
+    k_zfwd_pp2(const float *rho, float2 *Wa, float2 *Wb, FusedGeom g, YlmParams pa,
+               YlmParams pq,
                double z0, const float2 *__restrict__ tabz,
-               const float4 *__restrict__ rowtab_a,
-               const float4 *__restrict__ rowtab_b) {
+               const float4 *rowtab_a, const float4 *rowtab_b) {
   grid_chain();
   using Q = PP<L>;
   constexpr int RP = L + L / 8 + 1;
@@ -1217,7 +1206,7 @@ __global__ void __launch_bounds__(PP<L>::THREADS, 1024 / PP<L>::THREADS)
 
 // Per-row Horner coefficients of one (ell, m) (row_poly), two float4 per
 // row, so the z pass does no FP64 work per row.
-__global__ void k_rowpoly(float4 *__restrict__ tab, int64_t nrows, int n1,
+__global__ void k_rowpoly(float4 *tab, int64_t nrows, int n1,
                           YlmParams p, double x0, double y0) {
   grid_chain();
   for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

@@ -106,7 +106,7 @@ __device__ __forceinline__ void col_pass(const GPass &ps, const Tw *__restrict__
 // The first pass, read from device memory (columns at and above nb are
 // zero), into dst.
 template <int SIGN, int B, typename T>
-__device__ __forceinline__ void col_first(const GPass &ps, const C2<T> *__restrict__ src,
+__device__ __forceinline__ void col_first(const GPass &ps, const C2<T> *src,
                                           int64_t stride, int nb,
                                           typename GElem<T>::E *dst) {
   using GE = GElem<T>;
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kYThreads, sizeof(T) == 4 ? 2 : 1)
 
 template <typename T, int B>
 __global__ void __launch_bounds__(kYThreads, sizeof(T) == 4 ? 2 : 1)
-    k_gyinv(const C2<T> *__restrict__ Wr, C2<T> *__restrict__ Wry, FusedGeom g,
+    k_gyinv(const C2<T> *Wr, C2<T> *Wry, FusedGeom g,
             const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw) {
   grid_chain();
   using GE = GElem<T>;
@@ -266,8 +266,7 @@ __device__ __forceinline__ void split_elem(double2 *p, const double2 &z, const d
 // (fc_fused.h), two real columns to a complex one.
 template <typename T, int B, int MODE, bool EVEN>
 __global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
-    k_gx(const C2<T> *__restrict__ W, const C2<T> *__restrict__ G,
-         C2<T> *__restrict__ out, double *__restrict__ ksub, FusedGeom g,
+    k_gx(const C2<T> *W, const C2<T> *G, C2<T> *out, double *ksub, FusedGeom g,
          const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw,
          const T *__restrict__ ktab, T w00, int first) {
   grid_chain();
@@ -454,7 +453,7 @@ __device__ __forceinline__ double &comp(double2 &v, int c) { return c ? v.y : v.
 // of 2 W rows.
 template <typename T, int ELL>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
-    k_gzfwd(const T *__restrict__ rho, C2<T> *__restrict__ W, FusedGeom g,
+    k_gzfwd(const T *rho, C2<T> *W, FusedGeom g,
             const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw, int np,
             YlmParams p, double x0, double y0, double z0) {
   grid_chain();
@@ -551,7 +550,7 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
 // Pairs of rows of Wry to real rows, accumulated into the r-subgrid.
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
-    k_gzinv(const C2<T> *__restrict__ Wry, double *__restrict__ rsub, FusedGeom g,
+    k_gzinv(const C2<T> *Wry, double *rsub, FusedGeom g,
             const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw, int np,
             const T *__restrict__ rtab, int first) {
   grid_chain();

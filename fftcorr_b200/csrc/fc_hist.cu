@@ -67,8 +67,7 @@ __global__ void k_bin_fold(const double *partials, const int *chunk_first,
 // Persistent chunk reductions over the work items of any number of
 // histograms.
 __global__ void __launch_bounds__(kHistThreads)
-    k_hist_items(const HistItem *__restrict__ items, int n,
-                 double *__restrict__ partials) {
+    k_hist_items(const HistItem *__restrict__ items, int n, double *partials) {
   grid_chain();
   __shared__ double red[32];
   for (int it = blockIdx.x; it < n; it += gridDim.x) {
@@ -88,7 +87,7 @@ __global__ void __launch_bounds__(kHistThreads)
 
 // One thread per bin: its chunk partials folded in order.
 __global__ void k_hist_folds(const FoldItem *__restrict__ folds, int n,
-                             const double *__restrict__ partials) {
+                             const double *partials) {
   grid_chain();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += gridDim.x * blockDim.x) {
