@@ -57,6 +57,10 @@ constexpr uint32_t kWarpUnit = 32;
 // catalog then has 32 or fewer in a tenth of its units) every unit goes to a
 // CTA, and the warps' launches, 2 us a colour pass, are left out.
 constexpr int64_t kDenseUnit = 40;
+// With more than this the CTAs take their dense form (ScatterP::min_blocks; at
+// 48 a unit, 50M of a sector in 512^3, it takes 3.57 ms against 3.41), except
+// in a batch, whose boxes fill one another's waits (12 boxes 10.4 -> 10.6 ms).
+constexpr int64_t kDenseForm = 100;
 constexpr int kScatterThreads = 256;
 constexpr int kChunk = 256;      // particles staged per shared-memory chunk
 
@@ -477,10 +481,16 @@ struct ScatterP {
   static constexpr int W = Stencil<S>::W;
   static constexpr int W3 = W * W * W;
   static constexpr int THREADS = TX * 64;
-  // CTAs per SM: TSC's table and its 27 sums a thread leave room for five,
-  // the narrower stencils for eight (8M clustered points, CIC, 384^3 1.61 ->
-  // 1.51 ms; a batch of 12 boxes 11.1 -> 10.7 ms).
-  static constexpr int MIN_BLOCKS = TX == 2 ? (W == 3 ? 5 : 8) : kTile / TX;
+  // CTAs per SM.  TSC's table and its 27 sums a thread leave room for five.
+  // The narrower stencils' units of some dozens of particles are bound by
+  // latency and take eight (8M clustered points, CIC, 384^3, five: 1.62 ms,
+  // six: 1.59, eight: 1.51; a batch of 12 boxes 11.1 -> 10.7 ms); those of
+  // dense catalogs by the sums, which at eight spill (7.6M clustered points,
+  // CIC, 98^3: 1.27, 1.30 and 1.33 ms; 33M of a sector in 225^3: 1.98, 1.93,
+  // 2.04 ms; 300k in 64^3: 0.233, 0.235, 0.247 ms).
+  static constexpr int min_blocks(bool dense) {
+    return TX != 2 ? kTile / TX : W == 3 || dense ? 5 : 8;
+  }
   static constexpr int FX = TX + W - 1;     // footprint extent along x
   static constexpr int FY = kTile + W - 1;  // ... along y and z
   static constexpr int F3 = FX * FY * FY;
@@ -517,8 +527,8 @@ __device__ __forceinline__ size_t foot_cell(int fx, int fy, int fz, int o0,
 // (zero before the pass).
 // GT is the grid's cell type: each footprint cell's FP64 sum for the unit is
 // added to the cell in FP64 and rounded to GT once.
-template <int S, typename KeyT, int TX, typename GT>
-__global__ void __launch_bounds__(TX * 64, ScatterP<S, TX>::MIN_BLOCKS)
+template <int S, typename KeyT, int TX, typename GT, bool DENSE>
+__global__ void __launch_bounds__(TX * 64, (ScatterP<S, TX>::min_blocks(DENSE)))
     k_scatter_p(const double *__restrict__ posw, const KeyT *__restrict__ keys,
                 const uint32_t *__restrict__ vals,
                 const uint4 *__restrict__ ranges_end,
@@ -1008,27 +1018,26 @@ int stencil_width(int scheme, int *omin) {
   }
 }
 
-// Scatter kernels for scheme 0, 1 or 3, a key type and a cell type.
+// Scatter kernels for scheme 0, 1 or 3, a key type and a cell type; cta[1] is
+// the form for dense catalogs.
 struct ScatterFns {
-  const void *cta = nullptr, *warp = nullptr;
+  const void *cta[2] = {nullptr, nullptr}, *warp = nullptr;
   size_t smem = 0, warp_smem = 0;  // of their CTAs
 };
+template <int S, typename KeyT, typename GT>
+ScatterFns scatter_fns_of() {
+  // (TSC's two forms would be the same.)
+  return ScatterFns{{(const void *)k_scatter_p<S, KeyT, kUnitX, GT, false>,
+                     (const void *)k_scatter_p<S, KeyT, kUnitX, GT, S != 1>},
+                    (const void *)k_scatter_w<S, KeyT, GT>, ScatterP<S, kUnitX>::smem,
+                    kWarpsPerCta * ScatterW<S>::DOUBLES * sizeof(double)};
+}
 template <typename KeyT, typename GT>
 ScatterFns scatter_fns(int scheme) {
-  auto of = [](auto cta, auto warp, size_t smem, int doubles) {
-    return ScatterFns{(const void *)cta, (const void *)warp, smem,
-                      kWarpsPerCta * doubles * sizeof(double)};
-  };
   switch (scheme) {
-    case 0:
-      return of(k_scatter_p<0, KeyT, kUnitX, GT>, k_scatter_w<0, KeyT, GT>,
-                ScatterP<0, kUnitX>::smem, ScatterW<0>::DOUBLES);
-    case 1:
-      return of(k_scatter_p<1, KeyT, kUnitX, GT>, k_scatter_w<1, KeyT, GT>,
-                ScatterP<1, kUnitX>::smem, ScatterW<1>::DOUBLES);
-    default:
-      return of(k_scatter_p<3, KeyT, kUnitX, GT>, k_scatter_w<3, KeyT, GT>,
-                ScatterP<3, kUnitX>::smem, ScatterW<3>::DOUBLES);
+    case 0: return scatter_fns_of<0, KeyT, GT>();
+    case 1: return scatter_fns_of<1, KeyT, GT>();
+    default: return scatter_fns_of<3, KeyT, GT>();
   }
 }
 
@@ -1063,7 +1072,7 @@ struct Assignor {
                                        // units drawn, the CTAs' units
   std::vector<int64_t> color_offsets;  // per colour, into color_units
   ScatterFns scatter;                  // for this scheme, keys and cells
-  unsigned scatter_ctas = 0, scatter_w_ctas = 0;  // persistent CTAs of each
+  unsigned scatter_ctas[2] = {0, 0}, scatter_w_ctas = 0;  // persistent CTAs of each
   DeviceBuffer partials;               // K-key block partials
   DeviceBuffer totals;                 // [totw, totwsq]
   DeviceBuffer counts;                 // [num_added]
@@ -1120,13 +1129,15 @@ struct Assignor {
       else
         scatter = grid->fp32() ? scatter_fns<uint32_t, float>(scheme)
                                : scatter_fns<uint32_t, double>(scheme);
-      FC_CUDA(cudaFuncSetAttribute(scatter.cta,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)scatter.smem));
       int per_sm = 0;
-      FC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, scatter.cta, unit_x * 64, scatter.smem));
-      scatter_ctas = (unsigned)std::max(1, per_sm) * (unsigned)sm_count();
+      for (int d = 0; d < 2; ++d) {
+        FC_CUDA(cudaFuncSetAttribute(scatter.cta[d],
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)scatter.smem));
+        FC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, scatter.cta[d], unit_x * 64, scatter.smem));
+        scatter_ctas[d] = (unsigned)std::max(1, per_sm) * (unsigned)sm_count();
+      }
       FC_CUDA(cudaFuncSetAttribute(scatter.warp,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)scatter.warp_smem));
@@ -1485,6 +1496,7 @@ struct Assignor {
     cudaStream_t st = stream();
     if (!graph_mode) window_timer.start(st);
     const uint32_t warp_unit = n > kDenseUnit * nunits ? 0u : kWarpUnit;
+    const bool dense = !graph_mode && n > kDenseForm * nunits;
     const int unit_cells = unit_x * kTile * kTile;
     k_unit_starts<KeyT><<<grid_for(nunits + 1, 256), 256, 0, st>>>(
         sk, n, nunits, unit_cells, unit_start.as<uint32_t>());
@@ -1511,8 +1523,8 @@ struct Assignor {
       void *cta_args[] = {(void *)&pw,  (void *)&sk,  (void *)&sv, (void *)&cre,
                           (void *)&cnt, (void *)&nxt, (void *)&ga, (void *)&gp};
       if (n > warp_unit) {
-        FC_CUDA(cudaLaunchKernel(scatter.cta,
-                                 dim3((unsigned)std::min<int64_t>(nu, scatter_ctas)),
+        FC_CUDA(cudaLaunchKernel(scatter.cta[dense],
+                                 dim3((unsigned)std::min<int64_t>(nu, scatter_ctas[dense])),
                                  dim3(unit_x * 64), cta_args, scatter.smem, st));
         FC_LAUNCH_CHECK();
       }
