@@ -311,6 +311,15 @@ __device__ __forceinline__ void r8_twiddle(C *v, int k, int step,
   v[7] = cmul(v[7], cmul(w3, w4));
 }
 
+// The same with all seven twiddles from the table, each rounded once: the
+// product of two FP32 entries is off by three roundings.
+template <typename C, typename Tw>
+__device__ __forceinline__ void r8_twiddle_table(C *v, int k, int step,
+                                                 const Tw *__restrict__ tab, int sign) {
+#pragma unroll
+  for (int q = 1; q < 8; ++q) v[q] = cmul(v[q], tw_load(tab, q * k * step, sign));
+}
+
 // Outputs 0 and 7 of Dft<8> only (into v[0] and v[7]), by the same
 // operations, for transforms whose later use reads only the first and the
 // last TPC rows.
@@ -407,7 +416,11 @@ __device__ __forceinline__ void reg_fft(C *v, int t, Ex ex, Rd rd,
   for (int p = 0; p < P8; ++p) {
     if (p + 1 == P8) before_last();
     const int k = t & (Ns - 1);
-    if (Ns > 1) r8_twiddle(v, k, (L / (8 * Ns)) * tab_scale, tab, sign);
+    if (Ns > 1) {
+      // (Rows of 32 keep the table's accuracy, as the mixed-radix passes do.)
+      if constexpr (L == 32) r8_twiddle_table(v, k, (L / (8 * Ns)) * tab_scale, tab, sign);
+      else r8_twiddle(v, k, (L / (8 * Ns)) * tab_scale, tab, sign);
+    }
     if (p + 1 == P8 && edges_only)
       dft8_edges(v, sign);
     else
