@@ -399,7 +399,13 @@ struct RowCoef {
   T c[5], rxy2;
 };
 
-// Y_lm D of a cell at z: D (c0 + c1 z + .. + c4 z^4) / r^ell.
+// Y_lm D of a cell at z: D (c0 + c1 z + .. + c4 z^4) / r^ell.  In FP32 1 / r^2
+// is __fdividef's, off by 2 units in the last place at most, and z is rounded
+// once (RowZ).  Error against 64 bits (2-norm, mean of 6 fields) of 125 x 180 x
+// 126 surveys at ell <= 4: cross xi 8.6e-8 and P 8.1e-8 (rounded divide: 7.3e-8
+// and 7.7e-8; z rounded twice: 9.3e-8 and 8.7e-8; the passes with a rounded divide
+// before these: 1.16e-7 and 9.3e-8), auto xi 7.2e-8 (6.7e-8; 7.3e-8; 8.0e-8).
+// The rounded divide costs 250 x 360 x 378 cross correlations 5.06 -> 5.27 ms.
 template <typename T, int ELL>
 __device__ __forceinline__ T row_value(const RowCoef<T> &r, T D, T z) {
   const T z2 = z * z;
@@ -416,6 +422,27 @@ __device__ __forceinline__ T row_value(const RowCoef<T> &r, T D, T z) {
            ir2 * ir2;
   }
 }
+
+// z of the cell i of a row, z0 + i rounded to T once.
+template <typename T>
+struct RowZ;
+template <>
+struct RowZ<double> {
+  double z0;
+  __device__ explicit RowZ(double z) : z0(z) {}
+  __device__ double at(int i) const { return z0 + i; }
+};
+// FP32: Knuth's two-sum of the upper half and i, so that no cell converts from
+// FP64.
+template <>
+struct RowZ<float> {
+  float hi, lo;
+  __device__ explicit RowZ(double z) : hi((float)z), lo((float)(z - (double)(float)z)) {}
+  __device__ float at(int i) const {
+    const float x = (float)i, s = hi + x, b = s - hi;
+    return s + (((hi - (s - b)) + (x - b)) + lo);
+  }
+};
 
 // Shared index of element i of a row: one pad element in 8 spreads the
 // strided accesses over the banks.
@@ -483,6 +510,7 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
     __syncthreads();
   }
   const GPass &f = plan.p[0];
+  const RowZ<T> zs(z0);
   with_radix(f.R, [&]<int R>() {
     for (int bf = threadIdx.x; bf < f.LR * np; bf += blockDim.x) {
       const int b = gdiv(bf, f.LR, f.mLR);
@@ -503,13 +531,15 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
           v[q].y = v[q].y * (T)p.value0;
         }
       } else if constexpr (ELL > 0) {
-        const T zj = (T)(z0 + j);
+        T z[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) z[q] = zs.at(j + q * f.LR);
 #pragma unroll
         for (int c = 0; c < NR; ++c) {
           const RowCoef<T> a = rc[NR * b + c];
 #pragma unroll
           for (int q = 0; q < R; ++q)
-            comp(v[q], c) = row_value<T, ELL>(a, comp(v[q], c), zj + (T)(q * f.LR));
+            comp(v[q], c) = row_value<T, ELL>(a, comp(v[q], c), z[q]);
         }
       }
       GDft<R, -1, E>::run(v);
