@@ -1076,8 +1076,8 @@ struct Correlator {
     const size_t ncells = geo.ncells();
     const int maxell = 2 * (geo.nrows - 1);
     if (fused) {
-      const void *in = prepared ? fused->input(d.p, d.f32)
-                                : fused->prepare_input(d.p, d.f32, stream);
+      const FusedSurvey::Cells in = prepared ? fused->input(d.p, d.f32)
+                                             : fused->prepare_input(d.p, d.f32, stream);
       ProfHook hook(&prof, stream);
       PhaseHook *ph = prof.on ? &hook : nullptr;
       const KAxes ka = kaxes();

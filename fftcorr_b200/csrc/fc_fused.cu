@@ -1273,6 +1273,23 @@ __global__ void k_ktable(KT *__restrict__ tab, FusedGeom g, KAxes ax, YlmParams 
   }
 }
 
+// One term's unweighted k- and r-subgrids times their weights and `scale`,
+// added to the multipole's subgrids or (first) written over them.
+__global__ void k_add_term(double *ksub, double *rsub, const double *kterm,
+                           const double *rterm, const double *__restrict__ ktab,
+                           const double *__restrict__ rtab, size_t nk, size_t nr,
+                           double scale, int first) {
+  grid_chain();
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nk + nr;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const bool k = i < nk;
+    const size_t c = k ? i : i - nk;
+    double *dst = k ? ksub : rsub;
+    const double v = k ? ktab[c] * (scale * kterm[c]) : rtab[c] * (scale * rterm[c]);
+    dst[c] = first ? v : dst[c] + v;
+  }
+}
+
 __global__ void k_to_float(const double *__restrict__ in, float *__restrict__ out,
                            size_t n, double shift) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
@@ -1398,7 +1415,11 @@ FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
   if (survey) G.resize(nc * eb);
   Wr.resize((size_t)g.nri * g.n1 * g.hp * eb);
   Wry.resize((size_t)g.nri * g.rs * g.hp * eb);
-  if (!fp64) {
+  if (survey && wide()) {
+    kterm.resize(k_cells() * sizeof(double));
+    rterm.resize(r_cells() * sizeof(double));
+  }
+  if (!fp64 && !wide()) {
     rho32.resize((size_t)g.n0 * g.n1 * g.n2 * sizeof(float));
     if (survey) rowtab.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
     if (survey && pairs()) {
@@ -1426,22 +1447,23 @@ void FusedSurvey::set_smem_limits() {
   }
 }
 
-const void *FusedSurvey::prepare_input(const void *rho, bool f32,
-                                       cudaStream_t s) {
+FusedSurvey::Cells FusedSurvey::prepare_input(const void *rho, bool f32,
+                                              cudaStream_t s) {
   FC_REQUIRE(!(fp64_ && f32), FC_ERR_INVALID,
              "the FP64 passes take FP64 cells");
-  if (fp64_ || f32) return rho;
+  if (reads_as_is(f32)) return {rho, f32};
   const size_t n = (size_t)g.n0 * g.n1 * g.n2;
   k_to_float<<<grid_for(n, 256), 256, 0, s>>>(static_cast<const double *>(rho),
                                               rho32.as<float>(), n, 0.0);
   FC_LAUNCH_CHECK();
-  return rho32.get();
+  return {rho32.get(), true};
 }
 
 template <typename T>
-void FusedSurvey::zfwd(const void *rho, bool weight, const YlmParams &p,
-                       const double xyz0[3], cudaStream_t s) {
+void FusedSurvey::zfwd(Cells in, bool weight, const YlmParams &p, const double xyz0[3],
+                       cudaStream_t s) {
   if (p2_rows()) {
+    const void *rho = in.p;
     with_p2(g.m, [&]<int L>() {
       using Q = P2<T, L>;
       const int64_t nrows = (int64_t)g.n0 * g.n1;
@@ -1479,7 +1501,7 @@ void FusedSurvey::zfwd(const void *rho, bool weight, const YlmParams &p,
     FC_LAUNCH_CHECK();
     return;
   }
-  gen_zfwd<T>(gz, g, (const T *)rho, W.as<C2<T>>(), weight, p, xyz0, s);
+  gen_zfwd<T>(gz, g, in.p, in.f32, W.as<C2<T>>(), weight, p, xyz0, s);
 }
 
 template <typename T>
@@ -1612,9 +1634,9 @@ const void *FusedSurvey::r_table(int ell, int m, const double *raxis,
   if (it != rtabs.end()) return it->second.get();
   const size_t n = (size_t)g.nri * g.rs * g.rs;
   DeviceBuffer &b = rtabs[key];
-  // FP64 for the FP64 form, FP32 for the FP32-mixed form (the product with
-  // the transform and the accumulation stay FP64).
-  if (fp64_) {
+  // FP64 for the FP64 form and wide rows, else FP32 (the product with the
+  // transform and the accumulation stay FP64).
+  if (fp64_ || wide()) {
     b.resize(std::max<size_t>(n, 1) * sizeof(double));
     k_rtable<double><<<grid_for(n, 256), 256, 0, s>>>(b.as<double>(), g, raxis, pr);
   } else {
@@ -1642,9 +1664,9 @@ const void *FusedSurvey::k_table(int ell, int m, const KAxes &ka,
   const size_t n = k_cells();
   DeviceBuffer &b = ktabs[key];
   const YlmParams pk = make_ylm_params(ell, m, 4.0 * M_PI);
-  // FP64 weights for the FP64 form; the FP32 form keeps them in FP32 (a
-  // relative rounding of 6e-8, far inside its precision).
-  if (fp64_) {
+  // FP64 weights for the FP64 form and wide rows; the others keep them in FP32
+  // (a relative rounding of 6e-8, far inside their precision).
+  if (fp64_ || wide()) {
     b.resize(std::max<size_t>(n, 1) * sizeof(double));
     k_ktable<double><<<grid_for(n, 256), 256, 0, s>>>(
         b.as<double>(), g, ka, pk);
@@ -1657,17 +1679,17 @@ const void *FusedSurvey::k_table(int ell, int m, const KAxes &ka,
   return b.get();
 }
 
-void FusedSurvey::grid2(const void *rho_in, cudaStream_t s, const KAxes &ka) {
+void FusedSurvey::grid2(Cells in, cudaStream_t s, const KAxes &ka) {
   (void)ka;
   G.resize(W.bytes());
   YlmParams none = make_ylm_params(0, 0, 1.0);
   const double zero[3] = {0, 0, 0};
   if (fp64_) {
-    zfwd<double>(rho_in, false, none, zero, s);
+    zfwd<double>(in, false, none, zero, s);
     yfwd<double>(s);
     grid2_x<double>(s);
   } else {
-    zfwd<float>(rho_in, false, none, zero, s);
+    zfwd<float>(in, false, none, zero, s);
     yfwd<float>(s);
     grid2_x<float>(s);
   }
@@ -1678,7 +1700,7 @@ bool FusedSurvey::p2_rows() const {
 }
 bool FusedSurvey::pairs() const { return !fp64_ && p2_rows(); }
 
-void FusedSurvey::zfwd_pair(const void *rho_in, int ell_a, int m_a, int ell_b,
+void FusedSurvey::zfwd_pair(Cells in, int ell_a, int m_a, int ell_b,
                             int m_b, const double xyz0[3], cudaStream_t s,
                             PhaseHook *hook) {
   FC_REQUIRE(pairs() && ell_a > 0 && ell_b > 0, FC_ERR_STATE,
@@ -1697,7 +1719,7 @@ void FusedSurvey::zfwd_pair(const void *rho_in, int ell_a, int m_a, int ell_b,
     using PQ = PP<L>;
     const unsigned blocks = (unsigned)((nrows + PQ::PB - 1) / PQ::PB);
     launch_after(k_zfwd_pp2<L>, blocks, PQ::THREADS, p2_row_smem<float, L>(), s, 
-        static_cast<const float *>(rho_in), W.as<float2>(), W2.as<float2>(), g,
+        static_cast<const float *>(in.p), W.as<float2>(), W2.as<float2>(), g,
         pa, pb, xyz0[2], tabz.as<float2>(), rowtab.as<float4>(),
         rowtab2.as<float4>());
   });
@@ -1705,7 +1727,7 @@ void FusedSurvey::zfwd_pair(const void *rho_in, int ell_a, int m_a, int ell_b,
   if (hook) hook->end();
 }
 
-int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
+int FusedSurvey::term(Cells in, int ell, int m, const double xyz0[3],
                        double ncells, double *ksub, double *rsub,
                        const double *raxis, const KAxes &ka, cudaStream_t s,
                        PhaseHook *hook, bool first, bool g_of_input, bool z_done) {
@@ -1714,32 +1736,47 @@ int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
   const void *ktab = ksub ? k_table(ell, m, ka, s) : nullptr;
   const void *rtab = r_table(ell, m, raxis, pr, s);
   const bool from_g = ell == 0 && g_of_input;
+  // Wide rows: the passes leave the term's subgrids unweighted, and
+  // k_add_term weights them in FP64 (the constant of from_g among it).
+  const bool w = wide();
+  double *kdst = w && ksub ? kterm.as<double>() : ksub;
+  double *rdst = w ? rterm.as<double>() : rsub;
+  const void *kw = w ? nullptr : ktab, *rw = w ? nullptr : rtab;
+  const bool over = w || first;
   auto run = [&](auto tag) {
     using T = decltype(tag);
     if (from_g) {
       // The weight is the constant pw.value0, so the term's transform is
       // value0 * G (see k_xcorr_p2, MODE 2).
       if (hook) hook->begin("xcorr00");
-      xcorr<T>(2, ksub, ktab, pw.value0, first, s);
+      xcorr<T>(2, kdst, kw, w ? 1.0 : pw.value0, over, s);
       if (hook) hook->end();
     } else {
       if (!z_done) {
         if (hook) hook->begin("zfwd");
-        zfwd<T>(rho_in, true, pw, xyz0, s);
+        zfwd<T>(in, true, pw, xyz0, s);
         if (hook) hook->end();
       }
       if (hook) hook->begin("yfwd");
       yfwd<T>(s);
       if (hook) hook->end();
       if (hook) hook->begin("xcorr");
-      xcorr<T>(1, ksub, ktab, 0.0, first, s);
+      xcorr<T>(1, kdst, kw, 0.0, over, s);
       if (hook) hook->end();
     }
     if (hook) hook->begin("yinv");
     yinv<T>(s);
     if (hook) hook->end();
     if (hook) hook->begin("zinv");
-    zinv<T>(rsub, rtab, first, s);
+    zinv<T>(rdst, rw, over, s);
+    if (w) {
+      const size_t nk = ksub ? k_cells() : 0, nr = r_cells();
+      launch_small(k_add_term, grid_for(nk + nr, 256), 256, 0, s, ksub, rsub,
+                   kterm.as<double>(), rterm.as<double>(),
+                   static_cast<const double *>(ktab), static_cast<const double *>(rtab),
+                   nk, nr, from_g ? pw.value0 : 1.0, first);
+      FC_LAUNCH_CHECK();
+    }
     if (hook) hook->end();
   };
   if (fp64_)
@@ -1749,7 +1786,7 @@ int FusedSurvey::term(const void *rho_in, int ell, int m, const double xyz0[3],
   return from_g ? 1 : 2;
 }
 
-void FusedSurvey::periodic(const void *rho_in, bool cross, double *ksub, double *rsub,
+void FusedSurvey::periodic(Cells in, bool cross, double *ksub, double *rsub,
                            cudaStream_t s, PhaseHook *hook) {
   const YlmParams none = make_ylm_params(0, 0, 1.0);
   const double zero[3] = {0, 0, 0};
@@ -1760,7 +1797,7 @@ void FusedSurvey::periodic(const void *rho_in, bool cross, double *ksub, double 
   };
   auto run = [&](auto tag) {
     using T = decltype(tag);
-    phase("zfwd", [&] { zfwd<T>(rho_in, false, none, zero, s); });
+    phase("zfwd", [&] { zfwd<T>(in, false, none, zero, s); });
     phase("yfwd", [&] { yfwd<T>(s); });
     phase("xcorr", [&] { xcorr<T>(cross ? 1 : 3, ksub, nullptr, 0.0, true, s); });
     phase("yinv", [&] { yinv<T>(s); });

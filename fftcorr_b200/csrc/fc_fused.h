@@ -43,17 +43,21 @@ class FusedSurvey {
     return half_r_cell(g, ((size_t)g.ro * g.rs + g.ro) * g.rs + g.ro);
   }
 
-  // The grid in the arithmetic of the passes: rho itself when its cells
-  // already have the passes' type (f32: FP32 cells, in mixed precision
-  // only), else an FP32 copy of FP64 cells.
-  const void *prepare_input(const void *rho, bool f32, cudaStream_t s);
+  // Cells as the z passes read them.
+  struct Cells {
+    const void *p;
+    bool f32;
+  };
+  // The grid's cells as they are where the passes read that type (f32: FP32
+  // cells, in mixed precision only), else an FP32 copy of FP64 cells.
+  Cells prepare_input(const void *rho, bool f32, cudaStream_t s);
   // What prepare_input(rho, f32) last returned -- valid only while that
   // density is unchanged.
-  const void *input(const void *rho, bool f32) const {
-    return fp64_ || f32 ? rho : rho32.get();
+  Cells input(const void *rho, bool f32) const {
+    return reads_as_is(f32) ? Cells{rho, f32} : Cells{rho32.get(), true};
   }
   // G = 3-D DFT of the prepared grid (BaseCorrelator::set_grid2).
-  void grid2(const void *rho_in, cudaStream_t s, const KAxes &ka);
+  void grid2(Cells in, cudaStream_t s, const KAxes &ka);
   // Builds the r- (and, with with_k, k-) subgrid weight tables of every
   // (ell, m) up to maxell, so that later correlations allocate nothing.
   void prepare_tables(int maxell, double ncells, const double *raxis,
@@ -61,7 +65,7 @@ class FusedSurvey {
   // One (ell, m) term of Correlator::correlate_internal, accumulated into
   // the FP64 subgrids, or (first) written over them.
   // Returns the number of full-grid transforms run (1 or 2).
-  int term(const void *rho_in, int ell, int m, const double xyz0[3],
+  int term(Cells in, int ell, int m, const double xyz0[3],
             double ncells, double *ksub, double *rsub, const double *raxis,
             const KAxes &ka, cudaStream_t s, PhaseHook *hook, bool first,
             bool g_of_input, bool z_done);
@@ -69,7 +73,7 @@ class FusedSurvey {
   // of every multipole, |F|^2 or (cross) F conj(G), left unweighted in the
   // stored subgrids, P itself in ksub and its inverse transform in rsub.
   // The autocorrelation needs the even form.
-  void periodic(const void *rho_in, bool cross, double *ksub, double *rsub,
+  void periodic(Cells in, bool cross, double *ksub, double *rsub,
                 cudaStream_t s, PhaseHook *hook);
   // Whether two weighted terms can share one z pass (FP32, power-of-two
   // rows).  zfwd_pair runs the z pass of terms a and b (both ell > 0) in
@@ -83,7 +87,7 @@ class FusedSurvey {
   int nyq_group(bool k_extract) const {
     return (g.h - 1) % B == 0 && (!k_extract || g.ks2 / 2 < g.h - 1) ? 1 : 0;
   }
-  void zfwd_pair(const void *rho_in, int ell_a, int m_a, int ell_b, int m_b,
+  void zfwd_pair(Cells in, int ell_a, int m_a, int ell_b, int m_b,
                  const double xyz0[3], cudaStream_t s, PhaseHook *hook);
   void take_second() { std::swap(W, W2); }
 
@@ -103,9 +107,12 @@ class FusedSurvey {
   void set_smem_limits();
   // Whether the z passes are the power-of-two ones (even rows of m pairs).
   bool p2_rows() const;
+  // Whether the FP32 passes weight in FP64, cells, k- and r-subgrids alike.
+  bool wide() const { return !fp64_ && wide_rows(g.n2); }
+  bool reads_as_is(bool f32) const { return fp64_ || f32 || wide(); }
   template <typename T>
-  void zfwd(const void *rho, bool weight, const YlmParams &p,
-            const double xyz0[3], cudaStream_t s);
+  void zfwd(Cells in, bool weight, const YlmParams &p, const double xyz0[3],
+            cudaStream_t s);
   template <typename T>
   void yfwd(cudaStream_t s);
   template <typename T>
@@ -114,7 +121,7 @@ class FusedSurvey {
   void xcorr(int mode, double *ksub, const void *ktab, double w00, bool first,
              cudaStream_t s);
   // Weights of the k-subgrid cells for (ell, m), built on first use.
-  // (FP64 for the FP64 form, FP32 for the FP32-mixed form)
+  // (FP64 for the FP64 form and wide rows, else FP32)
   const void *k_table(int ell, int m, const KAxes &ka, cudaStream_t s);
   // Y_lm(r) of the r-subgrid cells for (ell, m), built on first use, in
   // the same type as the k weights.
@@ -130,6 +137,7 @@ class FusedSurvey {
   DeviceBuffer tabx, taby, tabz;
   DeviceBuffer W, G, Wr, Wry, rho32;
   DeviceBuffer W2, rowtab2;  // the second term of a paired z pass
+  DeviceBuffer kterm, rterm;  // a wide term's subgrids before their weights
   std::map<int, DeviceBuffer> ktabs;
   std::map<int, DeviceBuffer> rtabs;
   DeviceBuffer rowtab;  // per-row z-pass weight coefficients (FP32 form)

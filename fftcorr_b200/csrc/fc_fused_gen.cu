@@ -393,10 +393,10 @@ __global__ void __launch_bounds__(kXThreads, sizeof(T) == 4 ? 2 : 1)
 
 // ------------------------------------------------------------------ z
 // The z polynomial of Y_lm r^ell with the row's (x, y) fixed (row_poly in
-// fc_fused.cu), in the pass's precision, formed in FP64.
-template <typename T>
+// fc_fused.cu), in the weights' precision WT, formed in FP64.
+template <typename WT>
 struct RowCoef {
-  T c[5], rxy2;
+  WT c[5], rxy2;
 };
 
 // Y_lm D of a cell at z: D (c0 + c1 z + .. + c4 z^4) / r^ell.  In FP32 1 / r^2
@@ -406,24 +406,19 @@ struct RowCoef {
 // and 7.7e-8; z rounded twice: 9.3e-8 and 8.7e-8; the passes with a rounded divide
 // before these: 1.16e-7 and 9.3e-8), auto xi 7.2e-8 (6.7e-8; 7.3e-8; 8.0e-8).
 // The rounded divide costs 250 x 360 x 378 cross correlations 5.06 -> 5.27 ms.
-template <typename T, int ELL>
-__device__ __forceinline__ T row_value(const RowCoef<T> &r, T D, T z) {
-  const T z2 = z * z;
-  if constexpr (sizeof(T) == 4) {
-    const float ir2 = __fdividef(1.0f, r.rxy2 + z2 + 1e-20f);
-    if constexpr (ELL == 2) return D * ((r.c[2] * z + r.c[1]) * z + r.c[0]) * ir2;
-    // (1 / r^2 twice: its square is infinite in FP32 at the observer, r = 0.)
-    return D * ((((r.c[4] * z + r.c[3]) * z + r.c[2]) * z + r.c[1]) * z + r.c[0]) * ir2 *
-           ir2;
-  } else {
-    const double ir2 = 1.0 / (r.rxy2 + z2 + 1e-20);
-    if constexpr (ELL == 2) return D * ((r.c[2] * z + r.c[1]) * z + r.c[0]) * ir2;
-    return D * ((((r.c[4] * z + r.c[3]) * z + r.c[2]) * z + r.c[1]) * z + r.c[0]) *
-           ir2 * ir2;
-  }
+template <typename WT, int ELL>
+__device__ __forceinline__ WT row_value(const RowCoef<WT> &r, WT D, WT z) {
+  const WT z2 = z * z;
+  const WT r2 = r.rxy2 + z2 + (WT)1e-20;
+  WT ir2;
+  if constexpr (sizeof(WT) == 4) ir2 = __fdividef(1.0f, r2);
+  else ir2 = 1.0 / r2;
+  // (1 / r^2 twice: its square is infinite in FP32 at the observer, r = 0.)
+  if constexpr (ELL == 2) return D * ((r.c[2] * z + r.c[1]) * z + r.c[0]) * ir2;
+  return D * ((((r.c[4] * z + r.c[3]) * z + r.c[2]) * z + r.c[1]) * z + r.c[0]) * ir2 * ir2;
 }
 
-// z of the cell i of a row, z0 + i rounded to T once.
+// z of the cell i of a row, z0 + i rounded to its type once.
 template <typename T>
 struct RowZ;
 template <>
@@ -477,17 +472,18 @@ __device__ __forceinline__ float &comp(CPair &v, int c) {
 __device__ __forceinline__ double &comp(double2 &v, int c) { return c ? v.y : v.x; }
 
 // ELL: -1 unweighted, else the weight's multipole.  np elements per CTA, each
-// of 2 W rows.
-template <typename T, int ELL>
-__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
-    k_gzfwd(const T *rho, C2<T> *W, FusedGeom g,
+// of 2 W rows.  IN: the cells' type, WT: the precision in which they are
+// weighted; the result is rounded to T once.
+template <typename T, int ELL, typename IN, typename WT>
+__global__ void __launch_bounds__(kRowThreads, sizeof(WT) == 4 ? 5 : 4)
+    k_gzfwd(const IN *rho, C2<T> *W, FusedGeom g,
             const __grid_constant__ GPlan plan, const C2<T> *__restrict__ tw, int np,
             YlmParams p, double x0, double y0, double z0) {
   grid_chain();
   using E = typename GElem<T>::E;
   constexpr int NR = 2 * GElem<T>::W;  // grid rows per element
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ RowCoef<T> rc[NR * kGenMaxPairs];
+  __shared__ RowCoef<WT> rc[NR * kGenMaxPairs];
   const int N = g.n2;
   const int pitch = rpos(N - 1) + 1;
   E *buf = reinterpret_cast<E *>(smem_raw);
@@ -502,44 +498,49 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 5 : 4)
       const int y = (int)(row - (int64_t)x * g.n1);
       double c[5];
       row_poly_coefs(p, x0 + x * 1.0, y0 + y * 1.0, c);
-      RowCoef<T> r;
-      for (int i = 0; i < 5; ++i) r.c[i] = (T)c[i];
-      r.rxy2 = (T)((x0 + x) * (x0 + x) + (y0 + y) * (y0 + y));
+      RowCoef<WT> r;
+      for (int i = 0; i < 5; ++i) r.c[i] = (WT)c[i];
+      r.rxy2 = (WT)((x0 + x) * (x0 + x) + (y0 + y) * (y0 + y));
       rc[e] = r;
     }
     __syncthreads();
   }
   const GPass &f = plan.p[0];
-  const RowZ<T> zs(z0);
+  const RowZ<WT> zs(z0);
   with_radix(f.R, [&]<int R>() {
     for (int bf = threadIdx.x; bf < f.LR * np; bf += blockDim.x) {
       const int b = gdiv(bf, f.LR, f.mLR);
       const int j = bf - b * f.LR;
       const int64_t ra = row0 + NR * b;
-      const T *src = rho + (ra < nrows ? ra : 0) * N + j;
-      E v[R];
+      const IN *src = rho + (ra < nrows ? ra : 0) * N + j;
+      IN d[R][NR];
 #pragma unroll
       for (int c = 0; c < NR; ++c) {
         const bool on = ra + c < nrows;
 #pragma unroll
-        for (int q = 0; q < R; ++q) comp(v[q], c) = on ? src[c * N + q * f.LR] : (T)0;
+        for (int q = 0; q < R; ++q) d[q][c] = on ? src[c * N + q * f.LR] : (IN)0;
       }
-      if constexpr (ELL == 0) {
+      E v[R];
+      if constexpr (ELL < 0) {
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-          v[q].x = v[q].x * (T)p.value0;
-          v[q].y = v[q].y * (T)p.value0;
-        }
-      } else if constexpr (ELL > 0) {
-        T z[R];
+        for (int q = 0; q < R; ++q)
+#pragma unroll
+          for (int c = 0; c < NR; ++c) comp(v[q], c) = (T)d[q][c];
+      } else if constexpr (ELL == 0) {
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+#pragma unroll
+          for (int c = 0; c < NR; ++c) comp(v[q], c) = (T)((WT)d[q][c] * (WT)p.value0);
+      } else {
+        WT z[R];
 #pragma unroll
         for (int q = 0; q < R; ++q) z[q] = zs.at(j + q * f.LR);
 #pragma unroll
         for (int c = 0; c < NR; ++c) {
-          const RowCoef<T> a = rc[NR * b + c];
+          const RowCoef<WT> a = rc[NR * b + c];
 #pragma unroll
           for (int q = 0; q < R; ++q)
-            comp(v[q], c) = row_value<T, ELL>(a, comp(v[q], c), z[q]);
+            comp(v[q], c) = (T)row_value<WT, ELL>(a, (WT)d[q][c], z[q]);
         }
       }
       GDft<R, -1, E>::run(v);
@@ -711,10 +712,21 @@ void col_limits() {
 template <typename T>
 void set_limits(int L, bool row) {
   if (row) {
-    big_smem(k_gzfwd<T, -1>);
-    big_smem(k_gzfwd<T, 0>);
-    big_smem(k_gzfwd<T, 2>);
-    big_smem(k_gzfwd<T, 4>);
+    auto z_limits = [](auto in, auto wt) {
+      using IN = decltype(in);
+      using WT = decltype(wt);
+      big_smem(k_gzfwd<T, -1, IN, WT>);
+      big_smem(k_gzfwd<T, 0, IN, WT>);
+      big_smem(k_gzfwd<T, 2, IN, WT>);
+      big_smem(k_gzfwd<T, 4, IN, WT>);
+    };
+    z_limits(T(), T());
+    if constexpr (sizeof(T) == 4) {
+      if (wide_rows(L)) {
+        z_limits(T(), double());
+        z_limits(double(), double());
+      }
+    }
     big_smem(k_gzinv<T>);
   } else if (col_width(L) == 8) {
     col_limits<T, 8>();
@@ -750,21 +762,33 @@ void GenAxis::init(int L, bool row, bool fp64) {
 }
 
 template <typename T>
-void gen_zfwd(const GenAxis &a, const FusedGeom &g, const T *rho, C2<T> *W, bool weight,
-              const YlmParams &p, const double xyz0[3], cudaStream_t s) {
+void gen_zfwd(const GenAxis &a, const FusedGeom &g, const void *rho, bool f32, C2<T> *W,
+              bool weight, const YlmParams &p, const double xyz0[3], cudaStream_t s) {
   constexpr int NR = 2 * GElem<T>::W;
   const int64_t nrows = (int64_t)g.n0 * g.n1;
   const int np = row_elems(a.plan, (nrows + NR - 1) / NR);
   const unsigned blocks = (unsigned)((nrows + NR * np - 1) / (NR * np));
   const size_t sm = row_smem(g.n2, np);
-  auto go = [&](auto kernel) {
-    launch_small(kernel, blocks, row_threads(a.plan, np), sm, s, rho, W, g, a.plan, a.tw.as<C2<T>>(), np, p,
-                                           xyz0[0], xyz0[1], xyz0[2]);
+  auto run = [&](auto in, auto wt) {
+    using IN = decltype(in);
+    using WT = decltype(wt);
+    auto go = [&](auto kernel) {
+      launch_small(kernel, blocks, row_threads(a.plan, np), sm, s,
+                   static_cast<const IN *>(rho), W, g, a.plan, a.tw.as<C2<T>>(), np, p,
+                   xyz0[0], xyz0[1], xyz0[2]);
+    };
+    if (!weight) go(k_gzfwd<T, -1, IN, WT>);
+    else if (p.ell == 0) go(k_gzfwd<T, 0, IN, WT>);
+    else if (p.ell == 2) go(k_gzfwd<T, 2, IN, WT>);
+    else go(k_gzfwd<T, 4, IN, WT>);
   };
-  if (!weight) go(k_gzfwd<T, -1>);
-  else if (p.ell == 0) go(k_gzfwd<T, 0>);
-  else if (p.ell == 2) go(k_gzfwd<T, 2>);
-  else go(k_gzfwd<T, 4>);
+  if constexpr (sizeof(T) == 4) {
+    if (wide_rows(g.n2) && f32) run(T(), double());
+    else if (wide_rows(g.n2)) run(double(), double());
+    else run(T(), T());
+  } else {
+    run(T(), T());
+  }
   FC_LAUNCH_CHECK();
 }
 
@@ -826,8 +850,9 @@ void gen_zinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wry, double *rs
 }
 
 #define FC_GEN(T)                                                                      \
-  template void gen_zfwd<T>(const GenAxis &, const FusedGeom &, const T *, C2<T> *,    \
-                            bool, const YlmParams &, const double[3], cudaStream_t);   \
+  template void gen_zfwd<T>(const GenAxis &, const FusedGeom &, const void *, bool,    \
+                            C2<T> *, bool, const YlmParams &, const double[3],         \
+                            cudaStream_t);                                             \
   template void gen_yfwd<T>(const GenAxis &, const FusedGeom &, C2<T> *, cudaStream_t); \
   template void gen_x<T>(const GenAxis &, const FusedGeom &, int, const C2<T> *,       \
                          const C2<T> *, C2<T> *, double *, const T *, T, bool,        \
