@@ -1236,7 +1236,11 @@ __global__ void k_rowpoly(float4 *tab, int64_t nrows, int n1,
 
 // Per-cell r-subgrid weight of one (ell, m): Y_lm(r) with the r-subgrid
 // normalisation (make_ylm, correlator.h:477-480), computed once per
-// correlator and multipole so the z inverse pass does a multiply-add.
+// correlator and multipole so the z inverse pass does a multiply-add.  In the
+// even form a cell stands for its mirror image too, whose coordinates are not
+// its own with the sign changed to the last bit (start + i step, rounded): its
+// weight is the mean of the two, or the quadrupole near r = 0, where the cells
+// of a bin cancel, is off by those bits.
 template <typename RT>
 __global__ void k_rtable(RT *__restrict__ tab, FusedGeom g,
                          const double *__restrict__ raxis, YlmParams pr) {
@@ -1247,14 +1251,19 @@ __global__ void k_rtable(RT *__restrict__ tab, FusedGeom g,
     const int rk = (int)(i % g.rs);
     const int rj = (int)((i / g.rs) % g.rs);
     const int ri = (int)(i / ((size_t)g.rs * g.rs));
-    tab[i] = (RT)ylm_eval(pr, 1.0, raxis[x0 + ri], raxis[rj], raxis[rk]);
+    double y = ylm_eval(pr, 1.0, raxis[x0 + ri], raxis[rj], raxis[rk]);
+    if (x0 > 0) {
+      const int e = g.rs - 1;
+      y = 0.5 * (y + ylm_eval(pr, 1.0, raxis[e - x0 - ri], raxis[e - rj], raxis[e - rk]));
+    }
+    tab[i] = (RT)y;
   }
 }
 
 // Per-cell k-subgrid weight of one (ell, m): Y_lm(k) * 4 pi / (W(kx) W(ky)
 // W(kz)) with make_ylm's arithmetic (correlator.h:453-466), computed once
 // per correlator and multipole so the extraction in the x pass is a
-// multiply-add.
+// multiply-add; the mean of a cell's and of its mirror image's (k_rtable).
 template <typename KT>
 __global__ void k_ktable(KT *__restrict__ tab, FusedGeom g, KAxes ax, YlmParams pk) {
   const int oz = g.ks2 / 2;
@@ -1268,8 +1277,12 @@ __global__ void k_ktable(KT *__restrict__ tab, FusedGeom g, KAxes ax, YlmParams 
       tab[c] = (KT)0;
       continue;
     }
-    const double inv_w = 1.0 / (ax.wx[i] * ax.wy[j] * ax.wz[k]);
-    tab[c] = (KT)ylm_eval(pk, inv_w, ax.kx[i], ax.ky[j], ax.kz[k]);
+    auto weight = [&](int a, int b, int d) {
+      const double inv_w = 1.0 / (ax.wx[a] * ax.wy[b] * ax.wz[d]);
+      return ylm_eval(pk, inv_w, ax.kx[a], ax.ky[b], ax.kz[d]);
+    };
+    tab[c] = (KT)(0.5 * (weight(i, j, k) +
+                         weight(g.ks0 - 1 - i, g.ks1 - 1 - j, g.ks2 - 1 - k)));
   }
 }
 
