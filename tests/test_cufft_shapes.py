@@ -1,0 +1,69 @@
+"""Sides with a prime factor above 7, which run through cuFFT: the batched form
+beside fused boxes, and an FFT plan that cannot be made (raised on the host
+before the cuFFT call)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from conftest import clustered_catalog
+from oracle import fc_oracle as O
+
+import fftcorr_b200 as fb
+from fftcorr_b200 import _lib
+from test_batch import _batch, _single_box
+from test_gpu_parity import FP64_RTOL, _compare_results
+
+pytestmark = pytest.mark.gpu
+
+POSMIN = np.array([-160.0, -160.0, 20.0])
+
+
+@pytest.fixture(autouse=True)
+def _disarm():
+    yield
+    _lib.call("fc_fault_inject", _lib.FC_FAULT_FFT_PLAN, 0)
+
+
+def _device_bytes():
+    b = ctypes.c_size_t()
+    _lib.call("fc_device_bytes", ctypes.byref(b))
+    return b.value
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_batch_equals_single_box_path(precision):
+    boxes = []
+    for shape, n, seed in [((22, 22, 22), 20000, 1), ((33, 26, 39), 30000, 2),
+                           ((32, 32, 32), 30000, 3), ((26, 44, 22), 4000, 4)]:
+        posw = clustered_catalog(n, [0, 0, 0], 10.0 * np.array(shape), seed, ncenters=30)
+        boxes.append((shape, 10.0, posw))
+    b = _batch(boxes, precision)
+    b.run()
+    for i, (shape, cell, posw) in enumerate(boxes):
+        ref, _ = _single_box(shape, cell, posw, precision)
+        got = b.results(i)
+        for key in ("rcounts", "kcounts", "rhist", "khist"):
+            np.testing.assert_array_equal(got[key], ref[key], err_msg=f"box {i} {key}")
+        assert got["zerolag"] == ref["zerolag"]
+
+
+@pytest.mark.parametrize("kind", ["periodic", "survey"])
+def test_plan_failure_leaves_nothing_behind(kind):
+    shape, cell = (22, 26, 33), 10.0
+    if kind == "periodic":
+        args = (cell, 0, 60.0, 7.0, 0.25, 0.02, 2)
+        make, oracle = fb.PeriodicCorrelator, O.periodic_correlate
+    else:
+        args = (cell, POSMIN, 2, 60.0, 10.0, 0.2, 0.04, 2)
+        make, oracle = fb.Correlator, O.survey_correlate
+    before = _device_bytes()
+    _lib.call("fc_fault_inject", _lib.FC_FAULT_FFT_PLAN, 1)
+    with pytest.raises(_lib.FcError) as e:
+        make(shape, *args)
+    assert e.value.code == _lib.FC_ERR_CUFFT
+    assert _device_bytes() == before
+    grid = np.random.default_rng(5).standard_normal(shape)
+    c = make(shape, *args)
+    c.autocorrelate(grid)
+    _compare_results(c.results(), oracle(grid, *args), FP64_RTOL, kind)
