@@ -1324,7 +1324,10 @@ std::vector<C> root_table(int order) {
 
 // ----------------------------------------------------- power-of-two dispatch
 
-bool is_p2(int L) { return L >= 64 && L <= 2048 && (L & (L - 1)) == 0; }
+bool is_p2(int L) { return L >= 64 && L <= 1024 && (L & (L - 1)) == 0; }
+// Longest row (z) of the passes (longer ones go through cuFFT, whose weights are
+// FP64); columns end at 1280 (gen_supported).
+constexpr int kMaxRow = 2560;
 
 template <typename T, int L>
 size_t p2_col_smem() {
@@ -1335,18 +1338,22 @@ size_t p2_row_smem() {
   return (size_t)P2<T, L>::B * (L + L / 8 + 1) * sizeof(C2<T>);
 }
 
-// Calls f.template operator()<L>() for the power-of-two L.
+// Calls f.template operator()<L>() for the power-of-two L of a column, and of a
+// row's pairs.
 template <typename F>
 void with_p2(int L, F &&f) {
   switch (L) {
-    case 32: f.template operator()<32>(); break;
     case 64: f.template operator()<64>(); break;
     case 128: f.template operator()<128>(); break;
     case 256: f.template operator()<256>(); break;
     case 512: f.template operator()<512>(); break;
-    case 1024: f.template operator()<1024>(); break;
-    default: f.template operator()<2048>(); break;
+    default: f.template operator()<1024>(); break;
   }
+}
+template <typename F>
+void with_p2_row(int L, F &&f) {
+  if (L == 32) f.template operator()<32>();
+  else with_p2(L, f);
 }
 
 template <typename K>
@@ -1387,7 +1394,7 @@ void p2_set_limits() {
 }  // namespace
 
 bool FusedSurvey::supported(const int shape[3], int rsize) {
-  return gen_supported(shape[0], false) && gen_supported(shape[1], false) &&
+  return shape[2] <= kMaxRow && gen_supported(shape[0], false) && gen_supported(shape[1], false) &&
          gen_supported(shape[2], true) && rsize > 0;
 }
 
@@ -1454,9 +1461,9 @@ void FusedSurvey::set_smem_limits() {
   for (int L : {is_p2(g.n0) ? g.n0 : 0, is_p2(g.n1) ? g.n1 : 0, p2_rows() ? g.m : 0}) {
     if (L == 0) continue;
     if (fp64_)
-      with_p2(L, [&]<int LL>() { p2_set_limits<double, LL>(); });
+      with_p2_row(L, [&]<int LL>() { p2_set_limits<double, LL>(); });
     else
-      with_p2(L, [&]<int LL>() { p2_set_limits<float, LL>(); });
+      with_p2_row(L, [&]<int LL>() { p2_set_limits<float, LL>(); });
   }
 }
 
@@ -1477,7 +1484,7 @@ void FusedSurvey::zfwd(Cells in, bool weight, const YlmParams &p, const double x
                        cudaStream_t s) {
   if (p2_rows()) {
     const void *rho = in.p;
-    with_p2(g.m, [&]<int L>() {
+    with_p2_row(g.m, [&]<int L>() {
       using Q = P2<T, L>;
       const int64_t nrows = (int64_t)g.n0 * g.n1;
       const unsigned blocks = (unsigned)((nrows + Q::B - 1) / Q::B);
@@ -1627,7 +1634,7 @@ template <typename T>
 void FusedSurvey::zinv(double *rsub, const void *rtab_v, bool first, cudaStream_t s) {
   const T *rtab = static_cast<const T *>(rtab_v);
   if (p2_rows()) {
-    with_p2(g.m, [&]<int L>() {
+    with_p2_row(g.m, [&]<int L>() {
       using Q = P2<T, L>;
       const int nrows = g.nri * g.rs;
       const unsigned blocks = (unsigned)((nrows + Q::B - 1) / Q::B);
@@ -1728,7 +1735,7 @@ void FusedSurvey::zfwd_pair(Cells in, int ell_a, int m_a, int ell_b,
                                                  g.n1, pb, xyz0[0], xyz0[1]);
   FC_LAUNCH_CHECK();
   if (hook) hook->begin("zfwd2");
-  with_p2(g.m, [&]<int L>() {
+  with_p2_row(g.m, [&]<int L>() {
     using PQ = PP<L>;
     const unsigned blocks = (unsigned)((nrows + PQ::PB - 1) / PQ::PB);
     launch_after(k_zfwd_pp2<L>, blocks, PQ::THREADS, p2_row_smem<float, L>(), s, 

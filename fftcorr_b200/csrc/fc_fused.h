@@ -26,7 +26,7 @@ struct PhaseHook {
 class FusedSurvey {
  public:
   // True when every side factors into 2, 3, 5, 7 and the shared-memory tiles
-  // fit.
+  // fit: columns (x, y) of at most 1280 cells and rows (z) of at most 2560.
   static bool supported(const int shape[3], int rsize);
 
   // even: the r-subgrid's bins are those of its mirror image, so the inverse

@@ -1,4 +1,4 @@
-"""Sides with a prime factor above 7, which run through cuFFT: the batched form
+"""What runs through cuFFT, sides with a prime factor above 7 and long rows: the batched form
 beside fused boxes, and an FFT plan that cannot be made (raised on the host
 before the cuFFT call)."""
 import ctypes
@@ -67,3 +67,34 @@ def test_plan_failure_leaves_nothing_behind(kind):
     c = make(shape, *args)
     c.autocorrelate(grid)
     _compare_results(c.results(), oracle(grid, *args), FP64_RTOL, kind)
+
+
+@pytest.mark.parametrize("shape", [(4, 6, 4096), (5, 4, 2592), (2, 3, 2625)])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_long_rows(shape, precision, monkeypatch):
+    """Rows of more than 2560 cells: cuFFT's path by itself and when asked for
+    give the same bits; those of 2560 run through the fused passes."""
+    grid = np.random.default_rng(9).standard_normal(shape)
+    args = (10.0, POSMIN, 2, 10.0 * min(shape), 4.0, 0.1, 0.02, 4)
+    c = fb.Correlator(shape, *args, precision=precision)
+    c.autocorrelate(grid)
+    got = c.results()
+    monkeypatch.setenv("FFTCORR_B200_FFT", "cufft")
+    c = fb.Correlator(shape, *args, precision=precision)
+    c.autocorrelate(grid)
+    for key in ("rcounts", "kcounts", "rhist", "khist"):
+        np.testing.assert_array_equal(got[key], c.results()[key])
+    _compare_results(got, O.survey_correlate(grid, *args), FP64_RTOL, "long rows",
+                     fp32=precision == "fp32")
+
+
+@pytest.mark.parametrize("n2", [2048, 2500, 2560, 2401])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_longest_fused_rows(n2, precision):
+    shape = (4, 6, n2)
+    grid = np.random.default_rng(9).standard_normal(shape)
+    args = (10.0, POSMIN, 2, 40.0, 4.0, 0.1, 0.02, 4)
+    c = fb.Correlator(shape, *args, precision=precision)
+    c.autocorrelate(grid)
+    _compare_results(c.results(), O.survey_correlate(grid, *args), FP64_RTOL, "long rows",
+                     fp32=precision == "fp32")
