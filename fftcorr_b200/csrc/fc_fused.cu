@@ -1362,32 +1362,45 @@ void big_smem(K kernel) {
                                200 * 1024));
 }
 
+// Shared-memory limits of the kernels that a correlator launches, axis by axis.
 template <typename T, int L>
-void p2_set_limits() {
+void p2_z_limits(bool weighted, bool pairs) {
   big_smem(k_zinv_p2<T, L>);
+  if constexpr (std::is_same_v<T, double>) {
+    big_smem(k_zfwd_p2<L, false>);
+    if (weighted) big_smem(k_zfwd_p2<L, true>);
+  } else {
+    big_smem(k_zfwd_pp<L, false>);
+    if (weighted) big_smem(k_zfwd_pp<L, true>);
+    if (weighted && pairs) big_smem(k_zfwd_pp2<L>);
+  }
+}
+template <typename T, int L>
+void p2_y_limits() {
   if constexpr (std::is_same_v<T, double>) {
     big_smem(k_yfwd_p2<T, L>);
     big_smem(k_yinv_p2<T, L>);
-    big_smem(k_xcorr_p2<L, 0, false>);
-    big_smem(k_xcorr_p2<L, 1, false>);
-    big_smem(k_xcorr_p2<L, 2, false>);
-    big_smem(k_xcorr_p2<L, 1, true>);
-    big_smem(k_xcorr_p2<L, 2, true>);
-    big_smem(k_xcorr_p2<L, 3, true>);
-    big_smem(k_zfwd_p2<L, true>);
-    big_smem(k_zfwd_p2<L, false>);
   } else {
     big_smem(k_yfwd_pp<L>);
     big_smem(k_yinv_pp<L>);
-    big_smem(k_xfwd_pp<L>);
-    big_smem(k_xcorr_pp<L, 1, false>);
-    big_smem(k_xcorr_pp<L, 2, false>);
-    big_smem(k_xcorr_pp<L, 1, true>);
-    big_smem(k_xcorr_pp<L, 2, true>);
-    big_smem(k_xcorr_pp<L, 3, true>);
-    big_smem(k_zfwd_pp<L, true>);
-    big_smem(k_zfwd_pp<L, false>);
-    big_smem(k_zfwd_pp2<L>);
+  }
+}
+template <typename T, int L>
+void p2_x_limits(int mode, bool even) {
+  if constexpr (std::is_same_v<T, double>) {
+    if (mode == 0) big_smem(k_xcorr_p2<L, 0, false>);
+    else if (mode == 3) big_smem(k_xcorr_p2<L, 3, true>);
+    else if (mode == 2 && even) big_smem(k_xcorr_p2<L, 2, true>);
+    else if (mode == 2) big_smem(k_xcorr_p2<L, 2, false>);
+    else if (even) big_smem(k_xcorr_p2<L, 1, true>);
+    else big_smem(k_xcorr_p2<L, 1, false>);
+  } else {
+    if (mode == 0) big_smem(k_xfwd_pp<L>);
+    else if (mode == 3) big_smem(k_xcorr_pp<L, 3, true>);
+    else if (mode == 2 && even) big_smem(k_xcorr_pp<L, 2, true>);
+    else if (mode == 2) big_smem(k_xcorr_pp<L, 2, false>);
+    else if (even) big_smem(k_xcorr_pp<L, 1, true>);
+    else big_smem(k_xcorr_pp<L, 1, false>);
   }
 }
 
@@ -1417,19 +1430,17 @@ FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
   g.kp = (g.ks2 / 2 + 1 + 3) / 4 * 4;
   g.nri = even ? g.ro + 1 : g.rs;
   // Axes that the power-of-two passes do not take.
-  if (!is_p2(g.n0)) gx.init(g.n0, false, fp64);
-  if (!is_p2(g.n1)) gy.init(g.n1, false, fp64);
-  if (!p2_rows()) gz.init(g.n2, true, fp64);
+  if (!is_p2(g.n0)) gx.init(g.n0, fp64);
+  if (!is_p2(g.n1)) gy.init(g.n1, fp64);
+  if (!p2_rows()) gz.init(g.n2, fp64);
   const size_t eb = fp64 ? 16 : 8;
-  if (fp64) {
-    upload(tabx, root_table<double2>(g.n0));
-    upload(taby, root_table<double2>(g.n1));
-    upload(tabz, root_table<double2>(g.n2));
-  } else {
-    upload(tabx, root_table<float2>(g.n0));
-    upload(taby, root_table<float2>(g.n1));
-    upload(tabz, root_table<float2>(g.n2));
-  }
+  auto roots = [&](DeviceBuffer &tab, int n) {
+    if (fp64) upload(tab, root_table<double2>(n));
+    else upload(tab, root_table<float2>(n));
+  };
+  if (is_p2(g.n0)) roots(tabx, g.n0);
+  if (is_p2(g.n1)) roots(taby, g.n1);
+  if (p2_rows()) roots(tabz, g.n2);
   const size_t nc = (size_t)g.n0 * g.n1 * g.hp;
   W.resize(nc * eb);
   if (survey) G.resize(nc * eb);
@@ -1439,15 +1450,13 @@ FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
     kterm.resize(k_cells() * sizeof(double));
     rterm.resize(r_cells() * sizeof(double));
   }
-  if (!fp64 && !wide()) {
-    rho32.resize((size_t)g.n0 * g.n1 * g.n2 * sizeof(float));
-    if (survey) rowtab.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
-    if (survey && pairs()) {
-      W2.resize(nc * eb);
-      rowtab2.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
-    }
+  if (survey && pairs()) {
+    rowtab.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
+    W2.resize(nc * eb);
+    rowtab2.resize((size_t)g.n0 * g.n1 * 2 * sizeof(float4));
   }
-  set_smem_limits();
+  if (fp64) set_limits<double>(survey);
+  else set_limits<float>(survey);
 }
 
 template <typename V>
@@ -1457,14 +1466,36 @@ void FusedSurvey::upload(DeviceBuffer &dst, const std::vector<V> &v) {
                      cudaMemcpyHostToDevice));
 }
 
-void FusedSurvey::set_smem_limits() {
-  for (int L : {is_p2(g.n0) ? g.n0 : 0, is_p2(g.n1) ? g.n1 : 0, p2_rows() ? g.m : 0}) {
-    if (L == 0) continue;
-    if (fp64_)
-      with_p2_row(L, [&]<int LL>() { p2_set_limits<double, LL>(); });
-    else
-      with_p2_row(L, [&]<int LL>() { p2_set_limits<float, LL>(); });
+template <typename T>
+void FusedSurvey::x_limits(int mode) {
+  if (is_p2(g.n0)) with_p2(g.n0, [&]<int L>() { p2_x_limits<T, L>(mode, even()); });
+  else gen_x_limits<T>(g.n0, mode, even());
+}
+
+template <typename T>
+void FusedSurvey::set_limits(bool survey) {
+  if (p2_rows())
+    with_p2_row(g.m, [&]<int L>() { p2_z_limits<T, L>(survey, pairs()); });
+  else
+    gen_z_limits<T>(g.n2, survey);
+  if (is_p2(g.n1)) with_p2(g.n1, [&]<int L>() { p2_y_limits<T, L>(); });
+  else gen_y_limits<T>(g.n1);
+  if (survey) {
+    for (int mode : {0, 1, 2}) x_limits<T>(mode);
+    product_ready = true;
+  } else {
+    x_limits<T>(3);
   }
+}
+
+void FusedSurvey::prepare_product() {
+  G.resize(W.bytes());
+  if (product_ready) return;
+  for (int mode : {0, 1}) {
+    if (fp64_) x_limits<double>(mode);
+    else x_limits<float>(mode);
+  }
+  product_ready = true;
 }
 
 FusedSurvey::Cells FusedSurvey::prepare_input(const void *rho, bool f32,
@@ -1473,6 +1504,7 @@ FusedSurvey::Cells FusedSurvey::prepare_input(const void *rho, bool f32,
              "the FP64 passes take FP64 cells");
   if (reads_as_is(f32)) return {rho, f32};
   const size_t n = (size_t)g.n0 * g.n1 * g.n2;
+  rho32.resize(n * sizeof(float));  // (for the first FP64 cells)
   k_to_float<<<grid_for(n, 256), 256, 0, s>>>(static_cast<const double *>(rho),
                                               rho32.as<float>(), n, 0.0);
   FC_LAUNCH_CHECK();
@@ -1492,7 +1524,6 @@ void FusedSurvey::zfwd(Cells in, bool weight, const YlmParams &p, const double x
         using PQ = PP<L>;
         const float4 *rt = nullptr;
         if (weight && p.ell != 0) {
-          rowtab.resize((size_t)nrows * 2 * sizeof(float4));
           launch_after(k_rowpoly, grid_for(nrows, 256), 256, 0, s, 
               rowtab.as<float4>(), nrows, g.n1, p, xyz0[0], xyz0[1]);
           FC_LAUNCH_CHECK();
@@ -1701,7 +1732,7 @@ const void *FusedSurvey::k_table(int ell, int m, const KAxes &ka,
 
 void FusedSurvey::grid2(Cells in, cudaStream_t s, const KAxes &ka) {
   (void)ka;
-  G.resize(W.bytes());
+  prepare_product();
   YlmParams none = make_ylm_params(0, 0, 1.0);
   const double zero[3] = {0, 0, 0};
   if (fp64_) {

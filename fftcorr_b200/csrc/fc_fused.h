@@ -38,10 +38,6 @@ class FusedSurvey {
   // Cells of the stored subgrids (half_k_cell, half_r_cell).
   size_t k_cells() const { return (size_t)g.ks0 * g.ks1 * g.kp; }
   size_t r_cells() const { return (size_t)g.nri * g.rs * g.rs; }
-  // The stored cell of r = 0.
-  size_t zero_lag() const {
-    return half_r_cell(g, ((size_t)g.ro * g.rs + g.ro) * g.rs + g.ro);
-  }
 
   // Cells as the z passes read them.
   struct Cells {
@@ -94,7 +90,7 @@ class FusedSurvey {
   // G in the half-complex layout [N0][N1][N2/2+1] with rows g.hp elements
   // apart (FP64 or FP32 complex).
   void *g_data() {
-    G.resize(W.bytes());
+    prepare_product();
     return G.get();
   }
   bool fp64() const { return fp64_; }
@@ -104,7 +100,14 @@ class FusedSurvey {
  private:
   template <typename V>
   void upload(DeviceBuffer &dst, const std::vector<V> &v);
-  void set_smem_limits();
+  // Shared-memory limits of the kernels that this correlator launches: x's by
+  // the pass's mode (k_xcorr_p2).
+  template <typename T>
+  void set_limits(bool survey);
+  template <typename T>
+  void x_limits(int mode);
+  // What a product with a second grid needs beside the autocorrelation.
+  void prepare_product();
   // Whether the z passes are the power-of-two ones (even rows of m pairs).
   bool p2_rows() const;
   // Whether the FP32 passes weight in FP64, cells, k- and r-subgrids alike.
@@ -133,6 +136,7 @@ class FusedSurvey {
   void zinv(double *rsub, const void *rtab, bool first, cudaStream_t s);
 
   bool fp64_;
+  bool product_ready = false;
   GenAxis gx, gy, gz;  // of the axes that are not powers of two
   DeviceBuffer tabx, taby, tabz;
   DeviceBuffer W, G, Wr, Wry, rho32;

@@ -698,41 +698,22 @@ void big_smem(K kernel) {
                                (int)kGenSmem));
 }
 
-template <typename T, int B>
-void col_limits() {
-  big_smem(k_gyfwd<T, B>);
-  big_smem(k_gyinv<T, B>);
-  big_smem(k_gx<T, B, 0, false>);
-  big_smem(k_gx<T, B, 1, false>);
-  big_smem(k_gx<T, B, 2, false>);
-  big_smem(k_gx<T, B, 1, true>);
-  big_smem(k_gx<T, B, 2, true>);
-  big_smem(k_gx<T, B, 3, true>);
+// Calls f.template operator()<B>() for a length's column width.
+template <typename F>
+void with_width(int L, F &&f) {
+  if (col_width(L) == 8) f.template operator()<8>();
+  else f.template operator()<4>();
 }
-template <typename T>
-void set_limits(int L, bool row) {
-  if (row) {
-    auto z_limits = [](auto in, auto wt) {
-      using IN = decltype(in);
-      using WT = decltype(wt);
-      big_smem(k_gzfwd<T, -1, IN, WT>);
-      big_smem(k_gzfwd<T, 0, IN, WT>);
-      big_smem(k_gzfwd<T, 2, IN, WT>);
-      big_smem(k_gzfwd<T, 4, IN, WT>);
-    };
-    z_limits(T(), T());
-    if constexpr (sizeof(T) == 4) {
-      if (wide_rows(L)) {
-        z_limits(T(), double());
-        z_limits(double(), double());
-      }
-    }
-    big_smem(k_gzinv<T>);
-  } else if (col_width(L) == 8) {
-    col_limits<T, 8>();
-  } else {
-    col_limits<T, 4>();
-  }
+
+// Calls f(kernel) for the x kernel of a mode.
+template <typename T, int B, typename F>
+void x_kernel(int mode, bool even, F &&f) {
+  if (mode == 0) f(k_gx<T, B, 0, false>);
+  else if (mode == 3) f(k_gx<T, B, 3, true>);
+  else if (mode == 1 && even) f(k_gx<T, B, 1, true>);
+  else if (mode == 1) f(k_gx<T, B, 1, false>);
+  else if (even) f(k_gx<T, B, 2, true>);
+  else f(k_gx<T, B, 2, false>);
 }
 
 }  // namespace
@@ -744,7 +725,7 @@ bool gen_supported(int L, bool row) {
   return col_smem(L) <= kGenSmem;
 }
 
-void GenAxis::init(int L, bool row, bool fp64) {
+void GenAxis::init(int L, bool fp64) {
   FC_REQUIRE(gplan_length(L, &plan), FC_ERR_UNSUPPORTED,
              "grid size has a prime factor above 7");
   auto put = [&](const auto &t) {
@@ -752,13 +733,46 @@ void GenAxis::init(int L, bool row, bool fp64) {
     FC_CUDA(cudaMemcpy(tw.get(), t.data(), t.size() * sizeof(t[0]),
                        cudaMemcpyHostToDevice));
   };
-  if (fp64) {
-    put(gplan_twiddles<double2>(plan));
-    set_limits<double>(L, row);
+  if (fp64) put(gplan_twiddles<double2>(plan));
+  else put(gplan_twiddles<float2>(plan));
+}
+
+// Calls f(kernel) for every z kernel of a cell type and weights' precision.
+template <typename T, typename IN, typename WT, typename F>
+void z_kernels(bool weighted, F &&f) {
+  f(k_gzfwd<T, -1, IN, WT>);
+  if (!weighted) return;
+  f(k_gzfwd<T, 0, IN, WT>);
+  f(k_gzfwd<T, 2, IN, WT>);
+  f(k_gzfwd<T, 4, IN, WT>);
+}
+template <typename T>
+void gen_z_limits(int n2, bool weighted) {
+  auto set = [](auto kernel) { big_smem(kernel); };
+  if constexpr (sizeof(T) == 4) {
+    if (wide_rows(n2)) {
+      z_kernels<T, T, double>(weighted, set);
+      z_kernels<T, double, double>(weighted, set);
+    } else {
+      z_kernels<T, T, T>(weighted, set);
+    }
   } else {
-    put(gplan_twiddles<float2>(plan));
-    set_limits<float>(L, row);
+    z_kernels<T, T, T>(weighted, set);
   }
+  big_smem(k_gzinv<T>);
+}
+template <typename T>
+void gen_y_limits(int n1) {
+  with_width(n1, [&]<int B>() {
+    big_smem(k_gyfwd<T, B>);
+    big_smem(k_gyinv<T, B>);
+  });
+}
+template <typename T>
+void gen_x_limits(int n0, int mode, bool even) {
+  with_width(n0, [&]<int B>() {
+    x_kernel<T, B>(mode, even, [](auto kernel) { big_smem(kernel); });
+  });
 }
 
 template <typename T>
@@ -792,16 +806,9 @@ void gen_zfwd(const GenAxis &a, const FusedGeom &g, const void *rho, bool f32, C
   FC_LAUNCH_CHECK();
 }
 
-// Calls f.template operator()<B>() for the axis's column width.
-template <typename F>
-void with_width(const GenAxis &a, F &&f) {
-  if (col_width(a.plan.L) == 8) f.template operator()<8>();
-  else f.template operator()<4>();
-}
-
 template <typename T>
 void gen_yfwd(const GenAxis &a, const FusedGeom &g, C2<T> *W, cudaStream_t s) {
-  with_width(a, [&]<int B>() {
+  with_width(a.plan.L, [&]<int B>() {
     constexpr int NC = kCols<T, B>;
     launch_small(k_gyfwd<T, B>, dim3((g.h + NC - 1) / NC, g.n0), col_threads(a.plan, kYThreads), col_smem(g.n1), s, W, g, a.plan, a.tw.as<C2<T>>());
   });
@@ -811,19 +818,13 @@ void gen_yfwd(const GenAxis &a, const FusedGeom &g, C2<T> *W, cudaStream_t s) {
 template <typename T>
 void gen_x(const GenAxis &a, const FusedGeom &g, int mode, const C2<T> *W, const C2<T> *G,
            C2<T> *out, double *ksub, const T *ktab, T w00, bool first, cudaStream_t s) {
-  with_width(a, [&]<int B>() {
+  with_width(a.plan.L, [&]<int B>() {
     constexpr int NC = kCols<T, B>;
     auto go = [&](auto kernel) {
       launch_small(kernel, dim3((g.h + NC - 1) / NC, g.n1), col_threads(a.plan, kXThreads), col_smem(g.n0), s, 
           W, G, out, ksub, g, a.plan, a.tw.as<C2<T>>(), ktab, w00, first);
     };
-    const bool even = g.nri != g.rs;
-    if (mode == 0) go(k_gx<T, B, 0, false>);
-    else if (mode == 3) go(k_gx<T, B, 3, true>);
-    else if (mode == 1 && even) go(k_gx<T, B, 1, true>);
-    else if (mode == 1) go(k_gx<T, B, 1, false>);
-    else if (even) go(k_gx<T, B, 2, true>);
-    else go(k_gx<T, B, 2, false>);
+    x_kernel<T, B>(mode, g.nri != g.rs, go);
   });
   FC_LAUNCH_CHECK();
 }
@@ -831,7 +832,7 @@ void gen_x(const GenAxis &a, const FusedGeom &g, int mode, const C2<T> *W, const
 template <typename T>
 void gen_yinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wr, C2<T> *Wry,
               cudaStream_t s) {
-  with_width(a, [&]<int B>() {
+  with_width(a.plan.L, [&]<int B>() {
     constexpr int NC = kCols<T, B>;
     launch_small(k_gyinv<T, B>, dim3((g.h + NC - 1) / NC, g.nri), col_threads(a.plan, kYThreads), col_smem(g.n1), s, Wr, Wry, g, a.plan, a.tw.as<C2<T>>());
   });
@@ -850,6 +851,9 @@ void gen_zinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wry, double *rs
 }
 
 #define FC_GEN(T)                                                                      \
+  template void gen_z_limits<T>(int, bool);                                            \
+  template void gen_y_limits<T>(int);                                                  \
+  template void gen_x_limits<T>(int, int, bool);                                       \
   template void gen_zfwd<T>(const GenAxis &, const FusedGeom &, const void *, bool,    \
                             C2<T> *, bool, const YlmParams &, const double[3],         \
                             cudaStream_t);                                             \

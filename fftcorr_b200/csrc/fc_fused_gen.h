@@ -15,9 +15,15 @@ constexpr int kGenMaxPairs = 16;
 struct GenAxis {
   GPlan plan;
   DeviceBuffer tw;
-  // row: the z axis.
-  void init(int L, bool row, bool fp64);
+  void init(int L, bool fp64);
 };
+// Shared-memory limits of an axis's kernels.
+template <typename T>
+void gen_z_limits(int n2, bool weighted);
+template <typename T>
+void gen_y_limits(int n1);
+template <typename T>
+void gen_x_limits(int n0, int mode, bool even);
 
 // Whether an axis (of rows, or of columns) of this length fits, in either
 // precision.
