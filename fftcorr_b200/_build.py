@@ -29,8 +29,8 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 DEFAULT_REFERENCE = os.environ.get("FFTCORR_REFERENCE")
 
-SOURCES = ["fc_core.cu", "fc_hist.cu", "fc_assign.cu", "fc_fused.cu", "fc_fused_gen.cu", "fc_corr.cu",
-           "fc_batch.cu", "fc_catalog.cu", "fc_serve.cu"]
+SOURCES = ["fc_core.cu", "fc_hist.cu", "fc_assign.cu", "fc_fused.cu", "fc_fused_gen_f32.cu",
+           "fc_fused_gen_f64.cu", "fc_corr.cu", "fc_batch.cu", "fc_catalog.cu", "fc_serve.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -42,7 +42,7 @@ NVCC_FLAGS = [
 # the FFT passes, where fused multiply-adds only change rounding inside the
 # transform (which differs from FFTW's anyway) and halve the arithmetic.
 NO_FMAD = ["-fmad=false"]
-FMAD_OK = {"fc_fused.cu", "fc_fused_gen.cu"}
+FMAD_OK = {"fc_fused.cu", "fc_fused_gen_f32.cu", "fc_fused_gen_f64.cu"}
 
 
 def _run(cmd, cwd=None):

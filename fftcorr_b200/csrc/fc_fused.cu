@@ -134,7 +134,7 @@ __device__ __forceinline__ RowPoly load_row_poly(const float4 *tab, int64_t row,
 
 // --------------------------------------------------------------------------
 // Power-of-two lengths, with the register-resident engine (reg_fft in
-// fc_fft.cuh); other lengths are fc_fused_gen.cu's.  B2 columns per CTA keep the CTA at <= 1024
+// fc_fft.cuh); other lengths are fc_fused_gen.cuh's.  B2 columns per CTA keep the CTA at <= 1024
 // threads (TPC = L/8 threads per column).
 template <typename T, int L>
 struct P2 {

@@ -1,4 +1,4 @@
-// fc_fused_gen.cu -- the passes of the fused correlator (fc_fused.cu) along
+// fc_fused_gen.cuh -- the passes of the fused correlator (fc_fused.cu) along
 // an axis whose length is not a power of two, any product of 2, 3, 5 and 7,
 // even or odd, with the transform of fc_gfft.cuh.
 //
@@ -20,7 +20,10 @@
 // passes (two or three CTAs of an SM at up to 80 registers).  One column per
 // thread instead of two took y 91 us and x 184 us; 64-byte rows (half the
 // tile, more CTAs) y 76 and x 162 us, from bank conflicts and scattered
-// twiddle loads.
+// twiddle loads.  (fc_fused_gen_f32.cu and fc_fused_gen_f64.cu compile them,
+// side by side.)
+#pragma once
+
 #include <algorithm>
 
 #include "fc_fused_gen.h"
@@ -471,7 +474,7 @@ __device__ __forceinline__ float &comp(CPair &v, int c) {
 }
 __device__ __forceinline__ double &comp(double2 &v, int c) { return c ? v.y : v.x; }
 
-// ELL: -1 unweighted, else the weight's multipole.  np elements per CTA, each
+// ELL: the weight's multipole (unweighted: 0, with value0 = 1).  np elements per CTA, each
 // of 2 W rows.  IN: the cells' type, WT: the precision in which they are
 // weighted; the result is rounded to T once.
 template <typename T, int ELL, typename IN, typename WT>
@@ -521,12 +524,7 @@ __global__ void __launch_bounds__(kRowThreads, sizeof(WT) == 4 ? 5 : 4)
         for (int q = 0; q < R; ++q) d[q][c] = on ? src[c * N + q * f.LR] : (IN)0;
       }
       E v[R];
-      if constexpr (ELL < 0) {
-#pragma unroll
-        for (int q = 0; q < R; ++q)
-#pragma unroll
-          for (int c = 0; c < NR; ++c) comp(v[q], c) = (T)d[q][c];
-      } else if constexpr (ELL == 0) {
+      if constexpr (ELL == 0) {
 #pragma unroll
         for (int q = 0; q < R; ++q)
 #pragma unroll
@@ -718,31 +716,11 @@ void x_kernel(int mode, bool even, F &&f) {
 
 }  // namespace
 
-bool gen_supported(int L, bool row) {
-  GPlan p;
-  if (!gplan_length(L, &p)) return false;
-  if (row) return row_smem(L, 1) <= kGenSmem;
-  return col_smem(L) <= kGenSmem;
-}
-
-void GenAxis::init(int L, bool fp64) {
-  FC_REQUIRE(gplan_length(L, &plan), FC_ERR_UNSUPPORTED,
-             "grid size has a prime factor above 7");
-  auto put = [&](const auto &t) {
-    tw.resize(t.size() * sizeof(t[0]));
-    FC_CUDA(cudaMemcpy(tw.get(), t.data(), t.size() * sizeof(t[0]),
-                       cudaMemcpyHostToDevice));
-  };
-  if (fp64) put(gplan_twiddles<double2>(plan));
-  else put(gplan_twiddles<float2>(plan));
-}
-
 // Calls f(kernel) for every z kernel of a cell type and weights' precision.
 template <typename T, typename IN, typename WT, typename F>
 void z_kernels(bool weighted, F &&f) {
-  f(k_gzfwd<T, -1, IN, WT>);
-  if (!weighted) return;
   f(k_gzfwd<T, 0, IN, WT>);
+  if (!weighted) return;
   f(k_gzfwd<T, 2, IN, WT>);
   f(k_gzfwd<T, 4, IN, WT>);
 }
@@ -783,16 +761,17 @@ void gen_zfwd(const GenAxis &a, const FusedGeom &g, const void *rho, bool f32, C
   const int np = row_elems(a.plan, (nrows + NR - 1) / NR);
   const unsigned blocks = (unsigned)((nrows + NR * np - 1) / (NR * np));
   const size_t sm = row_smem(g.n2, np);
+  YlmParams one{};
+  one.value0 = 1.0;
   auto run = [&](auto in, auto wt) {
     using IN = decltype(in);
     using WT = decltype(wt);
     auto go = [&](auto kernel) {
       launch_small(kernel, blocks, row_threads(a.plan, np), sm, s,
-                   static_cast<const IN *>(rho), W, g, a.plan, a.tw.as<C2<T>>(), np, p,
-                   xyz0[0], xyz0[1], xyz0[2]);
+                   static_cast<const IN *>(rho), W, g, a.plan, a.tw.as<C2<T>>(), np,
+                   weight ? p : one, xyz0[0], xyz0[1], xyz0[2]);
     };
-    if (!weight) go(k_gzfwd<T, -1, IN, WT>);
-    else if (p.ell == 0) go(k_gzfwd<T, 0, IN, WT>);
+    if (!weight || p.ell == 0) go(k_gzfwd<T, 0, IN, WT>);
     else if (p.ell == 2) go(k_gzfwd<T, 2, IN, WT>);
     else go(k_gzfwd<T, 4, IN, WT>);
   };
@@ -865,7 +844,5 @@ void gen_zinv(const GenAxis &a, const FusedGeom &g, const C2<T> *Wry, double *rs
                             C2<T> *, cudaStream_t);                                    \
   template void gen_zinv<T>(const GenAxis &, const FusedGeom &, const C2<T> *,         \
                             double *, const T *, bool, cudaStream_t);
-FC_GEN(float)
-FC_GEN(double)
 
 }  // namespace fc

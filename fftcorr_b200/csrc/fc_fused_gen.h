@@ -1,5 +1,5 @@
 // fc_fused_gen.h -- launchers of the fused passes along axes whose length is
-// not a power of two (fc_fused_gen.cu).
+// not a power of two (fc_fused_gen.cuh).
 #pragma once
 
 #include "fc_common.cuh"

@@ -1,6 +1,6 @@
 // fc_gfft.cuh -- shared-memory FFT of any length with prime factors 2, 3, 5
 // and 7 (the lengths that the power-of-two engine of fc_fft.cuh does not
-// take), for the generic passes of fc_fused_gen.cu.
+// take), for the generic passes of fc_fused_gen.cuh.
 //
 // A length is split into as few radices of at most 10 as it has (378 = 9 x 7
 // x 6, 1000 = 10 x 10 x 10), one Stockham pass each.  The first pass reads

@@ -32,11 +32,11 @@ def test_chained_kernels_read_by_plain_loads(name):
 
 
 def test_the_passes_and_histograms_are_found():
-    text = "".join(_read(n) for n in ("fc_fused.cu", "fc_fused_gen.cu", "fc_hist.cu"))
+    text = "".join(_read(n) for n in ("fc_fused.cu", "fc_fused_gen.cuh", "fc_hist.cu"))
     chained = [k for k, _, body in KERNEL.findall(text) if "grid_chain()" in body]
     assert len(chained) == len(re.findall(r"^  grid_chain\(\);", text, re.M)) >= 18
 
 
-@pytest.mark.parametrize("name", ["fc_fused.cu", "fc_fused_gen.cu", "fc_hist.cu"])
+@pytest.mark.parametrize("name", ["fc_fused.cu", "fc_fused_gen.cuh", "fc_hist.cu"])
 def test_read_only_loads_are_of_tables(name):
     assert set(re.findall(r"__ldg\(&(\w+)", _read(name))) <= TABLES
