@@ -58,7 +58,7 @@ YlmParams make_ylm_params(int ell, int m, double coeff) {
   if (m != 0) isqpi *= sqrt(2.0);
   p.isqpi = isqpi;
   // The (ell, m) constant of each real-form Y_lm (spherical_harmonics.h:
-  // 107-176), folded with isqpi for the FP32 evaluator.
+  // 107-176), folded with isqpi for the row polynomials.
   double c = 1.0;
   if (ell == 2) {
     c = m == 2 ? sqrt(15.0 / 32.0) : m == 0 ? sqrt(5.0 / 16.0) : sqrt(15.0 / 8.0);
