@@ -1414,7 +1414,9 @@ bool FusedSurvey::supported(const int shape[3], int rsize) {
 FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
                          bool fp64, bool even, bool survey)
     : fp64_(fp64) {
-  if (fault_fires(kFaultFftPlan))
+  // (A planned failure takes a periodic correlator's plan, cuFFT's or this; a
+  // survey that makes no cuFFT plan passes it over.)
+  if (!survey && fault_fires(kFaultFftPlan))
     FC_THROW(FC_ERR_CUFFT, "injected FFT plan creation failure");
   g.n0 = shape[0];
   g.n1 = shape[1];

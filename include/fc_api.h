@@ -496,7 +496,8 @@ int fc_host_unregister(void *ptr);
  * would surface, before the CUDA or cuFFT call, so no GPU faults.  With
  * FC_FAULT_DEVICE_ALLOC, the n-th device allocation of the library from now
  * fails with FC_ERR_ALLOC.  With FC_FAULT_FFT_PLAN, the n-th FFT plan
- * creation (cuFFT's, or the fused passes' own) fails with FC_ERR_CUFFT.  n <= 0 disarms.  The reference fails
+ * creation (cuFFT's, or the fused passes' of a periodic correlator) fails with
+ * FC_ERR_CUFFT.  n <= 0 disarms.  The reference fails
  * the same way on an allocation or an FFTW plan that cannot be made
  * (cc/grid/fft_grid.cc:126,153). */
 enum { FC_FAULT_DEVICE_ALLOC = 1, FC_FAULT_FFT_PLAN = 2 };

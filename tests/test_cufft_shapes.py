@@ -69,6 +69,14 @@ def test_plan_failure_leaves_nothing_behind(kind):
     _compare_results(c.results(), oracle(grid, *args), FP64_RTOL, kind)
 
 
+def test_fused_surveys_make_no_plan_that_could_fail():
+    args = (10.0, POSMIN, 2, 60.0, 10.0, 0.2, 0.04, 2)
+    _lib.call("fc_fault_inject", _lib.FC_FAULT_FFT_PLAN, 1)
+    fb.Correlator((32, 30, 36), *args)
+    with pytest.raises(_lib.FcError):   # the planned failure is still to come
+        fb.Correlator((22, 26, 33), *args)
+
+
 @pytest.mark.parametrize("shape", [(4, 6, 4096), (5, 4, 2592), (2, 3, 2625)])
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
 def test_long_rows(shape, precision, monkeypatch):
