@@ -1274,8 +1274,9 @@ void correlator_time_kernels(Correlator *c, int which, cudaStream_t s) {
   }
 }
 
-// Device bytes of a correlator (see Correlator::allocate and make_plans);
-// the cuFFT work area is estimated as one complex grid.
+// Device bytes of a correlator for autocorrelations of grids whose cells have
+// its precision (see Correlator::allocate, FusedSurvey and make_plans); the
+// cuFFT work area is estimated as one complex grid.
 size_t correlator_footprint(int kind, const int shape[3], double cell,
                             double rmax, double kmax, int maxell,
                             int precision) {
@@ -1285,33 +1286,51 @@ size_t correlator_footprint(int kind, const int shape[3], double cell,
   size_t bytes = 0;
   const char *mode = std::getenv("FFTCORR_B200_FFT");
   const bool want_fused = !(mode && std::string(mode) == "cufft");
+  // Cells of a subgrid in the range of a histogram, at most: those of an
+  // ellipsoid of semi-axes a, b, c cells, grown by half a cell's diagonal.
+  auto in_range = [](size_t cells, double a, double b, double c) {
+    const double grow = 1.0 + 0.5 * sqrt(3.0) / std::min(a, std::min(b, c));
+    const double n = 4.0 / 3.0 * M_PI * a * b * c * grow * grow * grow;
+    return n < (double)cells ? (size_t)n + 1 : cells;
+  };
+  const double rr = rmax / cell, kk = kmax * cell / (2.0 * M_PI);
+  const size_t rin = in_range(g.rcells(), rr, rr, rr);
+  const size_t kin = in_range(g.kcells(), kk * shape[0], kk * shape[1], kk * shape[2]);
+  // A cell's separation is that of its mirror image where the axis is its own
+  // mirror image (otherwise the bins may differ, and the whole is counted).
+  bool mirrored = true;
+  for (int i = 0; i < g.rsize; ++i)
+    mirrored = mirrored && g.raxis[i] == -g.raxis[g.rsize - 1 - i];
   if (want_fused && FusedSurvey::supported(g.shape, g.rsize)) {
+    const bool survey = kind == FC_SURVEY;
+    const size_t rows = (size_t)g.shape[0] * g.shape[1];
     const size_t h = (g.shape[2] / 2 + 1 + 15) / 16 * 16;   // row pitch
-    // W, and G with a survey
-    bytes += (kind == FC_SURVEY ? 2 : 1) * (size_t)g.shape[0] * g.shape[1] * h * eb;
-    // Wr and Wry, and below the r-subgrid, whole: the even form keeps half.
-    bytes += (size_t)g.rsize * g.shape[1] * h * eb;
-    bytes += (size_t)g.rsize * g.rsize * h * eb;
-    if (precision != FC_FP64) {                              // FP32 density,
-      bytes += g.ncells() * 4;
-      if (kind == FC_SURVEY) bytes += (size_t)g.shape[0] * g.shape[1] * 32;  // row table
-      const int m = g.shape[2] / 2;
-      if (kind == FC_SURVEY && m >= 32 && m <= 2048 && (m & (m - 1)) == 0)        // paired z pass:
-        bytes += (size_t)g.shape[0] * g.shape[1] * (h * eb + 32);  // W2, table
-    }
-    if (kind == FC_SURVEY) {
+    const size_t rx = mirrored || !survey ? g.rsize / 2 + 1 : g.rsize;
+    bytes += (survey ? 2 : 1) * rows * h * eb;               // W, and a survey's G
+    bytes += rx * (g.shape[1] + g.rsize) * h * eb;           // Wr, Wry
+    // Stored cells of the subgrids.
+    const size_t rc = rx * g.rsize * g.rsize;
+    const size_t kc = (size_t)g.kshape[0] * g.kshape[1] * ((g.kshape[2] / 2 + 4) / 4 * 4);
+    const bool wide = precision != FC_FP64 && wide_rows(g.shape[2]);
+    const int m = g.shape[2] / 2;
+    if (survey && precision != FC_FP64 && !wide && m >= 32 && m <= 1024 &&
+        (m & (m - 1)) == 0)                                  // paired z pass:
+      bytes += rows * (h * eb + 2 * 32);                     // W2, row tables
+    if (survey) {
       const int nlm = maxell == 0 ? 1 : maxell == 2 ? 6 : 15;
-      bytes += (size_t)nlm * (g.kcells() + g.rcells()) * rb;   // weight tables
+      bytes += (size_t)nlm * (kc + rc) * (wide ? 8 : rb);    // weight tables
+      bytes += (size_t)(g.nrows + (wide ? 1 : 0)) * (kc + rc) * 8;  // subgrids
     } else {
-      bytes += (size_t)g.nrows * (g.kcells() + g.rcells()) * 8;  // bin weights
+      bytes += (kc + rc) * 8;                                // subgrids
+      bytes += (size_t)g.nrows * (rin + kin) * 8;              // bin weights
     }
   } else {
     bytes += g.nreal_padded() * rb;                          // work
     if (kind == FC_SURVEY) bytes += g.ncomplex() * eb;       // grid2 FFT
     bytes += g.ncomplex() * eb;                              // cuFFT work area
+    bytes += (g.rcells() + g.kcells()) * (size_t)(8 * g.nrows);  // subgrids
   }
-  // Subgrids per multipole and bin indices.
-  bytes += (g.rcells() + g.kcells()) * (size_t)(8 * g.nrows + 4);
+  bytes += (rin + kin) * 4;                                  // bin indices
   return bytes + (4 << 20);
 }
 

@@ -51,3 +51,32 @@ def test_density_copy_on_first_fp64_cells(kind):
         c.autocorrelate(grids["fp64"])
         assert _device_bytes() == before + 4 * values.size
         _compare_results(c.results(), ref, FP64_RTOL, "FP64 cells", fp32=True)
+
+
+@pytest.mark.parametrize("kind", ["periodic", "survey"])
+@pytest.mark.parametrize("n2", [128, 120, 105])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_footprint_of_a_correlator(kind, n2, precision):
+    """The bytes by which larger subgrids make a correlator grow, from the
+    server's estimate and from what is allocated: the estimate holds them, and
+    is at most a quarter above (cells in range are counted by volume)."""
+    shape, cell = (128, 96, n2), 10.0
+    data = catalog_spec(CAT_CLUSTERED_BOX, n=1000, boxsize=900.0, ncentres=10, sigma=5.0,
+                        seed=1)
+
+    def both(rmax, kmax):
+        job = JobSpec(kind, shape, cell, data, data if kind == "survey" else None,
+                      posmin=POSMIN, rmax=rmax, dr=rmax / 8, kmax=kmax, dk=kmax / 8,
+                      maxell=2, precision=precision)
+        args = (0, rmax, rmax / 8, kmax, kmax / 8, 2)
+        before = _device_bytes()
+        if kind == "periodic":
+            c = fb.PeriodicCorrelator(shape, cell, *args, precision=precision)
+        else:
+            c = fb.Correlator(shape, cell, POSMIN, *args, precision=precision)
+        made = _device_bytes() - before
+        del c
+        return job.footprint, made
+
+    estimate, made = np.subtract(both(397.0, 0.3), both(53.0, 0.05))
+    assert made <= estimate <= 1.25 * made, (estimate, made)
