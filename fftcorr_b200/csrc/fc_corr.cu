@@ -1307,7 +1307,8 @@ size_t correlator_footprint(int kind, const int shape[3], double cell,
     const size_t h = (g.shape[2] / 2 + 1 + 15) / 16 * 16;   // row pitch
     const size_t rx = mirrored || !survey ? g.rsize / 2 + 1 : g.rsize;
     bytes += (survey ? 2 : 1) * rows * h * eb;               // W, and a survey's G
-    bytes += rx * (g.shape[1] + g.rsize) * h * eb;           // Wr, Wry
+    bytes += rx * g.rsize * h * eb;                          // Wry
+    if (rx > (size_t)g.shape[0]) bytes += rx * g.shape[1] * h * eb;  // Wr
     // Stored cells of the subgrids.
     const size_t rc = rx * g.rsize * g.rsize;
     const size_t kc = (size_t)g.kshape[0] * g.kshape[1] * ((g.kshape[2] / 2 + 4) / 4 * 4);

@@ -1446,7 +1446,7 @@ FusedSurvey::FusedSurvey(const int shape[3], int rsize, const int kshape[3],
   const size_t nc = (size_t)g.n0 * g.n1 * g.hp;
   W.resize(nc * eb);
   if (survey) G.resize(nc * eb);
-  Wr.resize((size_t)g.nri * g.n1 * g.hp * eb);
+  if (g.nri > g.n0) Wr.resize((size_t)g.nri * g.n1 * g.hp * eb);
   Wry.resize((size_t)g.nri * g.rs * g.hp * eb);
   if (survey && wide()) {
     kterm.resize(k_cells() * sizeof(double));
@@ -1605,7 +1605,7 @@ void FusedSurvey::xcorr(int mode, double *ksub, const void *ktab_v, double w00,
                         bool first, cudaStream_t s) {
   const T *ktab = static_cast<const T *>(ktab_v);
   if (!is_p2(g.n0)) {
-    gen_x<T>(gx, g, mode, W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub,
+    gen_x<T>(gx, g, mode, W.as<C2<T>>(), G.as<C2<T>>(), inverse_rows<T>(), ksub,
              ktab, (T)w00, first, s);
     return;
   }
@@ -1614,7 +1614,7 @@ void FusedSurvey::xcorr(int mode, double *ksub, const void *ktab_v, double w00,
       using Y = PY<L, kXB>;
       auto go = [&](auto kernel, int nyq) {
         launch_after(kernel, dim3((g.h + Y::B - 1) / Y::B, g.n1), Y::THREADS, Y::smem, s, 
-            W.as<float2>(), G.as<float2>(), Wr.as<float2>(), ksub, g, tabx.as<float2>(),
+            W.as<float2>(), G.as<float2>(), inverse_rows<float>(), ksub, g, tabx.as<float2>(),
             ktab, (float)w00, nyq, first);
       };
       const int nyq = nyq_group<Y::B>(ksub != nullptr);
@@ -1627,7 +1627,7 @@ void FusedSurvey::xcorr(int mode, double *ksub, const void *ktab_v, double w00,
       using Q = P2<T, L>;
       auto go = [&](auto kernel) {
         launch_small(kernel, dim3((g.h + Q::B - 1) / Q::B, g.n1), Q::THREADS, p2_col_smem<T, L>(), s, 
-            W.as<C2<T>>(), G.as<C2<T>>(), Wr.as<C2<T>>(), ksub, g, tabx.as<C2<T>>(), ktab,
+            W.as<C2<T>>(), G.as<C2<T>>(), inverse_rows<T>(), ksub, g, tabx.as<C2<T>>(), ktab,
             w00, first);
       };
       if (mode == 3) go(k_xcorr_p2<L, 3, true>);
@@ -1649,18 +1649,18 @@ void FusedSurvey::yinv(cudaStream_t s) {
         using Y = PY<L>;
         dim3 grid((g.h + Y::B - 1) / Y::B, g.nri);
         launch_after(k_yinv_pp<L>, grid, Y::THREADS, Y::smem, s, 
-            Wr.as<float2>(), Wry.as<float2>(), g, taby.as<float2>(),
+            inverse_rows<float>(), Wry.as<float2>(), g, taby.as<float2>(),
             nyq_group<Y::B>(false));
       } else {
         dim3 grid((g.h + Q::B - 1) / Q::B, g.nri);
         launch_small(k_yinv_p2<T, L>, grid, Q::THREADS, p2_col_smem<T, L>(), s, 
-            Wr.as<C2<T>>(), Wry.as<C2<T>>(), g, taby.as<C2<T>>());
+            inverse_rows<T>(), Wry.as<C2<T>>(), g, taby.as<C2<T>>());
       }
     });
     FC_LAUNCH_CHECK();
     return;
   }
-  gen_yinv<T>(gy, g, Wr.as<C2<T>>(), Wry.as<C2<T>>(), s);
+  gen_yinv<T>(gy, g, inverse_rows<T>(), Wry.as<C2<T>>(), s);
 }
 
 template <typename T>

@@ -110,6 +110,13 @@ class FusedSurvey {
   void prepare_product();
   // Whether the z passes are the power-of-two ones (even rows of m pairs).
   bool p2_rows() const;
+  // Where the x pass leaves its inverse's rows: in W itself, whose columns a CTA
+  // has read before it writes them, unless the r-subgrid has more rows.
+  template <typename T>
+  typename Vec2<T>::type *inverse_rows() const {
+    using C = typename Vec2<T>::type;
+    return g.nri > g.n0 ? Wr.as<C>() : W.as<C>();
+  }
   // Whether the FP32 passes weight in FP64, cells, k- and r-subgrids alike.
   bool wide() const { return !fp64_ && wide_rows(g.n2); }
   bool reads_as_is(bool f32) const { return fp64_ || f32 || wide(); }
@@ -139,7 +146,7 @@ class FusedSurvey {
   bool product_ready = false;
   GenAxis gx, gy, gz;  // of the axes that are not powers of two
   DeviceBuffer tabx, taby, tabz;
-  DeviceBuffer W, G, Wr, Wry, rho32;
+  DeviceBuffer W, G, Wr, Wry, rho32;  // Wr: see inverse_rows
   DeviceBuffer W2, rowtab2;  // the second term of a paired z pass
   DeviceBuffer kterm, rterm;  // a wide term's subgrids before their weights
   std::map<int, DeviceBuffer> ktabs;
