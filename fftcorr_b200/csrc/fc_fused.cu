@@ -1,8 +1,9 @@
-// fc_fused.cu -- the survey correlator's per-(ell, m) work as five fused,
-// hand-written FFT passes over HBM (no cuFFT), with the Y_lm weighting, the
-// conjugate product, the k-subgrid extraction and the r-subgrid extraction
-// folded into them, and the inverse transform pruned to the rows the
-// r-subgrid needs.
+// fc_fused.cu -- correlations as five fused, hand-written FFT passes over HBM
+// (no cuFFT), with the Y_lm weighting, the conjugate product, the k-subgrid
+// extraction and the r-subgrid extraction folded into them, and the inverse
+// transform pruned to the rows the r-subgrid needs: a survey correlation's,
+// (ell, m) by (ell, m), and a periodic one's, once without the weights (those of
+// all its multipoles are in the histograms).
 //
 // Per (ell, m), for the half-complex work array W[x][y][kz] (kz < N2/2+1):
 //   zfwd   W[x][y][:] = R2C_z( Y_lm(cell) * rho[x][y][:] )   (make_ylm + r2c
@@ -11,7 +12,8 @@
 //   xcorr  per (ky, kz) column: F = DFT_x(W); P = F * conj(G)
 //          (array_ops.cc:139-163); ksub += Y_lm(k) W(k)^-2 4 pi Re P on the
 //          k-subgrid (fft_grid.cc:215-258); Wr[ri][ky][kz] = IDFT_x(P) only
-//          at the rs rows x = (N0 - rs/2 + ri) mod N0 of the r-subgrid
+//          at the rs rows x = (N0 - rs/2 + ri) mod N0 of the r-subgrid (in W's
+//          place, where it has no more rows than the grid)
 //   yinv   Wry[ri][rj][kz] = IDFT_y(Wr) at the rs rows of the r-subgrid
 //   zinv   rsub[ri][rj][rk] += Y_lm(r) 4 pi/N * C2R_z(Wry)[rk] (fft_grid.cc:
 //          182-210)
@@ -27,6 +29,17 @@
 // 14 us (a correlation 11.8 -> 10.8 ms); at 256^3 FP64: 105 -> 85 us, 15 -> 9
 // us, 9 -> 8 us; the x pass at 64^3, whose extraction walked the k-subgrid's
 // rows one after another, 27 -> 11 us.
+// Two columns that share a transform share its rounding too: the larger one's
+// reaches the smaller, of order 1e-7 (FP32) of the larger per value, and a
+// column of zeros beside one that is not comes out at that level instead of
+// zero.  The same holds of the rows that share one in fc_fused_gen.cuh.  The sum
+// of the squared errors is that of separate transforms, but the two halves of r
+// no longer average separate ones.  Errors of xi against 64 bits (2-norm, mean of
+// 6 fields; in brackets cuFFT's or the passes' before): survey 64^3 1.58e-7
+// (1.83e-7), 125 x 180 x 126 7.2e-8 (8.0e-8), 128^3 2.17e-7 (2.41e-7); periodic
+// 125 x 126 x 120 8.6e-8 (1.15e-7), 128^3 2.55e-7 (3.04e-7), 125 x 81 x 105
+// 1.27e-7 (1.05e-7) and in FP64 4.4e-16 (2.8e-16); survey 128^3 FP64 3.1e-16
+// (3.3e-16).
 // grid2's transform G (correlator.h:53-77) is zfwd (no weighting) + yfwd +
 // DFT_x.  Bytes per (ell, m) at 512^3 FP32: ~4 GB instead of ~11 GB for
 // separate make_ylm / cuFFT r2c / multiply / extract / cuFFT c2r passes.
@@ -88,10 +101,7 @@ __host__ __device__ __forceinline__ int row_poly_form(int ell, int m) {
 }
 
 // z of the cell `i` after the one at z0 (FP32: zt), rounded once in rows of 32
-// pairs: these stood with the mixed-radix rows before, which round it once.  With
-// the twiddles of r8_twiddle_table the error of 64^3 correlations at ell <= 4
-// against 64 bits (2-norm, mean of 6 fields) is 2.15e-7 in xi and 1.17e-7 in P,
-// against 2.34e-7 and 1.34e-7 without the two.
+// pairs, which stood with the mixed-radix rows before, as these round it.
 template <int L>
 __device__ __forceinline__ float row_z(double z0, float zt, int i) {
   if constexpr (L == 32) return (float)(z0 + i);
