@@ -57,10 +57,6 @@ constexpr uint32_t kWarpUnit = 32;
 // catalog then has 32 or fewer in a tenth of its units) every unit goes to a
 // CTA, and the warps' launches, 2 us a colour pass, are left out.
 constexpr int64_t kDenseUnit = 40;
-// With more than this the CTAs take their dense form (ScatterP::min_blocks; at
-// 48 a unit, 50M of a sector in 512^3, it takes 3.57 ms against 3.41), except
-// in a batch, whose boxes fill one another's waits (12 boxes 10.4 -> 10.6 ms).
-constexpr int64_t kDenseForm = 100;
 constexpr int kScatterThreads = 256;
 constexpr int kChunk = 256;      // particles staged per shared-memory chunk
 
@@ -484,12 +480,11 @@ struct ScatterP {
   // CTAs per SM.  TSC's table and its 27 sums a thread leave room for five.
   // The narrower stencils' units of some dozens of particles are bound by
   // latency and take eight (8M clustered points, CIC, 384^3, five: 1.62 ms,
-  // six: 1.59, eight: 1.51; a batch of 12 boxes 11.1 -> 10.7 ms); those of
-  // dense catalogs by the sums, which at eight spill (7.6M clustered points,
-  // CIC, 98^3: 1.27, 1.30 and 1.33 ms; 33M of a sector in 225^3: 1.98, 1.93,
-  // 2.04 ms; 300k in 64^3: 0.233, 0.235, 0.247 ms).
+  // six: 1.58, eight: 1.51; a batch of 12 boxes 11.1 -> 10.7 ms).  CIC's sums
+  // spill at eight, which the units of dense catalogs pay for: these take six
+  // (Assignor::dense_form).
   static constexpr int min_blocks(bool dense) {
-    return TX != 2 ? kTile / TX : W == 3 || dense ? 5 : 8;
+    return TX != 2 ? kTile / TX : W == 3 ? 5 : W == 2 && dense ? 6 : 8;
   }
   static constexpr int FX = TX + W - 1;     // footprint extent along x
   static constexpr int FY = kTile + W - 1;  // ... along y and z
@@ -1026,9 +1021,9 @@ struct ScatterFns {
 };
 template <int S, typename KeyT, typename GT>
 ScatterFns scatter_fns_of() {
-  // (TSC's two forms would be the same.)
+  // (Only CIC's two forms differ.)
   return ScatterFns{{(const void *)k_scatter_p<S, KeyT, kUnitX, GT, false>,
-                     (const void *)k_scatter_p<S, KeyT, kUnitX, GT, S != 1>},
+                     (const void *)k_scatter_p<S, KeyT, kUnitX, GT, S == 3>},
                     (const void *)k_scatter_w<S, KeyT, GT>, ScatterP<S, kUnitX>::smem,
                     kWarpsPerCta * ScatterW<S>::DOUBLES * sizeof(double)};
 }
@@ -1071,6 +1066,7 @@ struct Assignor {
   DeviceBuffer pass_counters;          // per colour: the warps' units, CTAs'
                                        // units drawn, the CTAs' units
   std::vector<int64_t> color_offsets;  // per colour, into color_units
+  int64_t most_units = 0;              // of a colour
   ScatterFns scatter;                  // for this scheme, keys and cells
   unsigned scatter_ctas[2] = {0, 0}, scatter_w_ctas = 0;  // persistent CTAs of each
   DeviceBuffer partials;               // K-key block partials
@@ -1201,6 +1197,7 @@ struct Assignor {
     for (auto &l : lists) {
       flat.insert(flat.end(), l.begin(), l.end());
       color_offsets.push_back((int64_t)flat.size());
+      most_units = std::max(most_units, color_offsets.back() - color_offsets.end()[-2]);
     }
     color_units.resize(flat.size() * sizeof(uint32_t));
     FC_CUDA(cudaMemcpy(color_units.get(), flat.data(),
@@ -1213,6 +1210,26 @@ struct Assignor {
   }
 
   size_t key_bytes() const { return wide_keys ? 8 : 4; }
+
+  // Whether a catalog that leaves the warps out (kDenseUnit) takes the CTAs'
+  // dense form: with more than 150 particles a unit on average, or where a colour
+  // has at most 16 units per CTA, whose last ones then weigh more; not in a batch,
+  // whose boxes fill one another's waits (12 boxes, five CTAs per SM: 10.4 -> 10.6
+  // ms).  CIC at eight / six / five CTAs per SM (one B200, us; s a sector, 30% of
+  // its box, c a clustered box):
+  //   64^3 c 100k (49 a unit)     226 /  215 /  217
+  //   98^3 c 1M (114)             502 /  477 /  474
+  //   128^3 s 2M (122)            393 /  379 /  383
+  //   180^3 c 12.9M (266)        1194 / 1184 / 1225
+  //   225^3 s 33.7M (346)        2050 / 1920 / 1978
+  //   225^3 c 40M (410)          2804 / 2790 / 2890
+  //   300^3 s 40M (182)          2205 / 2161 / 2199   (27000 units a colour)
+  //   384^3 c 50M (113)          4196 / 4367 / 4696   (55000)
+  //   512^3 s 50M (48)           3394 / 3437 / 3577   (131000)
+  bool dense_form(int64_t n) const {
+    return !graph_mode &&
+           (n > 150 * nunits || most_units <= 16 * (int64_t)scatter_ctas[1]);
+  }
 
   // Key/index buffers for assigning `need` particles straight from a
   // caller's device array (nothing is buffered).
@@ -1496,7 +1513,7 @@ struct Assignor {
     cudaStream_t st = stream();
     if (!graph_mode) window_timer.start(st);
     const uint32_t warp_unit = n > kDenseUnit * nunits ? 0u : kWarpUnit;
-    const bool dense = !graph_mode && n > kDenseForm * nunits;
+    const bool dense = warp_unit == 0 && dense_form(n);
     const int unit_cells = unit_x * kTile * kTile;
     k_unit_starts<KeyT><<<grid_for(nunits + 1, 256), 256, 0, st>>>(
         sk, n, nunits, unit_cells, unit_start.as<uint32_t>());
