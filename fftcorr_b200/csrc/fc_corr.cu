@@ -514,6 +514,7 @@ struct Correlator {
       const char *mode = std::getenv("FFTCORR_B200_FFT");
       const bool want_fused = !(mode && std::string(mode) == "cufft");
       upload_axes();
+      settle();
       bins_even = build_bins();
       // (A periodic autocorrelation's P is even whatever the bins are.)
       if (want_fused && FusedSurvey::supported(geo.shape, geo.rsize))
@@ -530,8 +531,7 @@ struct Correlator {
         fused->prepare_tables(2 * (geo.nrows - 1), (double)geo.ncells(),
                               d_raxis.as<double>(), kaxes(),
                               geo.kcells() > 0, stream);
-      // The tables are complete before any stream reads them.
-      FC_CUDA(cudaStreamSynchronize(stream));
+      settle();
     } catch (...) {
       // A failed construction leaves no stream, event or plan behind (the
       // buffers free themselves).
@@ -541,6 +541,14 @@ struct Correlator {
   }
 
   ~Correlator() { release_handles(); }
+
+  // Waits for what makes the tables: the correlator's stream, and the default
+  // one, whose fills and small copies from pageable memory are only enqueued when
+  // their calls return and which other streams do not wait for.
+  void settle() {
+    FC_CUDA(cudaStreamSynchronize(stream));
+    FC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  }
 
   void release_handles() {
     if (stream) cudaStreamSynchronize(stream);
@@ -932,6 +940,7 @@ struct Correlator {
     hist_items([&](int) { return r.as<double>(); }, rperm_full.as<uint32_t>(), it, fo);
     HistPlan h;
     h.upload(it, fo);
+    settle();
     rsub_cross = std::move(r);
     hist_cross = std::move(h);
     fused_cross = std::move(f);
