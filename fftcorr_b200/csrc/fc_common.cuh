@@ -225,7 +225,13 @@ struct LaunchShape {
 // kernels' shared memory differs from one to the next: a CTA that arrives
 // early runs with the split of L1 and shared memory that the kernel before it
 // chose.  launch_small takes the early start only for grids of at most four
-// CTAs per SM, where the latency counts.)
+// CTAs per SM, where the latency counts.  Whole correlations, us, with the line at
+// none / 1 / 2 / 4 / 8 / 16 / any number of CTAs per SM: surveys at ell <= 4, 64^3
+// FP64 588 / 576 / 546 / 487 / 485 / 486 / 481, 128^3 FP64 989 / 987 / 967 / 964 /
+// 960 / 861 / 843, 256^3 FP64 3528 / 3546 / 3520 / 3538 / 3523 / 3521 / 3712, 144^3
+// FP32 1130 / 1089 / 1087 / 1089 / 1017 / 1019 / 1017, 240^3 FP32 2766 / 2768 / 2765
+// / 2691 / 2682 / 2628 / 2591; periodic 64^3 to 192^3 within 2% from 4 on.  So what
+// loses does so above 16, and a line there would gain more than four does.)
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -13,15 +13,16 @@
 // Measured per launch on a 250 x 360 x 378 FP32 grid (34M cells, one B200),
 // against the engine before it (mixed radices chosen largest power of two
 // first, loads and stores as passes of their own through shared memory, one
-// column per thread, per-element modulos): z 339 -> 100 us, y 164 -> 67 us,
-// x with product and inverse 611 -> 134 us, inverse y 41 -> 19 us; a cross
-// correlation at ell <= 4 18.4 -> 5.6 ms.  The y pass moves 274 MB at 4.1
-// TB/s; all are bound by instruction issue and by barriers between the
-// passes (two or three CTAs of an SM at up to 80 registers).  One column per
-// thread instead of two took y 91 us and x 184 us; 64-byte rows (half the
-// tile, more CTAs) y 76 and x 162 us, from bank conflicts and scattered
-// twiddle loads.  (fc_fused_gen_f32.cu and fc_fused_gen_f64.cu compile them,
-// side by side.)
+// column per thread, per-element modulos): z 339 -> 104 us, y 164 -> 67 us,
+// x with product and inverse 611 -> 110 us (134 before the even form), inverse y
+// 41 -> 15 us (19); a cross correlation at ell <= 4 18.4 -> 5.05 ms.  The y pass
+// moves 274 MB at 4.1 TB/s; all are bound by instruction issue and by barriers
+// between the passes (two CTAs of an SM at 64 registers in y and at 80 in x, five
+// at up to 96 in z).  Before the even form, one column per thread instead of two
+// took y 91 us and x 184 us; 64-byte rows (half the tile, more CTAs) y 76 and x
+// 162 us, from bank conflicts and scattered twiddle loads.
+//
+// (fc_fused_gen_f32.cu and fc_fused_gen_f64.cu compile them, side by side.)
 #pragma once
 
 #include <algorithm>
