@@ -730,7 +730,8 @@ void gen_z_limits(int n2, bool weighted) {
   auto set = [](auto kernel) { big_smem(kernel); };
   if constexpr (sizeof(T) == 4) {
     if (wide_rows(n2)) {
-      z_kernels<T, T, double>(weighted, set);
+      z_kernels<T, T, T>(false, set);
+      if (weighted) z_kernels<T, T, double>(true, set);
       z_kernels<T, double, double>(weighted, set);
     } else {
       z_kernels<T, T, T>(weighted, set);
@@ -777,9 +778,9 @@ void gen_zfwd(const GenAxis &a, const FusedGeom &g, const void *rho, bool f32, C
     else go(k_gzfwd<T, 4, IN, WT>);
   };
   if constexpr (sizeof(T) == 4) {
-    if (wide_rows(g.n2) && f32) run(T(), double());
-    else if (wide_rows(g.n2)) run(double(), double());
-    else run(T(), T());
+    if (wide_rows(g.n2) && !f32) run(double(), double());
+    else if (wide_rows(g.n2) && weight) run(T(), double());
+    else run(T(), T());  // (the cells as they are)
   } else {
     run(T(), T());
   }

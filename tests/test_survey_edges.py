@@ -72,6 +72,34 @@ def test_odd_fp32_rows_take_either_cell_type(shape, cross):
         np.testing.assert_array_equal(results[0][key], results[1][key])
 
 
+@pytest.mark.parametrize("cross", [False, True])
+def test_odd_fp32_rows_of_periodic_grids(cross):
+    """The same of periodic correlations, which weight no cells."""
+    shape = (30, 64, 27)
+    rng = np.random.default_rng(13)
+    args = (CELL, TSC_ALIASED_CORRECTION, 50.0, 6.0, 0.15, 0.03, 4)
+    values = [rng.standard_normal(shape).astype(np.float32) for _ in range(2)]
+    results = []
+    for precision in ("fp32", "fp64"):
+        grids = []
+        for v in values:
+            g = fb.ConfigSpaceGrid.from_geometry(shape, np.zeros(3), CELL,
+                                                 precision=precision)
+            _lib.call("fc_grid_upload", g.handle, _lib.dptr(v.astype(np.float64)))
+            grids.append(g)
+        c = fb.PeriodicCorrelator(shape, *args, precision="fp32")
+        if cross:
+            c.cross_correlate(*grids)
+        else:
+            c.autocorrelate(grids[0])
+        results.append(c.results())
+    ref = O.periodic_correlate(values[0].astype(np.float64), *args,
+                               grid2=values[1].astype(np.float64) if cross else None)
+    _compare_results(results[0], ref, FP64_RTOL, "odd rows", fp32=True)
+    for key in ("rhist", "khist"):
+        np.testing.assert_array_equal(results[0][key], results[1][key])
+
+
 def test_axes_that_are_not_their_own_mirror_image():
     """cell = 17.1 rounds the r axis differently at r and -r (1e-14 of a cell),
     which has to cancel between the two in the sums of a bin.  The field is
