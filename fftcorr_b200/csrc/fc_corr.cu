@@ -29,7 +29,7 @@
 //   cuFFT c2r  in place
 //   k_rsub     rsub += Y_lm(r)*4pi/N*work on the r-subgrid
 // then the deterministic histograms of every multipole (fc_hist.cuh), two
-// launches.
+// launches (large subgrids: multipole by multipole, Correlator::one_pair_rule).
 #include <cufft.h>
 
 #include <algorithm>
@@ -446,6 +446,8 @@ struct Correlator {
   DeviceBuffer rweights, kweights;
   DeviceBuffer d_raxis, d_kaxes, d_kwin;
   DeviceBuffer d_out;  // r histograms | k histograms | zero lag
+  bool one_pair = false;
+  std::vector<HistPlan> row_r, row_k;  // of each multipole (one_pair)
   std::vector<HistItem> items;
   std::vector<FoldItem> folds;
   DeviceBuffer zero_cell;  // index of the subgrid cell r = 0
@@ -571,7 +573,8 @@ struct Correlator {
 
   void allocate() {
     if (!fused) work.resize(geo.nreal_padded() * real_bytes());
-    const int n = shared_subgrids() ? 1 : geo.nrows;
+    one_pair = !fused && one_pair_rule(geo, real_bytes());
+    const int n = shared_subgrids() || one_pair ? 1 : geo.nrows;
     rsub_l.resize(n);
     ksub_l.resize(n);
     for (int r = 0; r < n; ++r) {
@@ -582,6 +585,14 @@ struct Correlator {
     FC_CUDA(cudaMemset(d_out.get(), 0, d_out.bytes()));
   }
 
+  // Whether cuFFT's path uses one pair of subgrids for every multipole in turn and
+  // reduces each multipole's histograms before the next: where a pair each would
+  // hold more than the grid, and 256 MB more than one.  (They save two launches a
+  // multipole: 275 against 292 us at 64 x 70 x 85, nothing to speak of above.)
+  static bool one_pair_rule(const Geometry &g, size_t real_bytes) {
+    const size_t more = (g.nrows - 1) * (g.rcells() + g.kcells()) * sizeof(double);
+    return more > g.nreal_padded() * real_bytes && more > (size_t)256 << 20;
+  }
   // Whether every multipole reads the same subgrids.
   bool shared_subgrids() const { return fused && kind == FC_PERIODIC; }
   size_t out_len() const { return (size_t)geo.nrows * (geo.nr + geo.nk) + 1; }
@@ -590,8 +601,8 @@ struct Correlator {
     return d_out.as<double>() + (size_t)geo.nrows * geo.nr + (size_t)r * geo.nk;
   }
   double *zerolag_out() const { return d_out.as<double>() + out_len() - 1; }
-  double *rsub(int ell) const { return rsub_l[ell / 2].as<double>(); }
-  double *ksub(int ell) const { return ksub_l[ell / 2].as<double>(); }
+  double *rsub(int ell) const { return rsub_l[one_pair ? 0 : ell / 2].as<double>(); }
+  double *ksub(int ell) const { return ksub_l[one_pair ? 0 : ell / 2].as<double>(); }
   // Periodic weights (correlator.h:304-349): sqrt(4 pi (2 ell + 1)) times the
   // normalisations of P and of xi.
   double k_coeff(int ell) const {
@@ -608,19 +619,30 @@ struct Correlator {
   template <typename RsubOf>
   void hist_items(RsubOf rsub_of, const uint32_t *rcells, std::vector<HistItem> &it,
                   std::vector<FoldItem> &fo) const {
-    const bool sh = shared_subgrids();
     for (int r = 0; r < geo.nrows; ++r) {
-      rbins.append_work(rsub_of(r), rcells,
-                        sh ? rweights.as<double>() + r * rbins.ninrange : nullptr, 1.0,
-                        rhist_row(r), it, fo);
-      kbins.append_work(ksub_l[sh ? 0 : r].as<double>(), kbins.perm.as<uint32_t>(),
-                        sh ? kweights.as<double>() + r * kbins.ninrange : nullptr, 1.0,
-                        khist_row(r), it, fo);
+      r_items(rsub_of(r), rcells, r, it, fo);
+      k_items(r, it, fo);
     }
+    zero_item(rsub_of(0), rcells, it, fo);
+  }
+  void r_items(const double *rs, const uint32_t *rcells, int r, std::vector<HistItem> &it,
+               std::vector<FoldItem> &fo) const {
+    rbins.append_work(rs, rcells,
+                      shared_subgrids() ? rweights.as<double>() + r * rbins.ninrange : nullptr,
+                      1.0, rhist_row(r), it, fo);
+  }
+  void k_items(int r, std::vector<HistItem> &it, std::vector<FoldItem> &fo) const {
+    const bool sh = shared_subgrids();
+    kbins.append_work(ksub_l[sh || one_pair ? 0 : r].as<double>(), kbins.perm.as<uint32_t>(),
+                      sh ? kweights.as<double>() + r * kbins.ninrange : nullptr, 1.0,
+                      khist_row(r), it, fo);
+  }
+  void zero_item(const double *rs, const uint32_t *rcells, std::vector<HistItem> &it,
+                 std::vector<FoldItem> &fo) const {
     const uint32_t *zero = zero_cell.as<uint32_t>();
     fo.push_back(FoldItem{(int)it.size(), 1, zerolag_out()});
-    it.push_back(HistItem{rsub_of(0), zero, nullptr,
-                          sh ? make_ylm_params(0, 0, r_coeff(0)).value0 : 1.0,
+    it.push_back(HistItem{rs, zero, nullptr,
+                          shared_subgrids() ? make_ylm_params(0, 0, r_coeff(0)).value0 : 1.0,
                           rcells == rbins.perm.as<uint32_t>() ? 0u : 1u, 1});
   }
 
@@ -631,9 +653,25 @@ struct Correlator {
                               centre};
     zero_cell.resize(sizeof(zero));
     FC_CUDA(cudaMemcpy(zero_cell.get(), zero, sizeof(zero), cudaMemcpyHostToDevice));
+    const uint32_t *rcells = rbins.perm.as<uint32_t>();
+    if (one_pair) {
+      row_r = std::vector<HistPlan>(geo.nrows);
+      row_k = std::vector<HistPlan>(geo.nrows);
+      for (int r = 0; r < geo.nrows; ++r) {
+        std::vector<HistItem> it;
+        std::vector<FoldItem> fo;
+        r_items(rsub(0), rcells, r, it, fo);
+        if (r == 0) zero_item(rsub(0), rcells, it, fo);
+        row_r[r].upload(it, fo);
+        it.clear();
+        fo.clear();
+        k_items(r, it, fo);
+        row_k[r].upload(it, fo);
+      }
+      return;
+    }
     const bool sh = shared_subgrids();
-    hist_items([&](int r) { return rsub_l[sh ? 0 : r].as<double>(); },
-               rbins.perm.as<uint32_t>(), items, folds);
+    hist_items([&](int r) { return rsub_l[sh ? 0 : r].as<double>(); }, rcells, items, folds);
     hist.upload(items, folds);
   }
 
@@ -892,18 +930,29 @@ struct Correlator {
     FC_LAUNCH_CHECK();
   }
 
-  // Every histogram and the zero lag, unless the caller reduces them.
+  // Every histogram and the zero lag, unless the caller reduces them, or they
+  // have been, multipole by multipole.
   void reduce_hist(const HistPlan &h) {
     have_result = true;
-    if (deferred) return;
+    if (deferred || one_pair) return;
     Profiler::Scope ps(&prof, stream, "hist");
     h.run(stream);
   }
+  void reduce_row(const std::vector<HistPlan> &rows, int ell) {
+    if (!one_pair) return;
+    Profiler::Scope ps(&prof, stream, "hist");
+    rows[ell / 2].run(stream);
+  }
 
+  void zero_r(int ell) {
+    FC_CUDA(cudaMemsetAsync(rsub(ell), 0, rsub_cells() * sizeof(double), stream));
+  }
+  void zero_k(int ell) {
+    FC_CUDA(cudaMemsetAsync(ksub(ell), 0, ksub_cells() * sizeof(double), stream));
+  }
   void zero_sub(int ell) {
-    DeviceBuffer &r = rsub_l[ell / 2], &k = ksub_l[ell / 2];
-    FC_CUDA(cudaMemsetAsync(r.get(), 0, r.bytes(), stream));
-    FC_CUDA(cudaMemsetAsync(k.get(), 0, k.bytes(), stream));
+    zero_r(ell);
+    zero_k(ell);
   }
 
   // ----------------------------------------------------------- grid2
@@ -1040,11 +1089,16 @@ struct Correlator {
     conj_mul<T>(!cross);
     const int maxell = 2 * (geo.nrows - 1);
     for (int ell = 0; ell <= maxell; ell += 2) {
-      zero_sub(ell);
+      zero_k(ell);
       ksub_acc<T>(ell, 0, k_coeff(ell));
+      reduce_row(row_k, ell);
     }
     exec_c2r(work.get(), work.get());
-    for (int ell = 0; ell <= maxell; ell += 2) rsub_acc<T>(ell, 0, r_coeff(ell));
+    for (int ell = 0; ell <= maxell; ell += 2) {
+      zero_r(ell);
+      rsub_acc<T>(ell, 0, r_coeff(ell));
+      reduce_row(row_r, ell);
+    }
     reduce_hist(hist);
   }
 
@@ -1062,6 +1116,18 @@ struct Correlator {
     FC_REQUIRE(kind == FC_PERIODIC, FC_ERR_UNSUPPORTED,
                "deferred histograms are built for the periodic correlator");
     deferred = true;
+    if (!one_pair) return;
+    // All histograms at the end: a pair of subgrids each.
+    one_pair = false;
+    row_r.clear();
+    row_k.clear();
+    rsub_l.resize(geo.nrows);
+    ksub_l.resize(geo.nrows);
+    for (int r = 0; r < geo.nrows; ++r) {
+      rsub_l[r].resize(rsub_cells() * sizeof(double));
+      ksub_l[r].resize(ksub_cells() * sizeof(double));
+    }
+    build_hist();
   }
 
   // The histogram reductions of the deferred subgrids as work items.
@@ -1141,6 +1207,8 @@ struct Correlator {
         exec_c2r(work.get(), work.get());
         rsub_acc<T>(ell, m, 4.0 * M_PI / ncells);
       }
+      reduce_row(row_r, ell);
+      reduce_row(row_k, ell);
     }
     reduce_hist(hist);
   }
@@ -1338,7 +1406,8 @@ size_t correlator_footprint(int kind, const int shape[3], double cell,
     bytes += g.nreal_padded() * rb;                          // work
     if (kind == FC_SURVEY) bytes += g.ncomplex() * eb;       // grid2 FFT
     bytes += g.ncomplex() * eb;                              // cuFFT work area
-    bytes += (g.rcells() + g.kcells()) * (size_t)(8 * g.nrows);  // subgrids
+    const int pairs = Correlator::one_pair_rule(g, rb) ? 1 : g.nrows;
+    bytes += (g.rcells() + g.kcells()) * (size_t)(8 * pairs);  // subgrids
   }
   bytes += (rin + kin) * 4;                                  // bin indices
   return bytes + (4 << 20);

@@ -11,6 +11,7 @@ from oracle import fc_oracle as O
 
 import fftcorr_b200 as fb
 from fftcorr_b200 import _lib
+from fftcorr_b200.batch import PeriodicBatch
 from test_batch import _batch, _single_box
 from test_gpu_parity import FP64_RTOL, _compare_results
 
@@ -67,6 +68,60 @@ def test_plan_failure_leaves_nothing_behind(kind):
     c = make(shape, *args)
     c.autocorrelate(grid)
     _compare_results(c.results(), oracle(grid, *args), FP64_RTOL, kind)
+
+
+LARGE = (242, 264, 286)   # a k-subgrid of 18M cells, 150 MB in FP64
+
+
+@pytest.mark.parametrize("kind", ["periodic", "survey"])
+def test_large_subgrids_take_turns(kind):
+    """A k-subgrid that reaches the Nyquist frequency is larger than the grid:
+    at ell <= 4 the multipoles use one pair of subgrids in turn, and their
+    histograms are reduced one by one, which gives the bits of ell <= 2 (a pair
+    each) and holds less."""
+    grid = np.random.default_rng(6).standard_normal(LARGE)
+
+    def run(maxell):
+        args = (60.0, 7.0, 0.35, 0.03, maxell)
+        before = _device_bytes()
+        if kind == "periodic":
+            c = fb.PeriodicCorrelator(LARGE, 10.0, 0, *args, precision="fp32")
+        else:
+            c = fb.Correlator(LARGE, 10.0, POSMIN, 2, *args, precision="fp32")
+        made = _device_bytes() - before
+        c.autocorrelate(grid)
+        first = c.results()
+        c.autocorrelate(grid)
+        for key in ("rhist", "khist"):
+            np.testing.assert_array_equal(first[key], c.results()[key])
+        return made, first
+
+    made2, two = run(2)
+    made4, four = run(4)
+    assert made4 < made2
+    for key in ("rhist", "khist", "rcounts", "kcounts"):
+        np.testing.assert_array_equal(four[key][:2], two[key])
+        assert np.all(np.isfinite(four[key])) and np.any(four[key][2] != 0)
+    assert four["zerolag"] == two["zerolag"]
+
+
+def test_batch_with_large_subgrids():
+    """A batch reduces all histograms at its end, from a pair of subgrids each."""
+    posw = clustered_catalog(20000, [0, 0, 0], 10.0 * np.array(LARGE), 1, ncenters=30)
+    args = (60.0, 7.0, 0.35, 0.03, 4)
+    b = PeriodicBatch([(LARGE, 10.0, posw)], fb.DistributionScheme.CLOUD_IN_CELL, *args, 0,
+                      "fp32", tune=False)
+    b.run()
+    g = fb.ConfigSpaceGrid.from_geometry(LARGE, [0, 0, 0], 10.0, precision="fp32")
+    ma = fb.MassAssignor(g, fb.DistributionScheme.CLOUD_IN_CELL, True, 0)
+    ma.add_particles(posw)
+    mean = ma.totw / float(np.prod(LARGE))
+    g -= mean
+    g *= 1.0 / mean
+    c = fb.PeriodicCorrelator(LARGE, 10.0, 0, *args, precision="fp32")
+    c.autocorrelate(g)
+    for key in ("rcounts", "kcounts", "rhist", "khist"):
+        np.testing.assert_array_equal(b.results(0)[key], c.results()[key])
 
 
 def test_fused_surveys_make_no_plan_that_could_fail():
